@@ -73,9 +73,9 @@ struct gcz_ctx {
     int algo = 2;          // 1: fused single-warp kernels, 2: candidate sweep + second stage
     int parse_ctas = 3;    // second-stage CTAs per SM
     int seg_width = 1024;  // Zstd speculative segment: 1024 per 8-lane group, or 2048/4096/8192 per warp
-    int sweep_warps = 7;   // candidate-sweep windows per CTA (4-7)
-    int sweep_groups = 0;  // candidate sweep's equal-hash grouping: 0/1 after a read-back (match_any/ballots), 2/3 one block ahead
-    int sweep_prefetch = 4;  // candidate sweep's L2 prefetch distance of the input, in 128-byte blocks (0, 4, 8)
+    int sweep_warps = 7;   // warps that take turns on a window in the candidate sweep (4-7)
+    int sweep_groups = 0;  // odd: the sweep groups the lanes of every step by hash first
+    int sweep_prefetch = 4;  // accepted, without effect
     int lzma_ctas = 3;     // LZMA2 second-stage CTAs per SM
     int lzma_threads = 1024;  // LZMA2 second-stage threads per CTA (256, 512 or 1024)
     // profiling
@@ -224,7 +224,7 @@ int zstd_device_core(gcz_ctx *c, Scratch &sc, const uint8_t *d_src, size_t n, ui
     if (split) {
         uint16_t *cand = static_cast<uint16_t *>(sc.cand.p);
         GCZ_CUDA(c, gcz::launch_cand_sweep(d_src, n, kW, (uint32_t)nb, cand, c->num_sms, st, wins, c->sweep_warps,
-                                           c->sweep_groups, c->sweep_prefetch));
+                                           c->sweep_groups));
         gcz::Zstd2Launch l{};
         l.src = d_src;
         l.cand = cand;
@@ -278,7 +278,7 @@ int lzma_run(gcz_ctx *c, Scratch &sc, const gcz::LzmaLaunch &l, cudaStream_t st)
     if (split) {
         uint16_t *cand = static_cast<uint16_t *>(sc.cand.p);
         GCZ_CUDA(c, gcz::launch_cand_sweep(l.src, l.n, l.window, l.num_windows, cand, c->num_sms, st, l.wins,
-                                           c->sweep_warps, c->sweep_groups, c->sweep_prefetch));
+                                           c->sweep_warps, c->sweep_groups));
         gcz::LzmaLaunch lv = l;
         lv.ctas_per_sm = c->lzma_ctas;
         lv.threads = c->lzma_threads;
@@ -808,7 +808,7 @@ extern "C" int gcz_zstd_match_find_ref_layout_device(gcz_ctx *c, const uint8_t *
         ProfScope ps(c, st);
         uint16_t *cand = static_cast<uint16_t *>(c->sc.cand.p);
         GCZ_CUDA(c, gcz::launch_cand_sweep(d_input, n_eff, chunk_size, (uint32_t)nb, cand, c->num_sms, st, nullptr,
-                                           c->sweep_warps, c->sweep_groups, c->sweep_prefetch));
+                                           c->sweep_warps, c->sweep_groups));
         gcz::Zstd2Launch l{};
         l.src = d_input;
         l.cand = cand;
@@ -1393,7 +1393,7 @@ int server_launch(gcz_server *sv, ServerSlot &s) {
     if (nb) {
         GCZ_CUDA(c, cudaMemcpyAsync(s.wins.p, s.hwins.data(), nb * sizeof(gcz_window), cudaMemcpyHostToDevice, s.st));
         GCZ_CUDA(c, gcz::launch_cand_sweep(slab_p, slab, kW, (uint32_t)nb, cand, c->num_sms, s.st, dw, c->sweep_warps,
-                                           c->sweep_groups, c->sweep_prefetch));
+                                           c->sweep_groups));
     }
     const uint32_t nz = s.wb[kGrpLzma];  // Zstd windows: sequences and frames groups
     uint64_t *d_off = static_cast<uint64_t *>(s.offsets.p);

@@ -18,7 +18,8 @@ constexpr uint32_t kErrTmaTimeout = 1;
 constexpr uint32_t kErrCapacity = 2;
 
 // Multiplicative 4-byte hash, HASH4 in zstd_compress.cu:228 and lzma2_match_find.cu:92.
-__device__ __forceinline__ uint32_t hash4(uint32_t v) { return (v * 2654435761u) >> (32 - kHashLog); }
+constexpr uint32_t kHashMul = 2654435761u;
+__device__ __forceinline__ uint32_t hash4(uint32_t v) { return (v * kHashMul) >> (32 - kHashLog); }
 
 __device__ __forceinline__ uint32_t lanemask_lt() {
     uint32_t m;

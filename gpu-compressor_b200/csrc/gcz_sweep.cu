@@ -9,22 +9,30 @@
 // which this kernel computes for every position of every window; the match
 // finders then verify, extend and parse from it.
 //
-// One warp sweeps one window 32 positions per step.  Each lane reads its
-// bucket (the last position of earlier steps), writes its own position and
-// reads it back; when every lane reads back its own position no two lanes of
-// the step share a bucket, the values read are the candidates and the table
-// is up to date.  Otherwise (equal hashes inside a step) the table is restored
-// from that step on, and in each step with equal hashes __match_any_sync
-// groups the lanes: the in-step predecessor is the next lower lane of the
-// group and the highest lane writes the bucket.  Only the table lives in
-// shared memory (32 KiB), so seven windows are swept per SM; the input streams
-// through coalesced 128-byte loads.
+// Lookup and insertion are one shared-memory exchange per position: the entry
+// is {window epoch, position}, and what the exchange returns is the position
+// that was there.  One warp instruction covers 32 positions, lane l the l-th.
+// The lanes of one instruction that hit the same bucket are applied in some
+// order; on sm_100a that order is ascending, which makes every returned value
+// the candidate, equal hashes inside the step included.  Nothing rests on it:
+// the exchanges of a bucket form one chain, and if every one of them returns
+// an entry below its own, the chain ascends and each value is the highest
+// position before it.  A single returned entry that is not below its own makes
+// the CTA sweep its windows again with the lanes grouped first
+// (__match_any_sync), which is exact whatever the order.
+//
+// One window per CTA at a time, three CTAs (64 KiB tables) per SM.  The CTA's
+// warps take turns, 512 positions each, in window order: a warp hashes its
+// chunk before its turn and writes its candidates after it, so that the turn
+// is sixteen exchanges and a named-barrier handover.  The epoch in the entries
+// marks earlier windows' positions as empty, so that the table is cleared once
+// per launch (and every 65535 windows) and the turns run on from one window to
+// the next.
 #include "gcz_common.cuh"
 #include "gcz_kernels.h"
 
 namespace gcz {
 namespace {
-
 
 struct SweepArgs {
     const uint8_t *src;
@@ -35,290 +43,205 @@ struct SweepArgs {
     const WinDesc *wins;
 };
 
-// Lanes of this warp whose key equals this lane's (valid lanes only; an
-// invalid lane matches only itself): kBits ballots, one per key bit, combined
-// bit-sliced.  The ballots do not depend on each other, so their latency
-// overlaps, unlike one __match_any_sync.
-template <int kBits>
-__device__ __forceinline__ uint32_t same_key_lanes(uint32_t key, bool valid) {
-    uint32_t m = __ballot_sync(kFull, valid);
-#pragma unroll
-    for (int b = 0; b < kBits; ++b) {
-        const bool bit = (key >> b) & 1u;
-        const uint32_t bb = __ballot_sync(kFull, bit);
-        m &= bit ? bb : ~bb;
-    }
-    return valid ? m : (1u << lane_id());
+constexpr uint32_t kChunkSteps = 16;                 // exchanges of one turn
+constexpr uint32_t kChunkPos = 32u * kChunkSteps;    // positions of one turn
+constexpr uint32_t kSweepCtas = 3;                   // per SM: 3 x (64 KiB table + hash buffers)
+
+template <int kWarps>
+struct SweepSmem {
+    uint32_t T[kHashSize];
+    uint16_t h[kWarps][kChunkPos];  // a warp's chunk: byte offsets of its positions' buckets in T
+    uint32_t redo;
+};
+
+__device__ __forceinline__ void window_of(const SweepArgs &a, uint32_t w, uint64_t &start, uint32_t &size) {
+    start = a.wins ? a.wins[w].offset : static_cast<uint64_t>(w) * a.window;
+    size = a.wins ? a.wins[w].size : static_cast<uint32_t>(a.n - start < a.window ? a.n - start : a.window);
 }
 
-// The hashes of one 128-position block (independent of the table): step j,
-// lane l is position blk * 128 + 32 j + l.  Lane l holds word l of the block
-// (w0) and word l of the next block (w1; only lane 0's is used).
-__device__ __forceinline__ void block_hashes(uint32_t blk, uint32_t size, uint32_t w0, uint32_t w1, uint32_t *h,
-                                             bool *v) {
-    const uint32_t lane = lane_id();
-    const uint32_t up = __shfl_down_sync(kFull, w0, 1);
-    const uint32_t n0 = __shfl_sync(kFull, w1, 0);
-    const uint32_t w0n = lane == 31u ? n0 : up;  // word l+1
-#pragma unroll
-    for (uint32_t j = 0; j < 4; ++j) {
-        const uint32_t q = blk * 128u + j * 32u + lane;
-        const uint32_t src_lane = j * 8u + (lane >> 2);
-        const uint32_t lo = __shfl_sync(kFull, w0, src_lane);
-        const uint32_t hi = __shfl_sync(kFull, w0n, src_lane);
-        v[j] = q + 3u < size;
-        h[j] = hash4(__funnelshift_r(lo, hi, (lane & 3u) * 8u));
-    }
+// The words of one chunk: lane l holds words 2l, 2l+1 of each half (256
+// positions), lane 31 also the first word after the chunk.  0 past the window.
+struct ChunkWords {
+    uint2 a, b;
+    uint32_t next;
+};
+__device__ __forceinline__ uint2 load_words(const uint32_t *src32, uint32_t nwords, uint32_t i) {
+    if (i + 1u < nwords) return __ldg(reinterpret_cast<const uint2 *>(src32 + i));
+    return make_uint2(i < nwords ? __ldg(src32 + i) : 0u, 0u);
+}
+__device__ __forceinline__ ChunkWords load_chunk(const uint32_t *src32, uint32_t nwords, uint32_t ch) {
+    const uint32_t lane = lane_id(), i = ch * (kChunkPos / 4u) + 2u * lane, e = (ch + 1u) * (kChunkPos / 4u);
+    ChunkWords w;
+    w.a = load_words(src32, nwords, i);
+    w.b = load_words(src32, nwords, i + 64u);
+    w.next = lane == 31u && e < nwords ? __ldg(src32 + e) : 0u;
+    return w;
 }
 
-// The block's table work and candidates, from its hashes.
-template <bool kBallotGroups>
-__device__ __forceinline__ void block_table(uint16_t *T, uint16_t *out, uint32_t blk, uint32_t size,
-                                            const uint32_t *h, const bool *v, uint32_t lt, uint32_t gt) {
-    const uint32_t lane = lane_id();
-    // Step by step: read the bucket, write this position,
-    // read it back.  A lane that does not read back its own position
-    // shares its bucket with another lane of the same step.
-    uint32_t tv[4], dup = 0;
+// The bucket offsets (4 * hash4) of the eight positions whose bytes start in
+// w, packed in pairs; nx: the word after w.
+__device__ __forceinline__ uint4 bucket_offsets(uint2 w, uint32_t nx) {
+    uint32_t p[8];
 #pragma unroll
-    for (uint32_t j = 0; j < 4; ++j) {
-        const uint32_t q = blk * 128u + j * 32u + lane;
-        tv[j] = v[j] ? static_cast<uint32_t>(T[h[j]]) : 0xFFFFu;
-        __syncwarp();
-        if (v[j]) T[h[j]] = static_cast<uint16_t>(q);
-        __syncwarp();
-        if (v[j] && T[h[j]] != static_cast<uint16_t>(q)) dup |= 1u << j;
+    for (uint32_t k = 0; k < 4; ++k) {
+        p[k] = (k ? __funnelshift_r(w.x, w.y, 8u * k) : w.x) * kHashMul;
+        p[4 + k] = (k ? __funnelshift_r(w.y, nx, 8u * k) : w.y) * kHashMul;
     }
-    uint32_t g[4] = {1u << lane, 1u << lane, 1u << lane, 1u << lane};
-    const uint32_t dsteps = __reduce_or_sync(kFull, dup);  // steps with equal hashes in two lanes
-    if (dsteps) {
-        // One block in two on compressible data.  Steps before the
-        // first such step j0 wrote each bucket once and are exact.  Put
-        // the table back as it was before j0 (latest steps first, so
-        // each bucket ends with the value its earliest step from j0 on
-        // read) and redo from j0, grouping the lanes of the steps that
-        // share buckets.  Which lanes share a bucket depends only on
-        // the hashes, so the other steps need no groups.
-        const uint32_t j0 = static_cast<uint32_t>(__ffs(dsteps)) - 1u;
+    // hash4 = product >> 18, so 4 * hash4 is the product's upper half without its two low bits
+    uint4 r;
+    r.x = __byte_perm(p[0], p[1], 0x7632) & 0xFFFCFFFCu;
+    r.y = __byte_perm(p[2], p[3], 0x7632) & 0xFFFCFFFCu;
+    r.z = __byte_perm(p[4], p[5], 0x7632) & 0xFFFCFFFCu;
+    r.w = __byte_perm(p[6], p[7], 0x7632) & 0xFFFCFFFCu;
+    return r;
+}
+
+// Named barrier between the warp whose turn ends (arrive) and the next (sync).
+__device__ __forceinline__ void turn_wait(uint32_t id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+__device__ __forceinline__ void turn_pass(uint32_t id) { asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory"); }
+
+// Candidates of one window by one warp, 32 positions per step with the lanes
+// grouped by hash first: exact for any order of colliding lanes.  T: a table
+// of kHashSize entries (one warp at a time).
+__device__ void sweep_window_grouped(uint32_t *T, uint16_t *out, const uint32_t *src32, uint32_t size) {
+    const uint32_t lane = lane_id(), lt = lanemask_lt(), gt = lanemask_gt();
+    const uint32_t nwords = (size + 3u) >> 2;
+    for (uint32_t i = lane; i < kHashSize; i += 32u) T[i] = 0xFFFFu;
+    __syncwarp();
+    for (uint32_t q = lane; q - lane < size; q += 32u) {
+        const bool v = q + 3u < size;
+        const uint32_t i = q >> 2;
+        const uint32_t x = i < nwords ? __ldg(src32 + i) : 0u, y = i + 1u < nwords ? __ldg(src32 + i + 1u) : 0u;
+        const uint32_t h = hash4(__funnelshift_r(x, y, (q & 3u) * 8u));
+        const uint32_t g = __match_any_sync(kFull, v ? h : (0x80000000u | lane));
+        const uint32_t lower = g & lt;
+        uint32_t c = v ? T[h] : 0xFFFFu;
+        if (lower) c = q - lane + 31u - static_cast<uint32_t>(__clz(lower));
         __syncwarp();
-#pragma unroll
-        for (int j = 3; j >= 0; --j) {
-            if (static_cast<uint32_t>(j) >= j0) {
-                if (v[j]) T[h[j]] = static_cast<uint16_t>(tv[j]);
-                __syncwarp();
-            }
-        }
-#pragma unroll
-        for (uint32_t j = 0; j < 4; ++j) {
-            if (j < j0) continue;
-            const uint32_t q = blk * 128u + j * 32u + lane;
-            if ((dsteps >> j) & 1u) {
-                if constexpr (kBallotGroups) g[j] = same_key_lanes<kHashLog>(h[j], v[j]);
-                else g[j] = __match_any_sync(kFull, v[j] ? h[j] : (0x80000000u | lane));
-            }
-            tv[j] = v[j] ? static_cast<uint32_t>(T[h[j]]) : 0xFFFFu;
-            __syncwarp();
-            if (v[j] && !(g[j] & gt)) T[h[j]] = static_cast<uint16_t>(q);
-            __syncwarp();
-        }
-    }
-    // ... then the candidates.
-#pragma unroll
-    for (uint32_t j = 0; j < 4; ++j) {
-        const uint32_t q = blk * 128u + j * 32u + lane;
-        const uint32_t lower = g[j] & lt;
-        const uint32_t c = lower ? (q - lane + 31u - static_cast<uint32_t>(__clz(lower))) : tv[j];
+        if (v && !(g & gt)) T[h] = q;
+        __syncwarp();
         if (q < size) out[q] = static_cast<uint16_t>(c);
     }
 }
 
-// One 128-position block of a window's sweep: hashes, then table work.
-template <bool kBallotGroups>
-__device__ __forceinline__ void sweep_block(uint16_t *T, uint16_t *out, uint32_t blk, uint32_t size, uint32_t w0,
-                                            uint32_t w1, uint32_t lt, uint32_t gt) {
-    uint32_t h[4];
-    bool v[4];
-    block_hashes(blk, size, w0, w1, h, v);
-    block_table<kBallotGroups>(T, out, blk, size, h, v, lt, gt);
-}
-
-// Word l of block b of a window (0 past its end).
-__device__ __forceinline__ uint32_t block_word(const uint32_t *src32, uint32_t nwords, uint32_t b) {
-    const uint32_t i = b * 32u + lane_id();
-    return i < nwords ? __ldg(src32 + i) : 0u;
-}
-
-// kSweepWarpsPerCta windows per CTA, one 32 KiB table each (7 fill an SM's
-// shared memory); a schedule knob, the candidates do not depend on it.  So is
-// kBallotGroups: how the lanes of a step with equal hashes are grouped
-// (__match_any_sync, or bit-sliced ballots), and kPf, how many 128-byte
-// blocks ahead the input is prefetched into L2 (0: not at all; a compile-time
-// distance, which measured 0.4 ms per GiB faster than the same distance read
-// from the kernel's arguments).
-template <int kSweepWarpsPerCta, bool kBallotGroups, uint32_t kPf>
-__global__ void __launch_bounds__(32 * kSweepWarpsPerCta) cand_sweep_kernel(SweepArgs a) {
-    extern __shared__ __align__(16) uint8_t smem[];
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    uint16_t *T = reinterpret_cast<uint16_t *>(smem) + warp * kHashSize;
-    uint4 *T4 = reinterpret_cast<uint4 *>(T);
-    const uint32_t lt = lanemask_lt(), gt = lanemask_gt();
-    const uint32_t gwarps = gridDim.x * kSweepWarpsPerCta;
-    for (uint32_t w = blockIdx.x * kSweepWarpsPerCta + warp; w < a.num_windows; w += gwarps) {
-        const uint64_t start = a.wins ? a.wins[w].offset : static_cast<uint64_t>(w) * a.window;
-        const uint32_t size =
-            a.wins ? a.wins[w].size : static_cast<uint32_t>(a.n - start < a.window ? a.n - start : a.window);
-        for (uint32_t i = lane; i < kHashSize * 2 / 16; i += 32) T4[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
-        __syncwarp();
-        const uint32_t *src32 = reinterpret_cast<const uint32_t *>(a.src + start);
-        const uint32_t nwords = (size + 3u) >> 2;
-        uint16_t *out = a.cand + start;
-        const uint32_t nblk = (size + 127u) >> 7;
-        // 128-byte blocks: lane l holds word l.  Each block's words are loaded
-        // two blocks ahead of its sweep; with kPf > 0 lane 0 also prefetches
-        // block b + kPf into L2 while block b is swept, so that those loads hit
-        // L2 instead of waiting on DRAM.
-        uint32_t w0 = block_word(src32, nwords, 0), w1 = block_word(src32, nwords, 1);
-        for (uint32_t blk = 0; blk < nblk; ++blk) {
-            if constexpr (kPf > 0) {
-                const uint32_t pw = (blk + kPf) * 32u;
-                if (lane == 0 && pw < nwords) asm volatile("prefetch.global.L2 [%0];" ::"l"(src32 + pw));
+// kWarps warps take turns on a window (a schedule knob, 4-7).  kGrouped: every
+// window takes the grouped sweep (what an unexpected lane order would lead to).
+template <int kWarps, bool kGrouped>
+__global__ void __launch_bounds__(32 * kWarps, kSweepCtas) cand_sweep_kernel(SweepArgs a) {
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    SweepSmem<kWarps> &S = *reinterpret_cast<SweepSmem<kWarps> *>(smem_raw);
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    constexpr uint32_t kThreads = 32u * kWarps;
+    auto clear = [&] {
+        uint4 *T4 = reinterpret_cast<uint4 *>(S.T);
+        for (uint32_t i = tid; i < kHashSize / 4; i += kThreads) T4[i] = make_uint4(0u, 0u, 0u, 0u);
+    };
+    if (tid == 0) S.redo = kGrouped ? 1u : 0u;
+    clear();
+    __syncthreads();
+    bool bad = false;
+    if constexpr (!kGrouped) {
+        uint32_t first = 0;  // warp whose turn the window's first chunk is
+        uint32_t epoch = 0;
+        bool begun = false;  // some chunk of this CTA has been handed out
+        for (uint32_t w = blockIdx.x; w < a.num_windows; w += gridDim.x) {
+            if (++epoch == 0x10000u) {
+                __syncthreads();
+                clear();
+                __syncthreads();
+                epoch = 1u;
             }
-            const uint32_t w2 = block_word(src32, nwords, blk + 2u);
-            sweep_block<kBallotGroups>(T, out, blk, size, w0, w1, lt, gt);
-            w0 = w1;
-            w1 = w2;
-        }
-        __syncwarp();
-    }
-}
-
-// The same candidates with each step's lanes grouped by hash one block
-// ahead.  Which lanes of a step share a bucket depends only on the input
-// bytes, so the groups of block b+1 are formed (by __match_any_sync or by
-// bit-sliced ballots) while block b's table work runs, and their latency
-// overlaps it.  With the groups known, each step is one read (every lane reads
-// its bucket: the lowest lane of a group gets the table's candidate, the others
-// take the next lower lane's position) and one write (the highest lane of each
-// group), with no read-back and no redo.
-template <bool kBallots>
-__device__ __forceinline__ void block_hashes_groups(uint32_t blk, uint32_t size, uint32_t w0, uint32_t w1,
-                                                    uint32_t *h, bool *v, uint32_t *g) {
-    const uint32_t lane = lane_id();
-    const uint32_t up = __shfl_down_sync(kFull, w0, 1);
-    const uint32_t n0 = __shfl_sync(kFull, w1, 0);
-    const uint32_t w0n = lane == 31u ? n0 : up;  // word l+1
-#pragma unroll
-    for (uint32_t j = 0; j < 4; ++j) {
-        const uint32_t q = blk * 128u + j * 32u + lane;
-        const uint32_t src_lane = j * 8u + (lane >> 2);
-        const uint32_t lo = __shfl_sync(kFull, w0, src_lane);
-        const uint32_t hi = __shfl_sync(kFull, w0n, src_lane);
-        v[j] = q + 3u < size;
-        h[j] = hash4(__funnelshift_r(lo, hi, (lane & 3u) * 8u));
-    }
-#pragma unroll
-    for (uint32_t j = 0; j < 4; ++j) {
-        if constexpr (kBallots) g[j] = same_key_lanes<kHashLog>(h[j], v[j]);
-        else g[j] = __match_any_sync(kFull, v[j] ? h[j] : (0x80000000u | lane));
-    }
-}
-
-template <int kSweepWarpsPerCta, bool kBallots>
-__global__ void __launch_bounds__(32 * kSweepWarpsPerCta) cand_sweep_ahead_kernel(SweepArgs a) {
-    extern __shared__ __align__(16) uint8_t smem[];
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    uint16_t *T = reinterpret_cast<uint16_t *>(smem) + warp * kHashSize;
-    uint4 *T4 = reinterpret_cast<uint4 *>(T);
-    const uint32_t lt = lanemask_lt(), gt = lanemask_gt();
-    const uint32_t gwarps = gridDim.x * kSweepWarpsPerCta;
-    for (uint32_t w = blockIdx.x * kSweepWarpsPerCta + warp; w < a.num_windows; w += gwarps) {
-        const uint64_t start = a.wins ? a.wins[w].offset : static_cast<uint64_t>(w) * a.window;
-        const uint32_t size =
-            a.wins ? a.wins[w].size : static_cast<uint32_t>(a.n - start < a.window ? a.n - start : a.window);
-        for (uint32_t i = lane; i < kHashSize * 2 / 16; i += 32) T4[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
-        __syncwarp();
-        const uint32_t *src32 = reinterpret_cast<const uint32_t *>(a.src + start);
-        const uint32_t nwords = (size + 3u) >> 2;
-        uint16_t *out = a.cand + start;
-        uint32_t w0 = lane < nwords ? __ldg(src32 + lane) : 0u;
-        uint32_t w1 = 32u + lane < nwords ? __ldg(src32 + 32u + lane) : 0u;
-        uint32_t h[4], g[4];
-        bool v[4];
-        block_hashes_groups<kBallots>(0u, size, w0, w1, h, v, g);
-        for (uint32_t blk = 0; blk * 128u < size; ++blk) {
-            const uint32_t nw = (blk + 2u) * 32u + lane;
-            const uint32_t w2 = nw < nwords ? __ldg(src32 + nw) : 0u;
-            // the next block's hashes and groups: no dependence on the table
-            uint32_t hn[4], gn[4];
-            bool vn[4];
-            block_hashes_groups<kBallots>(blk + 1u, size, w1, w2, hn, vn, gn);
-#pragma unroll
-            for (uint32_t j = 0; j < 4; ++j) {
-                const uint32_t q = blk * 128u + j * 32u + lane;
-                const uint32_t tv = v[j] ? static_cast<uint32_t>(T[h[j]]) : 0xFFFFu;
+            uint64_t start;
+            uint32_t size;
+            window_of(a, w, start, size);
+            const uint32_t *src32 = reinterpret_cast<const uint32_t *>(a.src + start);
+            uint16_t *out = a.cand + start;
+            const uint32_t nwords = (size + 3u) >> 2;
+            const uint32_t nch = (size + kChunkPos - 1u) / kChunkPos;
+            const bool last_window = a.num_windows - w <= gridDim.x;
+            uint32_t ch = warp >= first ? warp - first : warp + kWarps - first;  // this warp's first chunk
+            ChunkWords cw = load_chunk(src32, nwords, ch);
+            for (; ch < nch; ch += kWarps) {
+                uint32_t nx = __shfl_down_sync(kFull, cw.a.x, 1);
+                const uint32_t b0 = __shfl_sync(kFull, cw.b.x, 0);
+                if (lane == 31u) nx = b0;
+                uint32_t ny = __shfl_down_sync(kFull, cw.b.x, 1);
+                if (lane == 31u) ny = cw.next;
+                uint4 *hb = reinterpret_cast<uint4 *>(S.h[warp]);
+                hb[lane] = bucket_offsets(cw.a, nx);
+                hb[32u + lane] = bucket_offsets(cw.b, ny);
                 __syncwarp();
-                if (v[j] && !(g[j] & gt)) T[h[j]] = static_cast<uint16_t>(q);
-                __syncwarp();
-                const uint32_t lower = g[j] & lt;
-                const uint32_t c = lower ? (q - lane + 31u - static_cast<uint32_t>(__clz(lower))) : tv;
-                if (q < size) out[q] = static_cast<uint16_t>(c);
-            }
+                cw = load_chunk(src32, nwords, ch + kWarps);  // the next chunk's words arrive while others take turns
+                uint32_t h[kChunkSteps], old[kChunkSteps];
 #pragma unroll
-            for (uint32_t j = 0; j < 4; ++j) {
-                h[j] = hn[j];
-                v[j] = vn[j];
-                g[j] = gn[j];
+                for (uint32_t j = 0; j < kChunkSteps; ++j) h[j] = S.h[warp][32u * j + lane];
+                const uint32_t q0 = ch * kChunkPos + lane, e0 = epoch << 16;
+                uint8_t *T = reinterpret_cast<uint8_t *>(S.T);
+                if (begun || ch > 0u) turn_wait(1u + warp);
+                const bool full = (ch + 1u) * kChunkPos + 3u <= size;  // every position has its four bytes
+                if (full) {
+#pragma unroll
+                    for (uint32_t j = 0; j < kChunkSteps; ++j)
+                        old[j] = atomicExch(reinterpret_cast<uint32_t *>(T + h[j]), e0 + q0 + 32u * j);
+                } else {
+#pragma unroll
+                    for (uint32_t j = 0; j < kChunkSteps; ++j) {
+                        old[j] = 0u;
+                        if (q0 + 32u * j + 3u < size)
+                            old[j] = atomicExch(reinterpret_cast<uint32_t *>(T + h[j]), e0 + q0 + 32u * j);
+                    }
+                }
+                if (!(last_window && ch + 1u == nch)) turn_pass(1u + (warp + 1u == kWarps ? 0u : warp + 1u));
+#pragma unroll
+                for (uint32_t j = 0; j < kChunkSteps; ++j) {
+                    const uint32_t q = q0 + 32u * j;
+                    bad = bad || old[j] >= e0 + q;
+                    const uint32_t c = min(old[j] - e0, 0xFFFFu);  // an earlier epoch's entry is below e0: none
+                    if (full || q < size) out[q] = static_cast<uint16_t>(c);
+                }
             }
-            w0 = w1;
-            w1 = w2;
+            if (nch) begun = true;
+            first = (first + nch) % kWarps;
         }
-        __syncwarp();
+        if (bad) S.redo = 1u;
+    }
+    __syncthreads();
+    if (S.redo && warp == 0) {
+        for (uint32_t w = blockIdx.x; w < a.num_windows; w += gridDim.x) {
+            uint64_t start;
+            uint32_t size;
+            window_of(a, w, start, size);
+            sweep_window_grouped(S.T, a.cand + start, reinterpret_cast<const uint32_t *>(a.src + start), size);
+            __syncwarp();
+        }
     }
 }
 
-}  // namespace
-
-namespace {
-template <int kWarps, int kMode, uint32_t kPf = 0>
+template <int kWarps, bool kGrouped>
 cudaError_t launch_sweep_variant(const SweepArgs &a, int num_sms, cudaStream_t st) {
-    constexpr bool kBallots = (kMode & 1) != 0, kAhead = kMode >= 2;
-    const auto kernel =
-        kAhead ? cand_sweep_ahead_kernel<kWarps, kBallots> : cand_sweep_kernel<kWarps, kBallots, kAhead ? 0u : kPf>;
-    const uint32_t smem = kWarps * kHashSize * sizeof(uint16_t);
+    const uint32_t smem = sizeof(SweepSmem<kWarps>);
+    static_assert((sizeof(SweepSmem<kWarps>) + 1024) * kSweepCtas <= 233472, "three CTAs per SM must fit");
     static SmemOnce smem_set{0};
-    cudaError_t e = set_smem_once(kernel, smem, smem_set);
+    cudaError_t e = set_smem_once(cand_sweep_kernel<kWarps, kGrouped>, smem, smem_set);
     if (e != cudaSuccess) return e;
-    // as many CTAs per SM as the tables allow (one for 5-7 warps, two for 4 or less)
-    const uint32_t per_sm = (227u * 1024u) / (smem + 1024u);
-    uint32_t ctas = (a.num_windows + kWarps - 1) / kWarps;
-    const uint32_t cap = static_cast<uint32_t>(num_sms) * (per_sm ? per_sm : 1u);
-    if (ctas > cap) ctas = cap;
-    kernel<<<ctas, 32 * kWarps, smem, st>>>(a);
+    uint32_t ctas = static_cast<uint32_t>(num_sms) * kSweepCtas;
+    if (ctas > a.num_windows) ctas = a.num_windows;
+    cand_sweep_kernel<kWarps, kGrouped><<<ctas, 32 * kWarps, smem, st>>>(a);
     return cudaGetLastError();
 }
+
 }  // namespace
 
 cudaError_t launch_cand_sweep(const uint8_t *src, uint64_t n, uint32_t window, uint32_t num_windows, uint16_t *cand,
-                              int num_sms, cudaStream_t st, const WinDesc *wins, int sweep_warps, int sweep_groups,
-                              int sweep_prefetch) {
+                              int num_sms, cudaStream_t st, const WinDesc *wins, int sweep_warps, int sweep_groups) {
     if (num_windows == 0) return cudaSuccess;
     SweepArgs a{src, n, window, num_windows, cand, wins};
-    // sweep_groups: 0 / 1 group equal-hash lanes (__match_any_sync / ballots)
-    // only in blocks that need it, after a read-back; 2 / 3 form every step's
-    // groups one block ahead.  sweep_prefetch: the read-back modes' L2
-    // prefetch distance of the input, 0, 4 or 8 128-byte blocks (other values
-    // are rounded down to one of these).
-    const int pf = sweep_groups >= 2 ? 0 : (sweep_prefetch >= 8 ? 2 : (sweep_prefetch >= 4 ? 1 : 0));
-    switch ((pf * 4 + sweep_groups) * 8 + sweep_warps) {
-#define GCZ_SWEEP_CASE(P, M, W) \
-    case (P * 4 + M) * 8 + W: return launch_sweep_variant<W, M, P * 4u>(a, num_sms, st);
-#define GCZ_SWEEP_MODE(P, M) \
-    GCZ_SWEEP_CASE(P, M, 4) GCZ_SWEEP_CASE(P, M, 5) GCZ_SWEEP_CASE(P, M, 6) GCZ_SWEEP_CASE(P, M, 7)
-        GCZ_SWEEP_MODE(0, 0) GCZ_SWEEP_MODE(0, 1) GCZ_SWEEP_MODE(0, 2) GCZ_SWEEP_MODE(0, 3)
-        GCZ_SWEEP_MODE(1, 0) GCZ_SWEEP_MODE(1, 1) GCZ_SWEEP_MODE(2, 0) GCZ_SWEEP_MODE(2, 1)
-#undef GCZ_SWEEP_MODE
-#undef GCZ_SWEEP_CASE
-    default: return launch_sweep_variant<7, 0, 8u>(a, num_sms, st);
+    const bool grouped = (sweep_groups & 1) != 0;
+    switch (sweep_warps) {
+    case 4: return grouped ? launch_sweep_variant<4, true>(a, num_sms, st) : launch_sweep_variant<4, false>(a, num_sms, st);
+    case 5: return grouped ? launch_sweep_variant<5, true>(a, num_sms, st) : launch_sweep_variant<5, false>(a, num_sms, st);
+    case 6: return grouped ? launch_sweep_variant<6, true>(a, num_sms, st) : launch_sweep_variant<6, false>(a, num_sms, st);
+    default: return grouped ? launch_sweep_variant<7, true>(a, num_sms, st) : launch_sweep_variant<7, false>(a, num_sms, st);
     }
 }
 

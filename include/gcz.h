@@ -77,13 +77,12 @@ const char *gcz_version(void);
  * memory with bulk copies, 0 reads it through L1; "parse_ctas" = Zstd
  * second-stage CTAs per SM (1-8); "parse_seg" = the Zstd second stage's
  * speculative segment: 1024 bytes per 8-lane group (default), 512 bytes per
- * 4-lane group, or 2048, 4096 or 8192 bytes per warp; "sweep_warps" = windows per candidate-sweep CTA
- * (4-7, default 7); "sweep_groups" = how the sweep groups the lanes of a step
- * that share a hash bucket: after a table read-back, only in blocks that have
- * such lanes, with __match_any_sync (0, default) or bit-sliced ballots (1), or
- * for every step one block ahead of the table work (2, 3 likewise);
- * "sweep_prefetch" = how many 128-byte blocks ahead of itself the read-back
- * sweep (groups 0, 1) prefetches its input into L2: 0, 4 (default) or 8;
+ * 4-lane group, or 2048, 4096 or 8192 bytes per warp; "sweep_warps" = warps that take turns on
+ * a window in the candidate sweep (4-7, default 7); "sweep_groups" = 0 (default)
+ * or 2: the sweep exchanges positions through its table and checks the order of
+ * colliding lanes, 1 or 3: it groups the lanes of every step by hash first
+ * (several times slower; the path an unexpected order leads to);
+ * "sweep_prefetch" = accepted (0 to 64) and without effect;
  * "lzma_ctas" = LZMA2 second-stage CTAs per SM (1-8, default 3; values above
  * what fits on an SM -- 3, or 2 with 1024 threads -- run as that many);
  * "lzma_threads" = LZMA2 second-stage threads per CTA (256, 512 or 1024,
