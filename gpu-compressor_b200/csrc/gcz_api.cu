@@ -72,7 +72,7 @@ struct gcz_ctx {
     int staged = 1;
     int algo = 2;          // 1: fused single-warp kernels, 2: candidate sweep + second stage
     int parse_ctas = 3;    // second-stage CTAs per SM
-    int seg_width = 1024;  // Zstd speculative segment: 1024 per 8-lane group, or 2048/4096/8192 per warp
+    int seg_width = 1024;  // Zstd parse: 512 or 1024 lane parse, 2048/4096/8192 one warp per segment of that many bytes
     int sweep_warps = 7;   // warps that take turns on a window in the candidate sweep (4-7)
     int sweep_groups = 0;  // odd: the sweep groups the lanes of every step by hash first
     int sweep_prefetch = 4;  // accepted, without effect
@@ -1417,7 +1417,6 @@ int server_launch(gcz_server *sv, ServerSlot &s) {
             l.num_sms = c->num_sms;
             l.ctas_per_sm = c->parse_ctas;
             l.seg_width = (uint32_t)c->seg_width;
-        l.seg_width = (uint32_t)c->seg_width;
             l.wins = dw + a;
             GCZ_CUDA(c, gcz::launch_zstd_parse(l, s.st));
         }

@@ -68,7 +68,7 @@ struct Zstd2Launch {
     int num_sms;
     int ctas_per_sm;
     const WinDesc *wins;    // optional window table (null: windows at window * w)
-    uint32_t seg_width = 4096;  // speculative segment bytes per warp: 2048, 4096 or 8192 (schedule only)
+    uint32_t seg_width = 1024;  // 2048, 4096 or 8192: segment parse, bytes per warp; else the lane parse (schedule only)
 };
 
 cudaError_t launch_zstd_match(const ZstdLaunch &l, cudaStream_t st);

@@ -4,42 +4,52 @@
 // (gcz_sweep.cu).  Output: the exact sequence list of zstd_match_find
 // (zstd_compress.cu:179-355) for every window.
 //
-// 1. The window is staged into shared memory with 1-D bulk copies.  Every
-//    position's hash candidate (empty == position 0, :195-200) is verified on
-//    3 bytes (:241-246); the results form a bitmap.
-// 2. Parse.  The reference parse is a deterministic state machine over
-//    (pos, rep0, rep1, rep2): the next match and the next state depend on
-//    nothing else.  The window is cut into 4 KiB segments, one warp each.
-//    Every warp parses its segment from a guessed state (the segment start,
-//    repeat offsets {1,4,8}); warp 0's guess is the true initial state.  Then
-//    each warp keeps parsing past its segment end, and as soon as one of its
-//    matches equals a match of a later warp's list -- same start, length and
-//    offset, and the same repeat offsets afterwards -- both parses are in the
-//    same state and stay identical, so that later list is exact from there on.
-//    A chain walk from warp 0 then picks, in order: warp 0's list, its
-//    continuation up to the meeting point, the met warp's list from there, and
-//    so on; every list on the chain is exact by induction.  (On the synthetic
-//    workload a guessed parse meets the true one after ~180 bytes, three
-//    matches, so the overlap costs ~4% extra parse work.)
-//    Each warp parses like the reference, one match at a time, but with all
-//    32 lanes: the hash-match bits of the next positions come from the
-//    bitmap, the lanes test the three repeat offsets (:259-275) on the
-//    positions before the first hash match -- one (position, offset) pair per
-//    lane when there are at most 10 of them, one position per lane up to 32,
-//    and four positions per lane (8-byte compares) over up to 128 positions
-//    that hold no hash match -- a ballot finds the first event, matches are
-//    extended 128 bytes per warp iteration, and one lazy step (:278-307)
-//    follows.
-// 3. The chain is written in one pass as packed {ll | (ml-3) << 16, off} (or
-//    the reference's {ll, ml-3, off} triples) at the per-window stride, each
-//    literal length taken from the entry before it, capped at
-//    max_seqs exactly like the reference's `num_seqs < max_sequences_per_chunk`
-//    test (:309): the capped parse emits the first max_seqs matches of the
-//    uncapped one and nothing after them.
-// In the 8- and 4-lane group layouts, once only one group of a warp is still
-// continuing, the whole warp finishes that continuation with warp-wide steps.
-// If a continuation does not meet a later list within kContCap matches the
-// CTA falls back to an exact warp-wide parse of the whole window.
+// The window is staged into shared memory with 1-D bulk copies, and every
+// position's hash candidate (empty == position 0, :195-200) is verified on 3
+// bytes (:241-246); the results form a bitmap.  Two parses work from it.
+//
+// Lane parse (zstd_lane_parse_kernel, the default).  The reference parse is a
+// state machine over (pos, rep0, rep1, rep2), but its repeat offsets
+// (:259-275) decide a match only a few times per window.  So:
+// 1. Parse without repeat offsets.  Its state is the position alone.  The
+//    window is cut into 128-byte segments; every lane parses one at a time
+//    from the segment's start and pulls the next of its warp's when done.
+// 2. Link.  Where a segment's parse ends, it joins the list of the segment
+//    that holds that position: at once when that list has no match across it
+//    (the state is the position, so both parses go on alike), else after a few
+//    more matches.  The links from segment 0 pick the list of the whole parse.
+// 3. Check.  The repeat offsets of every literal run are those of the three
+//    matches before it, so all runs are tested at once, 16 positions and three
+//    offsets per lane task, tasks of 32 runs spread evenly over the lanes.
+// 4. Mend.  A run with a repeat-offset match is parsed again from its start,
+//    with repeat offsets, by one warp, until it emits a match of the list with
+//    the list's repeat offsets after it: from there on the list is right.
+//    Mends lie side by side; one that starts inside an earlier one is dropped.
+//    Every literal run is then either checked or parsed exactly, so the
+//    sequences are the reference's by induction over the runs.
+// A window with many such runs (records with a fixed stride), or one that
+// overflows a list, takes the segment parse instead.
+//
+// Segment parse (zstd_seg_parse_kernel, and the lane parse's way out).  Each
+// warp parses one segment of 2-8 KiB from a guessed state (the segment start,
+// repeat offsets {1,4,8}), then goes on past its end until one of its matches
+// equals a match of a later warp's list -- same start, length and offset, and
+// the same repeat offsets afterwards.  A chain walk from warp 0 picks the
+// lists; every list on the chain is exact by induction.  A warp step takes the
+// hash-match bits of the next positions from the bitmap, and the lanes test
+// the three repeat offsets on the positions before the first hash match -- one
+// (position, offset) pair per lane when there are at most 10 of them, one
+// position per lane up to 32, and four positions per lane (8-byte compares)
+// over up to 128 positions that hold no hash match; a ballot finds the first
+// event, matches are extended 128 bytes per warp iteration, and one lazy step
+// (:278-307) follows.  If a continuation does not meet a later list within
+// kContCap matches, one warp parses the whole window exactly.
+//
+// Output: packed {ll | (ml-3) << 16, off} (or the reference's {ll, ml-3, off}
+// triples) at the per-window stride, each literal length taken from the entry
+// before it, capped at max_seqs exactly like the reference's
+// `num_seqs < max_sequences_per_chunk` test (:309): the capped parse emits the
+// first max_seqs matches of the uncapped one and nothing after them.
 #include <type_traits>
 
 #include "gcz_common.cuh"
@@ -49,45 +59,34 @@ namespace gcz {
 namespace {
 
 constexpr uint32_t kMinMatch = 3;                 // MIN_MATCH_LEN, zstd_compress.cu:28
-// Speculative segment width is a schedule knob: 2, 4 or 8 KiB parsed by one
-// warp each (32, 16 or 8 warps per window), 1 KiB parsed by an 8-lane group
-// (four segments per warp, 64 per window), or 512 bytes parsed by a 4-lane
-// group (eight segments per warp, 128 per window).  It never changes the
-// sequences.
-template <uint32_t SegW, uint32_t GL = 32>
+
+// Segment parse: segment width (a schedule knob: 2, 4 or 8 KiB, one warp each;
+// it never changes the sequences).
+template <uint32_t SegW>
 struct SegCfg {
     static constexpr uint32_t kSegW = SegW;
     static constexpr uint32_t kSegs = kMaxWindow / SegW;
-    static constexpr uint32_t kThreads = kSegs * GL;
-    static constexpr uint32_t kWarps = kThreads / 32;
+    static constexpr uint32_t kThreads = kSegs * 32;
     // A segment's own parse ends with a step that starts before seg_end and
-    // looks at most kLook positions ahead (a warp's wide scan 128, a group's
-    // scan 32), the lazy step one more; matches do not overlap and are >= 3
-    // bytes, so a list holds at most (SegW + kLook) / 3 + 1 entries; lists are
-    // written in 32-entry blocks.
-    static constexpr uint32_t kLook = GL == 32 ? 128 : 32;
-    static constexpr uint32_t kSpecCap = ((SegW + kLook) / 3 + 1 + 31) / 32 * 32;
-    // continuation matches before giving up (a guessed parse meets the true
-    // one after ~3 matches; the cap keeps every layout's lists within the
-    // 1 KiB layout's 32768 entries per window)
-    static constexpr uint32_t kContCap = GL == 32 ? 256 : (GL == 8 ? 128 : 64);
+    // looks at most 128 positions ahead, the lazy step one more; matches do
+    // not overlap and are >= 3 bytes, so a list holds at most
+    // (SegW + 128) / 3 + 1 entries; lists are written in 32-entry blocks.
+    static constexpr uint32_t kSpecCap = ((SegW + 128) / 3 + 1 + 31) / 32 * 32;
+    static constexpr uint32_t kContCap = 256;  // continuation matches before giving up (three meet nearly always)
     static constexpr uint32_t kLaneCap = kSpecCap + kContCap;
     static constexpr uint32_t kMinBlocks = kThreads >= 1024 ? 1 : 3;
 };
 constexpr uint32_t kNoWarp = 0xFFFFu;
 constexpr uint32_t kNoEntry = 0xFFFFu;
 
-constexpr uint32_t kPre = 64;                           // zero bytes before the window
+constexpr uint32_t kPre = 32;                           // zero bytes before the window
 constexpr uint32_t kDataBytes = kPre + kMaxWindow + 64; // + zero pad after it
 constexpr uint32_t kBmWords = kMaxWindow / 32 + 8;  // the wide scan reads up to 4 words past a step's first
 
+// Shared-memory fields of the segment parse (list lengths, indices and output
+// offsets of a window are below 2^15).
 template <uint32_t kSegs>
-struct SmemLayout {
-    uint8_t data[kDataBytes];
-    uint32_t bm[kBmWords];
-    // Per segment, 16 bits each (list lengths, indices and output offsets of
-    // a window are below 2^15; segment indices below 2^7), so that 128
-    // segments fit beside the window at three CTAs per SM.
+struct SegSmem {
     uint16_t spec_count[kSegs];
     uint16_t cont_count[kSegs];
     uint16_t sync_warp[kSegs];
@@ -96,10 +95,64 @@ struct SmemLayout {
     uint16_t out_off[kSegs];
     uint16_t on_chain[kSegs];
     uint16_t prev_last[kSegs];  // seg index of the entry before a chain segment's first copied one (kNoEntry: none)
-    uint32_t flags;
+};
+
+struct ParseScalars {
+    uint32_t flags;    // 1: the segment parse gives up, 2: staging failed, 4: the lane parse gives up
     uint32_t total;
     uint32_t covered;
+    uint32_t count;    // literal runs with a repeat-offset match found
+    uint32_t mends;    // mends of the window
+    uint32_t bigs;     // continuations that took a long list
+    uint32_t warp_sum[16];
     alignas(8) uint64_t bar;
+};
+
+// Lane parse.
+constexpr uint32_t kLThreads = 512, kLWarps = kLThreads / 32;
+constexpr uint32_t kLSegW = 128, kLSegs = kMaxWindow / kLSegW;  // four bitmap words per segment
+constexpr uint32_t kLPool = kLSegs / kLWarps;                   // segments of one warp
+constexpr uint32_t kLCap = (kLSegW + 2) / 3;                    // matches that start their search in a segment
+constexpr uint32_t kLCont = 12;                                 // matches before a segment's parse joins a list ...
+constexpr uint32_t kLBig = 16, kLBigCap = 128;                  // ... and lists for the few that take more
+constexpr uint32_t kFixes = 256, kFixCap = 255;                 // mends per window, most matches per mend
+// Entries in a window's scratch: the segments' lists, then the continuations;
+// once the list of the whole parse is known it takes the lists' place, and
+// the mends that of the continuations.
+constexpr uint32_t kLContBase = kLSegs * kLCap;
+constexpr uint32_t kLBigBase = kLContBase + kLSegs * kLCont;
+constexpr uint32_t kLEntries = kLBigBase + kLBig * kLBigCap;
+constexpr uint32_t kFixEntries = kLEntries - kLContBase;        // shared by a window's mends
+static_assert(kLContBase >= 21846, "the whole parse fits where the lists were");
+static_assert(kLCont + kLBigCap <= 255, "8-bit counts");
+
+struct LaneSmem {
+    union {
+        struct {
+            uint16_t link[kLSegs];   // parse end past the segment, then the segment joined, then the output offset
+            uint8_t count[kLSegs];   // list entries
+            uint8_t from[kLSegs];    // entry joined at, then the first entry on the chain
+            uint8_t cont[kLSegs];    // continuation entries
+            uint16_t big[kLBig];     // segments whose continuation goes on in a list of kLBigCap entries
+            uint32_t chain[kLSegs / 32];  // segments on the chain
+        };
+        struct {
+            uint16_t run[kFixes];    // literal runs with a repeat-offset match
+            uint16_t meet[kFixes];   // entry a mend ends at
+            int16_t shift[kFixes];   // output index minus list index from there on
+            uint8_t len[kFixes];     // entries of the mend
+            uint8_t list[kFixes];    // the mend's list in the scratch
+        } fix;
+        SegSmem<kLWarps> seg;
+    };
+};
+
+template <class P>
+struct SmemLayout {
+    uint8_t data[kDataBytes];
+    uint32_t bm[kBmWords];
+    P p;
+    ParseScalars s;
 };
 
 struct Zstd2Args {
@@ -410,40 +463,6 @@ __device__ __forceinline__ bool warp_step(const Win &w, const uint32_t *bm, Cand
     return true;
 }
 
-// Group-wide extension: the lanes of each GL-lane group compare 4 bytes each
-// (4 * GL per iteration) of their group's own (c, q, lim) and get the first
-// index in [0, lim) where bytes c+i and q+i differ, else lim; groups with
-// act == false get 0.  All 32 lanes call it (the loop runs while any group
-// is still extending).
-template <uint32_t GL>
-__device__ __forceinline__ uint32_t extend_group(const Win &w, uint32_t c, uint32_t q, uint32_t lim, bool act) {
-    const uint32_t lane = lane_id(), gl = lane & (GL - 1u), gb = lane & ~(GL - 1u);
-    uint32_t len = 0, out = 0;
-    bool done = !act;
-    while (__any_sync(kFull, !done)) {
-        const uint32_t k = len + 8u * gl;  // 8 bytes per lane
-        uint32_t res = k;
-        if (!done && k < lim) {
-            uint32_t ql, qh, cl, ch;
-            w.u64(static_cast<int>(q + k), ql, qh);
-            w.u64(static_cast<int>(c + k), cl, ch);
-            const uint32_t dl = ql ^ cl, dh = qh ^ ch;
-            const uint32_t fb = dl ? (static_cast<uint32_t>(__ffs(dl)) - 1u) >> 3
-                                   : (dh ? 4u + ((static_cast<uint32_t>(__ffs(dh)) - 1u) >> 3) : 8u);
-            const uint32_t rem = lim - k;
-            res = k + (fb < rem ? fb : rem);
-        }
-        const uint32_t sb = (__ballot_sync(kFull, !done && res < k + 8u) >> gb) & ((1u << GL) - 1u);
-        const uint32_t v = __shfl_sync(kFull, res, gb + (sb ? static_cast<uint32_t>(__ffs(sb)) - 1u : 0u));
-        if (!done && sb) {
-            out = v;
-            done = true;
-        }
-        len += 8u * GL;
-    }
-    return out;
-}
-
 // Bit t (t < 16) set when bytes q+t .. q+t+2 equal bytes q-r+t .. q-r+t+2
 // (zstd_compress.cu:259-275 tests one position at a time).  Both 18-byte
 // ranges are read as aligned words; a byte of x ^ y is zero exactly when its
@@ -473,137 +492,6 @@ __device__ __forceinline__ uint32_t rep3_scan16(const Win &w, uint32_t q, uint32
     return m;
 }
 
-// Bit t (t < 32) set when bytes q+t .. q+t+2 equal bytes q-r+t .. q-r+t+2:
-// rep3_scan16 over 32 positions (34-byte ranges, ten aligned words each).
-__device__ __forceinline__ uint32_t rep3_scan32(const Win &w, uint32_t q, uint32_t r) {
-    const uint32_t *wd = reinterpret_cast<const uint32_t *>(w.d - kPre);
-    const uint32_t ax = q + kPre, ay = q - r + kPre;
-    const uint32_t *px = wd + (ax >> 2), *py = wd + (ay >> 2);
-    const uint32_t sx = (ax & 3u) * 8u, sy = (ay & 3u) * 8u;
-    uint32_t z[9];
-    uint32_t xp = px[0], yp = py[0];
-#pragma unroll
-    for (uint32_t j = 0; j < 9; ++j) {
-        const uint32_t xn = px[j + 1], yn = py[j + 1];
-        const uint32_t d = __funnelshift_r(xp, xn, sx) ^ __funnelshift_r(yp, yn, sy);
-        z[j] = ~(((d & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | d | 0x7F7F7F7Fu);
-        xp = xn;
-        yp = yn;
-    }
-    uint32_t m = 0;
-#pragma unroll
-    for (uint32_t j = 0; j < 8; ++j) {
-        const uint32_t e = z[j] & __funnelshift_r(z[j], z[j + 1], 8) & __funnelshift_r(z[j], z[j + 1], 16);
-        m |= ((e * 0x00204081u) >> 28) << (4u * j);
-    }
-    return m;
-}
-
-// One step of the exact parse for every GL-lane group of the warp at once
-// (GL = 8 or 4), each from its own state s (group-uniform); groups with
-// run == false keep theirs.  A group looks at the 32 positions from s.p: the
-// hash-match bits come from the bitmap, and the lanes test the three repeat
-// offsets among the positions before the first hash match
-// (zstd_compress.cu:259-275) -- six lanes of 16 positions each (GL = 8) or
-// three of 32 (GL = 4).  The first event is the match, extended 8 * GL bytes
-// per group iteration, with the lazy step (:278-307) at f+1; with no event
-// the group moves over the 32 positions.  Returns whether the group found a
-// match (m set, s advanced past it, repeat offsets updated).
-template <uint32_t GL>
-__device__ __forceinline__ bool group_step(const Win &w, const uint32_t *bm, const uint16_t *cand, uint32_t size,
-                                           bool lazy, bool run, PState &s, Match &m) {
-    static_assert(GL == 8 || GL == 4, "8- or 4-lane groups");
-    const uint32_t lane = lane_id(), gl = lane & (GL - 1u), gb = lane & ~(GL - 1u);
-    const uint32_t p = run ? s.p : 0u;
-    const uint32_t lim = run ? size - 3u - p : 0u;
-    const uint32_t n32 = lim < 32u ? lim : 32u;
-    uint32_t H = __funnelshift_r(bm[p >> 5], bm[(p >> 5) + 1], p & 31u);
-    if (n32 < 32u) H &= (1u << n32) - 1u;
-    const uint32_t nh = H ? static_cast<uint32_t>(__ffs(H)) - 1u : n32;  // positions without a hash match
-    // The candidates at the first hash match and the position after it are
-    // loaded before the repeat-offset test, so that their latency overlaps
-    // it: the event is that hash match unless a repeat offset hits earlier
-    // (a few times per window), and only then is cand(f+1) loaded again.
-    const uint32_t fh = nh < n32 ? p + nh : 0u;
-    const uint32_t ch0 = cand[fh], ch1 = cand[fh + 1u];
-    uint32_t m0, m1, m2;  // per repeat offset: hits among the 32 positions
-    if constexpr (GL == 8) {
-        // Lane 2k+h (k < 3) tests repeat offset k on the 16 positions from
-        // p + 16h that come before the first hash match and whose source lies
-        // in the window; lanes 6 and 7 test nothing.
-        const uint32_t rk = gl >> 1, hh = gl & 1u;
-        const uint32_t q0 = p + 16u * hh;
-        const uint32_t rv = rk == 0u ? s.r0 : (rk == 1u ? s.r1 : s.r2);
-        const uint32_t lo = rv > q0 ? (rv - q0 < 16u ? rv - q0 : 16u) : 0u;
-        const uint32_t hi = (rk < 3u && nh > 16u * hh) ? (nh - 16u * hh < 16u ? nh - 16u * hh : 16u) : 0u;
-        const uint32_t vm = ((1u << hi) - 1u) & ~((1u << lo) - 1u);
-        const uint32_t mk = rep3_scan16(w, q0, rv <= q0 + 16u ? rv : 0u) & vm;
-        const uint32_t mo = __shfl_xor_sync(kFull, mk, 1);
-        const uint32_t mf = hh ? (mo | (mk << 16)) : (mk | (mo << 16));  // offset rk over all 32 positions
-        m0 = __shfl_sync(kFull, mf, gb);
-        m1 = __shfl_sync(kFull, mf, gb + 2u);
-        m2 = __shfl_sync(kFull, mf, gb + 4u);
-    } else {
-        // Lane k (k < 3) tests repeat offset k on the 32 positions from p
-        // that come before the first hash match and whose source lies in the
-        // window; lane 3 tests nothing.
-        const uint32_t rv = gl == 0u ? s.r0 : (gl == 1u ? s.r1 : s.r2);
-        const uint32_t lo = rv > p ? (rv - p < 32u ? rv - p : 32u) : 0u;
-        const uint32_t hi = gl < 3u ? nh : 0u;  // nh <= 32
-        const uint32_t vm = (hi >= 32u ? ~0u : (1u << hi) - 1u) & (lo >= 32u ? 0u : ~((1u << lo) - 1u));
-        const uint32_t mk = rep3_scan32(w, p, rv <= p + 32u ? rv : 0u) & vm;
-        m0 = __shfl_sync(kFull, mk, gb);
-        m1 = __shfl_sync(kFull, mk, gb + 1u);
-        m2 = __shfl_sync(kFull, mk, gb + 2u);
-    }
-    const uint32_t al = m0 | m1 | m2;
-    const bool rep = al != 0u;
-    const bool ev = run && (rep || nh < n32);
-    uint32_t f = p + nh, r = 0;
-    if (rep) {
-        const uint32_t t = static_cast<uint32_t>(__ffs(al)) - 1u;
-        f = p + t;
-        r = (m0 >> t) & 1u ? 0u : ((m1 >> t) & 1u ? 1u : 2u);
-    }
-    const uint32_t fc = ev ? f : 0u;
-    const uint32_t cf = zmap(ch0);
-    uint32_t cf1 = zmap(ch1);
-    if (rep) cf1 = zmap(cand[fc + 1u]);
-    uint32_t off, c0;
-    if (!rep) {
-        off = fc - cf;
-        c0 = cf;
-    } else {  // first repeat offset with 3 equal bytes wins
-        off = r == 0u ? s.r0 : (r == 1u ? s.r1 : s.r2);
-        c0 = fc - off;
-    }
-    // The lazy candidate at f+1 is skipped when it is the same match one byte on
-    // (cand(f+1) == c0 + 1): it is exactly one byte shorter, never taken.
-    const bool ltry = ev && lazy && fc + 4u < size && bm_bit(bm, fc + 1u) && cf1 != c0 + 1u;
-    const uint32_t e1 = extend_group<GL>(w, c0 + kMinMatch, fc + kMinMatch, ev ? size - fc - kMinMatch : 0u, ev);
-    const uint32_t e2 =
-        extend_group<GL>(w, cf1 + kMinMatch, fc + 1u + kMinMatch, ltry ? size - fc - 1u - kMinMatch : 0u, ltry);
-    uint32_t len = e1 + kMinMatch;
-    f = fc;
-    if (ltry && e2 + kMinMatch > len + 1u) {
-        f = fc + 1u;
-        len = e2 + kMinMatch;
-        off = f - cf1;
-    }
-    if (ev) {
-        m.start = f;
-        m.len = len;
-        m.off = off;
-        s.r2 = s.r1;
-        s.r1 = s.r0;
-        s.r0 = off;
-        s.p = f + len;
-    } else if (run) {
-        s.p = p + n32;
-    }
-    return ev;
-}
-
 __device__ __forceinline__ uint2 pack_entry(const Match &m) {
     return make_uint2(m.start | ((m.len - kMinMatch) << 16), m.off);
 }
@@ -631,34 +519,355 @@ struct ListWriter {
     }
 };
 
-// ---------------------------------------------------------------- kernel
-template <bool kRef, uint32_t SegW, uint32_t GL>
-__global__ void __launch_bounds__(SegCfg<SegW, GL>::kThreads, SegCfg<SegW, GL>::kMinBlocks)
-    zstd_parse_kernel(Zstd2Args a) {
-    using C = SegCfg<SegW, GL>;
-    constexpr uint32_t kSegW = C::kSegW, kWarps = C::kWarps, kThreads = C::kThreads, kSegs = C::kSegs;
+// ---------------------------------------------------------------- shared parts of the kernels
+// First byte and size of window wi.
+__device__ __forceinline__ void window_of(const Zstd2Args &a, uint32_t wi, uint64_t &start, uint32_t &size) {
+    start = a.wins ? a.wins[wi].offset : static_cast<uint64_t>(wi) * a.window;
+    size = a.wins ? a.wins[wi].size : static_cast<uint32_t>(a.n - start < a.window ? a.n - start : a.window);
+}
+
+// Verification bitmap of a staged window, by all kW warps of the CTA: bit q
+// set when q can start a match and its candidate matches on 3 bytes.
+template <uint32_t kW>
+__device__ __forceinline__ void verify_window(const Win &win, uint32_t *bm, const uint16_t *cand, uint32_t size) {
+    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+    // Lane l covers positions 4l .. 4l+3 of a 128-position chunk: one
+    // 8-byte load brings its four candidates (2-byte loads where the
+    // window's candidates are not 8-byte aligned or the chunk ends the
+    // window), one aligned 8-byte read its own bytes, and the 8 lanes of
+    // each bitmap word gather their four bits with three shuffles.  kVC
+    // chunks per batch: their candidate loads are all issued first.
+    constexpr uint32_t kChunks = kBmWords / 4u, kVC = 4;
+    static_assert(kBmWords % 4u == 0u, "bitmap words come in 128-position chunks");
+    const bool al8 = (reinterpret_cast<uintptr_t>(cand) & 7u) == 0u;
+    for (uint32_t c0 = warp * kVC; c0 < kChunks; c0 += kW * kVC) {
+        uint2 cv[kVC];
+#pragma unroll
+        for (uint32_t u = 0; u < kVC; ++u) {
+            const uint32_t q = (c0 + u) * 128u + 4u * lane;
+            if (al8 && q + 4u <= size) {
+                cv[u] = *reinterpret_cast<const uint2 *>(cand + q);
+            } else {
+                uint32_t e[4];
+#pragma unroll
+                for (uint32_t k = 0; k < 4; ++k) e[k] = q + k < size ? static_cast<uint32_t>(cand[q + k]) : 0u;
+                cv[u] = make_uint2(e[0] | (e[1] << 16), e[2] | (e[3] << 16));
+            }
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < kVC; ++u) {
+            const uint32_t ch = c0 + u;
+            const uint32_t q = ch * 128u + 4u * lane;
+            uint32_t nib = 0;
+            if (q < size) {
+                const uint32_t x0 = win.w32(q), x1 = win.w32(q + 4u);
+#pragma unroll
+                for (uint32_t k = 0; k < 4; ++k) {
+                    const uint32_t cw = k < 2u ? cv[u].x : cv[u].y;
+                    const uint32_t c = zmap((k & 1u) ? cw >> 16 : cw & 0xFFFFu);
+                    const uint32_t xk = k ? __funnelshift_r(x0, x1, 8u * k) : x0;
+                    const uint32_t qk = q + k;
+                    const bool hm = qk + 3u < size && qk > 0u && ((xk ^ win.u32(static_cast<int>(c))) & 0xFFFFFFu) == 0u;
+                    nib |= static_cast<uint32_t>(hm) << k;
+                }
+            }
+            uint32_t v = nib << (4u * (lane & 7u));
+            v |= __shfl_xor_sync(kFull, v, 1);
+            v |= __shfl_xor_sync(kFull, v, 2);
+            v |= __shfl_xor_sync(kFull, v, 4);
+            if ((lane & 7u) == 0u && ch < kChunks) bm[ch * 4u + (lane >> 3)] = v;
+        }
+    }
+}
+
+// Output entry o of window wi.
+template <bool kRef>
+__device__ __forceinline__ void write_seq(const Zstd2Args &a, uint32_t wi, uint32_t o, uint32_t ll, uint32_t mlm3,
+                                          uint32_t off) {
+    if constexpr (kRef) {
+        uint32_t *r = a.ref_seqs + (static_cast<uint64_t>(wi) * a.max_seqs + o) * 3u;
+        r[0] = ll;
+        r[1] = mlm3;
+        r[2] = off;
+    } else {
+        a.packed[static_cast<uint64_t>(wi) * a.max_seqs + o] = make_uint2(ll | (mlm3 << 16), off);
+    }
+}
+
+// ---------------------------------------------------------------- segment parse
+// All threads of the CTA (SegCfg<SegW>::kThreads) call it with the window
+// staged and verified, S.flags & 1 clear and S.covered zero.
+template <bool kRef, uint32_t SegW>
+__device__ __forceinline__ void parse_segments(const Zstd2Args &a, SegSmem<SegCfg<SegW>::kSegs> &G, ParseScalars &S,
+                                               const Win &win, const uint32_t *bm, const uint16_t *cand, uint2 *seg,
+                                               uint32_t wi, uint32_t size, bool lazy) {
+    using C = SegCfg<SegW>;
+    constexpr uint32_t kSegW = C::kSegW, kSegs = C::kSegs;
     constexpr uint32_t kSpecCap = C::kSpecCap, kLaneCap = C::kLaneCap, kContCap = C::kContCap;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t lim_pos = size > 3u ? size - 3u : 0u;  // positions q < lim_pos can start a match
+    // ---- 2a. speculative parse of each segment (one warp each)
+    const uint32_t seg_start = warp * kSegW, seg_end = seg_start + kSegW;
+    const bool active = seg_start < lim_pos;
+    const bool last_active = !(seg_end < lim_pos);
+    ListWriter lw(seg + warp * kLaneCap);
+    PState s{seg_start, 1u, 4u, 8u};
+    CandBuf cb{cand, size, 0u, 0u, 0u, 0u};
+    if (active) cb.init(seg_start);
+    if (active) {
+        const uint32_t stop = last_active ? size : seg_end;
+        Match m;
+        while (s.p < stop && s.p + 3u < size) {
+            if (warp_step(win, bm, cb, size, lazy, s, m)) lw.put(pack_entry(m));
+        }
+        lw.flush();
+    }
+    if (lane == 0) {
+        G.spec_count[warp] = lw.n;
+        G.cont_count[warp] = 0;
+        G.sync_warp[warp] = kNoWarp;
+        G.sync_idx[warp] = 0;
+    }
+    __syncthreads();
+
+    // ---- 2b. continue each warp's parse until it meets a later warp's list
+    if (active && !last_active) {
+        ListWriter cw(seg + warp * kLaneCap + kSpecCap);
+        uint32_t t = kNoWarp, j = 0;
+        Match m;
+        while (s.p + 3u < size) {
+            if (!warp_step(win, bm, cb, size, lazy, s, m)) continue;
+            const uint32_t tw = m.start / kSegW;  // warp whose segment holds this match start
+            if (tw != t) {
+                t = tw;
+                j = 0;
+            }
+            const uint32_t tcount = G.spec_count[t];
+            const uint2 *tl = seg + t * kLaneCap;
+            // first entry of t's list with start >= m.start (lists are sorted by start)
+            for (;;) {
+                const uint32_t idx = j + lane;
+                const bool ge = idx >= tcount || (tl[idx].x & 0xFFFFu) >= m.start;
+                const uint32_t b = __ballot_sync(kFull, ge);
+                if (b) {
+                    j += static_cast<uint32_t>(__ffs(b)) - 1u;
+                    break;
+                }
+                j += 32u;
+            }
+            bool met = false;
+            if (j < tcount) {
+                const uint2 e = tl[j];
+                if (e.x == pack_entry(m).x && e.y == m.off) {
+                    uint32_t e0, e1, e2;
+                    reps_after(tl, j, e0, e1, e2);
+                    met = e0 == s.r0 && e1 == s.r1 && e2 == s.r2;
+                }
+            }
+            if (met) {
+                if (lane == 0) {
+                    G.sync_warp[warp] = t;
+                    G.sync_idx[warp] = j;
+                }
+                break;
+            }
+            if (cw.n == kContCap) {
+                if (lane == 0) atomicOr(&S.flags, 1u);  // give up: exact fallback below
+                break;
+            }
+            cw.put(pack_entry(m));
+        }
+        cw.flush();
+        if (lane == 0) G.cont_count[warp] = cw.n;
+    }
+    __syncthreads();
+
+    if (!(S.flags & 1u)) {
+        // ---- 3. chain walk, then copy in chain order.  Nearly always every
+        // continuation meets the next segment's list, so the chain is
+        // segments 0..K in order (K: the first segment with no link): warp
+        // 0 then sets it up at once -- output offsets by a scan of the
+        // segments' contributions, each segment's preceding entry by a max
+        // scan (entry indices grow with the segment).  Otherwise one
+        // thread walks the links.
+        bool chained = false;
+        if (warp == 0 && lim_pos > 0) {
+            constexpr uint32_t kPer = (kSegs + 31u) / 32u;  // segments per lane, contiguous
+            uint32_t kf = kSegs;
+            bool gap = false;
+#pragma unroll
+            for (uint32_t u = 0; u < kPer; ++u) {
+                const uint32_t i = lane * kPer + u;
+                if (i < kSegs && G.sync_warp[i] == kNoWarp && i < kf) kf = i;
+            }
+            const uint32_t K = __reduce_min_sync(kFull, kf);  // segment 0 always parses, so K < kSegs
+#pragma unroll
+            for (uint32_t u = 0; u < kPer; ++u) {
+                const uint32_t i = lane * kPer + u;
+                if (i < K && G.sync_warp[i] != i + 1u) gap = true;
+            }
+            chained = !__any_sync(kFull, gap);
+            if (chained) {
+                uint32_t con[kPer], lst1[kPer], sum = 0, lmax = 0;
+#pragma unroll
+                for (uint32_t u = 0; u < kPer; ++u) {
+                    const uint32_t i = lane * kPer + u;
+                    con[u] = 0;
+                    lst1[u] = 0;
+                    if (i <= K) {
+                        const uint32_t from = i ? static_cast<uint32_t>(G.sync_idx[i - 1u]) : 0u;
+                        const uint32_t ns = G.spec_count[i], nc = G.cont_count[i];
+                        con[u] = ns - from + nc;
+                        if (con[u]) lst1[u] = 1u + i * kLaneCap + (nc ? kSpecCap + nc - 1u : ns - 1u);
+                    }
+                    sum += con[u];
+                    lmax = lst1[u] > lmax ? lst1[u] : lmax;
+                }
+                // exclusive scans over the lanes: sum of contributions, max of last entries (+1)
+                uint32_t incl = sum, mx = lmax;
+#pragma unroll
+                for (uint32_t d = 1; d < 32u; d <<= 1) {
+                    const uint32_t o = __shfl_up_sync(kFull, incl, d), om = __shfl_up_sync(kFull, mx, d);
+                    if (lane >= d) {
+                        incl += o;
+                        mx = om > mx ? om : mx;
+                    }
+                }
+                uint32_t acc = incl - sum, last1 = __shfl_up_sync(kFull, mx, 1);
+                if (lane == 0) last1 = 0;
+#pragma unroll
+                for (uint32_t u = 0; u < kPer; ++u) {
+                    const uint32_t i = lane * kPer + u;
+                    if (i >= kSegs) continue;
+                    const bool on = i <= K;
+                    G.on_chain[i] = on ? 1u : 0u;
+                    if (on) {
+                        G.chain_from[i] = i ? G.sync_idx[i - 1u] : 0u;
+                        G.out_off[i] = acc;
+                        G.prev_last[i] = last1 ? last1 - 1u : kNoEntry;
+                    }
+                    acc += con[u];
+                    last1 = lst1[u] > last1 ? lst1[u] : last1;
+                }
+                if (lane == 31u) S.total = incl;
+            }
+        }
+        chained = __syncthreads_or(chained);
+        if (tid == 0 && !chained) {
+            for (uint32_t i = 0; i < kSegs; ++i) G.on_chain[i] = 0;
+            uint32_t cur = 0, from = 0, acc = 0, last = kNoEntry;
+            if (lim_pos > 0) {
+                for (;;) {
+                    G.on_chain[cur] = 1;
+                    G.chain_from[cur] = from;
+                    G.out_off[cur] = acc;
+                    G.prev_last[cur] = last;
+                    const uint32_t ns = G.spec_count[cur], nc = G.cont_count[cur];
+                    acc += (ns - from) + nc;
+                    if (ns + nc > from) last = cur * kLaneCap + (nc ? kSpecCap + nc - 1u : ns - 1u);
+                    const uint32_t nx = G.sync_warp[cur];
+                    if (nx == kNoWarp) break;
+                    from = G.sync_idx[cur];
+                    cur = nx;
+                }
+            }
+            S.total = acc;
+        }
+        __syncthreads();
+        const uint32_t total = S.total;
+        const uint32_t keep = total < a.max_seqs ? total : a.max_seqs;
+        // Write {ll, ml-3, off} in chain order: an entry's literal length is
+        // its start minus the end of the entry before it -- the previous
+        // entry of the same list, or for a segment's first copied entry the
+        // last entry contributed before it, which the chain walk located.
+        const uint32_t csg = tid / 32u, csl = tid % 32u;  // segment whose list this thread copies
+        if (G.on_chain[csg]) {
+            const uint32_t from = G.chain_from[csg], ns = G.spec_count[csg], nc = G.cont_count[csg];
+            const uint32_t base = G.out_off[csg];
+            const uint2 *mine = seg + csg * kLaneCap;
+            uint32_t cov = 0;
+            for (uint32_t i = from + csl; i < ns + nc; i += 32u) {
+                const uint32_t o = base + (i - from);
+                if (o >= keep) break;
+                const uint2 e = mine[i < ns ? i : kSpecCap + (i - ns)];
+                const uint32_t pi =
+                    i > from ? csg * kLaneCap + (i - 1u < ns ? i - 1u : kSpecCap + (i - 1u - ns)) : G.prev_last[csg];
+                uint32_t pe = 0;
+                if (pi != kNoEntry) {
+                    const uint32_t px = seg[pi].x;
+                    pe = (px & 0xFFFFu) + (px >> 16) + kMinMatch;
+                }
+                const uint32_t st0 = e.x & 0xFFFFu, mlm3 = e.x >> 16;
+                const uint32_t ll = st0 - pe;
+                cov += mlm3 + kMinMatch;
+                if constexpr (kRef) {
+                    uint32_t *r = a.ref_seqs + (static_cast<uint64_t>(wi) * a.max_seqs + o) * 3u;
+                    r[0] = ll;
+                    r[1] = mlm3;
+                    r[2] = e.y;
+                } else {
+                    a.packed[static_cast<uint64_t>(wi) * a.max_seqs + o] = make_uint2(ll | (mlm3 << 16), e.y);
+                }
+            }
+            if (cov) atomicAdd(&S.covered, cov);
+        }
+        __syncthreads();
+        if (tid == 0) {
+            a.seq_counts[wi] = keep;
+            if (a.lit_counts) a.lit_counts[wi] = size - S.covered;
+        }
+    } else if (warp == 0) {
+        // ---- exact warp-wide parse of the whole window
+        PState fs{0u, 1u, 4u, 8u};
+        CandBuf fcb{cand, size, 0u, 0u, 0u, 0u};
+        fcb.init(0u);
+        uint32_t idx = 0, cov = 0, prev_end = 0;
+        Match m;
+        while (fs.p + 3u < size) {
+            if (!warp_step(win, bm, fcb, size, lazy, fs, m)) continue;
+            if (idx < a.max_seqs && lane == 0) {
+                const uint32_t ll = m.start - prev_end;
+                if constexpr (kRef) {
+                    uint32_t *r = a.ref_seqs + (static_cast<uint64_t>(wi) * a.max_seqs + idx) * 3u;
+                    r[0] = ll;
+                    r[1] = m.len - kMinMatch;
+                    r[2] = m.off;
+                } else {
+                    a.packed[static_cast<uint64_t>(wi) * a.max_seqs + idx] =
+                        make_uint2(ll | ((m.len - kMinMatch) << 16), m.off);
+                }
+            }
+            if (idx < a.max_seqs) cov += m.len;
+            ++idx;
+            prev_end = m.start + m.len;
+        }
+        if (lane == 0) {
+            a.seq_counts[wi] = idx < a.max_seqs ? idx : a.max_seqs;
+            if (a.lit_counts) a.lit_counts[wi] = size - cov;
+            atomicAdd(a.status + 1, 1u);  // fallback counter (diagnostics)
+        }
+    }
+}
+
+template <bool kRef, uint32_t SegW>
+__global__ void __launch_bounds__(SegCfg<SegW>::kThreads, SegCfg<SegW>::kMinBlocks)
+    zstd_seg_parse_kernel(Zstd2Args a) {
+    using C = SegCfg<SegW>;
     extern __shared__ __align__(128) uint8_t smem_raw[];
-    SmemLayout<kSegs> &S = *reinterpret_cast<SmemLayout<kSegs> *>(smem_raw);
+    SmemLayout<SegSmem<C::kSegs>> &M = *reinterpret_cast<SmemLayout<SegSmem<C::kSegs>> *>(smem_raw);
+    ParseScalars &S = M.s;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     uint32_t parity = 0;
     if (tid == 0) {
         mbar_init(&S.bar, 1);
         fence_mbar_init();
     }
-    for (uint32_t i = tid; i < kPre / 4; i += kThreads) reinterpret_cast<uint32_t *>(S.data)[i] = 0u;
-    __syncthreads();
-    Win win{S.data + kPre};
-    const bool lazy = a.lazy != 0;
-
+    for (uint32_t i = tid; i < kPre / 4; i += C::kThreads) reinterpret_cast<uint32_t *>(M.data)[i] = 0u;
+    Win win{M.data + kPre};
     for (uint32_t wi = blockIdx.x; wi < a.num_windows; wi += gridDim.x) {
-        const uint64_t start = a.wins ? a.wins[wi].offset : static_cast<uint64_t>(wi) * a.window;
-        const uint32_t size =
-            a.wins ? a.wins[wi].size : static_cast<uint32_t>(a.n - start < a.window ? a.n - start : a.window);
-        const uint16_t *cand = a.cand + start;
-        uint2 *seg = a.seg + static_cast<uint64_t>(wi) * a.seg_stride;
-
-        // ---- 1. stage the window (warp 0), verification bitmap (all warps)
+        uint64_t start;
+        uint32_t size;
+        window_of(a, wi, start, size);
         __syncthreads();  // previous window fully consumed
         if (tid == 0) {
             S.flags = 0;
@@ -666,502 +875,637 @@ __global__ void __launch_bounds__(SegCfg<SegW, GL>::kThreads, SegCfg<SegW, GL>::
         }
         __syncthreads();
         if (warp == 0) {
-            if (!stage_window(S.data + kPre, a.src + start, size, &S.bar, parity, a.status) && lane == 0)
+            if (!stage_window(M.data + kPre, a.src + start, size, &S.bar, parity, a.status) && lane == 0)
                 S.flags = 2u;
         }
         __syncthreads();
         if (S.flags & 2u) return;  // bulk copy never completed: status already recorded, all threads leave
-        // Lane l covers positions 4l .. 4l+3 of a 128-position chunk: one
-        // 8-byte load brings its four candidates (2-byte loads where the
-        // window's candidates are not 8-byte aligned or the chunk ends the
-        // window), one aligned 8-byte read its own bytes, and the 8 lanes of
-        // each bitmap word gather their four bits with three shuffles.  kVC
-        // chunks per batch: their candidate loads are all issued first.
-        constexpr uint32_t kChunks = kBmWords / 4u, kVC = 4;
-        static_assert(kBmWords % 4u == 0u, "bitmap words come in 128-position chunks");
-        const bool al8 = (reinterpret_cast<uintptr_t>(cand) & 7u) == 0u;
-        for (uint32_t c0 = warp * kVC; c0 < kChunks; c0 += kWarps * kVC) {
-            uint2 cv[kVC];
-#pragma unroll
-            for (uint32_t u = 0; u < kVC; ++u) {
-                const uint32_t q = (c0 + u) * 128u + 4u * lane;
-                if (al8 && q + 4u <= size) {
-                    cv[u] = *reinterpret_cast<const uint2 *>(cand + q);
-                } else {
-                    uint32_t e[4];
-#pragma unroll
-                    for (uint32_t k = 0; k < 4; ++k) e[k] = q + k < size ? static_cast<uint32_t>(cand[q + k]) : 0u;
-                    cv[u] = make_uint2(e[0] | (e[1] << 16), e[2] | (e[3] << 16));
-                }
+        verify_window<C::kThreads / 32>(win, M.bm, a.cand + start, size);
+        __syncthreads();
+        parse_segments<kRef, SegW>(a, M.p, S, win, M.bm, a.cand + start,
+                                   a.seg + static_cast<uint64_t>(wi) * a.seg_stride, wi, size, a.lazy != 0);
+    }
+}
+
+// ---------------------------------------------------------------- lane parse
+// First set bit of bm in [p, stop), else stop.
+__device__ __forceinline__ uint32_t next_bit(const uint32_t *bm, uint32_t p, uint32_t stop) {
+    if (p >= stop) return stop;
+    uint32_t i = p >> 5, b = bm[i] & (~0u << (p & 31u));
+    while (!b) {
+        if ((++i << 5) >= stop) return stop;
+        b = bm[i];
+    }
+    const uint32_t f = (i << 5) + static_cast<uint32_t>(__ffs(b)) - 1u;
+    return f < stop ? f : stop;
+}
+
+// Equal bytes (0-8) at the start of two 8-byte reads.
+__device__ __forceinline__ uint32_t equal8(const Win &w, uint32_t c, uint32_t q) {
+    uint32_t ql, qh, cl, ch;
+    w.u64(static_cast<int>(q), ql, qh);
+    w.u64(static_cast<int>(c), cl, ch);
+    const uint32_t dl = ql ^ cl, dh = qh ^ ch;
+    return dl ? (static_cast<uint32_t>(__ffs(dl)) - 1u) >> 3
+              : (dh ? 4u + ((static_cast<uint32_t>(__ffs(dh)) - 1u) >> 3) : 8u);
+}
+
+// Per lane: first index in [0, lim) where bytes c+i and q+i differ, else lim
+// (0 for lanes without act).  All lanes call it.  Three matches in four end in
+// the first 8 bytes, which each lane compares alone, as it does the next 32;
+// the lanes still open then are finished one by one by the whole warp, 128
+// bytes per iteration, so that a long match does not hold 31 lanes for long.
+__device__ __forceinline__ uint32_t extend_lanes(const Win &w, uint32_t c, uint32_t q, uint32_t lim, bool act) {
+    const uint32_t lane = lane_id();
+    uint32_t k = 0;
+    bool open = act && lim > 0u;
+    if (open) {
+        const uint32_t e = equal8(w, c, q);
+        k = e < lim ? e : lim;
+        open = e == 8u && lim > 8u;
+    }
+#pragma unroll 1
+    for (uint32_t r = 0; r < 2u; ++r) {
+        if (!__any_sync(kFull, open)) return k;
+        if (open) {
+            uint32_t e = equal8(w, c + k, q + k);
+            if (e == 8u) e += equal8(w, c + k + 8u, q + k + 8u);
+            open = e == 16u && lim > k + 16u;
+            k = k + e < lim ? k + e : lim;
+        }
+    }
+    for (uint32_t pend; (pend = __ballot_sync(kFull, open)) != 0u;) {
+        const uint32_t hl = static_cast<uint32_t>(__ffs(pend)) - 1u;
+        const uint32_t hk = __shfl_sync(kFull, k, hl);
+        const uint32_t hc = __shfl_sync(kFull, c, hl) + hk, hq = __shfl_sync(kFull, q, hl) + hk;
+        const uint32_t end = hq + extend_warp(w, hc, hq, __shfl_sync(kFull, lim, hl) - hk);
+        // lanes inside the same match at the same distance end there too
+        if (open && q - c == hq - hc && q + k >= hq && q + k <= end) {
+            k = end - q;
+            open = false;
+        }
+    }
+    return k;
+}
+
+// The match a parse without repeat offsets takes at its first hash-match
+// position f (lanes with act): extended, with the lazy step (:278-307).
+__device__ __forceinline__ void lane_match(const Win &w, const uint32_t *bm, const uint16_t *cand, uint32_t size,
+                                           bool lazy, bool act, uint32_t f, Match &m) {
+    const uint32_t fc = act ? f : 0u;
+    const uint32_t c0 = zmap(cand[fc]), c1 = zmap(cand[fc + 1u]);
+    // skipped when it is the same match one byte on, which is never longer (warp_step)
+    const bool ltry = act && lazy && fc + 4u < size && bm_bit(bm, fc + 1u) && c1 != c0 + 1u;
+    m.start = fc;
+    m.len = kMinMatch + extend_lanes(w, c0 + kMinMatch, fc + kMinMatch, act ? size - fc - kMinMatch : 0u, act);
+    m.off = fc - c0;
+    if (__any_sync(kFull, ltry)) {
+        const uint32_t l2 = kMinMatch + extend_lanes(w, c1 + kMinMatch, fc + 1u + kMinMatch,
+                                                     ltry ? size - fc - 1u - kMinMatch : 0u, ltry);
+        if (ltry && l2 > m.len + 1u) {
+            m.start = fc + 1u;
+            m.len = l2;
+            m.off = fc + 1u - c1;
+        }
+    }
+}
+
+// List entry of a match found at hash position f: {start | (ml-3) << 16,
+// offset | lazy << 16}, lazy: the match starts at f + 1.
+__device__ __forceinline__ uint2 lane_entry(const Match &m, uint32_t f) {
+    return make_uint2(m.start | ((m.len - kMinMatch) << 16), m.off | ((m.start - f) << 16));
+}
+__device__ __forceinline__ uint32_t entry_end(uint2 e) { return (e.x & 0xFFFFu) + (e.x >> 16) + kMinMatch; }
+
+// Repeat offsets before entry i of the list of a whole window.
+__device__ __forceinline__ void reps_before(const uint2 *list, uint32_t i, uint32_t &a, uint32_t &b, uint32_t &c) {
+    a = i >= 1u ? list[i - 1u].y & 0xFFFFu : 1u;
+    b = i >= 2u ? list[i - 2u].y & 0xFFFFu : (i == 1u ? 1u : 4u);
+    c = i >= 3u ? list[i - 3u].y & 0xFFFFu : (i == 2u ? 1u : (i == 1u ? 4u : 8u));
+}
+
+// Step 1: every lane parses segments of its warp's pool without repeat offsets.
+__device__ __forceinline__ void lane_parse(LaneSmem &N, const Win &win, const uint32_t *bm, const uint16_t *cand,
+                                           uint2 *seg, uint32_t size, uint32_t nact, bool lazy) {
+    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5, lt = lanemask_lt();
+    uint32_t next = warp * kLPool;
+    const uint32_t end = next + kLPool < nact ? next + kLPool : nact;
+    bool has = false;
+    uint32_t s = 0, p = 0, n = 0;
+    for (;;) {
+        const uint32_t need = __ballot_sync(kFull, !has);
+        if (need && next < end) {
+            const uint32_t mine = next + static_cast<uint32_t>(__popc(need & lt));
+            if (!has && mine < end) {
+                has = true;
+                s = mine;
+                p = s * kLSegW;
+                n = 0;
             }
-#pragma unroll
-            for (uint32_t u = 0; u < kVC; ++u) {
-                const uint32_t ch = c0 + u;
-                const uint32_t q = ch * 128u + 4u * lane;
-                uint32_t nib = 0;
-                if (q < size) {
-                    const uint32_t x0 = win.w32(q), x1 = win.w32(q + 4u);
-#pragma unroll
-                    for (uint32_t k = 0; k < 4; ++k) {
-                        const uint32_t cw = k < 2u ? cv[u].x : cv[u].y;
-                        const uint32_t c = zmap((k & 1u) ? cw >> 16 : cw & 0xFFFFu);
-                        const uint32_t xk = k ? __funnelshift_r(x0, x1, 8u * k) : x0;
-                        const uint32_t qk = q + k;
-                        const bool hm = qk + 3u < size && qk > 0u && ((xk ^ win.u32(static_cast<int>(c))) & 0xFFFFFFu) == 0u;
-                        nib |= static_cast<uint32_t>(hm) << k;
-                    }
-                }
-                uint32_t v = nib << (4u * (lane & 7u));
-                v |= __shfl_xor_sync(kFull, v, 1);
-                v |= __shfl_xor_sync(kFull, v, 2);
-                v |= __shfl_xor_sync(kFull, v, 4);
-                if ((lane & 7u) == 0u && ch < kChunks) S.bm[ch * 4u + (lane >> 3)] = v;
+            next += static_cast<uint32_t>(__popc(need));
+        }
+        if (!__any_sync(kFull, has)) break;
+        const uint32_t seg_end = (s + 1u) * kLSegW;
+        const uint32_t f = has ? next_bit(bm, p, seg_end) : seg_end;
+        const bool ev = has && f < seg_end;
+        if (__any_sync(kFull, ev)) {
+            Match m;
+            lane_match(win, bm, cand, size, lazy, ev, f, m);
+            if (ev) {
+                seg[s * kLCap + n] = lane_entry(m, f);
+                ++n;
+                p = m.start + m.len;
             }
         }
+        if (has && (!ev || p >= seg_end)) {  // no match left, or the last one ends past the segment
+            N.count[s] = static_cast<uint8_t>(n);
+            N.link[s] = static_cast<uint16_t>(ev ? p - seg_end : 0u);
+            has = false;
+        }
+    }
+}
+
+// Step 2, first half: where each segment's parse joins a later segment's list.
+__device__ __forceinline__ void lane_link(LaneSmem &N, ParseScalars &S, const Win &win, const uint32_t *bm,
+                                          const uint16_t *cand, uint2 *seg, uint32_t size, uint32_t nact,
+                                          uint32_t lim_pos, bool lazy) {
+    const uint32_t tid = threadIdx.x;
+#pragma unroll 1
+    for (uint32_t s = tid; s < kLSegs; s += kLThreads) {
+        uint32_t E = (s + 1u) * kLSegW + (s < nact ? N.link[s] : 0u);  // position the parse has reached
+        uint32_t t = kNoWarp, j = 0, cn = 0, big = 0;
+        bool run = s < nact;
+        for (;;) {
+            if (run && E >= lim_pos) run = false;  // the parse is over: no link
+            if (run) {
+                t = E / kLSegW;
+                j = 0;
+                uint32_t pe = t * kLSegW;  // end of the list's match before E
+                if (E != pe) {
+                    const uint32_t tc = N.count[t];
+                    for (; j < tc; ++j) {
+                        const uint2 e = seg[t * kLCap + j];
+                        if ((e.x & 0xFFFFu) - (e.y >> 16) >= E) break;  // found at or after E
+                        pe = entry_end(e);
+                    }
+                }
+                if (pe <= E) run = false;  // both go on from E without a match in between
+                else t = kNoWarp;
+            }
+            if (!__any_sync(kFull, run)) break;
+            const uint32_t f = run ? next_bit(bm, E, lim_pos) : lim_pos;
+            const bool ev = run && f < lim_pos;
+            if (run && !ev) run = false;
+            Match m;
+            lane_match(win, bm, cand, size, lazy, ev, f, m);
+            if (ev && cn == kLCont) {  // goes on in a long list
+                big = atomicAdd(&S.bigs, 1u);
+                if (big < kLBig) N.big[big] = static_cast<uint16_t>(s);
+            }
+            if (ev && (cn == kLCont + kLBigCap || (cn >= kLCont && big >= kLBig))) {
+                atomicOr(&S.flags, 4u);
+                run = false;
+            } else if (ev) {
+                seg[cn < kLCont ? kLContBase + s * kLCont + cn : kLBigBase + big * kLBigCap + (cn - kLCont)] =
+                    lane_entry(m, f);
+                ++cn;
+                E = m.start + m.len;
+            }
+        }
+        N.link[s] = static_cast<uint16_t>(t);
+        N.from[s] = static_cast<uint8_t>(j);
+        N.cont[s] = static_cast<uint8_t>(cn);
+        if (s >= nact) N.count[s] = 0;
+    }
+}
+
+// Step 2, second half (whole CTA): the segments on the chain from segment 0,
+// the entry each is joined at and its output offset; the chain's entries.
+// Marking doubles: when the marked segments are those fewer than 2^r links
+// from segment 0 and `link` leads 2^r links on, the marked ones mark theirs.
+__device__ __forceinline__ uint32_t lane_chain(LaneSmem &N, ParseScalars &S, bool any) {
+    constexpr uint32_t kPer = kLSegs / kLThreads;  // consecutive segments per thread
+    static_assert(kPer * kLThreads == kLSegs && 32u % kPer == 0u, "whole segments per thread");
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, s0 = tid * kPer;
+    uint32_t n[kPer], l[kPer], j[kPer];
+    bool on[kPer];
+#pragma unroll
+    for (uint32_t u = 0; u < kPer; ++u) {
+        n[u] = l[u] = N.link[s0 + u];
+        j[u] = N.from[s0 + u];
+        on[u] = any && s0 + u == 0u;
+    }
+    if (tid < kLSegs / 32u) N.chain[tid] = any && tid == 0 ? 1u : 0u;
+    __syncthreads();
+    for (;;) {
+        bool go = false;
+#pragma unroll
+        for (uint32_t u = 0; u < kPer; ++u) {
+            if (n[u] == kNoWarp) continue;
+            if (on[u]) atomicOr(&N.chain[n[u] >> 5], 1u << (n[u] & 31u));
+            n[u] = N.link[n[u]];
+            go = go || n[u] != kNoWarp;
+        }
+        go = __syncthreads_or(go);
+#pragma unroll
+        for (uint32_t u = 0; u < kPer; ++u) on[u] = (N.chain[s0 >> 5] >> ((s0 & 31u) + u)) & 1u;
+        if (!go) break;
+#pragma unroll
+        for (uint32_t u = 0; u < kPer; ++u) N.link[s0 + u] = static_cast<uint16_t>(n[u]);
+        __syncthreads();
+    }
+#pragma unroll
+    for (uint32_t u = 0; u < kPer; ++u)
+        if (on[u] && l[u] != kNoWarp) N.from[l[u]] = static_cast<uint8_t>(j[u]);
+    if (tid == 0) N.from[0] = 0;
+    __syncthreads();
+    uint32_t sum = 0;
+#pragma unroll
+    for (uint32_t u = 0; u < kPer; ++u) {
+        l[u] = sum;
+        if (on[u]) sum += N.count[s0 + u] - N.from[s0 + u] + N.cont[s0 + u];
+    }
+    uint32_t x = sum;
+#pragma unroll
+    for (uint32_t d = 1; d < 32u; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, x, d);
+        if (lane >= d) x += y;
+    }
+    if (lane == 31u) S.warp_sum[warp] = x;
+    __syncthreads();
+    uint32_t base = 0, total = 0;
+    for (uint32_t w = 0; w < kLWarps; ++w) {
+        const uint32_t v = S.warp_sum[w];
+        if (w < warp) base += v;
+        total += v;
+    }
+#pragma unroll
+    for (uint32_t u = 0; u < kPer; ++u) N.link[s0 + u] = static_cast<uint16_t>(base + x - sum + l[u]);
+    return total;
+}
+
+// Step 3: runs of literals in which a repeat offset matches on 3 bytes
+// (zstd_compress.cu:259-275), into N.fix.run (unsorted, repeats possible);
+// S.count counts them.  Run i lies before entry i of the list, the last one
+// after it.
+__device__ __forceinline__ void lane_check(LaneSmem &N, ParseScalars &S, const Win &win, const uint2 *list,
+                                           uint32_t total, uint32_t lim_pos) {
+    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+    for (uint32_t g = warp * 32u; g <= total; g += kLThreads) {
+        const uint32_t i = g + lane;
+        uint32_t lo = 0, hi = 0, r1 = 1, r2 = 4, r3 = 8;
+        if (i <= total) {
+            if (i) lo = entry_end(list[i - 1u]);
+            hi = lim_pos;
+            if (i < total) {  // up to the hash match (the byte before a lazy match's start)
+                const uint2 e = list[i];
+                hi = (e.x & 0xFFFFu) - (e.y >> 16);
+            }
+            reps_before(list, i, r1, r2, r3);
+        }
+        const uint32_t nt = hi > lo ? (hi - lo + 15u) >> 4 : 0u;  // tasks of 16 positions
+        uint32_t x = nt;
+#pragma unroll
+        for (uint32_t d = 1; d < 32u; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFull, x, d);
+            if (lane >= d) x += y;
+        }
+        const uint32_t T = __shfl_sync(kFull, x, 31), before = x - nt;
+        const uint32_t span = lo | (hi << 16), r12 = r1 | (r2 << 16);  // hi <= 65533
+        for (uint32_t b = 0; b < T; b += 32u) {
+            const uint32_t t = b + lane;
+            uint32_t o = 0;  // the run of task t: the first lane whose inclusive count is above t
+#pragma unroll
+            for (uint32_t d = 16; d >= 1u; d >>= 1)
+                if (__shfl_sync(kFull, x, o + d - 1u) <= t) o += d;
+            o &= 31u;  // t >= T: any
+            const uint32_t k = t - __shfl_sync(kFull, before, o);
+            const uint32_t sp = __shfl_sync(kFull, span, o), ra = __shfl_sync(kFull, r12, o),
+                           rc = __shfl_sync(kFull, r3, o);
+            bool hit = false;
+            if (t < T) {
+                const uint32_t q0 = (sp & 0xFFFFu) + 16u * k, left = (sp >> 16) - q0;
+                const uint32_t upto = left < 16u ? (1u << left) - 1u : 0xFFFFu;
+                uint32_t any = 0;
+#pragma unroll
+                for (uint32_t v = 0; v < 3u; ++v) {
+                    const uint32_t r = v == 0u ? ra & 0xFFFFu : (v == 1u ? ra >> 16 : rc);
+                    // sources before the window start do not count
+                    const uint32_t skip = r > q0 ? (r - q0 < 16u ? r - q0 : 16u) : 0u;
+                    any |= rep3_scan16(win, q0, skip < 16u ? r : 0u) & (0xFFFFu << skip) & (skip < 16u ? ~0u : 0u);
+                }
+                hit = (any & upto) != 0u;
+            }
+            if (__any_sync(kFull, hit)) {
+                const uint32_t po = __shfl_up_sync(kFull, o, 1);
+                const bool ph = __shfl_up_sync(kFull, hit ? 1u : 0u, 1) != 0u;
+                if (hit && !(lane > 0u && ph && po == o)) {
+                    const uint32_t at = atomicAdd(&S.count, 1u);
+                    if (at < kFixes) N.fix.run[at] = static_cast<uint16_t>(g + o);
+                }
+            }
+        }
+    }
+}
+
+// Step 4, first part (warp 0): the n recorded runs sorted, each once; returns
+// how many.
+__device__ __forceinline__ uint32_t sort_runs(LaneSmem &N, uint32_t n) {
+    const uint32_t lane = lane_id(), lt = lanemask_lt();
+    uint32_t m = 0;  // distinct runs, moved to the front (never past the ones still to be looked at)
+    for (uint32_t i0 = 0; i0 < n; i0 += 32u) {
+        const uint32_t i = i0 + lane, v = i < n ? N.fix.run[i] : 0u;
+        bool first = i < n;
+        for (uint32_t k = 0; k < m && first; ++k) first = N.fix.run[k] != v;
+        for (uint32_t k = i0; k < i && first; ++k) first = N.fix.run[k] != v;
+        __syncwarp();
+        const uint32_t f = __ballot_sync(kFull, first);
+        if (first) N.fix.run[m + static_cast<uint32_t>(__popc(f & lt))] = static_cast<uint16_t>(v);
+        m += static_cast<uint32_t>(__popc(f));
+        __syncwarp();
+    }
+    for (uint32_t i = lane; i < m; i += 32u) {  // each to its rank, through N.fix.meet
+        const uint32_t v = N.fix.run[i];
+        uint32_t rank = 0;
+        for (uint32_t k = 0; k < m; ++k) rank += N.fix.run[k] < v ? 1u : 0u;
+        N.fix.meet[rank] = static_cast<uint16_t>(v);
+    }
+    __syncwarp();
+    for (uint32_t i = lane; i < m; i += 32u) N.fix.run[i] = N.fix.meet[i];
+    return m;
+}
+
+// Step 4, second part: mend r (one warp) parses run i exactly from its start
+// until it emits entry `meet` of the list with the same repeat offsets.
+__device__ __noinline__ void mend_run(LaneSmem &N, ParseScalars &S, Win win, const uint32_t *bm, const uint16_t *cand,
+                                      uint2 *seg, uint32_t size, bool lazy, uint32_t total, uint32_t r,
+                                      uint32_t cap) {
+    const uint32_t lane = lane_id();
+    const uint32_t i = N.fix.run[r];
+    const uint2 *list = seg;
+    uint2 *out = seg + kLContBase + r * cap;
+    PState st;
+    st.p = i ? entry_end(list[i - 1u]) : 0u;
+    reps_before(list, i, st.r0, st.r1, st.r2);
+    CandBuf cb{cand, size, 0u, 0u, 0u, 0u};
+    cb.init(st.p);
+    uint32_t j = i, n = 0, meet = total;
+    while (st.p + 3u < size) {
+        Match m;
+        if (!warp_step(win, bm, cb, size, lazy, st, m)) continue;
+        for (;;) {  // first entry with start >= m.start
+            const uint32_t idx = j + lane;
+            const uint32_t b = __ballot_sync(kFull, idx >= total || (list[idx].x & 0xFFFFu) >= m.start);
+            if (b) {
+                j += static_cast<uint32_t>(__ffs(b)) - 1u;
+                break;
+            }
+            j += 32u;
+        }
+        if (j < total && list[j].x == pack_entry(m).x) {
+            uint32_t e0, e1, e2;
+            reps_before(list, j + 1u, e0, e1, e2);
+            if (e0 == st.r0 && e1 == st.r1 && e2 == st.r2) {
+                meet = j;
+                break;
+            }
+        }
+        if (n == cap) {
+            if (lane == 0) atomicOr(&S.flags, 4u);
+            break;
+        }
+        if (lane == 0) out[n] = pack_entry(m);
+        ++n;
+    }
+    if (lane == 0) {
+        N.fix.meet[r] = static_cast<uint16_t>(meet);
+        N.fix.len[r] = static_cast<uint8_t>(n);
+    }
+}
+
+template <bool kRef>
+__device__ __noinline__ void parse_segments_out(Zstd2Args a, SegSmem<kLWarps> &G, ParseScalars &S, Win win,
+                                                const uint32_t *bm, const uint16_t *cand, uint2 *seg, uint32_t wi,
+                                                uint32_t size, bool lazy) {
+    parse_segments<kRef, kMaxWindow / kLWarps>(a, G, S, win, bm, cand, seg, wi, size, lazy);
+}
+
+template <bool kRef>
+__global__ void __launch_bounds__(kLThreads, 3) zstd_lane_parse_kernel(Zstd2Args a) {
+    extern __shared__ __align__(128) uint8_t smem_raw[];
+    SmemLayout<LaneSmem> &M = *reinterpret_cast<SmemLayout<LaneSmem> *>(smem_raw);
+    ParseScalars &S = M.s;
+    LaneSmem &N = M.p;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    uint32_t parity = 0;
+    if (tid == 0) {
+        mbar_init(&S.bar, 1);
+        fence_mbar_init();
+    }
+    for (uint32_t i = tid; i < kPre / 4; i += kLThreads) reinterpret_cast<uint32_t *>(M.data)[i] = 0u;
+    const Win win{M.data + kPre};
+    const bool lazy = a.lazy != 0;
+    for (uint32_t wi = blockIdx.x; wi < a.num_windows; wi += gridDim.x) {
+        uint64_t start;
+        uint32_t size;
+        window_of(a, wi, start, size);
+        const uint16_t *cand = a.cand + start;
+        uint2 *seg = a.seg + static_cast<uint64_t>(wi) * a.seg_stride;
+        __syncthreads();  // previous window fully consumed
+        if (tid == 0) {
+            S.flags = 0;
+            S.covered = 0;
+            S.count = 0;
+            S.bigs = 0;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            if (!stage_window(M.data + kPre, a.src + start, size, &S.bar, parity, a.status) && lane == 0)
+                S.flags = 2u;
+        }
+        __syncthreads();
+        if (S.flags & 2u) return;  // bulk copy never completed: status already recorded, all threads leave
+        verify_window<kLWarps>(win, M.bm, cand, size);
         __syncthreads();
 
         const uint32_t lim_pos = size > 3u ? size - 3u : 0u;  // positions q < lim_pos can start a match
-        if constexpr (GL == 32) {
-            // ---- 2a. speculative parse of each segment (one warp each)
-            const uint32_t seg_start = warp * kSegW, seg_end = seg_start + kSegW;
-            const bool active = seg_start < lim_pos;
-            const bool last_active = !(seg_end < lim_pos);
-            ListWriter lw(seg + warp * kLaneCap);
-            PState s{seg_start, 1u, 4u, 8u};
-            CandBuf cb{cand, size, 0u, 0u, 0u, 0u};
-            if (active) cb.init(seg_start);
-            if (active) {
-                const uint32_t stop = last_active ? size : seg_end;
-                Match m;
-                while (s.p < stop && s.p + 3u < size) {
-                    if (warp_step(win, S.bm, cb, size, lazy, s, m)) lw.put(pack_entry(m));
-                }
-                lw.flush();
-            }
-            if (lane == 0) {
-                S.spec_count[warp] = lw.n;
-                S.cont_count[warp] = 0;
-                S.sync_warp[warp] = kNoWarp;
-                S.sync_idx[warp] = 0;
-            }
-            __syncthreads();
-
-            // ---- 2b. continue each warp's parse until it meets a later warp's list
-            if (active && !last_active) {
-                ListWriter cw(seg + warp * kLaneCap + kSpecCap);
-                uint32_t t = kNoWarp, j = 0;
-                Match m;
-                while (s.p + 3u < size) {
-                    if (!warp_step(win, S.bm, cb, size, lazy, s, m)) continue;
-                    const uint32_t tw = m.start / kSegW;  // warp whose segment holds this match start
-                    if (tw != t) {
-                        t = tw;
-                        j = 0;
-                    }
-                    const uint32_t tcount = S.spec_count[t];
-                    const uint2 *tl = seg + t * kLaneCap;
-                    // first entry of t's list with start >= m.start (lists are sorted by start)
-                    for (;;) {
-                        const uint32_t idx = j + lane;
-                        const bool ge = idx >= tcount || (tl[idx].x & 0xFFFFu) >= m.start;
-                        const uint32_t b = __ballot_sync(kFull, ge);
-                        if (b) {
-                            j += static_cast<uint32_t>(__ffs(b)) - 1u;
-                            break;
-                        }
-                        j += 32u;
-                    }
-                    bool met = false;
-                    if (j < tcount) {
-                        const uint2 e = tl[j];
-                        if (e.x == pack_entry(m).x && e.y == m.off) {
-                            uint32_t e0, e1, e2;
-                            reps_after(tl, j, e0, e1, e2);
-                            met = e0 == s.r0 && e1 == s.r1 && e2 == s.r2;
-                        }
-                    }
-                    if (met) {
-                        if (lane == 0) {
-                            S.sync_warp[warp] = t;
-                            S.sync_idx[warp] = j;
-                        }
-                        break;
-                    }
-                    if (cw.n == kContCap) {
-                        if (lane == 0) atomicOr(&S.flags, 1u);  // give up: exact fallback below
-                        break;
-                    }
-                    cw.put(pack_entry(m));
-                }
-                cw.flush();
-                if (lane == 0) S.cont_count[warp] = cw.n;
-            }
-            __syncthreads();
-        } else {
-            // ---- 2a. speculative parse of each segment (one 8-lane group each)
-            const uint32_t sg = tid / GL, gl = lane & (GL - 1u), gb = lane & ~(GL - 1u);
-            const uint32_t seg_start = sg * kSegW, seg_end = seg_start + kSegW;
-            const bool active = seg_start < lim_pos;
-            const bool last_active = !(seg_end < lim_pos);
-            const uint32_t stop = last_active ? size : seg_end;
-            uint2 *lst = seg + sg * kLaneCap;
-            PState s{seg_start, 1u, 4u, 8u};
-            uint32_t n = 0;
-            for (;;) {
-                const bool run = active && s.p < stop && s.p + 3u < size;
-                if (!__any_sync(kFull, run)) break;
-                Match m;
-                if (group_step<GL>(win, S.bm, cand, size, lazy, run, s, m)) {
-                    if (gl == 0) lst[n] = pack_entry(m);
-                    ++n;
-                }
-            }
-            if (gl == 0) {
-                S.spec_count[sg] = n;
-                S.cont_count[sg] = 0;
-                S.sync_warp[sg] = kNoWarp;
-                S.sync_idx[sg] = 0;
-            }
-            __syncthreads();
-
-            // ---- 2b. continue each group's parse until it meets a later segment's list
-            bool crun = active && !last_active;
-            uint32_t t = kNoWarp, j = 0, cn = 0;
-            uint2 *cl = lst + kSpecCap;
-            for (;;) {
-                const bool run = crun && s.p + 3u < size;
-                const uint32_t runners = __ballot_sync(kFull, run && gl == 0u);
-                if (!runners) break;
-                if ((runners & (runners - 1u)) == 0u) {
-                    // Only one group of the warp still runs (the slow tail of the
-                    // phase): the whole warp takes over its parse with warp-wide
-                    // steps (up to 128 positions scanned, 128 bytes extended per
-                    // iteration), same meeting test, then the loop ends.
-                    const uint32_t L = static_cast<uint32_t>(__ffs(runners)) - 1u;
-                    PState ws{__shfl_sync(kFull, s.p, L), __shfl_sync(kFull, s.r0, L), __shfl_sync(kFull, s.r1, L),
-                              __shfl_sync(kFull, s.r2, L)};
-                    const uint32_t wsg = __shfl_sync(kFull, sg, L);
-                    uint32_t wt = __shfl_sync(kFull, t, L), wj = __shfl_sync(kFull, j, L),
-                             wcn = __shfl_sync(kFull, cn, L);
-                    uint2 *wcl = seg + wsg * kLaneCap + kSpecCap;
-                    CandBuf wcb{cand, size, 0u, 0u, 0u, 0u};
-                    wcb.init(ws.p);
-                    while (ws.p + 3u < size) {
-                        Match m;
-                        if (!warp_step(win, S.bm, wcb, size, lazy, ws, m)) continue;
-                        const uint32_t tw = m.start / kSegW;  // segment that holds this match start
-                        if (tw != wt) {
-                            wt = tw;
-                            wj = 0;
-                        }
-                        const uint32_t tcount = S.spec_count[wt];
-                        const uint2 *tl = seg + wt * kLaneCap;
-                        // first entry of wt's list with start >= m.start, 32 per step
-                        for (;;) {
-                            const uint32_t idx = wj + lane;
-                            const bool ge = idx >= tcount || (tl[idx].x & 0xFFFFu) >= m.start;
-                            const uint32_t b = __ballot_sync(kFull, ge);
-                            if (b) {
-                                wj += static_cast<uint32_t>(__ffs(b)) - 1u;
-                                break;
-                            }
-                            wj += 32u;
-                        }
-                        bool met = false;
-                        if (wj < tcount) {
-                            const uint2 e = tl[wj];
-                            if (e.x == pack_entry(m).x && e.y == m.off) {
-                                uint32_t e0, e1, e2;
-                                reps_after(tl, wj, e0, e1, e2);
-                                met = e0 == ws.r0 && e1 == ws.r1 && e2 == ws.r2;
-                            }
-                        }
-                        if (met) {
-                            if (lane == 0) {
-                                S.sync_warp[wsg] = wt;
-                                S.sync_idx[wsg] = wj;
-                            }
-                            break;
-                        }
-                        if (wcn == kContCap) {
-                            if (lane == 0) atomicOr(&S.flags, 1u);  // give up: exact fallback below
-                            break;
-                        }
-                        if (lane == 0) wcl[wcn] = pack_entry(m);
-                        ++wcn;
-                    }
-                    if (lane >= L && lane < L + GL) {
-                        cn = wcn;
-                        crun = false;
-                    }
-                    break;
-                }
-                Match m;
-                const bool ev = group_step<GL>(win, S.bm, cand, size, lazy, run, s, m);
-                uint32_t tcount = 0;
-                const uint2 *tl = seg;
-                if (ev) {
-                    const uint32_t tw = m.start / kSegW;  // segment that holds this match start
-                    if (tw != t) {
-                        t = tw;
-                        j = 0;
-                    }
-                    tcount = S.spec_count[t];
-                    tl = seg + t * kLaneCap;
-                }
-                // first entry of t's list with start >= m.start (lists are sorted by start), 8 per step
-                bool found = !ev;
-                while (__any_sync(kFull, !found)) {
-                    const uint32_t idx = j + gl;
-                    const bool ge = !found && (idx >= tcount || (tl[idx].x & 0xFFFFu) >= m.start);
-                    const uint32_t b = (__ballot_sync(kFull, ge) >> gb) & ((1u << GL) - 1u);
-                    if (!found) {
-                        if (b) {
-                            j += static_cast<uint32_t>(__ffs(b)) - 1u;
-                            found = true;
-                        } else {
-                            j += GL;
-                        }
-                    }
-                }
-                if (!ev) {
-                    if (!run) crun = false;
-                    continue;
-                }
-                bool met = false;
-                if (j < tcount) {
-                    const uint2 e = tl[j];
-                    if (e.x == pack_entry(m).x && e.y == m.off) {
-                        uint32_t e0, e1, e2;
-                        reps_after(tl, j, e0, e1, e2);
-                        met = e0 == s.r0 && e1 == s.r1 && e2 == s.r2;
-                    }
-                }
-                if (met) {
-                    if (gl == 0) {
-                        S.sync_warp[sg] = t;
-                        S.sync_idx[sg] = j;
-                    }
-                    crun = false;
-                } else if (cn == kContCap) {
-                    if (gl == 0) atomicOr(&S.flags, 1u);  // give up: exact fallback below
-                    crun = false;
+        const uint32_t nact = (lim_pos + kLSegW - 1u) / kLSegW;
+        lane_parse(N, win, M.bm, cand, seg, size, nact, lazy);
+        __syncthreads();
+        lane_link(N, S, win, M.bm, cand, seg, size, nact, lim_pos, lazy);
+        __syncthreads();
+        uint32_t total = lane_chain(N, S, lim_pos > 0u);
+        __syncthreads();
+        const bool capped = total > a.max_seqs;
+        if (capped) total = a.max_seqs;
+        // The chain's entries in order into the output slots, then from there
+        // to the front of the scratch, over the lists.
+        uint2 *pk = kRef ? nullptr : a.packed + static_cast<uint64_t>(wi) * a.max_seqs;
+        uint32_t *rk = kRef ? a.ref_seqs + static_cast<uint64_t>(wi) * a.max_seqs * 3u : nullptr;
+        for (uint32_t s = tid >> 2; s < kLSegs; s += kLThreads / 4u) {
+            if (!((N.chain[s >> 5] >> (s & 31u)) & 1u)) continue;
+            const uint32_t from = N.from[s], ns = N.count[s], nc = N.cont[s];
+            uint32_t big = 0;
+            if (nc > kLCont)
+                while (N.big[big] != s) ++big;  // a segment with more than kLCont entries has a long list
+            for (uint32_t i = from + (tid & 3u); i < ns + nc; i += 4u) {
+                const uint32_t o = N.link[s] + (i - from);
+                if (o >= total) break;
+                const uint2 e = seg[i < ns            ? s * kLCap + i
+                                    : i < ns + kLCont ? kLContBase + s * kLCont + (i - ns)
+                                                      : kLBigBase + big * kLBigCap + (i - ns - kLCont)];
+                if constexpr (kRef) {
+                    rk[3u * o] = e.x;
+                    rk[3u * o + 1u] = e.y;
                 } else {
-                    if (gl == 0) cl[cn] = pack_entry(m);
-                    ++cn;
+                    pk[o] = e;
                 }
             }
-            if (gl == 0) S.cont_count[sg] = cn;
-            __syncthreads();
         }
-
-        if (!(S.flags & 1u)) {
-            // ---- 3. chain walk, then copy in chain order.  Nearly always every
-            // continuation meets the next segment's list, so the chain is
-            // segments 0..K in order (K: the first segment with no link): warp
-            // 0 then sets it up at once -- output offsets by a scan of the
-            // segments' contributions, each segment's preceding entry by a max
-            // scan (entry indices grow with the segment).  Otherwise one
-            // thread walks the links.
-            bool chained = false;
-            if (warp == 0 && lim_pos > 0) {
-                constexpr uint32_t kPer = (kSegs + 31u) / 32u;  // segments per lane, contiguous
-                uint32_t kf = kSegs;
-                bool gap = false;
-#pragma unroll
-                for (uint32_t u = 0; u < kPer; ++u) {
-                    const uint32_t i = lane * kPer + u;
-                    if (i < kSegs && S.sync_warp[i] == kNoWarp && i < kf) kf = i;
+        __syncthreads();
+        for (uint32_t i = tid; i < total; i += kLThreads) {
+            if constexpr (kRef) seg[i] = make_uint2(rk[3u * i], rk[3u * i + 1u]);
+            else seg[i] = pk[i];
+        }
+        __syncthreads();
+        lane_check(N, S, win, seg, total, capped ? 0u : lim_pos);
+        __syncthreads();
+        uint32_t nfix = S.count, fcap = 0;
+        if (nfix > 0u) {
+            if (capped || nfix > kFixes) {  // (uniform over the CTA)
+                if (tid == 0) S.flags = 4u;
+            } else {
+                if (warp == 0) {
+                    nfix = sort_runs(N, nfix);
+                    if (lane == 0) S.mends = nfix;
                 }
-                const uint32_t K = __reduce_min_sync(kFull, kf);  // segment 0 always parses, so K < kSegs
-#pragma unroll
-                for (uint32_t u = 0; u < kPer; ++u) {
-                    const uint32_t i = lane * kPer + u;
-                    if (i < K && S.sync_warp[i] != i + 1u) gap = true;
+                __syncthreads();
+                nfix = S.mends;
+                fcap = kFixEntries / nfix < kFixCap ? kFixEntries / nfix : kFixCap;
+                for (uint32_t r = warp; r < nfix; r += kLWarps)
+                    mend_run(N, S, win, M.bm, cand, seg, size, lazy, total, r, fcap);
+                __syncthreads();
+                if (tid == 0) {  // drop the mends that start inside an earlier one
+                    uint32_t kept = 0;
+                    int32_t shift = 0;
+                    for (uint32_t r = 0; r < nfix; ++r) {
+                        const uint32_t i = N.fix.run[r], j = N.fix.meet[r], n = N.fix.len[r];
+                        if (kept && i <= N.fix.meet[kept - 1u]) continue;
+                        shift += static_cast<int32_t>(n) - static_cast<int32_t>(j - i);
+                        N.fix.run[kept] = static_cast<uint16_t>(i);
+                        N.fix.meet[kept] = static_cast<uint16_t>(j);
+                        N.fix.shift[kept] = static_cast<int16_t>(shift);
+                        N.fix.len[kept] = static_cast<uint8_t>(n);
+                        N.fix.list[kept] = static_cast<uint8_t>(r);
+                        ++kept;
+                    }
+                    S.mends = kept;
+                    S.total = static_cast<uint32_t>(static_cast<int32_t>(total) + shift);
                 }
-                chained = !__any_sync(kFull, gap);
-                if (chained) {
-                    uint32_t con[kPer], lst1[kPer], sum = 0, lmax = 0;
-#pragma unroll
-                    for (uint32_t u = 0; u < kPer; ++u) {
-                        const uint32_t i = lane * kPer + u;
-                        con[u] = 0;
-                        lst1[u] = 0;
-                        if (i <= K) {
-                            const uint32_t from = i ? static_cast<uint32_t>(S.sync_idx[i - 1u]) : 0u;
-                            const uint32_t ns = S.spec_count[i], nc = S.cont_count[i];
-                            con[u] = ns - from + nc;
-                            if (con[u]) lst1[u] = 1u + i * kLaneCap + (nc ? kSpecCap + nc - 1u : ns - 1u);
-                        }
-                        sum += con[u];
-                        lmax = lst1[u] > lmax ? lst1[u] : lmax;
-                    }
-                    // exclusive scans over the lanes: sum of contributions, max of last entries (+1)
-                    uint32_t incl = sum, mx = lmax;
-#pragma unroll
-                    for (uint32_t d = 1; d < 32u; d <<= 1) {
-                        const uint32_t o = __shfl_up_sync(kFull, incl, d), om = __shfl_up_sync(kFull, mx, d);
-                        if (lane >= d) {
-                            incl += o;
-                            mx = om > mx ? om : mx;
-                        }
-                    }
-                    uint32_t acc = incl - sum, last1 = __shfl_up_sync(kFull, mx, 1);
-                    if (lane == 0) last1 = 0;
-#pragma unroll
-                    for (uint32_t u = 0; u < kPer; ++u) {
-                        const uint32_t i = lane * kPer + u;
-                        if (i >= kSegs) continue;
-                        const bool on = i <= K;
-                        S.on_chain[i] = on ? 1u : 0u;
-                        if (on) {
-                            S.chain_from[i] = i ? S.sync_idx[i - 1u] : 0u;
-                            S.out_off[i] = acc;
-                            S.prev_last[i] = last1 ? last1 - 1u : kNoEntry;
-                        }
-                        acc += con[u];
-                        last1 = lst1[u] > last1 ? lst1[u] : last1;
-                    }
-                    if (lane == 31u) S.total = incl;
-                }
-            }
-            chained = __syncthreads_or(chained);
-            if (tid == 0 && !chained) {
-                for (uint32_t i = 0; i < kSegs; ++i) S.on_chain[i] = 0;
-                uint32_t cur = 0, from = 0, acc = 0, last = kNoEntry;
-                if (lim_pos > 0) {
-                    for (;;) {
-                        S.on_chain[cur] = 1;
-                        S.chain_from[cur] = from;
-                        S.out_off[cur] = acc;
-                        S.prev_last[cur] = last;
-                        const uint32_t ns = S.spec_count[cur], nc = S.cont_count[cur];
-                        acc += (ns - from) + nc;
-                        if (ns + nc > from) last = cur * kLaneCap + (nc ? kSpecCap + nc - 1u : ns - 1u);
-                        const uint32_t nx = S.sync_warp[cur];
-                        if (nx == kNoWarp) break;
-                        from = S.sync_idx[cur];
-                        cur = nx;
-                    }
-                }
-                S.total = acc;
             }
             __syncthreads();
-            const uint32_t total = S.total;
-            const uint32_t keep = total < a.max_seqs ? total : a.max_seqs;
-            // Write {ll, ml-3, off} in chain order: an entry's literal length is
-            // its start minus the end of the entry before it -- the previous
-            // entry of the same list, or for a segment's first copied entry the
-            // last entry contributed before it, which the chain walk located.
-            const uint32_t csg = tid / GL, csl = tid % GL;  // segment whose list this thread copies
-            if (S.on_chain[csg]) {
-                const uint32_t from = S.chain_from[csg], ns = S.spec_count[csg], nc = S.cont_count[csg];
-                const uint32_t base = S.out_off[csg];
-                const uint2 *mine = seg + csg * kLaneCap;
-                uint32_t cov = 0;
-                for (uint32_t i = from + csl; i < ns + nc; i += GL) {
-                    const uint32_t o = base + (i - from);
-                    if (o >= keep) break;
-                    const uint2 e = mine[i < ns ? i : kSpecCap + (i - ns)];
-                    const uint32_t pi =
-                        i > from ? csg * kLaneCap + (i - 1u < ns ? i - 1u : kSpecCap + (i - 1u - ns)) : S.prev_last[csg];
-                    uint32_t pe = 0;
-                    if (pi != kNoEntry) {
-                        const uint32_t px = seg[pi].x;
-                        pe = (px & 0xFFFFu) + (px >> 16) + kMinMatch;
-                    }
-                    const uint32_t st0 = e.x & 0xFFFFu, mlm3 = e.x >> 16;
-                    const uint32_t ll = st0 - pe;
-                    cov += mlm3 + kMinMatch;
-                    if constexpr (kRef) {
-                        uint32_t *r = a.ref_seqs + (static_cast<uint64_t>(wi) * a.max_seqs + o) * 3u;
-                        r[0] = ll;
-                        r[1] = mlm3;
-                        r[2] = e.y;
-                    } else {
-                        a.packed[static_cast<uint64_t>(wi) * a.max_seqs + o] = make_uint2(ll | (mlm3 << 16), e.y);
-                    }
-                }
-                if (cov) atomicAdd(&S.covered, cov);
-            }
+            nfix = S.mends;
+        }
+        if (S.flags & 4u) {
             __syncthreads();
-            if (tid == 0) {
-                a.seq_counts[wi] = keep;
-                if (a.lit_counts) a.lit_counts[wi] = size - S.covered;
-            }
-        } else if (warp == 0) {
-            // ---- exact warp-wide parse of the whole window
-            PState fs{0u, 1u, 4u, 8u};
-            CandBuf fcb{cand, size, 0u, 0u, 0u, 0u};
-            fcb.init(0u);
-            uint32_t idx = 0, cov = 0, prev_end = 0;
-            Match m;
-            while (fs.p + 3u < size) {
-                if (!warp_step(win, S.bm, fcb, size, lazy, fs, m)) continue;
-                if (idx < a.max_seqs && lane == 0) {
-                    const uint32_t ll = m.start - prev_end;
-                    if constexpr (kRef) {
-                        uint32_t *r = a.ref_seqs + (static_cast<uint64_t>(wi) * a.max_seqs + idx) * 3u;
-                        r[0] = ll;
-                        r[1] = m.len - kMinMatch;
-                        r[2] = m.off;
-                    } else {
-                        a.packed[static_cast<uint64_t>(wi) * a.max_seqs + idx] =
-                            make_uint2(ll | ((m.len - kMinMatch) << 16), m.off);
-                    }
+            if (tid == 0) S.flags = 0u;
+            __syncthreads();
+            parse_segments_out<kRef>(a, N.seg, S, win, M.bm, cand, seg, wi, size, lazy);
+            continue;
+        }
+        const uint32_t out_n = nfix ? S.total : total;
+        const uint32_t keep = out_n < a.max_seqs ? out_n : a.max_seqs;
+        uint32_t cov = 0;
+        for (uint32_t x = tid; x < total; x += kLThreads) {
+            uint32_t o = x, pi = x;  // output index; the entry before x is prev[pi - 1]
+            const uint2 *prev = seg;
+            bool skip = false;
+            uint32_t z = 0;  // mends that start at or before x
+            for (uint32_t d = kFixes; d >= 1u; d >>= 1)
+                if (z + d <= nfix && N.fix.run[z + d - 1u] <= x) z += d;
+            if (z) {
+                --z;
+                const uint32_t j = N.fix.meet[z];
+                skip = x < j;
+                o = x + static_cast<uint32_t>(static_cast<int32_t>(N.fix.shift[z]));
+                if (x == j && N.fix.len[z]) {
+                    prev = seg + kLContBase + N.fix.list[z] * fcap;
+                    pi = N.fix.len[z];
                 }
-                if (idx < a.max_seqs) cov += m.len;
-                ++idx;
-                prev_end = m.start + m.len;
             }
-            if (lane == 0) {
-                a.seq_counts[wi] = idx < a.max_seqs ? idx : a.max_seqs;
-                if (a.lit_counts) a.lit_counts[wi] = size - cov;
-                atomicAdd(a.status + 1, 1u);  // fallback counter (diagnostics)
+            if (skip || o >= keep) continue;
+            const uint2 e = seg[x];
+            const uint32_t pe = pi ? entry_end(prev[pi - 1u]) : 0u;
+            cov += (e.x >> 16) + kMinMatch;
+            write_seq<kRef>(a, wi, o, (e.x & 0xFFFFu) - pe, e.x >> 16, e.y & 0xFFFFu);
+        }
+        for (uint32_t z = warp; z < nfix; z += kLWarps) {
+            const uint32_t i = N.fix.run[z], n = N.fix.len[z];
+            const uint32_t base = i + (z ? static_cast<uint32_t>(static_cast<int32_t>(N.fix.shift[z - 1u])) : 0u);
+            const uint2 *fl = seg + kLContBase + N.fix.list[z] * fcap;
+            for (uint32_t k = lane; k < n && base + k < keep; k += 32u) {
+                const uint2 e = fl[k];
+                const uint32_t pe = k ? entry_end(fl[k - 1u]) : (i ? entry_end(seg[i - 1u]) : 0u);
+                cov += (e.x >> 16) + kMinMatch;
+                write_seq<kRef>(a, wi, base + k, (e.x & 0xFFFFu) - pe, e.x >> 16, e.y);
             }
+        }
+        if (kRef && cov) atomicAdd(&S.covered, cov);
+        if (tid == 0) a.seq_counts[wi] = keep;
+        if (a.lit_counts) {
+            __syncthreads();
+            if (tid == 0) a.lit_counts[wi] = size - S.covered;
         }
     }
 }
 
 }  // namespace
 
-// Seg entries per window: the largest of the layouts, so that a buffer sized
-// once serves every segment width.
-template <uint32_t SegW, uint32_t GL = 32>
-constexpr uint32_t seg_entries() { return SegCfg<SegW, GL>::kSegs * SegCfg<SegW, GL>::kLaneCap; }
+// Scratch entries per window: the largest of the layouts, so that a buffer
+// sized once serves every segment width.
+template <uint32_t SegW>
+constexpr uint32_t seg_entries() { return SegCfg<SegW>::kSegs * SegCfg<SegW>::kLaneCap; }
 constexpr uint32_t kSegStride = []() constexpr {
-    uint32_t m = seg_entries<2048>();
+    uint32_t m = kLEntries;
+    if (seg_entries<2048>() > m) m = seg_entries<2048>();
     if (seg_entries<4096>() > m) m = seg_entries<4096>();
     if (seg_entries<8192>() > m) m = seg_entries<8192>();
-    if (seg_entries<1024, 8>() > m) m = seg_entries<1024, 8>();
-    if (seg_entries<512, 4>() > m) m = seg_entries<512, 4>();
     return m;
 }();
 
 size_t zstd2_seg_scratch_entries(uint32_t num_windows) { return static_cast<size_t>(num_windows) * kSegStride; }
 
 namespace {
-template <bool kRef, uint32_t SegW, uint32_t GL>
-cudaError_t launch_parse_variant(const Zstd2Args &a, int num_sms, int ctas_per_sm, cudaStream_t st) {
-    using C = SegCfg<SegW, GL>;
-    const uint32_t smem = sizeof(SmemLayout<C::kSegs>);
-    static_assert(sizeof(SmemLayout<C::kSegs>) + 1024 <= 233472 / 3, "three CTAs per SM must fit");
-    static SmemOnce smem_set{0};
-    cudaError_t e = set_smem_once(zstd_parse_kernel<kRef, SegW, GL>, smem, smem_set);
+template <class Kernel>
+cudaError_t launch_parse_kernel(Kernel kernel, uint32_t smem, uint32_t threads, SmemOnce &smem_set,
+                                const Zstd2Args &a, int num_sms, int ctas_per_sm, cudaStream_t st) {
+    cudaError_t e = set_smem_once(kernel, smem, smem_set);
     if (e != cudaSuccess) return e;
     int grid = num_sms * ctas_per_sm;
     if (static_cast<uint32_t>(grid) > a.num_windows) grid = static_cast<int>(a.num_windows);
-    zstd_parse_kernel<kRef, SegW, GL><<<grid, C::kThreads, smem, st>>>(a);
+    kernel<<<grid, threads, smem, st>>>(a);
     return cudaGetLastError();
+}
+
+template <bool kRef, uint32_t SegW>
+cudaError_t launch_seg_parse(const Zstd2Args &a, int num_sms, int ctas_per_sm, cudaStream_t st) {
+    using C = SegCfg<SegW>;
+    constexpr uint32_t smem = sizeof(SmemLayout<SegSmem<C::kSegs>>);
+    static_assert(smem + 1024 <= 233472 / 3, "three CTAs per SM must fit");
+    static SmemOnce smem_set{0};
+    return launch_parse_kernel(zstd_seg_parse_kernel<kRef, SegW>, smem, C::kThreads, smem_set, a, num_sms, ctas_per_sm,
+                               st);
 }
 
 template <bool kRef>
 cudaError_t launch_parse_ref(const Zstd2Args &a, uint32_t seg_width, int num_sms, int ctas_per_sm, cudaStream_t st) {
-    if (seg_width == 512) return launch_parse_variant<kRef, 512, 4>(a, num_sms, ctas_per_sm, st);
-    if (seg_width == 1024) return launch_parse_variant<kRef, 1024, 8>(a, num_sms, ctas_per_sm, st);
-    if (seg_width == 2048) return launch_parse_variant<kRef, 2048, 32>(a, num_sms, ctas_per_sm, st);
-    if (seg_width == 8192) return launch_parse_variant<kRef, 8192, 32>(a, num_sms, ctas_per_sm, st);
-    return launch_parse_variant<kRef, 4096, 32>(a, num_sms, ctas_per_sm, st);
+    if (seg_width == 2048) return launch_seg_parse<kRef, 2048>(a, num_sms, ctas_per_sm, st);
+    if (seg_width == 4096) return launch_seg_parse<kRef, 4096>(a, num_sms, ctas_per_sm, st);
+    if (seg_width == 8192) return launch_seg_parse<kRef, 8192>(a, num_sms, ctas_per_sm, st);
+    constexpr uint32_t smem = sizeof(SmemLayout<LaneSmem>);
+    static_assert(smem + 1024 <= 233472 / 3, "three CTAs per SM must fit");
+    static SmemOnce smem_set{0};
+    return launch_parse_kernel(zstd_lane_parse_kernel<kRef>, smem, kLThreads, smem_set, a, num_sms, ctas_per_sm, st);
 }
 }  // namespace
 

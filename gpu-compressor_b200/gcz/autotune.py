@@ -5,10 +5,8 @@ decide the sequences and matches); what may change is how the work is
 scheduled:
 
   Zstd   "sweep_warps"  warps that take turns on a window in the sweep (4-7)
-         "parse_seg"    speculative segment of the second stage: 2048, 4096 or
-                        8192 bytes per warp (32, 16 or 8 warps per window), or
-                        1024 bytes per 8-lane group (64 segments per window),
-                        or 512 bytes per 4-lane group (128 segments)
+         "parse_seg"    second stage: 1024 the lane parse, 2048, 4096 or 8192 one
+                        warp per segment of that many bytes
          "parse_ctas"   second-stage CTAs per SM
   LZMA2  "lzma_ctas"    second-stage CTAs per SM (the sweep is shared)
          "lzma_threads" second-stage threads per CTA (256, 512 or 1024)
@@ -37,7 +35,7 @@ TUNED_DIR = os.path.join(HERE, "tuned")
 ZSTD_CANDIDATES = [
     {"algo": 2, "sweep_warps": sw, "sweep_groups": 0, "parse_seg": seg, "parse_ctas": ctas}
     for sw in (7, 6, 5, 4)
-    for seg, ctas_list in ((4096, (3, 2)), (1024, (3, 2)), (512, (3, 2)), (8192, (3, 2)), (2048, (1,)))
+    for seg, ctas_list in ((4096, (3, 2)), (1024, (3, 2)), (8192, (3, 2)), (2048, (1,)))
     for ctas in ctas_list
 ]
 LZMA_CANDIDATES = [{"lzma_ctas": c, "lzma_threads": t} for t in (512, 256) for c in (3, 2, 1)] + [

@@ -76,8 +76,9 @@ const char *gcz_version(void);
  * single-warp kernels; "staged" (algo 1) = 1 stages each window into shared
  * memory with bulk copies, 0 reads it through L1; "parse_ctas" = Zstd
  * second-stage CTAs per SM (1-8); "parse_seg" = the Zstd second stage's
- * speculative segment: 1024 bytes per 8-lane group (default), 512 bytes per
- * 4-lane group, or 2048, 4096 or 8192 bytes per warp; "sweep_warps" = warps that take turns on
+ * parse: 1024 (default) or 512, one lane per 128-byte segment without repeat
+ * offsets, which are checked and mended afterwards; 2048, 4096 or 8192, one
+ * warp per segment of that many bytes with them; "sweep_warps" = warps that take turns on
  * a window in the candidate sweep (4-7, default 7); "sweep_groups" = 0 (default)
  * or 2: the sweep exchanges positions through its table and checks the order of
  * colliding lanes, 1 or 3: it groups the lanes of every step by hash first
