@@ -50,14 +50,14 @@ struct SmemWin {
     __device__ __forceinline__ uint32_t word(uint32_t i) const { return w[i]; }
     __device__ __forceinline__ uint32_t u32(uint32_t q) const {
         const uint32_t i = q >> 2;
-        return __funnelshift_r(w[i], w[i + 1], (q & 3u) * 8u);
+        return __funnelshift_r(w[i], w[i + 1], q << 3);  // the shift counts modulo 32
     }
     __device__ __forceinline__ uint32_t byte(uint32_t q) const {
         return reinterpret_cast<const uint8_t *>(w)[q];
     }
     // The 8 bytes at q: three aligned words, two funnel shifts.
     __device__ __forceinline__ void u64(uint32_t q, uint32_t &lo, uint32_t &hi) const {
-        const uint32_t i = q >> 2, sh = (q & 3u) * 8u;
+        const uint32_t i = q >> 2, sh = q << 3;
         const uint32_t w1 = w[i + 1];
         lo = __funnelshift_r(w[i], w1, sh);
         hi = __funnelshift_r(w1, w[i + 2], sh);

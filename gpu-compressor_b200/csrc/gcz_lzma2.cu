@@ -192,12 +192,29 @@ __global__ void __launch_bounds__(256) lzma_unpack_kernel(const uint32_t *packed
 // ---------------------------------------------------------------------------
 // Second stage after the candidate sweep (gcz_sweep.cu): the window is staged
 // into shared memory, cand(q) streams in from global memory, and every lane
-// verifies its own position.  Lengths use the structure of match runs: when
-// cand(q) == cand(q-1)+1 and both positions match on 4 bytes, the common run
-// at q is the one at q-1 shortened by one, so only the first lane of each run
-// (its head) extends, up to min(size-q, 273+31) bytes, and the other lanes of
-// the run derive min(273, E_head - (q - head)) from it -- the same value the
-// reference's per-position loop computes with its 273 cap.
+// verifies four consecutive positions, 128 per warp iteration.
+//
+// Lengths come from the ends of match runs.  Where q and q+1 both match on 4
+// bytes and cand(q+1) == cand(q) + 1, both matches end at the same byte, so
+// only a run's last position needs a comparison (about five of 128 positions
+// on the synthetic data, gathered and shared out to the lanes).  Each warp goes through its part of the window from
+// the back, so that a run's end is known when its earlier positions come up:
+// inside a lane, from the next lane that holds a run's end (one ballot, one
+// shuffle), or carried over from the block after it.  The cap of 273 bytes is
+// applied to the end of each run and again per position.
+//
+// Two cases need no comparison loop.  A candidate that fails on 4 bytes
+// matches on 2 at most: it has the same 14 upper bits of v * K (K odd), and
+// two values v that agree in their low 24 bits and differ above differ in the
+// upper 8 bits of the product.  A distance-1 run (lzma2_match_find.cu:164-181)
+// is looked for only where the candidate fails; four equal bytes after an
+// equal one would have made q-1 a candidate that matches, so it is 2 or 3 long
+// (with search_depth 0 there are no candidates, and it is measured).
+//
+// What bounds it: instruction issue.  One lane per position and one warp-wide
+// extension per run head took 378 K warp instructions per window, 6.55 ms per
+// GiB of the synthetic data; this form takes 199 K and 4.1 ms (the memory's own
+// time for cand, input and output would be 1.2 ms).
 constexpr uint32_t kL2Pre = 64;
 constexpr uint32_t kL2DataBytes = kL2Pre + kMaxWindow + 64;
 
@@ -205,7 +222,7 @@ struct L2Smem {
     uint8_t data[kL2DataBytes];
     uint32_t any;
     uint32_t flags;
-    alignas(8) uint64_t bar;
+    alignas(16) uint64_t bar;
 };
 
 struct L2Args {
@@ -224,17 +241,94 @@ struct L2Args {
     const WinDesc *wins;
 };
 
-// kL2Threads (256, 512 or 1024) is a schedule knob: the window's steps are
-// split into kL2Threads / 32 contiguous ranges, one per warp.  Three CTAs
-// share an SM (two of 1024 threads).  kRefOut: the reference layout's
-// per-position counts and match slots are written too (the parity entry
-// points); without it the step loop carries no code for them.
+// The candidates of positions q .. q+3 (none past the window).
+__device__ __forceinline__ uint2 load_cand4(const uint16_t *cand, uint32_t q, uint32_t size) {
+    if (q + 4u <= size) return *reinterpret_cast<const uint2 *>(cand + q);
+    uint32_t e[4];
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) e[k] = q + k < size ? static_cast<uint32_t>(cand[q + k]) : kNone;
+    return make_uint2(e[0] | (e[1] << 16), e[2] | (e[3] << 16));
+}
+
+// Lanes with `open` have k equal bytes at (c, q) and compare on, up to lim
+// (left: bytes to the window's end): one lane at a time, the whole warp 128
+// bytes per iteration.  Open lanes inside the same stretch of equal bytes at
+// the same distance share its end.
+__device__ __forceinline__ uint32_t finish_long(const SmemWin &win, uint32_t c, uint32_t q, uint32_t k, uint32_t lim,
+                                                uint32_t left, bool open) {
+    const uint32_t lane = lane_id();
+    for (uint32_t pend; (pend = __ballot_sync(kFull, open)) != 0u;) {
+        const uint32_t hl = static_cast<uint32_t>(__ffs(pend)) - 1u;
+        const uint32_t hc = __shfl_sync(kFull, c, hl), hq = __shfl_sync(kFull, q, hl);
+        const uint32_t hb = __shfl_sync(kFull, lim, hl);
+        const uint32_t h0 = __shfl_sync(kFull, k, hl);
+        uint32_t len = h0;
+        for (;;) {
+            const uint32_t i = len + 4u * lane;
+            uint32_t res = i;
+            if (i < hb) {
+                const uint32_t d = win.u32(hq + i) ^ win.u32(hc + i);
+                const uint32_t fb = d ? (static_cast<uint32_t>(__ffs(d)) - 1u) >> 3 : 4u;
+                res = i + (fb < hb - i ? fb : hb - i);
+            }
+            const uint32_t sb = __ballot_sync(kFull, res < i + 4u);
+            if (sb) {
+                len = __shfl_sync(kFull, res, static_cast<uint32_t>(__ffs(sb)) - 1u);
+                break;
+            }
+            len += 128u;
+        }
+        const uint32_t end = hq + len;  // a mismatch or the window's end, unless the cap of lane hl came first
+        const bool real = len < hb || hb == __shfl_sync(kFull, left, hl);
+        if (lane == hl) {
+            k = len;
+            open = false;
+        } else if (open && real && q - c == hq - hc && q + k >= hq + h0 && q + k <= end) {
+            k = end - q < lim ? end - q : lim;
+            open = false;
+        }
+    }
+    return k;
+}
+
+// Two rare cases of positions q .. q+3, whose packed results so far are `out`:
+// a candidate that fails on 4 bytes but matches on 2 comes before a run, and
+// with search_depth 0 a run is measured.  A call of its own, so that the step
+// loop holds no registers for it.
+__device__ __noinline__ uint4 short_matches(SmemWin win, uint2 cc, uint32_t q, uint32_t size, uint32_t depth,
+                                            uint4 out) {
+#pragma unroll 1
+    for (uint32_t k = 0; k < 4; ++k) {
+        const uint32_t p = q + k;
+        const uint32_t c = ((k & 2u ? cc.y : cc.x) >> (16u * (k & 1u))) & 0xFFFFu;
+        uint32_t o = k == 0u ? out.x : (k == 1u ? out.y : (k == 2u ? out.z : out.w));
+        if (c != kNone) {
+            const uint32_t d = win.u32(c) ^ win.u32(p);
+            if (d != 0u && (d & 0xFFFFu) == 0u) o = (2u << 16) | (p - c);
+        } else if (o && depth == 0) {
+            const uint32_t lim = size - p < kLzmaMaxMatch ? size - p : kLzmaMaxMatch;
+            o = (run_lane(win, p, win.byte(p), 2u, lim) << 16) | 1u;
+        }
+        if (k == 0u) out.x = o;
+        else if (k == 1u) out.y = o;
+        else if (k == 2u) out.z = o;
+        else out.w = o;
+    }
+    return out;
+}
+
+// kL2Threads (256, 512 or 1024) is a schedule knob: the window's 128-position
+// blocks are split into kL2Threads / 32 contiguous ranges, one per warp.
+// kRefOut: the reference layout's per-position counts and match slots are
+// written too (the parity entry points); without it the loop carries no code
+// for them.
 template <uint32_t kL2Threads, bool kRefOut>
 __global__ void __launch_bounds__(kL2Threads, kL2Threads == 1024 ? 2 : 3) lzma_verify_kernel(L2Args a) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     L2Smem &S = *reinterpret_cast<L2Smem *>(smem_raw);
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint32_t lt = lanemask_lt();
+    const uint32_t lt = lanemask_lt(), gt = lanemask_gt();
+    uint32_t *ends = reinterpret_cast<uint32_t *>(smem_raw + sizeof(L2Smem)) + warp * 128u;  // of one block's tails
     uint32_t parity = 0;
     if (tid == 0) {
         mbar_init(&S.bar, 1);
@@ -242,7 +336,8 @@ __global__ void __launch_bounds__(kL2Threads, kL2Threads == 1024 ? 2 : 3) lzma_v
     }
     for (uint32_t i = tid; i < kL2Pre / 4; i += kL2Threads) reinterpret_cast<uint32_t *>(S.data)[i] = 0u;
     __syncthreads();
-    SmemWin win{reinterpret_cast<const uint32_t *>(S.data + kL2Pre)};
+    const uint32_t *W = reinterpret_cast<const uint32_t *>(S.data + kL2Pre);
+    const SmemWin win{W};
     for (uint32_t wi = blockIdx.x; wi < a.num_windows; wi += gridDim.x) {
         const uint64_t start = a.wins ? a.wins[wi].offset : static_cast<uint64_t>(wi) * a.window;
         const uint32_t size =
@@ -261,119 +356,145 @@ __global__ void __launch_bounds__(kL2Threads, kL2Threads == 1024 ? 2 : 3) lzma_v
         if (S.flags) return;
         const uint16_t *cand = a.cand + start;
         uint32_t *packed = a.packed ? a.packed + start : nullptr;
+        const bool al16 = (reinterpret_cast<uintptr_t>(packed) & 15u) == 0u;
         uint32_t *rc = kRefOut && a.ref_counts ? a.ref_counts + start : nullptr;
         uint32_t *rm = kRefOut && a.ref_matches ? a.ref_matches + start * a.max_matches * 2u : nullptr;
         uint32_t any = 0;
-        const uint32_t nsteps = (size + 31u) >> 5;
-        // Each warp takes a contiguous range of steps, so a run of matches
-        // (cand(q) = cand(q-1) + 1) carries from one step's last lane into the
-        // next step's first: lane 0 then derives its length instead of
-        // extending again.  The carried length is exact when it is below 273
-        // (an extension is cut only at 273 + 31 bytes or at the window's end).
+        const uint32_t nblk = (size + 127u) >> 7;
         constexpr uint32_t kL2Warps = kL2Threads / 32;
-        const uint32_t per = (nsteps + kL2Warps - 1u) / kL2Warps;
-        const uint32_t s_begin = warp * per, s_end = min(nsteps, s_begin + per);
-        uint32_t carry_c = kNone, carry_e = 0;  // last lane of the previous step: candidate, length (0: none)
-        // The next step's candidates are loaded while this step is verified.
-        uint32_t c_next = (s_begin < s_end && s_begin * 32u + lane + 3u < size) ? cand[s_begin * 32u + lane] : kNone;
-        for (uint32_t st = s_begin; st < s_end; ++st) {
-            const uint32_t q = st * 32u + lane;
-            const bool inwin = q < size;
-            const bool valid4 = q + 3u < size;
-            const uint32_t x = win.u32(q);
-            const uint32_t c = valid4 ? c_next : kNone;
-            {
-                const uint32_t st2 = st + 1u, q2 = st2 * 32u + lane;
-                c_next = (st2 < s_end && q2 + 3u < size) ? static_cast<uint32_t>(cand[q2]) : kNone;
+        const uint32_t per = (nblk + kL2Warps - 1u) / kL2Warps;
+        const uint32_t b0 = warp * per < nblk ? warp * per : nblk, b1 = b0 + per < nblk ? b0 + per : nblk;
+        // Of the position after the block: candidate, 4-byte match (bit 16)
+        // and the end of its run.  Not known after a warp's last block.
+        constexpr uint32_t kUnknown = ~0u;
+        uint32_t after = kUnknown, after_end = 0;
+        uint2 cn = b1 > b0 ? load_cand4(cand, (b1 - 1u) * 128u + 4u * lane, size) : make_uint2(~0u, ~0u);
+        for (uint32_t blk = b1; blk-- > b0;) {
+            const uint32_t q = blk * 128u + 4u * lane, i = q >> 2;
+            // (search_depth 0: the chain loop never runs)
+            const uint2 cc = a.search_depth ? cn : make_uint2(~0u, ~0u);
+            const uint32_t c[4] = {cc.x & 0xFFFFu, cc.x >> 16, cc.y & 0xFFFFu, cc.y >> 16};
+            if (blk > b0) cn = load_cand4(cand, q - 128u, size);  // arrives while this block is worked on
+            const uint32_t x0 = W[i], x1 = W[i + 1u];
+            const uint32_t xm = W[static_cast<int>(i) - 1];
+            bool eq[4], rare = false;
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) {
+                // none: word 16383, inside the window's buffer (the shift counts modulo 32)
+                const uint32_t *y = reinterpret_cast<const uint32_t *>(S.data + kL2Pre + (c[k] & 0xFFFCu));
+                const uint32_t d = __funnelshift_r(y[0], y[1], c[k] << 3) ^ (k ? __funnelshift_r(x0, x1, 8u * k) : x0);
+                eq[k] = d == 0u && c[k] != kNone;
+                rare = rare || ((d & 0xFFFFu) == 0u && !eq[k]);  // fails on 4 bytes, may match on 2
             }
-            const bool has = valid4 && a.search_depth > 0 && c != kNone;
-            const uint32_t y = has ? win.u32(c) : ~x;
-            const bool eq4 = has && y == x;
-            // run structure inside the step
-            const uint32_t c_prev = __shfl_up_sync(kFull, c, 1);
-            const uint32_t eq4_bits = __ballot_sync(kFull, eq4);
-            const bool cont = lane > 0 && eq4 && ((eq4_bits >> (lane - 1)) & 1u) && c == c_prev + 1u;
-            const uint32_t heads = __ballot_sync(kFull, !cont);
-            const uint32_t head = 31u - static_cast<uint32_t>(__clz(heads & (lt | (1u << lane))));
-            // Run heads compare 8 more bytes (bytes 4-11) with one unaligned
-            // 8-byte read of each side, no loop; a head still matching after
-            // that is finished by the whole warp (128 bytes per iteration), so
-            // one long run does not leave 31 lanes idle.
-            uint32_t ext = 0;
-            const uint32_t bound = size - q < kLzmaMaxMatch + 31u ? size - q : kLzmaMaxMatch + 31u;
-            bool pending = false;
-            if (eq4 && !cont) {
-                if (lane == 0 && carry_e > 4u && carry_e < kLzmaMaxMatch && c == carry_c + 1u) {
-                    ext = carry_e - 1u;  // the previous step's last match, one byte on
+            // What follows each position: the next one's candidate and 4-byte
+            // match; the run goes on when that is this one's candidate plus 0x10001.
+            uint32_t v[5];
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) v[k] = eq[k] ? c[k] + 0x10000u : c[k];
+            v[4] = __shfl_down_sync(kFull, v[0], 1);
+            if (lane == 31u) v[4] = after;
+            uint32_t E[4];      // end of the run at a run's last position
+            bool tail[4];
+            uint32_t rank[4], ntail = 0;
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) {
+                tail[k] = eq[k] && v[k + 1u] - c[k] != 0x10001u;
+                const uint32_t m = __ballot_sync(kFull, tail[k]);
+                rank[k] = ntail + static_cast<uint32_t>(__popc(m & lt));
+                ntail += static_cast<uint32_t>(__popc(m));
+            }
+            if (ntail) {
+                // Five positions of the 128 on average: spread over the lanes through shared memory.
+#pragma unroll
+                for (uint32_t k = 0; k < 4; ++k)
+                    if (tail[k]) ends[rank[k]] = (q + k) | (c[k] << 16);
+                __syncwarp();
+                for (uint32_t t0 = 0; t0 < ntail; t0 += 32u) {
+                    const uint32_t t = t0 + lane;
+                    const uint32_t e = t < ntail ? ends[t] : 0u;
+                    const uint32_t tq = e & 0xFFFFu, tc = e >> 16;
+                    const uint32_t left = size - tq, lim = left < kLzmaMaxMatch ? left : kLzmaMaxMatch;
+                    uint32_t len = 4u;
+                    bool open = false;
+                    if (t < ntail) {
+                        uint32_t ql, qh, cl, ch;
+                        win.u64(tq + 4u, ql, qh);
+                        win.u64(tc + 4u, cl, ch);
+                        const uint32_t dl = ql ^ cl, dh = qh ^ ch;
+                        const uint32_t fb = dl ? (static_cast<uint32_t>(__ffs(dl)) - 1u) >> 3
+                                               : (dh ? 4u + ((static_cast<uint32_t>(__ffs(dh)) - 1u) >> 3) : 8u);
+                        len = 4u + fb < lim ? 4u + fb : lim;
+                        open = fb == 8u && lim > 12u;
+                    }
+                    if (__any_sync(kFull, open)) len = finish_long(win, tc, tq, len, lim, left, open);
+                    if (t < ntail) ends[t] = tq + len;
+                }
+                __syncwarp();
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) E[k] = tail[k] ? ends[rank[k]] : 0u;
+            if (ntail) __syncwarp();
+            // ends of the runs that go on past their lane
+            const bool has_tail = tail[0] || tail[1] || tail[2] || tail[3];
+            const uint32_t first = tail[0] ? E[0] : (tail[1] ? E[1] : (tail[2] ? E[2] : E[3]));
+            const uint32_t later = __ballot_sync(kFull, has_tail) & gt;
+            const uint32_t fl = __shfl_sync(kFull, first, later ? static_cast<uint32_t>(__ffs(later)) - 1u : 0u);
+            uint32_t run_end = later ? fl : after_end;
+            // distance-1 runs: byte t of D is zero where bytes q-1+t and q+t are equal;
+            // flags at bit 8k + 7 of two (f2) and three (f3) equal bytes from q + k
+            const uint32_t D0 = __funnelshift_r(xm, x0, 24) ^ x0, D1 = __funnelshift_r(x0, x1, 24) ^ x1;
+            const uint32_t z0 = ~(((D0 & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | D0 | 0x7F7F7F7Fu);
+            const uint32_t z1 = ~(((D1 & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | D1 | 0x7F7F7F7Fu);
+            uint32_t f2 = z0 & __funnelshift_r(z0, z1, 8), f3 = f2 & __funnelshift_r(z0, z1, 16);
+            if (blk == 0u && lane == 0u) f2 &= ~0x80u;  // position 0 has no byte before it
+            if (blk + 2u >= nblk) {                     // bytes past the window are not equal to anything
+                const uint32_t n2 = size - 1u > q ? size - 1u - q : 0u, n3 = n2 ? n2 - 1u : 0u;
+                f2 = n2 < 4u ? f2 & ((1u << (8u * n2)) - 1u) : f2;
+                f3 = n3 < 4u ? f3 & ((1u << (8u * n3)) - 1u) : f3;
+            }
+            uint32_t out[4];
+#pragma unroll
+            for (int k = 3; k >= 0; --k) {
+                const uint32_t p = q + static_cast<uint32_t>(k), bit = 0x80u << (8 * k);
+                if (tail[k]) run_end = E[k];
+                const uint32_t e = run_end - p;
+                const uint32_t run = (f2 & bit) ? ((f3 & bit) ? 0x30001u : 0x20001u) : 0u;
+                out[k] = eq[k] ? min(e, kLzmaMaxMatch) * 65536u + (p - c[k]) : run;
+            }
+            if (rare || a.search_depth == 0) {
+                const uint4 o = short_matches(win, cc, q, size, a.search_depth, make_uint4(out[0], out[1], out[2], out[3]));
+                out[0] = o.x;
+                out[1] = o.y;
+                out[2] = o.z;
+                out[3] = o.w;
+            }
+            any |= out[0] | out[1] | out[2] | out[3];
+            if constexpr (kRefOut) {
+#pragma unroll
+                for (uint32_t k = 0; k < 4; ++k) {
+                    const uint32_t p = q + k;
+                    if (p >= size) continue;
+                    if (rc) rc[p] = out[k] ? 1u : 0u;
+                    if (rm && out[k]) {
+                        uint32_t *slot = rm + static_cast<uint64_t>(p) * a.max_matches * 2u;
+                        slot[0] = out[k] & 0xFFFFu;
+                        slot[1] = out[k] >> 16;
+                    }
+                }
+            }
+            // of position q of lane 0, for the block before this one (a position
+            // past the window has no match, so out[] and any need no guard)
+            after = __shfl_sync(kFull, v[0], 0);
+            after_end = __shfl_sync(kFull, run_end, 0);
+            if (packed) {
+                if (al16 && q + 4u <= size) {
+                    *reinterpret_cast<uint4 *>(packed + q) = make_uint4(out[0], out[1], out[2], out[3]);
                 } else {
-                    const uint32_t lim1 = bound < 12u ? bound : 12u;  // bound >= 4 (q + 3 < size)
-                    uint32_t ql, qh, cl, ch;
-                    win.u64(q + 4u, ql, qh);
-                    win.u64(c + 4u, cl, ch);
-                    const uint32_t dl = ql ^ cl, dh = qh ^ ch;
-                    const uint32_t fb = dl ? (static_cast<uint32_t>(__ffs(dl)) - 1u) >> 3
-                                           : (dh ? 4u + ((static_cast<uint32_t>(__ffs(dh)) - 1u) >> 3) : 8u);
-                    ext = 4u + fb < lim1 ? 4u + fb : lim1;
-                    pending = ext == lim1 && lim1 < bound;
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; ++k)
+                        if (q + k < size) packed[q + k] = out[k];
                 }
             }
-            for (uint32_t pend = __ballot_sync(kFull, pending); pend; pend &= pend - 1u) {
-                const uint32_t hl = static_cast<uint32_t>(__ffs(pend)) - 1u;
-                const uint32_t hc = __shfl_sync(kFull, c, hl), hq = __shfl_sync(kFull, q, hl);
-                const uint32_t hb = __shfl_sync(kFull, bound, hl);
-                uint32_t len2 = __shfl_sync(kFull, ext, hl);
-                for (;;) {
-                    const uint32_t k = len2 + 4u * lane;
-                    uint32_t res = k;
-                    if (k < hb) {
-                        const uint32_t d = win.u32(hq + k) ^ win.u32(hc + k);
-                        const uint32_t fb = d ? (static_cast<uint32_t>(__ffs(d)) - 1u) >> 3 : 4u;
-                        res = k + (fb < hb - k ? fb : hb - k);
-                    }
-                    const uint32_t sb = __ballot_sync(kFull, res < k + 4u);
-                    if (sb) {
-                        len2 = __shfl_sync(kFull, res, static_cast<uint32_t>(__ffs(sb)) - 1u);
-                        break;
-                    }
-                    len2 += 128u;
-                }
-                if (lane == hl) ext = len2;
-            }
-            const uint32_t ext_head = __shfl_sync(kFull, ext, head);
-            {
-                const uint32_t e31 = eq4 ? ext_head - (lane - head) : 0u;
-                carry_e = __shfl_sync(kFull, e31, 31);
-                carry_c = __shfl_sync(kFull, c, 31);
-            }
-            uint32_t dist = 0, len = 0;
-            if (inwin && q + 1u < size) {
-                if (eq4) {
-                    const uint32_t e = ext_head - (lane - head);
-                    len = e < kLzmaMaxMatch ? e : kLzmaMaxMatch;
-                    dist = q - c;
-                } else if (has && ((y ^ x) & 0xFFFFu) == 0u) {
-                    len = ((y ^ x) & 0xFF0000u) == 0u ? 3u : 2u;  // :134-139 (byte 3 differs)
-                    dist = q - c;
-                }
-                if (len == 0 && q > 0) {  // distance-1 run (:164-181)
-                    const uint32_t b0 = x & 0xFFu, b1 = (x >> 8) & 0xFFu;
-                    if (b1 == b0 && win.byte(q - 1u) == b0) {
-                        const uint32_t lim = size - q < kLzmaMaxMatch ? size - q : kLzmaMaxMatch;
-                        len = run_lane(win, q, b0, 2u, lim);
-                        dist = 1;
-                    }
-                }
-            }
-            if (inwin) {
-                if (packed) packed[q] = len ? ((len << 16) | dist) : 0u;
-                if (kRefOut && rc) rc[q] = len ? 1u : 0u;
-                if (kRefOut && rm && len) {
-                    uint32_t *slot = rm + static_cast<uint64_t>(q) * a.max_matches * 2u;
-                    slot[0] = dist;
-                    slot[1] = len;
-                }
-            }
-            any |= len;
         }
         if (kRefOut && rc)
             for (uint32_t q = size + tid; q < a.window; q += kL2Threads) rc[q] = 0u;  // :188-190
@@ -427,7 +548,8 @@ cudaError_t launch_lzma_unpack(const uint32_t *packed, uint64_t n, uint32_t wind
 namespace {
 template <uint32_t kThreads, bool kRefOut>
 cudaError_t launch_verify_variant(const L2Args &a, const LzmaLaunch &l, cudaStream_t st) {
-    const uint32_t smem = sizeof(L2Smem);
+    const uint32_t smem = sizeof(L2Smem) + kThreads / 32 * 128 * sizeof(uint32_t);
+    static_assert((sizeof(L2Smem) + kThreads * 16 + 1024) * (kThreads == 1024 ? 2 : 3) <= 233472, "CTAs of one wave must fit");
     static SmemOnce smem_set{0};
     cudaError_t e = set_smem_once(lzma_verify_kernel<kThreads, kRefOut>, smem, smem_set);
     if (e != cudaSuccess) return e;
@@ -461,7 +583,12 @@ cudaError_t launch_lzma_verify(const LzmaLaunch &l, const uint16_t *cand, cudaSt
         if (l.threads == 512) return launch_verify_variant<512, true>(a, l, st);
         return launch_verify_variant<1024, true>(a, l, st);
     }
-    if (l.threads == 256) return launch_verify_variant<256, false>(a, l, st);
+    // 1024 threads finish a window soonest (1 window: 64 us against 90 for 256
+    // threads, 256 windows 115 against 124); once there are several windows per
+    // CTA, 256 threads with their 64 registers have the higher throughput
+    // (1036 windows 390 us against 407, 16384 windows 5.11 ms against 5.25).
+    const bool many = l.num_windows > 6u * static_cast<uint32_t>(l.num_sms);
+    if (l.threads == 256 || (l.threads != 512 && many)) return launch_verify_variant<256, false>(a, l, st);
     if (l.threads == 512) return launch_verify_variant<512, false>(a, l, st);
     return launch_verify_variant<1024, false>(a, l, st);
 }

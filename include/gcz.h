@@ -87,7 +87,7 @@ const char *gcz_version(void);
  * "lzma_ctas" = LZMA2 second-stage CTAs per SM (1-8, default 3; values above
  * what fits on an SM -- 3, or 2 with 1024 threads -- run as that many);
  * "lzma_threads" = LZMA2 second-stage threads per CTA (256, 512 or 1024,
- * default 1024);
+ * default 1024, which takes 256 where there are several windows per CTA);
  * "slice_windows" = windows per slice of the host-buffer
  * pipelines (default 512 = 32 MiB; four slots, three slices in flight;
  * slices ramp up from a quarter of it and back down at the end);
