@@ -22,7 +22,7 @@
 //   zenc_huf_plan_kernel   (one warp):   Huffman code and tree description
 //   zenc_huf_write_kernel  (one CTA):    RLE or Huffman-coded literal section
 //                                        where that is smaller
-//   zenc_sequences_kernel  (one warp):   repeat-code pass, FSE chains, bitstream,
+//   zenc_sequences_kernel  (one CTA):    repeat-code pass, FSE chains, bitstream,
 //                                        block header, frame size
 //   zenc_compact_kernel    (one CTA):    frames back to back at scanned offsets
 // Frames are built in per-window slots of kZencSlot bytes first, because a
@@ -47,93 +47,53 @@ __constant__ int8_t kOFNorm[29] = {1, 1, 1, 1, 1, 1, 2, 2, 2, 1, 1, 1, 1, 1, 1,
 constexpr uint32_t kLLLog = 6, kMLLog = 6, kOFLog = 5;
 constexpr uint32_t kLLSyms = 36, kMLSyms = 53, kOFSyms = 29;
 
-// Literal-length and match-length codes (RFC 8878 3.1.1.3.2.1.1): baseline and
-// number of extra bits per code.
-__constant__ uint32_t kLLBase[36] = {0,  1,  2,  3,  4,  5,   6,   7,   8,    9,    10,   11,
-                                     12, 13, 14, 15, 16, 18,  20,  22,  24,   28,   32,   40,
-                                     48, 64, 128, 256, 512, 1024, 2048, 4096, 8192, 16384, 32768, 65536};
-__constant__ uint8_t kLLBits[36] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 1, 1,
-                                    1, 1, 2, 2, 3, 3, 4, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16};
-__constant__ uint32_t kMLBase[53] = {3,  4,  5,  6,  7,  8,  9,  10, 11, 12, 13,  14,  15,   16,   17,   18,   19,   20,
-                                     21, 22, 23, 24, 25, 26, 27, 28, 29, 30, 31,  32,  33,   34,   35,   37,   39,   41,
-                                     43, 47, 51, 59, 67, 83, 99, 131, 259, 515, 1027, 2051, 4099, 8195, 16387, 32771, 65539};
-__constant__ uint8_t kMLBits[53] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0,  0,  0,  0,  0,  0,  0,  0,  0, 0, 0,
-                                    0, 0, 0, 0, 0, 1, 1, 1, 1, 2, 2, 3, 3, 4, 4, 5, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16};
-
 __device__ __forceinline__ uint32_t highbit(uint32_t x) { return 31u - static_cast<uint32_t>(__clz(x)); }
 
-// Largest code whose baseline is <= v (bases ascending).
-__device__ __forceinline__ uint32_t code_of(const uint32_t *base, uint32_t ncodes, uint32_t v) {
-    uint32_t lo = 0, hi = ncodes - 1;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        if (base[mid] <= v) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
-
-// Code tables copied to shared memory (lanes of a warp look up different
-// codes): baselines, extra bits, and codes of the small values; above those,
-// codes follow the highest set bit.
+// Codes and extra-bit counts of the small values in shared memory (lanes of a
+// warp look up different ones); above those, codes follow the highest set bit.
+// Every code's baseline (less 3 for match lengths) is a multiple of 2^(its
+// extra bits), so the extra bits are the value's low bits.
 struct CodeTables {
-    uint32_t ll_base[kLLSyms];
-    uint32_t ml_base[kMLSyms];
-    uint8_t ll_bits[kLLSyms];
-    uint8_t ml_bits[kMLSyms];
-    uint8_t ll_lut[64];   // code of literal length v < 64
-    uint8_t ml_lut[128];  // code of match length v + 3, v < 128
+    uint16_t ll_lut[64];   // literal length v < 64: code | extra bits << 8
+    uint16_t ml_lut[128];  // match length v + 3, v < 128
     __device__ void build() {
-        for (uint32_t i = threadIdx.x; i < kLLSyms; i += blockDim.x) {
-            ll_base[i] = kLLBase[i];
-            ll_bits[i] = kLLBits[i];
-        }
-        for (uint32_t i = threadIdx.x; i < kMLSyms; i += blockDim.x) {
-            ml_base[i] = kMLBase[i];
-            ml_bits[i] = kMLBits[i];
-        }
-        for (uint32_t v = threadIdx.x; v < 64u; v += blockDim.x) ll_lut[v] = static_cast<uint8_t>(code_of(kLLBase, kLLSyms, v));
-        for (uint32_t v = threadIdx.x; v < 128u; v += blockDim.x)
-            ml_lut[v] = static_cast<uint8_t>(code_of(kMLBase, kMLSyms, v + 3u));
-    }
-    // Literal lengths >= 64 take code 19 + highbit (64 -> 25, ..., 65536 -> 35).
-    __device__ __forceinline__ uint32_t ll_code(uint32_t ll) const { return ll < 64u ? ll_lut[ll] : highbit(ll) + 19u; }
-    // Match lengths >= 131 take code 36 + highbit(ml - 3) (131 -> 43, ..., 65539 -> 52).
-    __device__ __forceinline__ uint32_t ml_code(uint32_t ml) const {
-        const uint32_t v = ml - 3u;
-        return v < 128u ? ml_lut[v] : highbit(v) + 36u;
-    }
-};
-
-// Forward bit writer (the decoder reads the stream backwards from its end
-// marker).  Bytes go to global memory one at a time: frame positions have no
-// alignment.
-struct BitWriter {
-    uint8_t *out;
-    uint32_t pos;  // bytes written
-    uint64_t acc;
-    uint32_t nbits;
-    __device__ __forceinline__ void add(uint32_t v, uint32_t nb) {
-        acc |= static_cast<uint64_t>(v) << nbits;
-        nbits += nb;
-        if (nbits >= 32u) {
-            const uint32_t w = static_cast<uint32_t>(acc);
-            out[pos] = static_cast<uint8_t>(w);
-            out[pos + 1] = static_cast<uint8_t>(w >> 8);
-            out[pos + 2] = static_cast<uint8_t>(w >> 16);
-            out[pos + 3] = static_cast<uint8_t>(w >> 24);
-            pos += 4u;
-            acc >>= 32;
-            nbits -= 32u;
+        for (uint32_t v = threadIdx.x; v < 128u; v += blockDim.x) {
+            uint32_t c, b;
+            if (v < 64u) {
+                if (v < 16u) c = v, b = 0u;
+                else if (v < 24u) c = 16u + ((v - 16u) >> 1), b = 1u;
+                else if (v < 32u) c = 20u + ((v - 24u) >> 2), b = 2u;
+                else if (v < 48u) c = 22u + ((v - 32u) >> 3), b = 3u;
+                else c = 24u, b = 4u;
+                ll_lut[v] = static_cast<uint16_t>(c | (b << 8));
+            }
+            if (v < 32u) c = v, b = 0u;
+            else if (v < 40u) c = 32u + ((v - 32u) >> 1), b = 1u;
+            else if (v < 48u) c = 36u + ((v - 40u) >> 2), b = 2u;
+            else if (v < 64u) c = 38u + ((v - 48u) >> 3), b = 3u;
+            else if (v < 96u) c = 40u + ((v - 64u) >> 4), b = 4u;
+            else c = 42u, b = 5u;
+            ml_lut[v] = static_cast<uint16_t>(c | (b << 8));
         }
     }
-    __device__ __forceinline__ void close() {
-        add(1u, 1u);  // end marker
-        while (nbits > 0u) {
-            out[pos++] = static_cast<uint8_t>(acc);
-            acc >>= 8;
-            nbits = nbits > 8u ? nbits - 8u : 0u;
-        }
+    // Literal lengths >= 64 take code 19 + highbit (64 -> 25, ..., 65536 -> 35) with highbit extra bits.
+    __device__ __forceinline__ void ll(uint32_t v, uint32_t &code, uint32_t &bits) const {
+        const uint32_t e = v < 64u ? ll_lut[v] : 0u, hb = highbit(v | 1u);
+        code = v < 64u ? e & 0xFFu : hb + 19u;
+        bits = v < 64u ? e >> 8 : hb;
+    }
+    // Match lengths >= 131 take code 36 + highbit(ml - 3) (131 -> 43, ..., 65539 -> 52) likewise.
+    __device__ __forceinline__ void ml(uint32_t m, uint32_t &code, uint32_t &bits) const {
+        const uint32_t v = m - 3u, e = v < 128u ? ml_lut[v] : 0u, hb = highbit(v | 1u);
+        code = v < 128u ? e & 0xFFu : hb + 36u;
+        bits = v < 128u ? e >> 8 : hb;
+    }
+    // Extra bits by code.
+    __device__ __forceinline__ uint32_t ll_bits(uint32_t c) const {
+        return c >= 25u ? c - 19u : (c < 16u ? 0u : static_cast<uint32_t>(0x433221111ull >> (4u * (c - 16u))) & 0xFu);
+    }
+    __device__ __forceinline__ uint32_t ml_bits(uint32_t c) const {
+        return c >= 43u ? c - 36u : (c < 32u ? 0u : static_cast<uint32_t>(0x54433221111ull >> (4u * (c - 32u))) & 0xFu);
     }
 };
 
@@ -881,22 +841,30 @@ __global__ void __launch_bounds__(kLitThreads) zenc_huf_write_kernel(ZencArgs a)
 }
 
 // ---------------------------------------------------------------- sequences
-// One warp per window, kSeqWarps windows per CTA.  Sequences pass through
-// shared memory in chunks of kChunk; the only serial work -- the
-// repeat-offset history, the three tables and the three FSE state chains --
-// runs on single lanes over shared memory, the rest is spread over the warp:
-//   R. ascending chunks: lane 0 computes each Offset_Value from the decoder's
-//      repeat history; the values go to a per-window global scratch; the
-//      lanes count the LL, ML and OF codes.
-//   T. lanes 0-2 pick the table of LL, OF and ML (RFC 8878 3.1.1.3.2.1):
-//      RLE_Mode when one code is used, else FSE_Compressed_Mode or
-//      Predefined_Mode, whichever costs fewer bits by an integer estimate
-//      (below); then spread the table and list each code's states.
-//   E. descending chunks (the bitstream starts with the last sequence):
-//      codes in parallel; lanes 0-2 run the LL / ML / OF chains; a warp scan
-//      gives each sequence's bit position; every lane ORs its sequences'
-//      fields into the warp's bit buffer; whole 32-bit words are stored, the
-//      partial last word carries into the next chunk.
+// One CTA of kSeqThreads threads per window; each thread owns a run of
+// consecutive sequences.  The serial parts of the format are run by all
+// threads at once from guessed states, which are then checked against the
+// state the thread before left, and run again where they differ:
+//   R. ascending: each Offset_Value from the decoder's repeat history.  A
+//      thread guesses the history as the three offsets before its run; the
+//      values go to a per-window global scratch, the LL, ML and OF codes are
+//      counted.
+//   T. one warp each picks and builds the table of LL, ML and OF (RFC 8878
+//      3.1.1.3.2.1): RLE_Mode when one code is used, else FSE_Compressed_Mode
+//      or Predefined_Mode, whichever costs fewer bits by an integer estimate
+//      (below).
+//   E. in bitstream order (the last sequence first), kChunk sequences at a time:
+//      codes by all threads; one warp per FSE chain, each lane a run of
+//      kChunk / 32 symbols; then every thread's bit count, a scan, and every
+//      thread writes the bits of its sequences.  An encoder state says little
+//      about the states a few symbols on: a lane starts kWarmUp symbols before
+//      its run from any state and has mostly met the true chain at its start.
+//      Where it has not, its run is repeated from the state before it, round
+//      by round (about 30 % of the runs, some over several rounds: runs of one
+//      frequent code keep two chains apart).
+// What bounds it: latency of the dependent table reads.  With one warp per
+// window, the history and the three chains on single lanes, 17 windows took
+// 554 us and 4096 windows 978 us; this form takes 75 us and 341 us.
 // The cost estimate counts, per code c used k times, k * (A - log2(n_c))
 // bits, with log2 taken piecewise linear between powers of two in 1/256 bit
 // (lg256 below), plus the table description's bytes.  FSE_Compressed_Mode
@@ -910,43 +878,44 @@ __global__ void __launch_bounds__(kLitThreads) zenc_huf_write_kernel(ZencArgs a)
 // numbered x = n .. 2n-1; for the next decoder state D' the encoder takes the
 // state x = (D' + 2^A) >> b, with b the bit count that puts x in [n, 2n), and
 // writes the low b bits of D' + 2^A.
-constexpr uint32_t kChunk = 128;
-constexpr uint32_t kSeqWarps = 4;
-constexpr uint32_t kPerLane = kChunk / 32;
-constexpr uint32_t kBufWords = kChunk * 74u / 32u + 4u;  // <= 74 bits per sequence, plus the carried word
+constexpr uint32_t kSeqThreads = 128;
+constexpr uint32_t kChunk = 1024;                        // sequences per pass of step E
+constexpr uint32_t kRun = kChunk / 32;                   // symbols per lane of a chain
+constexpr uint32_t kWarmUp = 8;                          // symbols before a run that its chain starts at
+constexpr uint32_t kOwn = kChunk / kSeqThreads;          // sequences per thread of a chunk
 constexpr uint32_t kMaxAl = 9;                           // Accuracy_Log limit of LL and ML (OF: 8)
 constexpr uint32_t kTabDesc = 128;                       // bytes of one table description
 constexpr uint32_t kOFCodes = 32;                        // offset codes counted (a window's are <= 16)
 
 // One field's (LL, ML or OF) table for one window.
 struct FieldTab {
-    uint16_t stl[1u << kMaxAl];  // each code's decoder states, ascending, code after code
-    uint8_t sym[1u << kMaxAl];   // spread table (building only)
-    uint16_t cumul[64];          // first stl entry of code c
-    uint16_t norm[64];           // normalised count (>= 1 where used; "less than 1" counts as 1)
     uint32_t hist[64];           // uses of code c in the window
-    uint8_t desc[kTabDesc];      // FSE table description, or the RLE code
+    // Code c with n states: x = (D' + 2^A) >> nb, nb = (D' + 2^A + enc.x) >> 16
+    // (enc.x = (hi << 16) - (n << hi), hi = A - floor(log2(n))), next state
+    // stl[x + enc.y] (enc.y: the code's first entry - n).
+    uint2 enc[64];
+    uint32_t desc[kTabDesc / 4]; // FSE table description, or the RLE code
+    uint16_t stl[1u << kMaxAl];  // each code's decoder states, ascending, code after code
+    uint16_t cumul[64];          // states of the codes before c
+    uint16_t fill[64];           // next stl entry of code c (building only)
+    uint16_t norm[64];           // normalised counts (building only)
+    uint8_t sym[1u << kMaxAl];   // spread table (building only)
     uint32_t al;                 // accuracy log (0 for RLE_Mode)
     uint32_t mode;               // 0 Predefined_Mode, 1 RLE_Mode, 2 FSE_Compressed_Mode
     uint32_t desc_len;
 };
 
-struct WarpSeq {
-    uint4 q[kChunk];          // the chunk's records, in bitstream order (last sequence first)
-    uint32_t ov[kChunk];      // Offset_Value
-    uint8_t code[3][kChunk];  // LL, ML, OF codes
-    uint16_t upd[3][kChunk];  // state-update bits: value | nbBits << 12 (LL, ML, OF)
-    uint32_t pos[kChunk];     // bit position within the chunk
-    uint32_t buf[kBufWords];
-    uint32_t state[3];
-    FieldTab tab[3];          // LL, ML, OF
-};
-
 struct SeqSmem {
     CodeTables C;
-    WarpSeq W[kSeqWarps];
+    FieldTab tab[3];                    // LL, ML, OF
+    uint32_t out_state[3][kSeqThreads]; // repeat offsets that each thread's run leaves
+    uint32_t state[3];                  // chain states after the chunk
+    uint32_t warp_bits[kSeqThreads / 32];
+    // Of the chunk's sequences: codes, and update bits (value | count << 12),
+    // lane by lane with a gap that spreads the lanes over the banks.
+    alignas(4) uint8_t code[3][kChunk + 4 * 32];
+    alignas(4) uint16_t upd[3][kChunk + 2 * 32];
 };
-static_assert(sizeof(SeqSmem) * 4 + 4 * 1024 <= 233472, "four sequence CTAs per SM");
 
 // log2(x) * 256, piecewise linear between powers of two (x >= 1).
 __device__ __forceinline__ uint32_t lg256(uint32_t x) {
@@ -954,346 +923,480 @@ __device__ __forceinline__ uint32_t lg256(uint32_t x) {
     return 256u * h + ((x << 8) >> h) - 256u;
 }
 
-// Picks and builds field f's table from its code histogram (one lane).
-// pre: the predefined distribution (-1 = "less than 1"), pre_n codes.
+__device__ __forceinline__ void or_desc(uint32_t *d, uint32_t bitpos, uint64_t v, uint32_t nb) {
+    if (nb == 0u) return;
+    const uint32_t w = bitpos >> 5, sh = bitpos & 31u;
+    const uint64_t lo = v << sh;  // nb <= 48, so v << sh spans at most 80 bits: three words
+    atomicOr(d + w, static_cast<uint32_t>(lo));
+    if (sh + nb > 32u) atomicOr(d + w + 1, static_cast<uint32_t>(lo >> 32));
+    if (sh + nb > 64u) atomicOr(d + w + 2, static_cast<uint32_t>(v >> (64u - sh)));
+}
+
+__device__ __forceinline__ uint32_t scan_incl(uint32_t x) {
+    const uint32_t lane = lane_id();
+#pragma unroll
+    for (uint32_t d = 1; d < 32u; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, x, d);
+        if (lane >= d) x += y;
+    }
+    return x;
+}
+
+// Picks and builds a field's table from its code histogram (one warp; lane l
+// holds codes l and l + 32).  pre: the predefined distribution (-1 = "less
+// than 1"), pre_n codes.
 __device__ void build_field_table(FieldTab &T, uint32_t ns, uint32_t ncodes, uint32_t amax, const int8_t *pre,
                                   uint32_t pre_n, uint32_t pre_al) {
-    uint32_t used = 0, last = 0;
-    for (uint32_t c = 0; c < ncodes; ++c)
-        if (T.hist[c]) {
-            ++used;
-            last = c;
-        }
+    const uint32_t lane = lane_id(), lt = lanemask_lt();
+    uint32_t h[2], n[2];
+    int32_t pn[2];
+    bool no_pre = false;
+#pragma unroll
+    for (uint32_t u = 0; u < 2u; ++u) {
+        const uint32_t c = lane + 32u * u;
+        h[u] = c < ncodes ? T.hist[c] : 0u;
+        pn[u] = c < pre_n ? pre[c] : 0;
+        no_pre = no_pre || (h[u] && pn[u] == 0);  // a used code without a predefined state
+    }
+    const uint32_t m0 = __ballot_sync(kFull, h[0] != 0u), m1 = __ballot_sync(kFull, h[1] != 0u);
+    const uint32_t used = static_cast<uint32_t>(__popc(m0) + __popc(m1));
+    const uint32_t last = m1 ? 32u + highbit(m1) : highbit(m0);
+    if (lane < kTabDesc / 4u) T.desc[lane] = 0u;
+    __syncwarp();
     if (used == 1u) {  // RLE_Mode: one code, no state
-        T.mode = 1;
-        T.al = 0;
-        T.desc[0] = static_cast<uint8_t>(last);
-        T.desc_len = 1;
+        if (lane == 0) {
+            T.mode = 1;
+            T.al = 0;
+            T.desc[0] = last;
+            T.desc_len = 1;
+            T.enc[last] = make_uint2(0u - 1u, 0u - 1u);
+            T.stl[0] = 0;
+        }
         return;
     }
-    // Predefined cost (impossible when a used code has no predefined state).
-    uint64_t cost_pre = 0;
-    bool pre_ok = true;
-    for (uint32_t c = 0; c <= last; ++c) {
-        if (!T.hist[c]) continue;
-        if (c >= pre_n || pre[c] == 0) {
-            pre_ok = false;
-            break;
-        }
-        const uint32_t n = pre[c] < 0 ? 1u : static_cast<uint32_t>(pre[c]);
-        cost_pre += static_cast<uint64_t>(T.hist[c]) * (256u * pre_al - lg256(n));
-    }
-    // FSE_Compressed_Mode: accuracy, normalised counts, description.
+    const bool pre_ok = !__any_sync(kFull, no_pre);
+    // FSE_Compressed_Mode: accuracy, normalised counts.
     uint32_t al = 32u - static_cast<uint32_t>(__clz(ns - 1u));  // bit length of ns - 1
     al = al > 2u ? al - 2u : 0u;
     al = al < amax ? al : amax;
     al = al > 5u ? al : 5u;
     while ((1u << al) < 2u * used && al < amax) ++al;
     const uint32_t size = 1u << al;
-    int32_t sum = 0;
-    uint32_t top = 0;
-    for (uint32_t c = 0; c < 64u; ++c) {
-        uint32_t n = 0;
-        if (c <= last && T.hist[c]) {
-            n = (T.hist[c] * size + ns / 2u) / ns;
-            n = n > 1u ? n : 1u;
-            if (T.hist[c] > T.hist[top]) top = c;
-        }
-        T.norm[c] = static_cast<uint16_t>(n);
-        sum += static_cast<int32_t>(n);
+#pragma unroll
+    for (uint32_t u = 0; u < 2u; ++u) n[u] = h[u] ? max((h[u] * size + ns / 2u) / ns, 1u) : 0u;
+    int32_t d = static_cast<int32_t>(size) - static_cast<int32_t>(__reduce_add_sync(kFull, n[0] + n[1]));
+    // the lowest code among those with the largest key
+    auto top_of = [&](uint32_t k0, uint32_t k1) {
+        const uint32_t a = (k0 << 6) | (63u - lane), b = (k1 << 6) | (31u - lane);
+        return 63u - (__reduce_max_sync(kFull, a > b ? a : b) & 63u);
+    };
+    if (d > 0) {
+        const uint32_t top = top_of(h[0], h[1]);
+        if (top == lane) n[0] += static_cast<uint32_t>(d);
+        if (top == lane + 32u) n[1] += static_cast<uint32_t>(d);
     }
-    int32_t d = static_cast<int32_t>(size) - sum;
-    if (d > 0) T.norm[top] = static_cast<uint16_t>(T.norm[top] + d);
     for (; d < 0; ++d) {
-        uint32_t big = 0;
-        for (uint32_t c = 1; c <= last; ++c)
-            if (T.norm[c] > T.norm[big]) big = c;
-        T.norm[big] = static_cast<uint16_t>(T.norm[big] - 1u);
+        const uint32_t big = top_of(n[0], n[1]);
+        if (big == lane) --n[0];
+        if (big == lane + 32u) --n[1];
     }
-    SmemBits wr{T.desc, kTabDesc, 0u, 0u, 0ull, false};
-    {
-        wr.add(al - 5u, 4u);
-        int remaining = static_cast<int>(size) + 1, threshold = static_cast<int>(size);
-        uint32_t nb = al + 1u;
-        for (int c = 0; c <= static_cast<int>(last); ++c) {
-            const int n = T.norm[c];
-            const int v = n + 1, mx = (2 * threshold - 1) - remaining;
-            if (v < mx) wr.add(static_cast<uint32_t>(v), nb - 1u);
-            else if (v < threshold) wr.add(static_cast<uint32_t>(v), nb);
-            else wr.add(static_cast<uint32_t>(v + mx), nb);
-            remaining -= n;
-            while (remaining < threshold) {
-                --nb;
-                threshold >>= 1;
-            }
-            if (n == 0) {
-                int z = 0;
-                while (c + 1 + z < static_cast<int>(last) && T.norm[c + 1 + z] == 0) ++z;
-                c += z;
-                for (; z >= 3; z -= 3) wr.add(3u, 2u);
-                wr.add(static_cast<uint32_t>(z), 2u);
-            }
+    // Table description (RFC 8878 4.1.1).  The width of a count's field follows
+    // from the counts before it; of a run of zeros the first is a count, the
+    // others are two-bit repeat flags.
+    const uint32_t s0 = scan_incl(n[0]), sum0 = __shfl_sync(kFull, s0, 31), s1 = scan_incl(n[1]) + sum0;
+    const uint64_t zeros = ~((static_cast<uint64_t>(m1) << 32) | m0);  // codes with no uses
+    uint64_t fv[2];
+    uint32_t fb[2];
+#pragma unroll
+    for (uint32_t u = 0; u < 2u; ++u) {
+        const uint32_t c = lane + 32u * u;
+        fv[u] = 0;
+        fb[u] = 0;
+        const bool follows = c > 0u && ((zeros >> (c - 1u)) & 1u) != 0u && n[u] == 0u;  // inside a run of zeros
+        if (c > last || follows) continue;
+        const uint32_t before = (u ? s1 : s0) - n[u];
+        const uint32_t remaining = size + 1u - before;
+        // the threshold halves while it is above `remaining`, from 2^al on
+        const uint32_t tlog = min(highbit(remaining), al), threshold = 1u << tlog;
+        const uint32_t v = n[u] + 1u, mx = 2u * threshold - 1u - remaining;
+        if (v < mx) {
+            fv[u] = v;
+            fb[u] = tlog;
+        } else {
+            fv[u] = v < threshold ? v : v + mx;
+            fb[u] = tlog + 1u;
         }
-        wr.flush();
+        if (n[u] == 0u) {
+            const uint64_t rest = ~(zeros >> (c + 1u));  // c < last < 63
+            const uint32_t z = static_cast<uint32_t>(__ffsll(static_cast<long long>(rest))) - 1u;  // zeros after c
+            uint32_t b = fb[u];
+            for (uint32_t k = 0; k < z / 3u; ++k, b += 2u) fv[u] |= 3ull << b;
+            fv[u] |= static_cast<uint64_t>(z % 3u) << b;
+            fb[u] = b + 2u;
+        }
     }
-    uint64_t cost_fse = 2048ull * wr.pos;
-    for (uint32_t c = 0; c <= last; ++c)
-        if (T.hist[c]) cost_fse += static_cast<uint64_t>(T.hist[c]) * (256u * al - lg256(T.norm[c]));
-    const bool fse = !wr.ovf && (!pre_ok || cost_fse < cost_pre);
-    uint32_t high = 0;
+    const uint32_t b0 = scan_incl(fb[0]), bsum0 = __shfl_sync(kFull, b0, 31), b1 = scan_incl(fb[1]);
+    const uint32_t bits = 4u + bsum0 + __shfl_sync(kFull, b1, 31), bytes = (bits + 7u) >> 3;
+    uint32_t cp = 0, cf = 0;
+#pragma unroll
+    for (uint32_t u = 0; u < 2u; ++u) {
+        if (!h[u]) continue;
+        if (pre_ok) cp += h[u] * (256u * pre_al - lg256(pn[u] < 0 ? 1u : static_cast<uint32_t>(pn[u])));
+        cf += h[u] * (256u * al - lg256(n[u]));
+    }
+    // (sums of at most 21845 * 9 * 256)
+    const uint32_t cost_pre = __reduce_add_sync(kFull, cp), cost_fse = __reduce_add_sync(kFull, cf) + 2048u * bytes;
+    const bool fse = bytes <= kTabDesc && (!pre_ok || cost_fse < cost_pre);
+    uint32_t high, tal;
     if (fse) {
-        T.mode = 2;
-        T.al = al;
-        T.desc_len = wr.pos;
+        if (lane == 0) or_desc(T.desc, 0u, al - 5u, 4u);
+        or_desc(T.desc, 4u + b0 - fb[0], fv[0], fb[0]);
+        or_desc(T.desc, 4u + bsum0 + b1 - fb[1], fv[1], fb[1]);
+        tal = al;
         high = size - 1u;
-    } else {  // Predefined_Mode
-        T.mode = 0;
-        T.al = pre_al;
-        T.desc_len = 0;
-        high = (1u << pre_al) - 1u;
-        for (uint32_t c = 0; c < 64u; ++c) T.norm[c] = c < pre_n ? static_cast<uint16_t>(pre[c] < 0 ? 1 : pre[c]) : 0;
+    } else {  // Predefined_Mode; "less than 1" codes take the top states, one each
+        const uint32_t l0 = __ballot_sync(kFull, pn[0] < 0), l1 = __ballot_sync(kFull, pn[1] < 0);
+        tal = pre_al;
+        const uint32_t top = (1u << pre_al) - 1u;
+        high = top - static_cast<uint32_t>(__popc(l0) + __popc(l1));
+        if (pn[0] < 0) T.sym[top - static_cast<uint32_t>(__popc(l0 & lt))] = static_cast<uint8_t>(lane);
+        if (pn[1] < 0) T.sym[top - static_cast<uint32_t>(__popc(l0) + __popc(l1 & lt))] = static_cast<uint8_t>(lane + 32u);
+#pragma unroll
+        for (uint32_t u = 0; u < 2u; ++u) n[u] = pn[u] < 0 ? 1u : static_cast<uint32_t>(pn[u]);
     }
-    // Spread (RFC 8878 4.1.1): "less than 1" codes at the top, the others
-    // stepped through the remaining states.
-    const uint32_t tsize = 1u << T.al, mask = tsize - 1u, step = (tsize >> 1) + (tsize >> 3) + 3u;
-    const uint32_t ntab = fse ? last + 1u : pre_n;
-    for (uint32_t c = 0; c < ntab; ++c)
-        if (!fse && pre[c] < 0) T.sym[high--] = static_cast<uint8_t>(c);
-    uint32_t pos = 0;
-    for (uint32_t c = 0; c < ntab; ++c) {
-        const int n = fse ? static_cast<int>(T.norm[c]) : static_cast<int>(pre[c]);
-        for (int i = 0; i < n; ++i) {
+    const uint32_t tsize = 1u << tal, mask = tsize - 1u, step = (tsize >> 1) + (tsize >> 3) + 3u;
+    // states before each code: all of them (cumul), and those that are spread (fill, for the search below)
+    const bool sp0 = fse || pn[0] > 0, sp1 = fse || pn[1] > 0;
+    const uint32_t a0 = scan_incl(n[0]), asum = __shfl_sync(kFull, a0, 31), a1 = scan_incl(n[1]) + asum;
+    const uint32_t q0 = scan_incl(sp0 ? n[0] : 0u), qsum = __shfl_sync(kFull, q0, 31), q1 = scan_incl(sp1 ? n[1] : 0u) + qsum;
+    T.cumul[lane] = static_cast<uint16_t>(a0 - n[0]);
+    T.cumul[lane + 32u] = static_cast<uint16_t>(a1 - n[1]);
+    T.fill[lane] = static_cast<uint16_t>(q0 - (sp0 ? n[0] : 0u));
+    T.fill[lane + 32u] = static_cast<uint16_t>(q1 - (sp1 ? n[1] : 0u));
+#pragma unroll
+    for (uint32_t u = 0; u < 2u; ++u) {
+        const uint32_t c = lane + 32u * u, before = (u ? a1 : a0) - n[u];
+        const uint32_t hi = n[u] ? tal - highbit(n[u]) : 0u;
+        T.enc[c] = make_uint2((hi << 16) - (n[u] << hi), before - n[u]);
+    }
+    __syncwarp();
+    // Spread (RFC 8878 4.1.1): the codes' states in order, stepped through the
+    // table, past the positions above `high`.  The k-th state placed belongs to
+    // the last code with at most k spread states before it.
+    uint32_t placed = 0;
+    for (uint32_t i0 = 0; i0 < tsize; i0 += 32u) {
+        const uint32_t pos = ((i0 + lane) * step) & mask;
+        const uint32_t ok = __ballot_sync(kFull, pos <= high);
+        const uint32_t k = placed + static_cast<uint32_t>(__popc(ok & lt));
+        if (pos <= high) {
+            uint32_t c = 0;
+#pragma unroll
+            for (uint32_t dd = 32; dd >= 1u; dd >>= 1)
+                if (T.fill[c + dd] <= k) c += dd;  // c + dd <= 63
             T.sym[pos] = static_cast<uint8_t>(c);
-            do {
-                pos = (pos + step) & mask;
-            } while (pos > high);
+        }
+        placed += static_cast<uint32_t>(__popc(ok));
+    }
+    __syncwarp();
+    T.fill[lane] = T.cumul[lane];
+    T.fill[lane + 32u] = T.cumul[lane + 32u];
+    __syncwarp();
+    for (uint32_t u0 = 0; u0 < tsize; u0 += 32u) {
+        const uint32_t s = T.sym[u0 + lane], base = T.fill[s];
+        const uint32_t g = __match_any_sync(kFull, s);
+        T.stl[base + static_cast<uint32_t>(__popc(g & lt))] = static_cast<uint16_t>(u0 + lane);
+        __syncwarp();
+        if (!(g & ~lt & ~(1u << lane))) T.fill[s] = static_cast<uint16_t>(base + static_cast<uint32_t>(__popc(g)));
+        __syncwarp();
+    }
+    if (lane == 0) {
+        T.mode = fse ? 2u : 0u;
+        T.al = tal;
+        T.desc_len = fse ? bytes : 0u;
+    }
+}
+
+// Places of chunk sequence j in SeqSmem::code and ::upd.
+__device__ __forceinline__ uint32_t code_at(uint32_t j) { return j + 4u * (j / kRun); }
+__device__ __forceinline__ uint32_t upd_at(uint32_t j) { return j + 2u * (j / kRun); }
+
+// One FSE chain over a chunk of len symbols (one warp): update bits of every
+// symbol into up; D: the state before the chunk, then the one after it.
+// fresh: the chunk's first symbol takes any state of its code, without bits.
+__device__ void fse_chain(const FieldTab &T, const uint8_t *cd, uint16_t *up, uint32_t len, bool fresh, uint32_t &D) {
+    const uint32_t lane = lane_id(), size = 1u << T.al;
+    const uint32_t j0 = lane * kRun, n = len > j0 ? min(kRun, len - j0) : 0u;
+    const uint32_t *cw = reinterpret_cast<const uint32_t *>(cd + code_at(j0));  // (rounded up to four codes)
+    uint32_t *uw = reinterpret_cast<uint32_t *>(up + upd_at(j0));
+    uint32_t in = D;
+    if (lane > 0u && n) {  // a guess: the state kWarmUp symbols on from any state
+        in = 0u;
+        for (uint32_t j = j0 - kWarmUp; j < j0; ++j) {
+            const uint2 e = T.enc[cd[code_at(j)]];
+            const uint32_t v = in + size, nb = (v + e.x) >> 16;
+            in = T.stl[(v >> nb) + e.y];
         }
     }
-    uint32_t acc = 0;
-    for (uint32_t c = 0; c < 64u; ++c) {
-        T.cumul[c] = static_cast<uint16_t>(acc);
-        acc += T.norm[c];
+    uint32_t out = in;
+    for (bool again = n > 0u; __any_sync(kFull, again);) {
+        if (again) {
+            out = in;
+            // Four symbols at a time; the codes' entries, which do not depend
+            // on the state, are read one group ahead of the chain.
+            uint32_t w = cw[0];
+            uint2 e[4];
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) e[k] = T.enc[(w >> (8u * k)) & 0xFFu];
+#pragma unroll 1
+            for (uint32_t j = 0; j < n; j += 4u) {
+                uint2 f[4];
+                const bool more = j + 4u < n;
+                if (more) w = cw[j / 4u + 1u];
+#pragma unroll
+                for (uint32_t k = 0; k < 4; ++k) f[k] = T.enc[(w >> (8u * k)) & 0xFFu];
+                uint32_t u[4];
+#pragma unroll
+                for (uint32_t k = 0; k < 4; ++k) {
+                    const uint32_t v = out + size, nb = (v + e[k].x) >> 16, x = v >> nb;
+                    u[k] = (v - (x << nb)) | (nb << 12);
+                    if (j + k < n) out = T.stl[x + e[k].y];
+                }
+                uw[j / 2u] = u[0] | (u[1] << 16);
+                uw[j / 2u + 1u] = u[2] | (u[3] << 16);
+#pragma unroll
+                for (uint32_t k = 0; k < 4; ++k) e[k] = f[k];
+            }
+            if (fresh && lane == 0u) up[0] = 0;
+        }
+        const uint32_t p = __shfl_up_sync(kFull, out, 1);
+        again = lane > 0u && n && p != in;
+        if (again) in = p;
     }
-    uint16_t fill[64];
-    for (uint32_t c = 0; c < 64u; ++c) fill[c] = T.cumul[c];
-    for (uint32_t u = 0; u < tsize; ++u) T.stl[fill[T.sym[u]]++] = static_cast<uint16_t>(u);
+    D = __shfl_sync(kFull, out, (len - 1u) / kRun);
 }
 
-// Decoder state before code c when the next decoder state is dn: the state
-// and, in `up`, the bits the decoder reads (value | count << 12).
-__device__ __forceinline__ uint32_t fse_encode(const FieldTab &T, uint32_t c, uint32_t dn, uint16_t &up) {
-    const uint32_t n = T.norm[c], v = dn + (1u << T.al);
-    const uint32_t hi = T.al - highbit(n);
-    const uint32_t nb = v >= (n << hi) ? hi : hi - 1u;
-    const uint32_t x = v >> nb;
-    up = static_cast<uint16_t>((v - (x << nb)) | (nb << 12));
-    return T.stl[T.cumul[c] + x - n];
+// 32-bit words of `out` from bit `bitpos` on; words shared with a neighbour
+// are ORed in, the others stored.
+struct RunWriter {
+    uint32_t *out;
+    uint64_t word, acc;
+    uint32_t nb;
+    bool first;
+    __device__ __forceinline__ RunWriter(uint32_t *o, uint64_t bitpos)
+        : out(o), word(bitpos >> 5), acc(0), nb(static_cast<uint32_t>(bitpos & 31u)), first(true) {}
+    __device__ __forceinline__ void add(uint32_t v, uint32_t len) {  // len <= 32
+        acc |= static_cast<uint64_t>(v) << nb;
+        nb += len;
+        if (nb >= 32u) {
+            if (first) atomicOr(out + word, static_cast<uint32_t>(acc));
+            else out[word] = static_cast<uint32_t>(acc);
+            first = false;
+            ++word;
+            acc >>= 32;
+            nb -= 32u;
+        }
+    }
+    __device__ __forceinline__ void close() {
+        if (nb) atomicOr(out + word, static_cast<uint32_t>(acc));
+    }
+};
+
+// Step R for one thread's run [i0, i1): Offset_Values from the repeat history
+// r1, r2, r3, which it leaves as it is after the run.
+__device__ __forceinline__ void offset_values(const uint4 *sq, uint32_t *ovg, uint32_t i0, uint32_t i1, uint32_t &r1,
+                                              uint32_t &r2, uint32_t &r3) {
+    uint4 q = i0 < i1 ? sq[i0] : make_uint4(0u, 0u, 0u, 0u);
+    for (uint32_t i = i0; i < i1; ++i) {
+        const uint32_t o = q.x, z = q.y == 0u ? 1u : 0u;
+        if (i + 1u < i1) q = sq[i + 1u];
+        uint32_t v;
+        if (!z) v = o == r1 ? 1u : (o == r2 ? 2u : (o == r3 ? 3u : o + 3u));
+        else v = o == r2 ? 1u : (o == r3 ? 2u : (o == r1 - 1u ? 3u : o + 3u));
+        const uint32_t idx = v > 3u ? 3u : v - 1u + z;
+        // idx 0: rep1 kept; 1: rep2 swapped to the front; else: o in front, the rest shift
+        if (idx >= 2u) r3 = r2;
+        if (idx >= 1u) {
+            r2 = r1;
+            r1 = o;
+        }
+        ovg[i] = v;
+    }
 }
 
-__device__ __forceinline__ void or_bits(uint32_t *buf, uint32_t bitpos, uint64_t v, uint32_t nb) {
-    if (nb == 0u) return;
-    const uint32_t w = bitpos >> 5, sh = bitpos & 31u;
-    const uint64_t lo = v << sh;  // nb <= 48, so v << sh spans at most 80 bits: three words
-    atomicOr(buf + w, static_cast<uint32_t>(lo));
-    if (sh + nb > 32u) atomicOr(buf + w + 1, static_cast<uint32_t>(lo >> 32));
-    if (sh + nb > 64u) atomicOr(buf + w + 2, static_cast<uint32_t>(v >> (64u - sh)));
-}
-
-// Returns the frame's block content size, or 0 when a raw block is smaller.
-__device__ uint32_t encode_sequences_warp(const ZencArgs &a, const SeqSmem &G, WarpSeq &S, uint32_t b, uint32_t w,
-                                          uint32_t fh, uint8_t *slot, uint32_t sec) {
-    const uint32_t lane = lane_id();
+// The frame's block content size, or 0 when a raw block is smaller (the whole
+// CTA gets it).
+__device__ uint32_t encode_sequences(const ZencArgs &a, SeqSmem &G, uint32_t b, uint32_t w, uint32_t fh,
+                                     uint8_t *slot, uint32_t sec) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint64_t s0 = a.seq_offsets[b];
     const uint32_t ns = static_cast<uint32_t>(a.seq_offsets[b + 1] - s0);
     const uint4 *sq = a.seqs + s0;
     uint32_t *ovg = a.ovs + static_cast<uint64_t>(b) * kZencMaxSeqs;
+    const uint32_t per = (ns + kSeqThreads - 1u) / kSeqThreads;
+    const uint32_t i0 = min(tid * per, ns), i1 = min(i0 + per, ns);
 
-    for (uint32_t k = lane; k < 64u; k += 32u) S.tab[0].hist[k] = S.tab[1].hist[k] = S.tab[2].hist[k] = 0u;
-    __syncwarp();
-    // ---- R: Offset_Values, ascending, with the decoder's repeat history (lane 0); code counts
-    uint32_t r1 = 1, r2 = 4, r3 = 8;
-    for (uint32_t lo = 0; lo < ns; lo += kChunk) {
-        const uint32_t len = min(kChunk, ns - lo);
-        for (uint32_t k = lane; k < len; k += 32u) {
-            const uint4 q = sq[lo + k];
-            S.pos[k] = q.x;               // offset
-            S.ov[k] = q.y == 0u ? 1u : 0u;  // literal length is zero
-            atomicAdd(&S.tab[0].hist[G.C.ll_code(q.y)], 1u);
-            atomicAdd(&S.tab[1].hist[G.C.ml_code(q.z)], 1u);
-        }
-        __syncwarp();
-        if (lane == 0) {
-            for (uint32_t k = 0; k < len; ++k) {
-                const uint32_t o = S.pos[k], z = S.ov[k];
-                uint32_t v;
-                if (!z) v = o == r1 ? 1u : (o == r2 ? 2u : (o == r3 ? 3u : o + 3u));
-                else v = o == r2 ? 1u : (o == r3 ? 2u : (o == r1 - 1u ? 3u : o + 3u));
-                const uint32_t idx = v > 3u ? 3u : v - 1u + z;
-                // idx 0: rep1 kept; 1: rep2 swapped to the front; else: o in front, the rest shift
-                if (idx == 1u) {
-                    r2 = r1;
-                    r1 = o;
-                } else if (idx >= 2u) {
-                    r3 = r2;
-                    r2 = r1;
-                    r1 = o;
-                }
-                S.ov[k] = v;
-            }
-        }
-        __syncwarp();
-        for (uint32_t k = lane; k < len; k += 32u) {
-            ovg[lo + k] = S.ov[k];
-            atomicAdd(&S.tab[2].hist[highbit(S.ov[k])], 1u);
-        }
-        __syncwarp();
+    for (uint32_t k = tid; k < 64u; k += kSeqThreads) G.tab[0].hist[k] = G.tab[1].hist[k] = G.tab[2].hist[k] = 0u;
+    __syncthreads();
+    // ---- R: Offset_Values and code counts
+    uint32_t in1 = 1, in2 = 4, in3 = 8;
+    if (i0 < i1 && i0 >= 1u) {
+        in3 = i0 >= 3u ? sq[i0 - 3u].x : (i0 == 2u ? 1u : 4u);
+        in2 = i0 >= 2u ? sq[i0 - 2u].x : 1u;
+        in1 = sq[i0 - 1u].x;
     }
+    for (uint32_t i = tid; i < ns; i += kSeqThreads) {
+        const uint4 q = sq[i];
+        uint32_t c, nb;
+        G.C.ll(q.y, c, nb);
+        atomicAdd(&G.tab[0].hist[c], 1u);
+        G.C.ml(q.z, c, nb);
+        atomicAdd(&G.tab[1].hist[c], 1u);
+    }
+    for (bool again = true;;) {
+        if (again) {
+            uint32_t r1 = in1, r2 = in2, r3 = in3;
+            offset_values(sq, ovg, i0, i1, r1, r2, r3);
+            G.out_state[0][tid] = r1;
+            G.out_state[1][tid] = r2;
+            G.out_state[2][tid] = r3;
+        }
+        __syncthreads();
+        again = false;
+        if (tid > 0u && i0 < i1) {
+            const uint32_t p1 = G.out_state[0][tid - 1u], p2 = G.out_state[1][tid - 1u], p3 = G.out_state[2][tid - 1u];
+            again = p1 != in1 || p2 != in2 || p3 != in3;
+            in1 = p1;
+            in2 = p2;
+            in3 = p3;
+        }
+        if (!__syncthreads_or(again)) break;  // (a thread's history is right once the one before it is)
+    }
+    for (uint32_t i = i0; i < i1; ++i) atomicAdd(&G.tab[2].hist[highbit(ovg[i])], 1u);
+    __syncthreads();
 
-    // ---- T: the three tables (lane 0: LL, lane 1: ML, lane 2: OF)
-    if (lane == 0) build_field_table(S.tab[0], ns, kLLSyms, kMaxAl, kLLNorm, kLLSyms, kLLLog);
-    else if (lane == 1) build_field_table(S.tab[1], ns, kMLSyms, kMaxAl, kMLNorm, kMLSyms, kMLLog);
-    else if (lane == 2) build_field_table(S.tab[2], ns, kOFCodes, 8u, kOFNorm, kOFSyms, kOFLog);
-    __syncwarp();
+    // ---- T: the three tables
+    if (warp == 0) build_field_table(G.tab[0], ns, kLLSyms, kMaxAl, kLLNorm, kLLSyms, kLLLog);
+    else if (warp == 1) build_field_table(G.tab[1], ns, kMLSyms, kMaxAl, kMLNorm, kMLSyms, kMLLog);
+    else if (warp == 2) build_field_table(G.tab[2], ns, kOFCodes, 8u, kOFNorm, kOFSyms, kOFLog);
+    __syncthreads();
 
-    // ---- header: Number_of_Sequences, modes, table descriptions (LL, OF, ML)
+    // header: Number_of_Sequences, modes, table descriptions (LL, OF, ML)
     uint8_t *hp = slot + sec;
     const uint32_t nsb = ns < 128u ? 1u : 2u;
-    const uint32_t d_ll = S.tab[0].desc_len, d_of = S.tab[2].desc_len, d_ml = S.tab[1].desc_len;
+    const uint32_t d_ll = G.tab[0].desc_len, d_of = G.tab[2].desc_len, d_ml = G.tab[1].desc_len;
     const uint32_t hl = nsb + 1u + d_ll + d_of + d_ml;
-    if (lane == 0) {
+    if (sec + hl >= fh + 3u + w) return 0u;  // the literals alone fill the window
+    if (tid == 0) {
         if (ns < 128u) {
             hp[0] = static_cast<uint8_t>(ns);
         } else {
             hp[0] = static_cast<uint8_t>((ns >> 8) + 0x80u);
             hp[1] = static_cast<uint8_t>(ns);
         }
-        hp[nsb] = static_cast<uint8_t>((S.tab[0].mode << 6) | (S.tab[2].mode << 4) | (S.tab[1].mode << 2));
+        hp[nsb] = static_cast<uint8_t>((G.tab[0].mode << 6) | (G.tab[2].mode << 4) | (G.tab[1].mode << 2));
     }
-    for (uint32_t k = lane; k < d_ll + d_of + d_ml; k += 32u) {
-        const uint8_t v = k < d_ll ? S.tab[0].desc[k]
-                                   : (k < d_ll + d_of ? S.tab[2].desc[k - d_ll] : S.tab[1].desc[k - d_ll - d_of]);
-        hp[nsb + 1u + k] = v;
+    for (uint32_t k = tid; k < d_ll + d_of + d_ml; k += kSeqThreads) {
+        const uint8_t *t0 = reinterpret_cast<const uint8_t *>(G.tab[0].desc);
+        const uint8_t *t1 = reinterpret_cast<const uint8_t *>(G.tab[1].desc);
+        const uint8_t *t2 = reinterpret_cast<const uint8_t *>(G.tab[2].desc);
+        hp[nsb + 1u + k] = k < d_ll ? t0[k] : (k < d_ll + d_of ? t2[k - d_ll] : t1[k - d_ll - d_of]);
     }
-    uint8_t *bs = hp + hl;
-    // bitstream bytes at which the block stops paying (none when the literals alone fill the window)
-    const int32_t room = static_cast<int32_t>(fh + 3u + w) - static_cast<int32_t>(sec + hl);
-    if (room <= 0) return 0u;
-    uint32_t carry_word = 0, carry_bits = 0, out_pos = 0;
-    uint32_t D = 0;  // chain state of lanes 0-2
-    for (uint32_t hi = ns; hi > 0u;) {
-        const uint32_t lo = hi > kChunk ? hi - kChunk : 0u, len = hi - lo;
-        // codes, in bitstream order j (sequence hi - 1 - j)
-        for (uint32_t j = lane; j < len; j += 32u) {
-            const uint32_t i = hi - 1u - j;
+    // ---- E: chunks in bitstream order (sequence ns - 1 - j)
+    uint32_t *wslot = reinterpret_cast<uint32_t *>(slot);
+    const uint32_t sb = sec + hl;                 // first byte of the stream
+    const uint32_t room = 8u * (fh + 3u + w - sb);  // stream bits at which the block stops paying
+    if (tid < ((4u - (sb & 3u)) & 3u)) slot[sb + tid] = 0;  // to the first whole word; the words follow chunk by chunk
+    uint32_t zeroed = (sb + 3u) >> 2;             // words below are zero or written (runs OR their shared words in)
+    uint32_t pos = 8u * sb, D = 0;
+    for (uint32_t c0 = 0; c0 < ns; c0 += kChunk) {
+        const uint32_t len = min(kChunk, ns - c0);
+        for (uint32_t j = tid; j < len; j += kSeqThreads) {
+            const uint32_t i = ns - 1u - c0 - j;
             const uint4 q = sq[i];
-            const uint32_t v = ovg[i];
-            S.q[j] = q;
-            S.ov[j] = v;
-            S.code[0][j] = static_cast<uint8_t>(G.C.ll_code(q.y));
-            S.code[1][j] = static_cast<uint8_t>(G.C.ml_code(q.z));
-            S.code[2][j] = static_cast<uint8_t>(highbit(v));
+            uint32_t lc, mc, nb;
+            G.C.ll(q.y, lc, nb);
+            G.C.ml(q.z, mc, nb);
+            G.code[0][code_at(j)] = static_cast<uint8_t>(lc);
+            G.code[1][code_at(j)] = static_cast<uint8_t>(mc);
+            G.code[2][code_at(j)] = static_cast<uint8_t>(highbit(ovg[i]));
         }
-        for (uint32_t k = lane; k < kBufWords; k += 32u) S.buf[k] = 0u;
-        __syncwarp();
-        if (lane < 3u) {  // the three FSE chains
-            const FieldTab &T = S.tab[lane];
-            const uint8_t *cd = S.code[lane];
-            uint16_t *up = S.upd[lane];
-            uint32_t j = 0;
-            if (T.mode == 1u) {  // RLE_Mode: no state, no bits
-                for (; j < len; ++j) up[j] = 0;
-            } else {
-                if (hi == ns) {  // last sequence: any state of its code, no bits
-                    uint16_t dummy;
-                    D = fse_encode(T, cd[0], 0u, dummy);
-                    up[0] = 0;
-                    j = 1;
-                }
-                for (; j < len; ++j) D = fse_encode(T, cd[j], D, up[j]);
+        if (tid < 3u)  // the chains read four codes at a time
+            for (uint32_t j = len; j & 3u; ++j) G.code[tid][code_at(j)] = 0;
+        __syncthreads();
+        if (warp < 3u) {
+            fse_chain(G.tab[warp], G.code[warp], G.upd[warp], len, c0 == 0u, D);
+            if (lane == 0) G.state[warp] = D;
+        }
+        __syncthreads();
+        const uint32_t j0 = min(tid * kOwn, len), j1 = min(j0 + kOwn, len);
+        uint32_t bits = 0;
+        for (uint32_t j = j0; j < j1; ++j) {
+            const uint32_t u = upd_at(j), c = code_at(j);
+            bits += (G.upd[0][u] >> 12) + (G.upd[1][u] >> 12) + (G.upd[2][u] >> 12) + G.C.ll_bits(G.code[0][c]) +
+                    G.C.ml_bits(G.code[1][c]) + G.code[2][c];
+        }
+        const uint32_t incl = scan_incl(bits);
+        if (lane == 31u) G.warp_bits[warp] = incl;
+        __syncthreads();
+        uint32_t before = incl - bits, total = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < kSeqThreads / 32u; ++k) {
+            const uint32_t x = G.warp_bits[k];
+            if (k < warp) before += x;
+            total += x;
+        }
+        if (pos + total - 8u * sb >= room) return 0u;
+        // this chunk's words (and room for the final states), then its bits
+        const uint32_t wend = ((pos + total + 31u) >> 5) + 1u;
+        for (uint32_t k = zeroed + tid; k < wend; k += kSeqThreads) wslot[k] = 0u;
+        __syncthreads();
+        if (j0 < j1) {
+            RunWriter wr(wslot, pos + before);
+            for (uint32_t j = j0; j < j1; ++j) {
+                const uint32_t u = upd_at(j), c = code_at(j), i = ns - 1u - c0 - j;
+                const uint4 q = sq[i];
+                const uint32_t uo = G.upd[2][u], um = G.upd[1][u], ul = G.upd[0][u];
+                const uint32_t no = uo >> 12, nm = um >> 12, nl = ul >> 12;
+                const uint32_t lb = G.C.ll_bits(G.code[0][c]), mb = G.C.ml_bits(G.code[1][c]), oc = G.code[2][c];
+                // updates: OF, ML, LL (the decoder, reading backwards, takes LL, ML, OF); extra bits: LL, ML, OF
+                wr.add((uo & 0xFFFu) | ((um & 0xFFFu) << no) | ((ul & 0xFFFu) << (no + nm)), no + nm + nl);
+                wr.add((q.y & ((1u << lb) - 1u)) | (((q.z - 3u) & ((1u << mb) - 1u)) << lb), lb + mb);
+                wr.add(ovg[i] - (1u << oc), oc);
             }
+            wr.close();
         }
-        __syncwarp();
-        // bit widths and their exclusive scan (each lane: kPerLane consecutive j)
-        uint32_t wsum = 0;
-        const uint32_t j0 = lane * kPerLane;
-        for (uint32_t u = 0; u < kPerLane; ++u) {
-            const uint32_t j = j0 + u;
-            uint32_t nb = 0;
-            if (j < len) {
-                nb = (S.upd[0][j] >> 12) + (S.upd[1][j] >> 12) + (S.upd[2][j] >> 12) + G.C.ll_bits[S.code[0][j]] +
-                     G.C.ml_bits[S.code[1][j]] + S.code[2][j];
-            }
-            S.pos[j] = wsum;
-            wsum += nb;
-        }
-        uint32_t x = wsum;
-        for (uint32_t d = 1; d < 32; d <<= 1) {
-            const uint32_t y = __shfl_up_sync(kFull, x, d);
-            if (lane >= d) x += y;
-        }
-        const uint32_t chunk_bits = __shfl_sync(kFull, x, 31);
-        const uint32_t base = carry_bits + x - wsum;
-        if (lane == 0) S.buf[0] = carry_word;
-        __syncwarp();
-        for (uint32_t u = 0; u < kPerLane; ++u) {
-            const uint32_t j = j0 + u;
-            if (j >= len) break;
-            const uint32_t p0 = base + S.pos[j];
-            // updates: OF, ML, LL (the decoder, reading backwards, takes LL, ML, OF)
-            const uint32_t uo = S.upd[2][j], um = S.upd[1][j], ul = S.upd[0][j];
-            const uint32_t no = uo >> 12, nm = um >> 12, nl = ul >> 12;
-            const uint64_t ga = static_cast<uint64_t>(uo & 0xFFFu) | (static_cast<uint64_t>(um & 0xFFFu) << no) |
-                                (static_cast<uint64_t>(ul & 0xFFFu) << (no + nm));
-            or_bits(S.buf, p0, ga, no + nm + nl);
-            // extra bits: LL, ML, OF
-            const uint4 q = S.q[j];
-            const uint32_t lc = S.code[0][j], mc = S.code[1][j], oc = S.code[2][j];
-            const uint32_t lb = G.C.ll_bits[lc], mb = G.C.ml_bits[mc];
-            const uint64_t gb = static_cast<uint64_t>(q.y - G.C.ll_base[lc]) |
-                                (static_cast<uint64_t>(q.z - G.C.ml_base[mc]) << lb) |
-                                (static_cast<uint64_t>(S.ov[j] - (1u << oc)) << (lb + mb));
-            or_bits(S.buf, p0 + no + nm + nl, gb, lb + mb + oc);
-        }
-        __syncwarp();
-        // store the whole words; the partial one carries over
-        const uint32_t total = carry_bits + chunk_bits, nfull = total >> 5;
-        if (static_cast<int32_t>(out_pos + 4u * nfull) >= room) return 0u;  // warp-uniform
-        for (uint32_t k = lane; k < 4u * nfull; k += 32u)
-            bs[out_pos + k] = static_cast<uint8_t>(S.buf[k >> 2] >> ((k & 3u) * 8u));
-        carry_word = S.buf[nfull];
-        carry_bits = total & 31u;
-        out_pos += 4u * nfull;
-        __syncwarp();
-        hi = lo;
+        zeroed = wend;
+        pos += total;
+        __syncthreads();
     }
-    if (lane < 3u) S.state[lane] = D;
-    __syncwarp();
-    uint32_t content = 0;
-    if (lane == 0) {
-        BitWriter bw{bs, out_pos, carry_word, carry_bits};
-        bw.add(S.state[1], S.tab[1].al);
-        bw.add(S.state[2], S.tab[2].al);
-        bw.add(S.state[0], S.tab[0].al);
-        bw.close();
-        content = sec + hl + bw.pos - (fh + 3u);
+    // the final states ML, OF, LL and the end marker
+    const uint32_t al0 = G.tab[0].al, al1 = G.tab[1].al, al2 = G.tab[2].al;
+    const uint32_t stream = (pos - 8u * sb + al0 + al1 + al2 + 1u + 7u) >> 3;
+    const uint32_t content = sb + stream - (fh + 3u);
+    if (content >= w) return 0u;
+    if (tid == 0) {
+        RunWriter wr(wslot, pos);
+        wr.add(G.state[1], al1);
+        wr.add(G.state[2], al2);
+        wr.add(G.state[0], al0);
+        wr.add(1u, 1u);
+        wr.close();
     }
-    content = __shfl_sync(kFull, content, 0);
-    return content < w ? content : 0u;
+    return content;
 }
 
-__global__ void __launch_bounds__(32 * kSeqWarps) zenc_sequences_kernel(ZencArgs a) {
-    extern __shared__ __align__(128) uint8_t smem_raw[];
-    SeqSmem &G = *reinterpret_cast<SeqSmem *>(smem_raw);
-    const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
+__global__ void __launch_bounds__(kSeqThreads, 8) zenc_sequences_kernel(ZencArgs a) {
+    __shared__ SeqSmem G;
+    const uint32_t tid = threadIdx.x;
     G.C.build();
     __syncthreads();
-    for (uint32_t b = blockIdx.x * kSeqWarps + wid; b < a.num_windows; b += gridDim.x * kSeqWarps) {
+    for (uint32_t b = blockIdx.x; b < a.num_windows; b += gridDim.x) {
         const uint32_t w = win_size(a, b);
         const uint32_t fh = frame_header_bytes(w);
         uint8_t *slot = a.slots + static_cast<uint64_t>(b) * kZencSlot;
         const uint32_t sec = a.sec_off[b];
-        const uint32_t content = sec != 0u ? encode_sequences_warp(a, G, G.W[wid], b, w, fh, slot, sec) : 0u;
-        if (lane == 0) {
+        const uint32_t content = sec != 0u ? encode_sequences(a, G, b, w, fh, slot, sec) : 0u;
+        if (tid == 0) {
             if (content) {
                 write_block_header(slot + fh, 2u, content);
                 a.fsize[b] = fh + 3u + content;
@@ -1304,7 +1407,7 @@ __global__ void __launch_bounds__(32 * kSeqWarps) zenc_sequences_kernel(ZencArgs
                 a.raw[b] = 1;
             }
         }
-        __syncwarp();
+        __syncthreads();
     }
 }
 
@@ -1351,7 +1454,7 @@ ZencArgs args_of(const ZencLaunch &l) {
     return a;
 }
 
-SmemOnce g_lit_smem_set{0}, g_seq_smem_set{0}, g_plan_smem_set{0}, g_write_smem_set{0};
+SmemOnce g_lit_smem_set{0}, g_plan_smem_set{0}, g_write_smem_set{0};
 
 }  // namespace
 
@@ -1375,11 +1478,9 @@ cudaError_t launch_zenc(const ZencLaunch &l, cudaStream_t st) {
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     zenc_huf_write_kernel<<<grid, kLitThreads, kWriteSmem, st>>>(a);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = set_smem_once(zenc_sequences_kernel, sizeof(SeqSmem), g_seq_smem_set)) != cudaSuccess) return e;
-    grid = l.num_sms * 4;  // 4 CTAs of ~56 KB per SM
-    const uint32_t need = (l.num_windows + kSeqWarps - 1) / kSeqWarps;
-    if (static_cast<uint32_t>(grid) > need) grid = static_cast<int>(need);
-    zenc_sequences_kernel<<<grid, 32 * kSeqWarps, sizeof(SeqSmem), st>>>(a);
+    grid = l.num_sms * 8;  // 64 registers per thread
+    if (static_cast<uint32_t>(grid) > l.num_windows) grid = static_cast<int>(l.num_windows);
+    zenc_sequences_kernel<<<grid, kSeqThreads, 0, st>>>(a);
     return cudaGetLastError();
 }
 
