@@ -223,8 +223,8 @@ int zstd_device_core(gcz_ctx *c, Scratch &sc, const uint8_t *d_src, size_t n, ui
     ProfScope ps(c, st);
     if (split) {
         uint16_t *cand = static_cast<uint16_t *>(sc.cand.p);
-        GCZ_CUDA(c, gcz::launch_cand_sweep(d_src, n, kW, (uint32_t)nb, cand, c->num_sms, st, wins, c->sweep_warps,
-                                           c->sweep_groups));
+        GCZ_CUDA(c, gcz::launch_cand_sweep(d_src, n, kW, (uint32_t)nb, cand, (uint32_t)nb, c->num_sms, st, wins,
+                                           c->sweep_warps, c->sweep_groups));
         gcz::Zstd2Launch l{};
         l.src = d_src;
         l.cand = cand;
@@ -277,7 +277,7 @@ int lzma_run(gcz_ctx *c, Scratch &sc, const gcz::LzmaLaunch &l, cudaStream_t st)
     ProfScope ps(c, st);
     if (split) {
         uint16_t *cand = static_cast<uint16_t *>(sc.cand.p);
-        GCZ_CUDA(c, gcz::launch_cand_sweep(l.src, l.n, l.window, l.num_windows, cand, c->num_sms, st, l.wins,
+        GCZ_CUDA(c, gcz::launch_cand_sweep(l.src, l.n, l.window, l.num_windows, cand, 0u, c->num_sms, st, l.wins,
                                            c->sweep_warps, c->sweep_groups));
         gcz::LzmaLaunch lv = l;
         lv.ctas_per_sm = c->lzma_ctas;
@@ -807,7 +807,7 @@ extern "C" int gcz_zstd_match_find_ref_layout_device(gcz_ctx *c, const uint8_t *
         if ((r = ensure_dev(c, c->sc.seg, gcz::zstd2_seg_scratch_entries((uint32_t)nb) * 8)) != GCZ_OK) return r;
         ProfScope ps(c, st);
         uint16_t *cand = static_cast<uint16_t *>(c->sc.cand.p);
-        GCZ_CUDA(c, gcz::launch_cand_sweep(d_input, n_eff, chunk_size, (uint32_t)nb, cand, c->num_sms, st, nullptr,
+        GCZ_CUDA(c, gcz::launch_cand_sweep(d_input, n_eff, chunk_size, (uint32_t)nb, cand, (uint32_t)nb, c->num_sms, st, nullptr,
                                            c->sweep_warps, c->sweep_groups));
         gcz::Zstd2Launch l{};
         l.src = d_input;
@@ -1392,8 +1392,8 @@ int server_launch(gcz_server *sv, ServerSlot &s) {
         if (q->n) GCZ_CUDA(c, cudaMemcpyAsync(slab_p + q->slab_off, q->src, q->n, cudaMemcpyHostToDevice, s.st));
     if (nb) {
         GCZ_CUDA(c, cudaMemcpyAsync(s.wins.p, s.hwins.data(), nb * sizeof(gcz_window), cudaMemcpyHostToDevice, s.st));
-        GCZ_CUDA(c, gcz::launch_cand_sweep(slab_p, slab, kW, (uint32_t)nb, cand, c->num_sms, s.st, dw, c->sweep_warps,
-                                           c->sweep_groups));
+        GCZ_CUDA(c, gcz::launch_cand_sweep(slab_p, slab, kW, (uint32_t)nb, cand, s.wb[kGrpLzma], c->num_sms, s.st, dw,
+                                           c->sweep_warps, c->sweep_groups));
     }
     const uint32_t nz = s.wb[kGrpLzma];  // Zstd windows: sequences and frames groups
     uint64_t *d_off = static_cast<uint64_t *>(s.offsets.p);

@@ -5,7 +5,8 @@
 // order, each lookup at q happening after all p < q were written
 // (zstd_compress.cu:231-235,280,303,328-331; lzma2_match_find.cu:104-108).  The
 // candidate either of them sees at q is therefore
-//     cand(q) = max{ p < q : hash4(p) == hash4(q) }       (0xFFFF if none)
+//     cand(q) = max{ p < q : hash4(p) == hash4(q) }       (none: 0xFFFF, the
+// LZMA2 table's empty entry; or 0, the Zstd one's, which stands for position 0)
 // which this kernel computes for every position of every window; the match
 // finders then verify, extend and parse from it.
 //
@@ -41,6 +42,7 @@ struct SweepArgs {
     uint32_t num_windows;
     uint16_t *cand;  // one entry per input byte, same offsets as src
     const WinDesc *wins;
+    uint32_t zero_windows;  // windows whose positions without a candidate get 0 (0xFFFF in the others)
 };
 
 constexpr uint32_t kChunkSteps = 16;                 // exchanges of one turn
@@ -103,10 +105,11 @@ __device__ __forceinline__ void turn_pass(uint32_t id) { asm volatile("bar.arriv
 // Candidates of one window by one warp, 32 positions per step with the lanes
 // grouped by hash first: exact for any order of colliding lanes.  T: a table
 // of kHashSize entries (one warp at a time).
-__device__ void sweep_window_grouped(uint32_t *T, uint16_t *out, const uint32_t *src32, uint32_t size) {
+__device__ void sweep_window_grouped(uint32_t *T, uint16_t *out, const uint32_t *src32, uint32_t size,
+                                     uint32_t none) {
     const uint32_t lane = lane_id(), lt = lanemask_lt(), gt = lanemask_gt();
     const uint32_t nwords = (size + 3u) >> 2;
-    for (uint32_t i = lane; i < kHashSize; i += 32u) T[i] = 0xFFFFu;
+    for (uint32_t i = lane; i < kHashSize; i += 32u) T[i] = none;
     __syncwarp();
     for (uint32_t q = lane; q - lane < size; q += 32u) {
         const bool v = q + 3u < size;
@@ -115,7 +118,7 @@ __device__ void sweep_window_grouped(uint32_t *T, uint16_t *out, const uint32_t 
         const uint32_t h = hash4(__funnelshift_r(x, y, (q & 3u) * 8u));
         const uint32_t g = __match_any_sync(kFull, v ? h : (0x80000000u | lane));
         const uint32_t lower = g & lt;
-        uint32_t c = v ? T[h] : 0xFFFFu;
+        uint32_t c = v ? T[h] : none;
         if (lower) c = q - lane + 31u - static_cast<uint32_t>(__clz(lower));
         __syncwarp();
         if (v && !(g & gt)) T[h] = q;
@@ -159,6 +162,7 @@ __global__ void __launch_bounds__(32 * kWarps, kSweepCtas) cand_sweep_kernel(Swe
             const uint32_t nwords = (size + 3u) >> 2;
             const uint32_t nch = (size + kChunkPos - 1u) / kChunkPos;
             const bool last_window = a.num_windows - w <= gridDim.x;
+            const uint32_t none = w < a.zero_windows ? 0u : 0xFFFFu;
             uint32_t ch = warp >= first ? warp - first : warp + kWarps - first;  // this warp's first chunk
             ChunkWords cw = load_chunk(src32, nwords, ch);
             for (; ch < nch; ch += kWarps) {
@@ -196,8 +200,8 @@ __global__ void __launch_bounds__(32 * kWarps, kSweepCtas) cand_sweep_kernel(Swe
                 for (uint32_t j = 0; j < kChunkSteps; ++j) {
                     const uint32_t q = q0 + 32u * j;
                     bad = bad || old[j] >= e0 + q;
-                    const uint32_t c = min(old[j] - e0, 0xFFFFu);  // an earlier epoch's entry is below e0: none
-                    if (full || q < size) out[q] = static_cast<uint16_t>(c);
+                    const uint32_t c = old[j] - e0;  // an earlier epoch's entry is below e0: none
+                    if (full || q < size) out[q] = static_cast<uint16_t>(c < 0x10000u ? c : none);
                 }
             }
             if (nch) begun = true;
@@ -211,7 +215,8 @@ __global__ void __launch_bounds__(32 * kWarps, kSweepCtas) cand_sweep_kernel(Swe
             uint64_t start;
             uint32_t size;
             window_of(a, w, start, size);
-            sweep_window_grouped(S.T, a.cand + start, reinterpret_cast<const uint32_t *>(a.src + start), size);
+            sweep_window_grouped(S.T, a.cand + start, reinterpret_cast<const uint32_t *>(a.src + start), size,
+                                 w < a.zero_windows ? 0u : 0xFFFFu);
             __syncwarp();
         }
     }
@@ -233,9 +238,10 @@ cudaError_t launch_sweep_variant(const SweepArgs &a, int num_sms, cudaStream_t s
 }  // namespace
 
 cudaError_t launch_cand_sweep(const uint8_t *src, uint64_t n, uint32_t window, uint32_t num_windows, uint16_t *cand,
-                              int num_sms, cudaStream_t st, const WinDesc *wins, int sweep_warps, int sweep_groups) {
+                              uint32_t zero_windows, int num_sms, cudaStream_t st, const WinDesc *wins,
+                              int sweep_warps, int sweep_groups) {
     if (num_windows == 0) return cudaSuccess;
-    SweepArgs a{src, n, window, num_windows, cand, wins};
+    SweepArgs a{src, n, window, num_windows, cand, wins, zero_windows};
     const bool grouped = (sweep_groups & 1) != 0;
     switch (sweep_warps) {
     case 4: return grouped ? launch_sweep_variant<4, true>(a, num_sms, st) : launch_sweep_variant<4, false>(a, num_sms, st);

@@ -138,6 +138,7 @@ struct LaneSmem {
         };
         struct {
             uint16_t run[kFixes];    // literal runs with a repeat-offset match
+            uint16_t pos[kFixes];    // position at or less than 16 before the run's first one
             uint16_t meet[kFixes];   // entry a mend ends at
             int16_t shift[kFixes];   // output index minus list index from there on
             uint8_t len[kFixes];     // entries of the mend
@@ -179,7 +180,7 @@ struct Win {
     __device__ __forceinline__ uint32_t u32(int q) const {
         const uint32_t *w = reinterpret_cast<const uint32_t *>(d - kPre);
         const uint32_t a = static_cast<uint32_t>(q + static_cast<int>(kPre));
-        return __funnelshift_r(w[a >> 2], w[(a >> 2) + 1], (a & 3u) * 8u);
+        return __funnelshift_r(w[a >> 2], w[(a >> 2) + 1], a << 3);  // the shift counts modulo 32
     }
     // The 4 bytes at q, q a multiple of 4.
     __device__ __forceinline__ uint32_t w32(uint32_t q) const { return reinterpret_cast<const uint32_t *>(d)[q >> 2]; }
@@ -187,7 +188,7 @@ struct Win {
     __device__ __forceinline__ void u64(int q, uint32_t &lo, uint32_t &hi) const {
         const uint32_t *w = reinterpret_cast<const uint32_t *>(d - kPre);
         const uint32_t a = static_cast<uint32_t>(q + static_cast<int>(kPre));
-        const uint32_t i = a >> 2, sh = (a & 3u) * 8u;
+        const uint32_t i = a >> 2, sh = a << 3;
         const uint32_t w1 = w[i + 1];
         lo = __funnelshift_r(w[i], w1, sh);
         hi = __funnelshift_r(w1, w[i + 2], sh);
@@ -296,8 +297,6 @@ __device__ __forceinline__ bool eq3(const Win &w, uint32_t a, uint32_t b) {
 }
 
 __device__ __forceinline__ uint32_t bm_bit(const uint32_t *bm, uint32_t q) { return (bm[q >> 5] >> (q & 31u)) & 1u; }
-
-__device__ __forceinline__ uint32_t zmap(uint32_t c) { return c == 0xFFFFu ? 0u : c; }  // empty entry = position 0
 
 struct PState {
     uint32_t p, r0, r1, r2;
@@ -424,8 +423,8 @@ __device__ __forceinline__ bool warp_step(const Win &w, const uint32_t *bm, Cand
         }
     }
     cb.advance(f);  // a wide scan's event can lie past the buffer
-    const uint32_t cf = zmap(cb.get(f));
-    const uint32_t cf1 = zmap(cb.get(f + 1u));
+    const uint32_t cf = cb.get(f);
+    const uint32_t cf1 = cb.get(f + 1u);
     uint32_t off, c0;
     if (hash) {
         off = f - cf;
@@ -492,6 +491,47 @@ __device__ __forceinline__ uint32_t rep3_scan16(const Win &w, uint32_t q, uint32
     return m;
 }
 
+// Whether any position of q .. q+min(n,16)-1 (n >= 1) has its three bytes equal
+// to those at one of the three distances ro (all <= q).  Per word of positions
+// and distance: y = OR of the difference bytes at t, t+1 and t+2, which is zero
+// at a match; (y - 0x01..) & ~y has 0x80 at the lowest zero byte (and maybe
+// above it, which does not change whether there is one).
+__device__ __forceinline__ bool rep3_any16(const Win &w, uint32_t q, const uint32_t *ro, uint32_t n) {
+    const uint32_t *wd = reinterpret_cast<const uint32_t *>(w.d - kPre);
+    const uint32_t ax = q + kPre;
+    const uint32_t *px = wd + (ax >> 2);
+    uint32_t x[5], a[4] = {0u, 0u, 0u, 0u}, xp = px[0];
+#pragma unroll
+    for (uint32_t j = 0; j < 5; ++j) {
+        const uint32_t xn = px[j + 1];
+        x[j] = __funnelshift_r(xp, xn, ax << 3);
+        xp = xn;
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < 3; ++k) {
+        const uint32_t ay = ax - ro[k];
+        const uint32_t *py = wd + (ay >> 2);
+        uint32_t yp = py[0], yn = py[1], d = x[0] ^ __funnelshift_r(yp, yn, ay << 3);
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+            yp = yn;
+            yn = py[j + 2];
+            const uint32_t dn = x[j + 1] ^ __funnelshift_r(yp, yn, ay << 3);
+            const uint32_t y = d | __funnelshift_r(d, dn, 8) | __funnelshift_r(d, dn, 16);
+            a[j] |= (y - 0x01010101u) & ~y;
+            d = dn;
+        }
+    }
+    if (n < 16u) {
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+            const uint32_t t = n > 4u * j ? n - 4u * j : 0u;  // positions of word j that count
+            if (t < 4u) a[j] &= (1u << (8u * t)) - 1u;
+        }
+    }
+    return ((a[0] | a[1] | a[2] | a[3]) & 0x80808080u) != 0u;
+}
+
 __device__ __forceinline__ uint2 pack_entry(const Match &m) {
     return make_uint2(m.start | ((m.len - kMinMatch) << 16), m.off);
 }
@@ -532,22 +572,22 @@ template <uint32_t kW>
 __device__ __forceinline__ void verify_window(const Win &win, uint32_t *bm, const uint16_t *cand, uint32_t size) {
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
     // Lane l covers positions 4l .. 4l+3 of a 128-position chunk: one
-    // 8-byte load brings its four candidates (2-byte loads where the
-    // window's candidates are not 8-byte aligned or the chunk ends the
-    // window), one aligned 8-byte read its own bytes, and the 8 lanes of
-    // each bitmap word gather their four bits with three shuffles.  kVC
-    // chunks per batch: their candidate loads are all issued first.
-    constexpr uint32_t kChunks = kBmWords / 4u, kVC = 4;
+    // 8-byte load brings its four candidates, one aligned 8-byte read its own
+    // bytes, and the 8 lanes of each bitmap word gather their four bits with
+    // three shuffles.  kVC chunks per batch: their candidate loads are all
+    // issued first.  Words up to four past the window's last are set.
+    constexpr uint32_t kVC = 4;
     static_assert(kBmWords % 4u == 0u, "bitmap words come in 128-position chunks");
-    const bool al8 = (reinterpret_cast<uintptr_t>(cand) & 7u) == 0u;
-    for (uint32_t c0 = warp * kVC; c0 < kChunks; c0 += kW * kVC) {
+    const uint32_t nch = (size >> 7) + 2u, lim_pos = size > 3u ? size - 3u : 0u;
+    for (uint32_t c0 = warp * kVC; c0 < nch; c0 += kW * kVC) {
         uint2 cv[kVC];
 #pragma unroll
         for (uint32_t u = 0; u < kVC; ++u) {
             const uint32_t q = (c0 + u) * 128u + 4u * lane;
-            if (al8 && q + 4u <= size) {
+            cv[u] = make_uint2(0u, 0u);
+            if (q + 4u <= size) {
                 cv[u] = *reinterpret_cast<const uint2 *>(cand + q);
-            } else {
+            } else if (q < lim_pos) {
                 uint32_t e[4];
 #pragma unroll
                 for (uint32_t k = 0; k < 4; ++k) e[k] = q + k < size ? static_cast<uint32_t>(cand[q + k]) : 0u;
@@ -557,25 +597,27 @@ __device__ __forceinline__ void verify_window(const Win &win, uint32_t *bm, cons
 #pragma unroll
         for (uint32_t u = 0; u < kVC; ++u) {
             const uint32_t ch = c0 + u;
-            const uint32_t q = ch * 128u + 4u * lane;
-            uint32_t nib = 0;
-            if (q < size) {
-                const uint32_t x0 = win.w32(q), x1 = win.w32(q + 4u);
+            if (ch >= nch) break;
+            const uint32_t q = min(ch * 128u + 4u * lane, kMaxWindow);
+            const uint32_t x0 = win.w32(q), x1 = win.w32(q + 4u);
+            uint32_t v = 0;
 #pragma unroll
-                for (uint32_t k = 0; k < 4; ++k) {
-                    const uint32_t cw = k < 2u ? cv[u].x : cv[u].y;
-                    const uint32_t c = zmap((k & 1u) ? cw >> 16 : cw & 0xFFFFu);
-                    const uint32_t xk = k ? __funnelshift_r(x0, x1, 8u * k) : x0;
-                    const uint32_t qk = q + k;
-                    const bool hm = qk + 3u < size && qk > 0u && ((xk ^ win.u32(static_cast<int>(c))) & 0xFFFFFFu) == 0u;
-                    nib |= static_cast<uint32_t>(hm) << k;
-                }
+            for (uint32_t k = 0; k < 4; ++k) {
+                const uint32_t cw = k < 2u ? cv[u].x : cv[u].y;
+                const uint32_t c = (k & 1u) ? cw >> 16 : cw & 0xFFFFu;
+                const uint32_t xk = k ? __funnelshift_r(x0, x1, 8u * k) : x0;
+                if (((xk ^ win.u32(static_cast<int>(c))) & 0xFFFFFFu) == 0u) v |= 1u << k;
             }
-            uint32_t v = nib << (4u * (lane & 7u));
+            v <<= 4u * (lane & 7u);
             v |= __shfl_xor_sync(kFull, v, 1);
             v |= __shfl_xor_sync(kFull, v, 2);
             v |= __shfl_xor_sync(kFull, v, 4);
-            if ((lane & 7u) == 0u && ch < kChunks) bm[ch * 4u + (lane >> 3)] = v;
+            if (ch == 0u && lane == 0u) v &= ~1u;  // position 0 has nothing before it
+            if (ch * 128u + 128u > lim_pos) {      // positions from lim_pos on start no match
+                const uint32_t p = ch * 128u + 32u * (lane >> 3), in = lim_pos > p ? lim_pos - p : 0u;
+                if (in < 32u) v &= (1u << in) - 1u;
+            }
+            if ((lane & 7u) == 0u) bm[ch * 4u + (lane >> 3)] = v;
         }
     }
 }
@@ -953,7 +995,7 @@ __device__ __forceinline__ uint32_t extend_lanes(const Win &w, uint32_t c, uint3
 __device__ __forceinline__ void lane_match(const Win &w, const uint32_t *bm, const uint16_t *cand, uint32_t size,
                                            bool lazy, bool act, uint32_t f, Match &m) {
     const uint32_t fc = act ? f : 0u;
-    const uint32_t c0 = zmap(cand[fc]), c1 = zmap(cand[fc + 1u]);
+    const uint32_t c0 = cand[fc], c1 = cand[fc + 1u];
     // skipped when it is the same match one byte on, which is never longer (warp_step)
     const bool ltry = act && lazy && fc + 4u < size && bm_bit(bm, fc + 1u) && c1 != c0 + 1u;
     m.start = fc;
@@ -1151,7 +1193,12 @@ __device__ __forceinline__ uint32_t lane_chain(LaneSmem &N, ParseScalars &S, boo
 __device__ __forceinline__ void lane_check(LaneSmem &N, ParseScalars &S, const Win &win, const uint2 *list,
                                            uint32_t total, uint32_t lim_pos) {
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-    for (uint32_t g = warp * 32u; g <= total; g += kLThreads) {
+    // Few groups of 32 runs (long runs, so many tasks each) are shared by
+    // several warps, each of which repeats the group's scan: 16 warps up to 8
+    // groups, 4 up to 16 (a window of random bytes is one run of 4096 tasks).
+    const uint32_t groups = total / 32u + 1u;
+    const uint32_t team = groups <= 8u ? kLWarps : (groups <= kLWarps ? 4u : 1u);
+    for (uint32_t g = warp / team * 32u; g <= total; g += kLWarps / team * 32u) {
         const uint32_t i = g + lane;
         uint32_t lo = 0, hi = 0, r1 = 1, r2 = 4, r3 = 8;
         if (i <= total) {
@@ -1172,7 +1219,7 @@ __device__ __forceinline__ void lane_check(LaneSmem &N, ParseScalars &S, const W
         }
         const uint32_t T = __shfl_sync(kFull, x, 31), before = x - nt;
         const uint32_t span = lo | (hi << 16), r12 = r1 | (r2 << 16);  // hi <= 65533
-        for (uint32_t b = 0; b < T; b += 32u) {
+        for (uint32_t b = warp % team * 32u; b < T; b += team * 32u) {
             const uint32_t t = b + lane;
             uint32_t o = 0;  // the run of task t: the first lane whose inclusive count is above t
 #pragma unroll
@@ -1185,58 +1232,90 @@ __device__ __forceinline__ void lane_check(LaneSmem &N, ParseScalars &S, const W
             bool hit = false;
             if (t < T) {
                 const uint32_t q0 = (sp & 0xFFFFu) + 16u * k, left = (sp >> 16) - q0;
-                const uint32_t upto = left < 16u ? (1u << left) - 1u : 0xFFFFu;
-                uint32_t any = 0;
-#pragma unroll
-                for (uint32_t v = 0; v < 3u; ++v) {
-                    const uint32_t r = v == 0u ? ra & 0xFFFFu : (v == 1u ? ra >> 16 : rc);
-                    // sources before the window start do not count
-                    const uint32_t skip = r > q0 ? (r - q0 < 16u ? r - q0 : 16u) : 0u;
-                    any |= rep3_scan16(win, q0, skip < 16u ? r : 0u) & (0xFFFFu << skip) & (skip < 16u ? ~0u : 0u);
+                const uint32_t ro[3] = {ra & 0xFFFFu, ra >> 16, rc};
+                if (max(max(ro[0], ro[1]), ro[2]) <= q0) {
+                    hit = rep3_any16(win, q0, ro, left);
+                } else {  // sources before the window start do not count
+                    const uint32_t upto = left < 16u ? (1u << left) - 1u : 0xFFFFu;
+                    uint32_t any = 0;
+#pragma unroll 1
+                    for (uint32_t v = 0; v < 3u; ++v) {
+                        const uint32_t r = v == 0u ? ro[0] : (v == 1u ? ro[1] : ro[2]);
+                        const uint32_t skip = r > q0 ? r - q0 : 0u;
+                        if (skip < 16u) any |= rep3_scan16(win, q0, r) & (0xFFFFu << skip);
+                    }
+                    hit = (any & upto) != 0u;
                 }
-                hit = (any & upto) != 0u;
             }
             if (__any_sync(kFull, hit)) {
                 const uint32_t po = __shfl_up_sync(kFull, o, 1);
                 const bool ph = __shfl_up_sync(kFull, hit ? 1u : 0u, 1) != 0u;
                 if (hit && !(lane > 0u && ph && po == o)) {
                     const uint32_t at = atomicAdd(&S.count, 1u);
-                    if (at < kFixes) N.fix.run[at] = static_cast<uint16_t>(g + o);
+                    if (at < kFixes) {
+                        N.fix.run[at] = static_cast<uint16_t>(g + o);
+                        N.fix.pos[at] = static_cast<uint16_t>((sp & 0xFFFFu) + 16u * k);
+                    }
                 }
             }
         }
     }
 }
 
-// Step 4, first part (warp 0): the n recorded runs sorted, each once; returns
-// how many.
+// Step 4, first part (warp 0): the n recorded runs sorted, each once, with its
+// lowest recorded position; returns how many.
 __device__ __forceinline__ uint32_t sort_runs(LaneSmem &N, uint32_t n) {
     const uint32_t lane = lane_id(), lt = lanemask_lt();
-    uint32_t m = 0;  // distinct runs, moved to the front (never past the ones still to be looked at)
-    for (uint32_t i0 = 0; i0 < n; i0 += 32u) {
-        const uint32_t i = i0 + lane, v = i < n ? N.fix.run[i] : 0u;
-        bool first = i < n;
-        for (uint32_t k = 0; k < m && first; ++k) first = N.fix.run[k] != v;
-        for (uint32_t k = i0; k < i && first; ++k) first = N.fix.run[k] != v;
-        __syncwarp();
-        const uint32_t f = __ballot_sync(kFull, first);
-        if (first) N.fix.run[m + static_cast<uint32_t>(__popc(f & lt))] = static_cast<uint16_t>(v);
-        m += static_cast<uint32_t>(__popc(f));
-        __syncwarp();
-    }
-    for (uint32_t i = lane; i < m; i += 32u) {  // each to its rank, through N.fix.meet
-        const uint32_t v = N.fix.run[i];
+    auto key = [&](uint32_t i) { return (static_cast<uint32_t>(N.fix.run[i]) << 16) | N.fix.pos[i]; };
+    uint32_t m = 0;
+    for (uint32_t i = lane; i < n; i += 32u) {  // each to its rank, through meet and shift
+        const uint32_t v = key(i);
         uint32_t rank = 0;
-        for (uint32_t k = 0; k < m; ++k) rank += N.fix.run[k] < v ? 1u : 0u;
-        N.fix.meet[rank] = static_cast<uint16_t>(v);
+        for (uint32_t k = 0; k < n; ++k) {
+            const uint32_t o = key(k);
+            rank += o < v || (o == v && k < i) ? 1u : 0u;
+        }
+        N.fix.meet[rank] = static_cast<uint16_t>(v >> 16);
+        N.fix.shift[rank] = static_cast<int16_t>(v & 0xFFFFu);
     }
     __syncwarp();
-    for (uint32_t i = lane; i < m; i += 32u) N.fix.run[i] = N.fix.meet[i];
+    for (uint32_t i0 = 0; i0 < n; i0 += 32u) {  // the first of each run, moved together
+        const uint32_t i = i0 + lane;
+        const bool first = i < n && (i == 0u || N.fix.meet[i] != N.fix.meet[i - 1u]);
+        const uint32_t f = __ballot_sync(kFull, first), at = m + static_cast<uint32_t>(__popc(f & lt));
+        if (first) {
+            N.fix.run[at] = N.fix.meet[i];
+            N.fix.pos[at] = static_cast<uint16_t>(N.fix.shift[i]);
+        }
+        m += static_cast<uint32_t>(__popc(f));
+    }
+    __syncwarp();
     return m;
 }
 
-// Step 4, second part: mend r (one warp) parses run i exactly from its start
-// until it emits entry `meet` of the list with the same repeat offsets.
+// Past literals that start no match, 512 at a time (16 per lane), for long
+// stretches without a hash match (a window of random bytes is one): a position
+// from which on the state is the same.
+__device__ __noinline__ uint32_t skip_literals(Win win, const uint32_t *bm, uint32_t lim_pos, PState st) {
+    const uint32_t lane = lane_id();
+    const uint32_t ro[3] = {st.r0, st.r1, st.r2};
+    while (st.p + 512u <= lim_pos && max(max(ro[0], ro[1]), ro[2]) <= st.p) {
+        const uint32_t sh = st.p & 31u;
+        uint32_t b = lane <= 16u ? bm[(st.p >> 5) + lane] : 0u;
+        if (lane == 0u) b &= ~0u << sh;
+        if (lane == 16u) b &= (1u << sh) - 1u;
+        if (__any_sync(kFull, b != 0u)) break;
+        const uint32_t hit = __ballot_sync(kFull, rep3_any16(win, st.p + 16u * lane, ro, 16u));
+        if (hit) return st.p + 16u * (static_cast<uint32_t>(__ffs(hit)) - 1u);
+        st.p += 512u;
+    }
+    return st.p;
+}
+
+// Step 4, second part: mend r (one warp) parses run i exactly from its first
+// repeat-offset match (less than 16 positions before it; the literals up to
+// there are checked) until it emits entry `meet` of the list with the same
+// repeat offsets.
 __device__ __noinline__ void mend_run(LaneSmem &N, ParseScalars &S, Win win, const uint32_t *bm, const uint16_t *cand,
                                       uint2 *seg, uint32_t size, bool lazy, uint32_t total, uint32_t r,
                                       uint32_t cap) {
@@ -1244,13 +1323,16 @@ __device__ __noinline__ void mend_run(LaneSmem &N, ParseScalars &S, Win win, con
     const uint32_t i = N.fix.run[r];
     const uint2 *list = seg;
     uint2 *out = seg + kLContBase + r * cap;
+    const uint32_t lim_pos = size - 3u;  // a window with a run to mend has more than 3 bytes
     PState st;
-    st.p = i ? entry_end(list[i - 1u]) : 0u;
+    st.p = N.fix.pos[r];
     reps_before(list, i, st.r0, st.r1, st.r2);
     CandBuf cb{cand, size, 0u, 0u, 0u, 0u};
     cb.init(st.p);
     uint32_t j = i, n = 0, meet = total;
     while (st.p + 3u < size) {
+        const uint32_t *ahead = bm + (st.p >> 5);
+        if ((ahead[1] | ahead[2] | ahead[3]) == 0u) st.p = skip_literals(win, bm, lim_pos, st);
         Match m;
         if (!warp_step(win, bm, cb, size, lazy, st, m)) continue;
         for (;;) {  // first entry with start >= m.start
