@@ -47,7 +47,7 @@ struct Scratch {
 struct Slot {
     Scratch sc;
     DevBuf in, offsets, seqs, lz_packed, lz_has, frames, foff;
-    HostBuf h_off, h_packed, h_foff;
+    HostBuf h_off, h_packed, h_foff, h_has;
     cudaStream_t st = nullptr;
     cudaEvent_t ev = nullptr;      // the slice's kernels (and small copies) are done
     cudaEvent_t ev_out = nullptr;  // the slice's results have left its device buffers
@@ -187,6 +187,12 @@ struct ProfScope {
     }
 };
 
+int status_error(gcz_ctx *c, uint32_t h) {
+    if (h & 2u) return fail(c, GCZ_ECAPACITY, "output capacity exceeded (device status %u)", h);
+    if (h & 4u) return fail(c, GCZ_EINVAL, "sequences do not describe their windows (device status %u)", h);
+    return fail(c, GCZ_EDEVICE, "kernel reported status %u (bounded wait expired)", h);
+}
+
 int read_status(gcz_ctx *c, cudaStream_t st) {
     uint32_t h = 0;
     GCZ_CUDA(c, cudaMemcpyAsync(&h, c->d_status, 4, cudaMemcpyDeviceToHost, st));
@@ -194,9 +200,7 @@ int read_status(gcz_ctx *c, cudaStream_t st) {
     if (h) {
         GCZ_CUDA(c, cudaMemsetAsync(c->d_status, 0, 4, st));
         GCZ_CUDA(c, cudaStreamSynchronize(st));
-        if (h & 2u) return fail(c, GCZ_ECAPACITY, "output capacity exceeded (device status %u)", h);
-        if (h & 4u) return fail(c, GCZ_EINVAL, "sequences do not describe their windows (device status %u)", h);
-        return fail(c, GCZ_EDEVICE, "kernel reported status %u (bounded wait expired)", h);
+        return status_error(c, h);
     }
     return GCZ_OK;
 }
@@ -208,7 +212,7 @@ size_t nwin(size_t n) { return (n + kW - 1) / kW; }
 // With `wins`, n is the slab size and nbw the number of windows in the table.
 int zstd_device_core(gcz_ctx *c, Scratch &sc, const uint8_t *d_src, size_t n, uint32_t depth, void *d_seqs,
                      uint64_t capacity, uint64_t *d_offsets, cudaStream_t st, const gcz::WinDesc *wins = nullptr,
-                     size_t nbw = 0, bool rec8 = false) {
+                     size_t nbw = 0, bool rec8 = false, uint32_t *status_out = nullptr) {
     const size_t nb = wins ? nbw : nwin(n);
     int r;
     if ((r = ensure_dev(c, sc.packed, nb * (size_t)kMaxSeqs * 8)) != GCZ_OK) return r;
@@ -259,14 +263,9 @@ int zstd_device_core(gcz_ctx *c, Scratch &sc, const uint8_t *d_src, size_t n, ui
         GCZ_CUDA(c, gcz::launch_zstd_match(l, st));
         c->all_launches += 1;
     }
-    GCZ_CUDA(c, gcz::launch_scan_counts(counts, (uint32_t)nb, d_offsets, st));
-    if (rec8)
-        GCZ_CUDA(c, gcz::launch_compact_seqs(sc.packed.p, counts, d_offsets, (uint32_t)nb, kMaxSeqs, d_seqs, capacity,
-                                             c->d_status, c->num_sms, st));
-    else
-        GCZ_CUDA(c, gcz::launch_expand_seqs(sc.packed.p, counts, d_offsets, (uint32_t)nb, kMaxSeqs, d_seqs, capacity,
-                                            c->d_status, c->num_sms, st));
-    c->all_launches += 2;
+    GCZ_CUDA(c, gcz::launch_expand_seqs(sc.packed.p, counts, d_offsets, (uint32_t)nb, kMaxSeqs, d_seqs, capacity,
+                                        c->d_status, c->num_sms, st, rec8, status_out));
+    c->all_launches += nb <= gcz::kFusedScan ? 1 : 2;
     return GCZ_OK;
 }
 
@@ -320,9 +319,8 @@ int zenc_core(gcz_ctx *c, Scratch &sc, const uint8_t *d_src, size_t n, const voi
     l.num_sms = c->num_sms;
     l.wins = wins;
     GCZ_CUDA(c, gcz::launch_zenc(l, st));
-    GCZ_CUDA(c, gcz::launch_scan_counts(l.fsize, (uint32_t)nb, d_frame_offsets, st));
     GCZ_CUDA(c, gcz::launch_zenc_compact(l, d_frame_offsets, d_out, out_capacity, st));
-    c->all_launches += 6;
+    c->all_launches += nb <= gcz::kFusedScan ? 5 : 6;
     return GCZ_OK;
 }
 
@@ -400,7 +398,7 @@ extern "C" void gcz_destroy(gcz_ctx *c) {
             free_scratch(sl.sc);
             for (DevBuf *b : {&sl.in, &sl.offsets, &sl.seqs, &sl.lz_packed, &sl.lz_has, &sl.frames, &sl.foff})
                 if (b->p) cudaFree(b->p);
-            for (HostBuf *b : {&sl.h_off, &sl.h_packed, &sl.h_foff})
+            for (HostBuf *b : {&sl.h_off, &sl.h_packed, &sl.h_foff, &sl.h_has})
                 if (b->p) cudaFreeHost(b->p);
             if (sl.ev) cudaEventDestroy(sl.ev);
             if (sl.ev_out) cudaEventDestroy(sl.ev_out);
@@ -625,6 +623,46 @@ int drain_slots(gcz_ctx *c) {
 // (two slots, finishing slice k-1: 47.7 GB/s for 1 GiB; four: 48.8, against
 // 51.8 for the same copies with no kernels).
 namespace {
+// Inputs of at most this size take one slice whose kernels write offsets,
+// records and the status word straight into pinned host memory: one
+// synchronisation, and no copy back that would have to wait for the offsets
+// (4 KiB: 84 -> 47 us, 200 KB: 160 -> 126 us). Above, the host copy out of the
+// pinned memory costs more than the synchronisation it saves.
+constexpr size_t kDirectBytes = 256u << 10;
+
+int zstd_host_direct(gcz_ctx *c, const uint8_t *src, size_t n, uint32_t search_depth, void *seqs, size_t seq_capacity,
+                     uint64_t *offsets, uint32_t rec_bytes) {
+    const size_t nb = nwin(n), cap = gcz_zstd_max_sequences(n);
+    Slot &sl = c->slots[0];
+    int r;
+    if ((r = ensure_dev(c, sl.in, nb * (size_t)kW + 64)) != GCZ_OK) return r;
+    // sized once for the largest direct input: status word, offsets, records
+    const size_t off_bytes = (16 + (kDirectBytes / kW + 1) * 8 + 15) & ~size_t(15);  // records are 16-byte stores
+    if ((r = ensure_host(c, sl.h_off, off_bytes + gcz_zstd_max_sequences(kDirectBytes) * 16)) != GCZ_OK) return r;
+    uint8_t *h = static_cast<uint8_t *>(sl.h_off.p);
+    uint32_t *h_status = reinterpret_cast<uint32_t *>(h);
+    uint64_t *h_off = reinterpret_cast<uint64_t *>(h + 16);
+    uint8_t *h_rec = h + off_bytes;
+    GCZ_CUDA(c, cudaMemcpyAsync(sl.in.p, src, n, cudaMemcpyHostToDevice, sl.st));
+    if ((r = zstd_device_core(c, sl.sc, static_cast<const uint8_t *>(sl.in.p), n, search_depth, h_rec, cap, h_off,
+                              sl.st, nullptr, 0, rec_bytes == 8, h_status)) != GCZ_OK)
+        return r;
+    GCZ_CUDA(c, cudaStreamSynchronize(sl.st));
+    if (*h_status) {
+        GCZ_CUDA(c, cudaMemsetAsync(c->d_status, 0, 4, sl.st));
+        GCZ_CUDA(c, cudaStreamSynchronize(sl.st));
+        return status_error(c, *h_status);
+    }
+    const uint64_t total = h_off[nb];
+    if (total > seq_capacity)
+        return fail(c, GCZ_ECAPACITY, "need %llu sequences, capacity %zu", (unsigned long long)total, seq_capacity);
+    memcpy(offsets, h_off, (nb + 1) * 8);
+    if (total) memcpy(seqs, h_rec, total * rec_bytes);
+    return GCZ_OK;
+}
+}  // namespace
+
+namespace {
 // The host-buffer Zstd pipeline: records of rec_bytes (16: ZSTD_Sequence, 8:
 // packed {ll | (ml-3) << 16, off}) back to back in `seqs`.
 int zstd_host_pipeline(gcz_ctx *c, const uint8_t *src, size_t n, uint32_t search_depth, void *seqs,
@@ -632,6 +670,9 @@ int zstd_host_pipeline(gcz_ctx *c, const uint8_t *src, size_t n, uint32_t search
     DeviceGuard g(c->device);
     const size_t nb = nwin(n);
     offsets[0] = 0;
+    if (n == 0) return read_status(c, c->stream);
+    if (n <= kDirectBytes && nb <= c->slice_windows)
+        return zstd_host_direct(c, src, n, search_depth, seqs, seq_capacity, offsets, rec_bytes);
     int r = GCZ_OK;
     uint64_t done = 0;  // sequences copied so far
     constexpr size_t kS = sizeof(c->slots) / sizeof(c->slots[0]);
@@ -880,6 +921,7 @@ int lzma_host_slices(gcz_ctx *c, const uint8_t *src, size_t n, uint32_t depth, u
     auto finish = [&](Slot &sl) -> int {
         GCZ_CUDA(c, cudaEventSynchronize(sl.ev));
         sl.busy = false;
+        if (has_out) memcpy(has_out + sl.b0, sl.h_has.p, sl.sb);
         consume(sl.off, sl.len, packed_out ? packed_out + sl.off : static_cast<const uint32_t *>(sl.h_packed.p));
         return GCZ_OK;
     };
@@ -908,7 +950,10 @@ int lzma_host_slices(gcz_ctx *c, const uint8_t *src, size_t n, uint32_t depth, u
             }
             GCZ_CUDA(c, cudaMemcpyAsync(dst, sl.lz_packed.p, sl.len * 4, cudaMemcpyDeviceToHost, sl.st));
         }
-        if (has_out) GCZ_CUDA(c, cudaMemcpyAsync(has_out + b0, sl.lz_has.p, sb, cudaMemcpyDeviceToHost, sl.st));
+        if (has_out) {  // through pinned memory: a copy to pageable memory would hold up the host until the slice is done
+            if ((r = ensure_host(c, sl.h_has, sb)) != GCZ_OK) break;
+            GCZ_CUDA(c, cudaMemcpyAsync(sl.h_has.p, sl.lz_has.p, sb, cudaMemcpyDeviceToHost, sl.st));
+        }
         GCZ_CUDA(c, cudaEventRecord(sl.ev, sl.st));
         sl.busy = true;
         if (k >= kS - 1) {  // finish slice k-(S-1), in slice order
@@ -1420,7 +1465,6 @@ int server_launch(gcz_server *sv, ServerSlot &s) {
             l.wins = dw + a;
             GCZ_CUDA(c, gcz::launch_zstd_parse(l, s.st));
         }
-        GCZ_CUDA(c, gcz::launch_scan_counts(counts, nz, d_off, s.st));
         GCZ_CUDA(c, gcz::launch_expand_seqs(s.packed.p, counts, d_off, nz, kMaxSeqs, s.seqs.p,
                                             s.seqs.cap / 16, status, c->num_sms, s.st));
         if (s.wb[kGrpFramesLazy])  // offsets of the sequences groups
@@ -1448,7 +1492,6 @@ int server_launch(gcz_server *sv, ServerSlot &s) {
         l.wins = dw + f0;
         uint64_t *d_foff = static_cast<uint64_t *>(s.foff.p);
         GCZ_CUDA(c, gcz::launch_zenc(l, s.st));
-        GCZ_CUDA(c, gcz::launch_scan_counts(l.fsize, nf, d_foff, s.st));
         GCZ_CUDA(c, gcz::launch_zenc_compact(l, d_foff, static_cast<uint8_t *>(s.frames.p), s.frames.cap, s.st));
         GCZ_CUDA(c, cudaMemcpyAsync(s.h_foff.p, d_foff, (nf + 1) * 8, cudaMemcpyDeviceToHost, s.st));
     }

@@ -81,6 +81,22 @@ struct GlobalWin {
     }
 };
 
+// Sum of counts[0 .. w), for every thread of a CTA of 256.
+__device__ __forceinline__ uint64_t cta_sum_before(const uint32_t *counts, uint32_t w) {
+    __shared__ uint64_t part[8];
+    uint64_t s = 0;
+    for (uint32_t i = threadIdx.x; i < w; i += 256u) s += counts[i];
+#pragma unroll
+    for (uint32_t o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
+    __syncthreads();  // the last call's sums have been read
+    if ((threadIdx.x & 31u) == 0u) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    s = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) s += part[k];
+    return s;
+}
+
 // One bit per device: the kernel's shared-memory limit is set there.  Atomic,
 // because contexts on different host threads launch concurrently.
 using SmemOnce = std::atomic<unsigned long long>;

@@ -83,13 +83,16 @@ cudaError_t launch_cand_sweep(const uint8_t *src, uint64_t n, uint32_t window, u
 size_t zstd2_seg_scratch_entries(uint32_t num_windows);
 cudaError_t launch_zstd_parse(const Zstd2Launch &l, cudaStream_t st);
 cudaError_t launch_scan_counts(const uint32_t *counts, uint32_t num, uint64_t *offsets, cudaStream_t st);
-cudaError_t launch_expand_seqs(const void *packed, const uint32_t *counts, const uint64_t *offsets, uint32_t num,
+// Up to this many windows the kernels that need the offsets compute them, each
+// CTA those of its windows: one launch less (3 us of 37 for one window). Above,
+// scan_counts_kernel's single pass is cheaper than every CTA's.
+constexpr uint32_t kFusedScan = 1024;
+// Per-window offsets (num + 1) from the counts, and the records back to back:
+// ZSTD_Sequence, or with rec8 8 bytes {ll | (ml-3) << 16, off}.  status_out
+// (at most kFusedScan windows): copy of the status word.
+cudaError_t launch_expand_seqs(const void *packed, const uint32_t *counts, uint64_t *offsets, uint32_t num,
                                uint32_t max_seqs, void *out, uint64_t capacity, uint32_t *status, int num_sms,
-                               cudaStream_t st);
-// 8-byte records {ll | (ml-3) << 16, off} instead of ZSTD_Sequence.
-cudaError_t launch_compact_seqs(const void *packed, const uint32_t *counts, const uint64_t *offsets, uint32_t num,
-                                uint32_t max_seqs, void *out, uint64_t capacity, uint32_t *status, int num_sms,
-                                cudaStream_t st);
+                               cudaStream_t st, bool rec8 = false, uint32_t *status_out = nullptr);
 cudaError_t launch_zstd_literals(const uint8_t *src, uint64_t n, uint32_t window, uint32_t num_windows,
                                  const uint32_t *ref_seqs, const uint32_t *seq_counts, uint32_t max_seqs, uint8_t *lits,
                                  int num_sms, cudaStream_t st);
@@ -117,7 +120,8 @@ struct ZencLaunch {
     const WinDesc *wins = nullptr;  // optional window table (16-byte-aligned offsets)
 };
 cudaError_t launch_zenc(const ZencLaunch &l, cudaStream_t st);
-cudaError_t launch_zenc_compact(const ZencLaunch &l, const uint64_t *frame_offsets, uint8_t *out, uint64_t capacity,
+// Frame offsets (num_windows + 1) from l.fsize, and the frames back to back.
+cudaError_t launch_zenc_compact(const ZencLaunch &l, uint64_t *frame_offsets, uint8_t *out, uint64_t capacity,
                                 cudaStream_t st);
 
 cudaError_t launch_lzma_match(const LzmaLaunch &l, cudaStream_t st);

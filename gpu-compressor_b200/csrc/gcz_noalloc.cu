@@ -95,7 +95,6 @@ int na_run(int device, const uint8_t *d_src, size_t n, uint32_t search_depth, gc
     l.num_sms = d.num_sms;
     l.staged = 1;
     if (gcz::launch_zstd_match(l, st) != cudaSuccess ||
-        gcz::launch_scan_counts(counts, nb, d_offsets, st) != cudaSuccess ||
         gcz::launch_expand_seqs(d.scratch, counts, d_offsets, nb, GCZ_ZSTD_MAX_SEQ_PER_WINDOW, d_seqs, seq_capacity,
                                 status, d.num_sms, st) != cudaSuccess)
         return GCZ_ECUDA;

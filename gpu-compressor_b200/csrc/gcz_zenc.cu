@@ -1538,7 +1538,9 @@ __global__ void __launch_bounds__(kSeqThreads, 8) zenc_sequences_kernel(ZencArgs
 // ---------------------------------------------------------------- compaction
 // blockIdx.y of gridDim.y parts of a frame (multiples of 16 bytes): few
 // windows are copied by several CTAs each.
-__global__ void __launch_bounds__(256) zenc_compact_kernel(ZencArgs a, const uint64_t *foff, uint8_t *out,
+// kScan: the frame offsets are computed here too (few windows).
+template <bool kScan>
+__global__ void __launch_bounds__(256) zenc_compact_kernel(ZencArgs a, uint64_t *foff, uint8_t *out,
                                                            uint64_t capacity) {
     const uint32_t tid = threadIdx.x;
     // the part [lo, hi) of n bytes
@@ -1547,7 +1549,18 @@ __global__ void __launch_bounds__(256) zenc_compact_kernel(ZencArgs a, const uin
         if (lo < n) cta_copy(d + lo, s + lo, n - lo < per ? n - lo : per);
     };
     for (uint32_t b = blockIdx.x; b < a.num_windows; b += gridDim.x) {
-        const uint64_t o = foff[b], size = foff[b + 1] - o;
+        uint64_t o, size;
+        if constexpr (kScan) {
+            o = cta_sum_before(a.fsize, b);
+            size = a.fsize[b];
+            if (tid == 0 && blockIdx.y == 0u) {
+                foff[b] = o;
+                if (b + 1u == a.num_windows) foff[b + 1u] = o + size;
+            }
+        } else {
+            o = foff[b];
+            size = foff[b + 1] - o;
+        }
         if (o + size > capacity) {
             if (tid == 0) atomicOr(a.status, kErrCapacity);
             continue;
@@ -1615,14 +1628,20 @@ cudaError_t launch_zenc(const ZencLaunch &l, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_zenc_compact(const ZencLaunch &l, const uint64_t *frame_offsets, uint8_t *out, uint64_t capacity,
+cudaError_t launch_zenc_compact(const ZencLaunch &l, uint64_t *frame_offsets, uint8_t *out, uint64_t capacity,
                                 cudaStream_t st) {
     if (l.num_windows == 0) return cudaSuccess;
     const uint32_t most = static_cast<uint32_t>(l.num_sms) * 8u;
     const uint32_t grid = most < l.num_windows ? most : l.num_windows;
     // up to 16 parts of a frame (about 4 KiB each) while CTAs are left
     const uint32_t parts = grid * 16u <= most ? 16u : most / grid;
-    zenc_compact_kernel<<<dim3(grid, parts), 256, 0, st>>>(args_of(l), frame_offsets, out, capacity);
+    if (l.num_windows <= kFusedScan) {
+        zenc_compact_kernel<true><<<dim3(grid, parts), 256, 0, st>>>(args_of(l), frame_offsets, out, capacity);
+    } else {
+        const cudaError_t e = launch_scan_counts(l.fsize, l.num_windows, frame_offsets, st);
+        if (e != cudaSuccess) return e;
+        zenc_compact_kernel<false><<<dim3(grid, parts), 256, 0, st>>>(args_of(l), frame_offsets, out, capacity);
+    }
     return cudaGetLastError();
 }
 

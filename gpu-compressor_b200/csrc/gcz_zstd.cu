@@ -290,14 +290,30 @@ __global__ void __launch_bounds__(1024) scan_counts_kernel(const uint32_t *count
     if (tid == 0) offsets[num] = carry_s;
 }
 
-// Packed sequences at stride max_seqs -> compact ZSTD_Sequence records
-// (offset, litLength, matchLength = ml-3+3, rep = 0), compress_zstd_custom.rs:140-153.
+// Packed sequences at stride max_seqs -> compact records: ZSTD_Sequence
+// (offset, litLength, matchLength = ml-3+3, rep = 0), compress_zstd_custom.rs:140-153,
+// or with k8 8 bytes each, {litLength | (matchLength-3) << 16, offset} (a
+// window's lengths and offsets are below 65536).  kScan: the offsets are
+// computed here too (few windows), each CTA summing the counts before its
+// window, and status_out, if any, takes the status word of the kernels before.
+template <bool k8, bool kScan>
 __global__ void __launch_bounds__(256) expand_seqs_kernel(const uint2 *packed, const uint32_t *counts,
-                                                          const uint64_t *offsets, uint32_t num, uint32_t max_seqs,
-                                                          uint4 *out, uint64_t capacity, uint32_t *status) {
+                                                          uint64_t *offsets, uint32_t num, uint32_t max_seqs,
+                                                          void *out, uint64_t capacity, uint32_t *status,
+                                                          uint32_t *status_out) {
     for (uint32_t w = blockIdx.x; w < num; w += gridDim.x) {
         const uint32_t cnt = counts[w];
-        const uint64_t o = offsets[w];
+        uint64_t o;
+        if constexpr (kScan) {
+            o = cta_sum_before(counts, w);
+            if (threadIdx.x == 0) {
+                offsets[w] = o;
+                if (w + 1u == num) offsets[num] = o + cnt;
+                if (w == 0u && status_out) *status_out = *status;
+            }
+        } else {
+            o = offsets[w];
+        }
         const uint2 *src = packed + static_cast<uint64_t>(w) * max_seqs;
         if (o + cnt > capacity) {
             if (threadIdx.x == 0) atomicOr(status, kErrCapacity);
@@ -305,25 +321,9 @@ __global__ void __launch_bounds__(256) expand_seqs_kernel(const uint2 *packed, c
         }
         for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) {
             const uint2 v = src[i];
-            out[o + i] = make_uint4(v.y, v.x & 0xFFFFu, (v.x >> 16) + kZstdMinMatch, 0u);
+            if constexpr (k8) static_cast<uint2 *>(out)[o + i] = v;
+            else static_cast<uint4 *>(out)[o + i] = make_uint4(v.y, v.x & 0xFFFFu, (v.x >> 16) + kZstdMinMatch, 0u);
         }
-    }
-}
-
-// The same records compacted as 8 bytes each: {litLength | (matchLength-3) << 16,
-// offset} (a window's lengths and offsets are below 65536).
-__global__ void __launch_bounds__(256) compact_seqs_kernel(const uint2 *packed, const uint32_t *counts,
-                                                           const uint64_t *offsets, uint32_t num, uint32_t max_seqs,
-                                                           uint2 *out, uint64_t capacity, uint32_t *status) {
-    for (uint32_t w = blockIdx.x; w < num; w += gridDim.x) {
-        const uint32_t cnt = counts[w];
-        const uint64_t o = offsets[w];
-        const uint2 *src = packed + static_cast<uint64_t>(w) * max_seqs;
-        if (o + cnt > capacity) {
-            if (threadIdx.x == 0) atomicOr(status, kErrCapacity);
-            continue;
-        }
-        for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) out[o + i] = src[i];
     }
 }
 
@@ -412,26 +412,35 @@ cudaError_t launch_scan_counts(const uint32_t *counts, uint32_t num, uint64_t *o
     return cudaGetLastError();
 }
 
-cudaError_t launch_expand_seqs(const void *packed, const uint32_t *counts, const uint64_t *offsets, uint32_t num,
-                               uint32_t max_seqs, void *out, uint64_t capacity, uint32_t *status, int num_sms,
-                               cudaStream_t st) {
-    if (num == 0) return cudaSuccess;
+namespace {
+template <bool k8>
+cudaError_t launch_records(const void *packed, const uint32_t *counts, uint64_t *offsets, uint32_t num,
+                           uint32_t max_seqs, void *out, uint64_t capacity, uint32_t *status, uint32_t *status_out,
+                           int num_sms, cudaStream_t st) {
     int grid = num_sms * 8;
     if (static_cast<uint32_t>(grid) > num) grid = static_cast<int>(num);
-    expand_seqs_kernel<<<grid, 256, 0, st>>>(reinterpret_cast<const uint2 *>(packed), counts, offsets, num, max_seqs,
-                                             reinterpret_cast<uint4 *>(out), capacity, status);
+    const uint2 *pk = reinterpret_cast<const uint2 *>(packed);
+    if (num <= kFusedScan) {
+        expand_seqs_kernel<k8, true><<<grid, 256, 0, st>>>(pk, counts, offsets, num, max_seqs, out, capacity, status,
+                                                           status_out);
+    } else {
+        const cudaError_t e = launch_scan_counts(counts, num, offsets, st);
+        if (e != cudaSuccess) return e;
+        expand_seqs_kernel<k8, false><<<grid, 256, 0, st>>>(pk, counts, offsets, num, max_seqs, out, capacity, status,
+                                                            nullptr);
+    }
     return cudaGetLastError();
 }
+}  // namespace
 
-cudaError_t launch_compact_seqs(const void *packed, const uint32_t *counts, const uint64_t *offsets, uint32_t num,
-                                uint32_t max_seqs, void *out, uint64_t capacity, uint32_t *status, int num_sms,
-                                cudaStream_t st) {
+cudaError_t launch_expand_seqs(const void *packed, const uint32_t *counts, uint64_t *offsets, uint32_t num,
+                               uint32_t max_seqs, void *out, uint64_t capacity, uint32_t *status, int num_sms,
+                               cudaStream_t st, bool rec8, uint32_t *status_out) {
     if (num == 0) return cudaSuccess;
-    int grid = num_sms * 8;
-    if (static_cast<uint32_t>(grid) > num) grid = static_cast<int>(num);
-    compact_seqs_kernel<<<grid, 256, 0, st>>>(reinterpret_cast<const uint2 *>(packed), counts, offsets, num, max_seqs,
-                                              reinterpret_cast<uint2 *>(out), capacity, status);
-    return cudaGetLastError();
+    return rec8 ? launch_records<true>(packed, counts, offsets, num, max_seqs, out, capacity, status, status_out,
+                                       num_sms, st)
+                : launch_records<false>(packed, counts, offsets, num, max_seqs, out, capacity, status, status_out,
+                                        num_sms, st);
 }
 
 cudaError_t launch_zstd_literals(const uint8_t *src, uint64_t n, uint32_t window, uint32_t num_windows,
