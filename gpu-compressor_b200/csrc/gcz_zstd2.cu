@@ -111,7 +111,6 @@ struct ParseScalars {
 // Lane parse.
 constexpr uint32_t kLThreads = 512, kLWarps = kLThreads / 32;
 constexpr uint32_t kLSegW = 128, kLSegs = kMaxWindow / kLSegW;  // four bitmap words per segment
-constexpr uint32_t kLPool = kLSegs / kLWarps;                   // segments of one warp
 constexpr uint32_t kLCap = (kLSegW + 2) / 3;                    // matches that start their search in a segment
 constexpr uint32_t kLCont = 12;                                 // matches before a segment's parse joins a list ...
 constexpr uint32_t kLBig = 16, kLBigCap = 128;                  // ... and lists for the few that take more
@@ -1030,8 +1029,11 @@ __device__ __forceinline__ void reps_before(const uint2 *list, uint32_t i, uint3
 __device__ __forceinline__ void lane_parse(LaneSmem &N, const Win &win, const uint32_t *bm, const uint16_t *cand,
                                            uint2 *seg, uint32_t size, uint32_t nact, bool lazy) {
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5, lt = lanemask_lt();
-    uint32_t next = warp * kLPool;
-    const uint32_t end = next + kLPool < nact ? next + kLPool : nact;
+    // A short window's segments are spread over all warps: fewer lanes of a warp
+    // wait for one another.
+    const uint32_t pool = (nact + kLWarps - 1u) / kLWarps;
+    uint32_t next = warp * pool;
+    const uint32_t end = next + pool < nact ? next + pool : nact;
     bool has = false;
     uint32_t s = 0, p = 0, n = 0;
     for (;;) {
