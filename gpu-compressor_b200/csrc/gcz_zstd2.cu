@@ -163,7 +163,7 @@ struct Zstd2Args {
     uint32_t num_windows;
     uint32_t lazy;
     uint32_t max_seqs;
-    uint2 *seg;          // per window: kSegs * kLaneCap entries {start | (ml-3)<<16, off} (the widest layout's stride)
+    uint2 *seg;          // per window: seg_stride entries {start | (ml-3)<<16, off}
     uint2 *packed;       // packed output at stride max_seqs (or null)
     uint32_t *ref_seqs;  // reference triples at stride max_seqs (or null)
     uint32_t *seq_counts;
