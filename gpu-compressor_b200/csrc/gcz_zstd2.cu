@@ -104,12 +104,11 @@ struct ParseScalars {
     uint32_t count;    // literal runs with a repeat-offset match found
     uint32_t mends;    // mends of the window
     uint32_t bigs;     // continuations that took a long list
-    uint32_t warp_sum[16];
+    uint32_t warp_sum[32];
     alignas(8) uint64_t bar;
 };
 
 // Lane parse.
-constexpr uint32_t kLThreads = 512, kLWarps = kLThreads / 32;
 constexpr uint32_t kLSegW = 128, kLSegs = kMaxWindow / kLSegW;  // four bitmap words per segment
 constexpr uint32_t kLCap = (kLSegW + 2) / 3;                    // matches that start their search in a segment
 constexpr uint32_t kLCont = 12;                                 // matches before a segment's parse joins a list ...
@@ -125,6 +124,7 @@ constexpr uint32_t kFixEntries = kLEntries - kLContBase;        // shared by a w
 static_assert(kLContBase >= 21846, "the whole parse fits where the lists were");
 static_assert(kLCont + kLBigCap <= 255, "8-bit counts");
 
+template <uint32_t kWarps>
 struct LaneSmem {
     union {
         struct {
@@ -143,7 +143,7 @@ struct LaneSmem {
             uint8_t len[kFixes];     // entries of the mend
             uint8_t list[kFixes];    // the mend's list in the scratch
         } fix;
-        SegSmem<kLWarps> seg;
+        SegSmem<kWarps> seg;
     };
 };
 
@@ -1026,12 +1026,13 @@ __device__ __forceinline__ void reps_before(const uint2 *list, uint32_t i, uint3
 }
 
 // Step 1: every lane parses segments of its warp's pool without repeat offsets.
-__device__ __forceinline__ void lane_parse(LaneSmem &N, const Win &win, const uint32_t *bm, const uint16_t *cand,
+template <uint32_t kWarps>
+__device__ __forceinline__ void lane_parse(LaneSmem<kWarps> &N, const Win &win, const uint32_t *bm, const uint16_t *cand,
                                            uint2 *seg, uint32_t size, uint32_t nact, bool lazy) {
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5, lt = lanemask_lt();
     // A short window's segments are spread over all warps: fewer lanes of a warp
     // wait for one another.
-    const uint32_t pool = (nact + kLWarps - 1u) / kLWarps;
+    const uint32_t pool = (nact + kWarps - 1u) / kWarps;
     uint32_t next = warp * pool;
     const uint32_t end = next + pool < nact ? next + pool : nact;
     bool has = false;
@@ -1070,12 +1071,13 @@ __device__ __forceinline__ void lane_parse(LaneSmem &N, const Win &win, const ui
 }
 
 // Step 2, first half: where each segment's parse joins a later segment's list.
-__device__ __forceinline__ void lane_link(LaneSmem &N, ParseScalars &S, const Win &win, const uint32_t *bm,
+template <uint32_t kWarps>
+__device__ __forceinline__ void lane_link(LaneSmem<kWarps> &N, ParseScalars &S, const Win &win, const uint32_t *bm,
                                           const uint16_t *cand, uint2 *seg, uint32_t size, uint32_t nact,
                                           uint32_t lim_pos, bool lazy) {
     const uint32_t tid = threadIdx.x;
 #pragma unroll 1
-    for (uint32_t s = tid; s < kLSegs; s += kLThreads) {
+    for (uint32_t s = tid; s < kLSegs; s += 32u * kWarps) {
         uint32_t E = (s + 1u) * kLSegW + (s < nact ? N.link[s] : 0u);  // position the parse has reached
         uint32_t t = kNoWarp, j = 0, cn = 0, big = 0;
         bool run = s < nact;
@@ -1127,48 +1129,32 @@ __device__ __forceinline__ void lane_link(LaneSmem &N, ParseScalars &S, const Wi
 // the entry each is joined at and its output offset; the chain's entries.
 // Marking doubles: when the marked segments are those fewer than 2^r links
 // from segment 0 and `link` leads 2^r links on, the marked ones mark theirs.
-__device__ __forceinline__ uint32_t lane_chain(LaneSmem &N, ParseScalars &S, bool any) {
-    constexpr uint32_t kPer = kLSegs / kLThreads;  // consecutive segments per thread
-    static_assert(kPer * kLThreads == kLSegs && 32u % kPer == 0u, "whole segments per thread");
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, s0 = tid * kPer;
-    uint32_t n[kPer], l[kPer], j[kPer];
-    bool on[kPer];
-#pragma unroll
-    for (uint32_t u = 0; u < kPer; ++u) {
-        n[u] = l[u] = N.link[s0 + u];
-        j[u] = N.from[s0 + u];
-        on[u] = any && s0 + u == 0u;
-    }
+template <uint32_t kWarps>
+__device__ __forceinline__ uint32_t lane_chain(LaneSmem<kWarps> &N, ParseScalars &S, bool any) {
+    static_assert(32u * kWarps >= kLSegs, "a thread for every segment");
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const bool mine = tid < kLSegs;  // thread s keeps segment s
+    uint32_t n = mine ? N.link[tid] : kNoWarp, l = n, j = mine ? N.from[tid] : 0u;
+    bool on = any && tid == 0u;
     if (tid < kLSegs / 32u) N.chain[tid] = any && tid == 0 ? 1u : 0u;
     __syncthreads();
     for (;;) {
         bool go = false;
-#pragma unroll
-        for (uint32_t u = 0; u < kPer; ++u) {
-            if (n[u] == kNoWarp) continue;
-            if (on[u]) atomicOr(&N.chain[n[u] >> 5], 1u << (n[u] & 31u));
-            n[u] = N.link[n[u]];
-            go = go || n[u] != kNoWarp;
+        if (n != kNoWarp) {
+            if (on) atomicOr(&N.chain[n >> 5], 1u << (n & 31u));
+            n = N.link[n];
+            go = n != kNoWarp;
         }
         go = __syncthreads_or(go);
-#pragma unroll
-        for (uint32_t u = 0; u < kPer; ++u) on[u] = (N.chain[s0 >> 5] >> ((s0 & 31u) + u)) & 1u;
+        if (mine) on = (N.chain[tid >> 5] >> (tid & 31u)) & 1u;
         if (!go) break;
-#pragma unroll
-        for (uint32_t u = 0; u < kPer; ++u) N.link[s0 + u] = static_cast<uint16_t>(n[u]);
+        if (mine) N.link[tid] = static_cast<uint16_t>(n);
         __syncthreads();
     }
-#pragma unroll
-    for (uint32_t u = 0; u < kPer; ++u)
-        if (on[u] && l[u] != kNoWarp) N.from[l[u]] = static_cast<uint8_t>(j[u]);
+    if (on && l != kNoWarp) N.from[l] = static_cast<uint8_t>(j);
     if (tid == 0) N.from[0] = 0;
     __syncthreads();
-    uint32_t sum = 0;
-#pragma unroll
-    for (uint32_t u = 0; u < kPer; ++u) {
-        l[u] = sum;
-        if (on[u]) sum += N.count[s0 + u] - N.from[s0 + u] + N.cont[s0 + u];
-    }
+    const uint32_t sum = on ? N.count[tid] - N.from[tid] + N.cont[tid] : 0u;
     uint32_t x = sum;
 #pragma unroll
     for (uint32_t d = 1; d < 32u; d <<= 1) {
@@ -1178,13 +1164,12 @@ __device__ __forceinline__ uint32_t lane_chain(LaneSmem &N, ParseScalars &S, boo
     if (lane == 31u) S.warp_sum[warp] = x;
     __syncthreads();
     uint32_t base = 0, total = 0;
-    for (uint32_t w = 0; w < kLWarps; ++w) {
+    for (uint32_t w = 0; w < kWarps; ++w) {
         const uint32_t v = S.warp_sum[w];
         if (w < warp) base += v;
         total += v;
     }
-#pragma unroll
-    for (uint32_t u = 0; u < kPer; ++u) N.link[s0 + u] = static_cast<uint16_t>(base + x - sum + l[u]);
+    if (mine) N.link[tid] = static_cast<uint16_t>(base + x - sum);
     return total;
 }
 
@@ -1192,15 +1177,16 @@ __device__ __forceinline__ uint32_t lane_chain(LaneSmem &N, ParseScalars &S, boo
 // (zstd_compress.cu:259-275), into N.fix.run (unsorted, repeats possible);
 // S.count counts them.  Run i lies before entry i of the list, the last one
 // after it.
-__device__ __forceinline__ void lane_check(LaneSmem &N, ParseScalars &S, const Win &win, const uint2 *list,
+template <uint32_t kWarps>
+__device__ __forceinline__ void lane_check(LaneSmem<kWarps> &N, ParseScalars &S, const Win &win, const uint2 *list,
                                            uint32_t total, uint32_t lim_pos) {
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
     // Few groups of 32 runs (long runs, so many tasks each) are shared by
     // several warps, each of which repeats the group's scan: 16 warps up to 8
     // groups, 4 up to 16 (a window of random bytes is one run of 4096 tasks).
     const uint32_t groups = total / 32u + 1u;
-    const uint32_t team = groups <= 8u ? kLWarps : (groups <= kLWarps ? 4u : 1u);
-    for (uint32_t g = warp / team * 32u; g <= total; g += kLWarps / team * 32u) {
+    const uint32_t team = groups <= 8u ? kWarps : (groups <= kWarps ? 4u : 1u);
+    for (uint32_t g = warp / team * 32u; g <= total; g += kWarps / team * 32u) {
         const uint32_t i = g + lane;
         uint32_t lo = 0, hi = 0, r1 = 1, r2 = 4, r3 = 8;
         if (i <= total) {
@@ -1266,7 +1252,8 @@ __device__ __forceinline__ void lane_check(LaneSmem &N, ParseScalars &S, const W
 
 // Step 4, first part (warp 0): the n recorded runs sorted, each once, with its
 // lowest recorded position; returns how many.
-__device__ __forceinline__ uint32_t sort_runs(LaneSmem &N, uint32_t n) {
+template <uint32_t kWarps>
+__device__ __forceinline__ uint32_t sort_runs(LaneSmem<kWarps> &N, uint32_t n) {
     const uint32_t lane = lane_id(), lt = lanemask_lt();
     auto key = [&](uint32_t i) { return (static_cast<uint32_t>(N.fix.run[i]) << 16) | N.fix.pos[i]; };
     uint32_t m = 0;
@@ -1318,7 +1305,8 @@ __device__ __noinline__ uint32_t skip_literals(Win win, const uint32_t *bm, uint
 // repeat-offset match (less than 16 positions before it; the literals up to
 // there are checked) until it emits entry `meet` of the list with the same
 // repeat offsets.
-__device__ __noinline__ void mend_run(LaneSmem &N, ParseScalars &S, Win win, const uint32_t *bm, const uint16_t *cand,
+template <uint32_t kWarps>
+__device__ __noinline__ void mend_run(LaneSmem<kWarps> &N, ParseScalars &S, Win win, const uint32_t *bm, const uint16_t *cand,
                                       uint2 *seg, uint32_t size, bool lazy, uint32_t total, uint32_t r,
                                       uint32_t cap) {
     const uint32_t lane = lane_id();
@@ -1367,26 +1355,27 @@ __device__ __noinline__ void mend_run(LaneSmem &N, ParseScalars &S, Win win, con
     }
 }
 
-template <bool kRef>
-__device__ __noinline__ void parse_segments_out(Zstd2Args a, SegSmem<kLWarps> &G, ParseScalars &S, Win win,
+template <bool kRef, uint32_t kWarps>
+__device__ __noinline__ void parse_segments_out(Zstd2Args a, SegSmem<kWarps> &G, ParseScalars &S, Win win,
                                                 const uint32_t *bm, const uint16_t *cand, uint2 *seg, uint32_t wi,
                                                 uint32_t size, bool lazy) {
-    parse_segments<kRef, kMaxWindow / kLWarps>(a, G, S, win, bm, cand, seg, wi, size, lazy);
+    parse_segments<kRef, kMaxWindow / kWarps>(a, G, S, win, bm, cand, seg, wi, size, lazy);
 }
 
-template <bool kRef>
-__global__ void __launch_bounds__(kLThreads, 3) zstd_lane_parse_kernel(Zstd2Args a) {
+template <bool kRef, uint32_t kWarps>
+__global__ void __launch_bounds__(32 * kWarps, kWarps == 16 ? 3 : 1) zstd_lane_parse_kernel(Zstd2Args a) {
+    constexpr uint32_t kThreads = 32u * kWarps;
     extern __shared__ __align__(128) uint8_t smem_raw[];
-    SmemLayout<LaneSmem> &M = *reinterpret_cast<SmemLayout<LaneSmem> *>(smem_raw);
+    SmemLayout<LaneSmem<kWarps>> &M = *reinterpret_cast<SmemLayout<LaneSmem<kWarps>> *>(smem_raw);
     ParseScalars &S = M.s;
-    LaneSmem &N = M.p;
+    LaneSmem<kWarps> &N = M.p;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     uint32_t parity = 0;
     if (tid == 0) {
         mbar_init(&S.bar, 1);
         fence_mbar_init();
     }
-    for (uint32_t i = tid; i < kPre / 4; i += kLThreads) reinterpret_cast<uint32_t *>(M.data)[i] = 0u;
+    for (uint32_t i = tid; i < kPre / 4; i += kThreads) reinterpret_cast<uint32_t *>(M.data)[i] = 0u;
     const Win win{M.data + kPre};
     const bool lazy = a.lazy != 0;
     for (uint32_t wi = blockIdx.x; wi < a.num_windows; wi += gridDim.x) {
@@ -1409,7 +1398,7 @@ __global__ void __launch_bounds__(kLThreads, 3) zstd_lane_parse_kernel(Zstd2Args
         }
         __syncthreads();
         if (S.flags & 2u) return;  // bulk copy never completed: status already recorded, all threads leave
-        verify_window<kLWarps>(win, M.bm, cand, size);
+        verify_window<kWarps>(win, M.bm, cand, size);
         __syncthreads();
 
         const uint32_t lim_pos = size > 3u ? size - 3u : 0u;  // positions q < lim_pos can start a match
@@ -1426,7 +1415,7 @@ __global__ void __launch_bounds__(kLThreads, 3) zstd_lane_parse_kernel(Zstd2Args
         // to the front of the scratch, over the lists.
         uint2 *pk = kRef ? nullptr : a.packed + static_cast<uint64_t>(wi) * a.max_seqs;
         uint32_t *rk = kRef ? a.ref_seqs + static_cast<uint64_t>(wi) * a.max_seqs * 3u : nullptr;
-        for (uint32_t s = tid >> 2; s < kLSegs; s += kLThreads / 4u) {
+        for (uint32_t s = tid >> 2; s < kLSegs; s += kThreads / 4u) {
             if (!((N.chain[s >> 5] >> (s & 31u)) & 1u)) continue;
             const uint32_t from = N.from[s], ns = N.count[s], nc = N.cont[s];
             uint32_t big = 0;
@@ -1447,7 +1436,7 @@ __global__ void __launch_bounds__(kLThreads, 3) zstd_lane_parse_kernel(Zstd2Args
             }
         }
         __syncthreads();
-        for (uint32_t i = tid; i < total; i += kLThreads) {
+        for (uint32_t i = tid; i < total; i += kThreads) {
             if constexpr (kRef) seg[i] = make_uint2(rk[3u * i], rk[3u * i + 1u]);
             else seg[i] = pk[i];
         }
@@ -1466,7 +1455,7 @@ __global__ void __launch_bounds__(kLThreads, 3) zstd_lane_parse_kernel(Zstd2Args
                 __syncthreads();
                 nfix = S.mends;
                 fcap = kFixEntries / nfix < kFixCap ? kFixEntries / nfix : kFixCap;
-                for (uint32_t r = warp; r < nfix; r += kLWarps)
+                for (uint32_t r = warp; r < nfix; r += kWarps)
                     mend_run(N, S, win, M.bm, cand, seg, size, lazy, total, r, fcap);
                 __syncthreads();
                 if (tid == 0) {  // drop the mends that start inside an earlier one
@@ -1494,13 +1483,13 @@ __global__ void __launch_bounds__(kLThreads, 3) zstd_lane_parse_kernel(Zstd2Args
             __syncthreads();
             if (tid == 0) S.flags = 0u;
             __syncthreads();
-            parse_segments_out<kRef>(a, N.seg, S, win, M.bm, cand, seg, wi, size, lazy);
+            parse_segments_out<kRef, kWarps>(a, N.seg, S, win, M.bm, cand, seg, wi, size, lazy);
             continue;
         }
         const uint32_t out_n = nfix ? S.total : total;
         const uint32_t keep = out_n < a.max_seqs ? out_n : a.max_seqs;
         uint32_t cov = 0;
-        for (uint32_t x = tid; x < total; x += kLThreads) {
+        for (uint32_t x = tid; x < total; x += kThreads) {
             uint32_t o = x, pi = x;  // output index; the entry before x is prev[pi - 1]
             const uint2 *prev = seg;
             bool skip = false;
@@ -1523,7 +1512,7 @@ __global__ void __launch_bounds__(kLThreads, 3) zstd_lane_parse_kernel(Zstd2Args
             cov += (e.x >> 16) + kMinMatch;
             write_seq<kRef>(a, wi, o, (e.x & 0xFFFFu) - pe, e.x >> 16, e.y & 0xFFFFu);
         }
-        for (uint32_t z = warp; z < nfix; z += kLWarps) {
+        for (uint32_t z = warp; z < nfix; z += kWarps) {
             const uint32_t i = N.fix.run[z], n = N.fix.len[z];
             const uint32_t base = i + (z ? static_cast<uint32_t>(static_cast<int32_t>(N.fix.shift[z - 1u])) : 0u);
             const uint2 *fl = seg + kLContBase + N.fix.list[z] * fcap;
@@ -1581,15 +1570,26 @@ cudaError_t launch_seg_parse(const Zstd2Args &a, int num_sms, int ctas_per_sm, c
                                st);
 }
 
+template <bool kRef, uint32_t kWarps>
+cudaError_t launch_lane_parse(const Zstd2Args &a, int num_sms, int ctas_per_sm, cudaStream_t st) {
+    constexpr uint32_t smem = sizeof(SmemLayout<LaneSmem<kWarps>>);
+    static_assert(smem + 1024 <= 233472 / 3, "three CTAs per SM must fit");
+    static SmemOnce smem_set{0};
+    return launch_parse_kernel(zstd_lane_parse_kernel<kRef, kWarps>, smem, 32 * kWarps, smem_set, a, num_sms,
+                               ctas_per_sm, st);
+}
+
 template <bool kRef>
 cudaError_t launch_parse_ref(const Zstd2Args &a, uint32_t seg_width, int num_sms, int ctas_per_sm, cudaStream_t st) {
     if (seg_width == 2048) return launch_seg_parse<kRef, 2048>(a, num_sms, ctas_per_sm, st);
     if (seg_width == 4096) return launch_seg_parse<kRef, 4096>(a, num_sms, ctas_per_sm, st);
     if (seg_width == 8192) return launch_seg_parse<kRef, 8192>(a, num_sms, ctas_per_sm, st);
-    constexpr uint32_t smem = sizeof(SmemLayout<LaneSmem>);
-    static_assert(smem + 1024 <= 233472 / 3, "three CTAs per SM must fit");
-    static SmemOnce smem_set{0};
-    return launch_parse_kernel(zstd_lane_parse_kernel<kRef>, smem, kLThreads, smem_set, a, num_sms, ctas_per_sm, st);
+    // At most one window per SM: 32 warps share it instead of 16, with all of
+    // the SM's registers.  Sweep to records, 1 window 100.3 -> 89.3 us, 148
+    // windows 109.6 -> 96.6; a 4 KiB window takes the same 26.7.  From two
+    // windows per SM on the 16-warp form runs them side by side (149 windows: 119).
+    if (a.num_windows <= static_cast<uint32_t>(num_sms)) return launch_lane_parse<kRef, 32>(a, num_sms, 1, st);
+    return launch_lane_parse<kRef, 16>(a, num_sms, ctas_per_sm, st);
 }
 }  // namespace
 
