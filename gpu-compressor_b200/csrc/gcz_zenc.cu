@@ -481,7 +481,7 @@ constexpr uint32_t kPlanWarps = 4;
 struct PlanSmem {  // one per warp
     uint32_t leafw[258];  // leaf weights ascending, then two sentinels
     uint32_t node[258];   // internal weights in the order they are made, sentinels where none is yet
-    uint32_t bl[64];
+    uint32_t bl[32];
     uint32_t start[16];
     uint32_t cw[12];
     uint16_t leaf[256];
@@ -556,7 +556,7 @@ __device__ uint32_t plan_fse_weights(PlanSmem &P, uint32_t N) {
     if (!(p0 | p1)) return 0;
     const uint32_t s_prev = p0 ? static_cast<uint32_t>(__ffs(p0)) - 1u : 31u + static_cast<uint32_t>(__ffs(p1));
     __syncwarp();
-    uint32_t size = 0;
+    uint32_t desc = 0;
     if (lane == 0) {
         // table description (RFC 8878 4.1.1)
         SmemBits wr{P.tree + 1, 127u, 0u, 0u, 0ull, false};
@@ -591,37 +591,71 @@ __device__ uint32_t plan_fse_weights(PlanSmem &P, uint32_t N) {
             if (norm[s2] == 0) zeros = 0;
         }
         wr.flush();
-        // The two chains alternate, so each step's table read overlaps the one before it.
-        uint8_t *out = P.tree + 1 + wr.pos;
-        const uint32_t cap = 127u > wr.pos ? 127u - wr.pos : 0u;
-        uint32_t pos = 0, nbits = 0, pa = s_last, pb = s_prev;
-        uint64_t bits = 0;
-        auto put = [&](uint32_t v, uint32_t n) {
-            bits |= static_cast<uint64_t>(v) << nbits;
-            nbits += n;
-            if (nbits >= 32u) {
-#pragma unroll
-                for (uint32_t k = 0; k < 4; ++k)
-                    if (pos + k < cap) out[pos + k] = static_cast<uint8_t>(bits >> (8u * k));
-                pos += 4u;
-                bits >>= 32;
-                nbits -= 32u;
-            }
-        };
-        for (int i = static_cast<int>(N) - 3; i >= 0; --i) {
-            const uint32_t e = P.fenc[P.wts[i] * 64u + pa], n = e >> 6;
-            put((pa + 64u) & ((1u << n) - 1u), n);
-            pa = pb;
-            pb = e & 63u;
-        }
-        put(pa, 6u);  // state of weight 1, then of weight 0
-        put(pb, 6u);
-        put(1u, 1u);  // end marker
-        for (; nbits > 0u; nbits = nbits > 8u ? nbits - 8u : 0u, bits >>= 8, ++pos)
-            if (pos < cap) out[pos] = static_cast<uint8_t>(bits);
-        if (!wr.ovf && wr.pos + pos <= 127u) size = wr.pos + pos;
+        desc = wr.pos;
     }
-    return __shfl_sync(kFull, size, 0);
+    desc = __shfl_sync(kFull, desc, 0);
+    // Entry u of the bitstream: state | bit count << 6, for weights N-3 .. 0,
+    // then the states of weights 1 and 0 and the end marker.  The two chains
+    // alternate; lanes 0 and 1 run one each, four weights read ahead of it.
+    uint16_t *ent = P.anc[0];
+    uint32_t *words = reinterpret_cast<uint32_t *>(P.anc[1]);
+    const uint32_t M = N - 2u, T = M + 3u;
+    if (lane < 2u) {
+        uint32_t x = lane ? s_prev : s_last, u = lane;
+        for (; u + 6u < M; u += 8u) {
+            uint32_t w[4], o[4];
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) w[k] = 64u * P.wts[M - 1u - u - 2u * k];
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) {
+                const uint32_t e = P.fenc[w[k] + x];
+                o[k] = x | (e & ~63u);
+                x = e & 63u;
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) ent[u + 2u * k] = static_cast<uint16_t>(o[k]);
+        }
+        for (; u < M; u += 2u) {
+            const uint32_t e = P.fenc[64u * P.wts[M - 1u - u] + x];
+            ent[u] = static_cast<uint16_t>(x | (e & ~63u));
+            x = e & 63u;
+        }
+        ent[u] = static_cast<uint16_t>(x | (6u << 6));  // u: M or M + 1
+    }
+    if (lane == 2u) ent[T - 1u] = 1u | (1u << 6);
+    for (uint32_t i = lane; i < 52u; i += 32u) words[i] = 0u;
+    __syncwarp();
+    uint64_t v = 0;  // this lane's eight entries, at most 48 bits
+    uint32_t nv = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) {
+        const uint32_t u = 8u * lane + k;
+        if (u < T) {
+            const uint32_t e = ent[u], n = e >> 6;
+            v |= static_cast<uint64_t>(e & ((1u << n) - 1u)) << nv;
+            nv += n;
+        }
+    }
+    uint32_t end = nv;
+#pragma unroll
+    for (uint32_t d = 1; d < 32u; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, end, d);
+        if (lane >= d) end += y;
+    }
+    if (nv) {
+        const uint32_t at = end - nv, sh = at & 31u;
+        const uint64_t lo = v << sh;
+        atomicOr(&words[at >> 5], static_cast<uint32_t>(lo));
+        atomicOr(&words[(at >> 5) + 1u], static_cast<uint32_t>(lo >> 32));
+        if (sh) atomicOr(&words[(at >> 5) + 2u], static_cast<uint32_t>(v >> (64u - sh)));
+    }
+    const uint32_t bytes = (__shfl_sync(kFull, end, 31) + 7u) >> 3;
+    if (desc + bytes > 127u) return 0;
+    __syncwarp();
+    const uint8_t *wb = reinterpret_cast<const uint8_t *>(words);
+    for (uint32_t i = lane; i < bytes; i += 32u) P.tree[1u + desc + i] = wb[i];
+    __syncwarp();
+    return desc + bytes;
 }
 
 // The 256 keys of a warp in ascending order (bitonic network); lane l holds
@@ -653,7 +687,10 @@ __device__ __forceinline__ void sort256(uint32_t *v) {
     }
 }
 
-// One warp per window: the Huffman code of the window's literals.
+// One warp per window: the Huffman code of the window's literals.  One window is
+// bound by latency, so what one lane did in order (255 merges, 253 FSE steps with
+// their bits, moves of leaves one by one) is done by the warp in few rounds:
+// 17 windows 69 -> 36 us, 4096 windows 134 -> 62.
 __global__ void __launch_bounds__(32 * kPlanWarps) zenc_huf_plan_kernel(ZencArgs a) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
@@ -692,69 +729,104 @@ __global__ void __launch_bounds__(32 * kPlanWarps) zenc_huf_plan_kernel(ZencArgs
                 }
                 if (lane < 2u) P.leafw[256u + lane] = P.node[256u + lane] = ~0u;
                 __syncwarp();
-                // Two-queue Huffman construction (serial): the two lightest of the
-                // next two leaves and the next two internal nodes, a leaf first
-                // on equal weights; sentinels stand for what is not there.
-                if (lane == 0) {
-                    uint32_t li = 0, ii = 0;
-                    for (uint32_t m = 0; m + 1u < n; ++m) {
-                        const uint32_t l0 = P.leafw[li], l1 = P.leafw[li + 1u], n0 = P.node[ii], n1 = P.node[ii + 1u];
-                        const bool a = l0 <= n0;                       // the first is a leaf
-                        const bool b2 = a ? l1 <= n0 : l0 <= n1;       // the second is a leaf
-                        const uint32_t w = (a ? l0 : n0) + (a ? (b2 ? l1 : n0) : (b2 ? l0 : n1));
-                        const uint32_t first = a ? li : n + ii;
-                        const uint32_t second = b2 ? li + (a ? 1u : 0u) : n + ii + (a ? 0u : 1u);
-                        P.node[m] = w;
-                        P.anc[0][first] = P.anc[0][second] = static_cast<uint16_t>(n + m);
-                        const uint32_t used = (a ? 1u : 0u) + (b2 ? 1u : 0u);
-                        li += used;
-                        ii += 2u - used;
-                    }
-                }
-                __syncwarp();
-                // depths by pointer jumping (parent links, the root points to itself)
-                const uint32_t nn = 2u * n - 1u, root = nn - 1u;
-                for (uint32_t k = lane; k < nn; k += 32u) {
-                    if (k == root) P.anc[0][k] = static_cast<uint16_t>(root);
-                    P.dep[0][k] = k == root ? 0u : 1u;
-                }
-                if (lane < 64u) P.bl[lane] = 0u;
-                if (lane + 32u < 64u) P.bl[lane + 32u] = 0u;
-                __syncwarp();
-                uint32_t cur = 0;
-                for (uint32_t r = 0; r < 9; ++r) {
-                    for (uint32_t k = lane; k < nn; k += 32u) {
-                        const uint32_t an = P.anc[cur][k];
-                        P.dep[cur ^ 1u][k] = static_cast<uint8_t>(P.dep[cur][k] + P.dep[cur][an]);
-                        P.anc[cur ^ 1u][k] = P.anc[cur][an];
+                // Two-queue Huffman construction: the two lightest of the leaves and
+                // internal nodes left are merged, a leaf first on equal weights,
+                // an older node before a newer one; sentinels stand for what is
+                // not there.  No new node is lighter than the first pair's sum,
+                // so all items up to that sum pair up in order, at once (an odd
+                // last one waits), and the sums at least double every other round.
+                uint32_t *srt = reinterpret_cast<uint32_t *>(P.anc[1]);
+                for (uint32_t li = 0, ii = 0, m = 0; m + 1u < n;) {
+                    const uint32_t l0 = P.leafw[li], l1 = P.leafw[li + 1u], n0 = P.node[ii], n1 = P.node[ii + 1u];
+                    const uint32_t sum = l0 <= n0 ? l0 + min(l1, n0) : n0 + min(l0, n1);
+                    auto upto = [&](const uint32_t *w, uint32_t from) {  // items from `from` on up to sum
+                        for (uint32_t c = 0;;) {
+                            const uint32_t k = from + c + lane;
+                            const uint32_t bal = __ballot_sync(kFull, k < 256u && w[k] <= sum);
+                            c += static_cast<uint32_t>(__popc(bal));
+                            if (bal != kFull) return c;
+                        }
+                    };
+                    const uint32_t nl = upto(P.leafw, li), ni = upto(P.node, ii), k = nl + ni, paired = k & ~1u;
+                    const bool leaf_last = nl && (!ni || P.leafw[li + nl - 1u] > P.node[ii + ni - 1u]);
+                    for (uint32_t j = lane; j < k; j += 32u) {  // to its rank among both
+                        const bool lf = j < nl;
+                        const uint32_t jj = lf ? j : j - nl, w = lf ? P.leafw[li + jj] : P.node[ii + jj];
+                        const uint32_t *other = lf ? P.node + ii : P.leafw + li;
+                        const uint32_t cnt = lf ? ni : nl, below = lf ? w : w + 1u;
+                        uint32_t r = 0;
+                        if (nl && ni)
+                            for (uint32_t d = 1u << highbit(max(nl, ni)); d; d >>= 1)
+                                if (r + d <= cnt && other[r + d - 1u] < below) r += d;
+                        r += jj;
+                        srt[r] = w;
+                        if (r < paired) P.anc[0][lf ? li + jj : n + ii + jj] = static_cast<uint16_t>(n + m + (r >> 1));
                     }
                     __syncwarp();
-                    cur ^= 1u;
+                    for (uint32_t j = lane; j < paired / 2u; j += 32u) P.node[m + j] = srt[2u * j] + srt[2u * j + 1u];
+                    __syncwarp();
+                    m += paired / 2u;
+                    li += nl - (k != paired && leaf_last ? 1u : 0u);
+                    ii += ni - (k != paired && !leaf_last ? 1u : 0u);
                 }
-                for (uint32_t k = lane; k < n; k += 32u) atomicAdd(&P.bl[min(static_cast<uint32_t>(P.dep[cur][k]), 63u)], 1u);
+                // depths by pointer jumping (parent links, the root points to itself)
+                const uint32_t nn = 2u * n - 1u, root = nn - 1u;
+                for (uint32_t k = lane; k < ((nn + 127u) & ~127u); k += 32u) {
+                    if (k >= root) P.anc[0][k] = static_cast<uint16_t>(root);
+                    P.dep[0][k] = k >= root ? 0u : 1u;
+                }
+                P.bl[lane] = 0u;
                 __syncwarp();
-                const uint32_t lens = __ballot_sync(kFull, P.bl[lane] != 0u), lens2 = __ballot_sync(kFull, P.bl[lane + 32u] != 0u);
-                const uint32_t maxlen = lens2 ? 32u + highbit(lens2) : highbit(lens);
-                if (lane == 0) {  // limit to 11 bits, keeping the code complete
-                    for (uint32_t i = maxlen; i > kHufMaxBits; --i) {
-                        while (P.bl[i] > 0) {
-                            uint32_t j = i - 2u;
-                            while (P.bl[j] == 0) --j;
-                            P.bl[i] -= 2u;
-                            P.bl[i - 1] += 1u;
-                            P.bl[j + 1] += 2u;
-                            P.bl[j] -= 1u;
+                uint32_t cur = 0;
+                for (bool open = true; open; cur ^= 1u) {
+                    open = false;
+                    for (uint32_t k = lane; k < nn; k += 128u) {
+                        uint32_t an[4], a2[4], d[4];
+#pragma unroll
+                        for (uint32_t u = 0; u < 4; ++u) an[u] = P.anc[cur][k + 32u * u];
+#pragma unroll
+                        for (uint32_t u = 0; u < 4; ++u) {
+                            a2[u] = P.anc[cur][an[u]];
+                            d[u] = P.dep[cur][k + 32u * u] + P.dep[cur][an[u]];
+                        }
+#pragma unroll
+                        for (uint32_t u = 0; u < 4; ++u) {
+                            P.anc[cur ^ 1u][k + 32u * u] = static_cast<uint16_t>(a2[u]);
+                            P.dep[cur ^ 1u][k + 32u * u] = static_cast<uint8_t>(d[u]);
+                            open = open || a2[u] != root;
                         }
                     }
-                    uint32_t maxb = 0;
-                    for (uint32_t L = kHufMaxBits; L >= 1u && !maxb; --L)
-                        if (P.bl[L]) maxb = L;
-                    P.start[maxb] = 0;
-                    for (uint32_t L = maxb - 1; L >= 1u; --L) P.start[L] = (P.start[L + 1] + P.bl[L + 1]) >> 1;
-                    P.start[0] = maxb;
+                    open = __any_sync(kFull, open);
+                    __syncwarp();
                 }
+                // (65536 literals: no depth above 22)
+                for (uint32_t k = lane; k < n; k += 32u) atomicAdd(&P.bl[min(static_cast<uint32_t>(P.dep[cur][k]), 31u)], 1u);
                 __syncwarp();
-                const uint32_t maxb = P.start[0];
+                // Limit to 11 bits, keeping the code complete: two leaves at level i
+                // become one at i - 1, and the deepest leaf at most at i - 2 two
+                // one level below it.  Lane L holds level L; as long as that leaf
+                // is at i - 2 itself, its whole level goes at once.
+                uint32_t lv = P.bl[lane];
+                for (uint32_t i = highbit(__ballot_sync(kFull, lv != 0u)); i > kHufMaxBits; --i) {
+                    for (uint32_t at_i; (at_i = __shfl_sync(kFull, lv, i)) != 0u;) {
+                        const uint32_t j = highbit(__ballot_sync(kFull, lv != 0u) & ((1u << (i - 1u)) - 1u));
+                        const uint32_t at_j = __shfl_sync(kFull, lv, j);
+                        const uint32_t t = j + 2u == i ? min(at_i / 2u, at_j) : 1u;
+                        if (lane == i) lv -= 2u * t;
+                        if (lane == i - 1u) lv += t;
+                        if (lane == j + 1u) lv += 2u * t;
+                        if (lane == j) lv -= t;
+                    }
+                }
+                const uint32_t maxb = highbit(__ballot_sync(kFull, lv != 0u));
+                uint32_t code0 = 0, mine = 0;  // first code of level L
+                for (uint32_t L = maxb - 1u; L >= 1u; --L) {
+                    code0 = (code0 + __shfl_sync(kFull, lv, L + 1u)) >> 1;
+                    if (lane == L) mine = code0;
+                }
+                P.bl[lane] = lv;
+                if (lane < 16u) P.start[lane] = mine;
+                __syncwarp();
                 // lengths: the longest codes to the least frequent bytes
                 for (uint32_t i = 0; i < 8; ++i) P.len[lane * 8u + i] = 0;
                 __syncwarp();
