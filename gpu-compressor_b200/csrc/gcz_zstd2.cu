@@ -1362,8 +1362,9 @@ __device__ __noinline__ void parse_segments_out(Zstd2Args a, SegSmem<kWarps> &G,
     parse_segments<kRef, kMaxWindow / kWarps>(a, G, S, win, bm, cand, seg, wi, size, lazy);
 }
 
-template <bool kRef, uint32_t kWarps>
-__global__ void __launch_bounds__(32 * kWarps, kWarps == 16 ? 3 : 1) zstd_lane_parse_kernel(Zstd2Args a) {
+// kCtas: CTAs of an SM.
+template <bool kRef, uint32_t kWarps, int kCtas>
+__global__ void __launch_bounds__(32 * kWarps, kCtas) zstd_lane_parse_kernel(Zstd2Args a) {
     constexpr uint32_t kThreads = 32u * kWarps;
     extern __shared__ __align__(128) uint8_t smem_raw[];
     SmemLayout<LaneSmem<kWarps>> &M = *reinterpret_cast<SmemLayout<LaneSmem<kWarps>> *>(smem_raw);
@@ -1570,13 +1571,13 @@ cudaError_t launch_seg_parse(const Zstd2Args &a, int num_sms, int ctas_per_sm, c
                                st);
 }
 
-template <bool kRef, uint32_t kWarps>
+template <bool kRef, uint32_t kWarps, int kCtas>
 cudaError_t launch_lane_parse(const Zstd2Args &a, int num_sms, int ctas_per_sm, cudaStream_t st) {
     constexpr uint32_t smem = sizeof(SmemLayout<LaneSmem<kWarps>>);
     static_assert(smem + 1024 <= 233472 / 3, "three CTAs per SM must fit");
     static SmemOnce smem_set{0};
-    return launch_parse_kernel(zstd_lane_parse_kernel<kRef, kWarps>, smem, 32 * kWarps, smem_set, a, num_sms,
-                               ctas_per_sm, st);
+    return launch_parse_kernel(zstd_lane_parse_kernel<kRef, kWarps, kCtas>, smem, 32 * kWarps, smem_set, a, num_sms,
+                               ctas_per_sm < kCtas ? ctas_per_sm : kCtas, st);
 }
 
 template <bool kRef>
@@ -1586,10 +1587,13 @@ cudaError_t launch_parse_ref(const Zstd2Args &a, uint32_t seg_width, int num_sms
     if (seg_width == 8192) return launch_seg_parse<kRef, 8192>(a, num_sms, ctas_per_sm, st);
     // At most one window per SM: 32 warps share it instead of 16, with all of
     // the SM's registers.  Sweep to records, 1 window 100.3 -> 89.3 us, 148
-    // windows 109.6 -> 96.6; a 4 KiB window takes the same 26.7.  From two
-    // windows per SM on the 16-warp form runs them side by side (149 windows: 119).
-    if (a.num_windows <= static_cast<uint32_t>(num_sms)) return launch_lane_parse<kRef, 32>(a, num_sms, 1, st);
-    return launch_lane_parse<kRef, 16>(a, num_sms, ctas_per_sm, st);
+    // windows 109.6 -> 96.6; a 4 KiB window takes the same 26.7.  At most two:
+    // 16 warps each, 64 registers instead of 40 and no spills, 256 windows
+    // 127.7 -> 121.4.  More: three CTAs per SM (4096 windows 1.31 ms, two 1.72).
+    const uint32_t sms = static_cast<uint32_t>(num_sms);
+    if (a.num_windows <= sms) return launch_lane_parse<kRef, 32, 1>(a, num_sms, ctas_per_sm, st);
+    if (a.num_windows <= 2u * sms) return launch_lane_parse<kRef, 16, 2>(a, num_sms, ctas_per_sm, st);
+    return launch_lane_parse<kRef, 16, 3>(a, num_sms, ctas_per_sm, st);
 }
 }  // namespace
 

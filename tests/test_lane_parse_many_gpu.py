@@ -1,5 +1,5 @@
-"""The Zstd lane parse has two forms: one for at most one window per SM, one for
-more windows.  Both against the oracle, on the data that takes its rarer paths."""
+"""The Zstd lane parse has three forms: for at most one window per SM, at most
+two, and more.  Each against the oracle, on the data that takes its rarer paths."""
 import numpy as np
 import pytest
 
@@ -9,8 +9,8 @@ from test_lane_parse_gpu import CASES
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("copies", [1, 12])
-def test_both_forms_vs_oracle(ctx, copies):
+@pytest.mark.parametrize("copies", [1, 6, 12])
+def test_each_form_vs_oracle(ctx, copies):
     files = [make(n, 7 + n, *args) for _, make, args in CASES for n in (133, 4096, 65535)]
     assert (len(files) * copies <= 148) == (copies == 1)  # 148 SMs, one window per file
     for depth in (1, 16):
