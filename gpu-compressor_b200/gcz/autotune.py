@@ -9,7 +9,7 @@ scheduled:
                         warp per segment of that many bytes
          "parse_ctas"   second-stage CTAs per SM
   LZMA2  "lzma_ctas"    second-stage CTAs per SM (the sweep is shared)
-         "lzma_threads" second-stage threads per CTA (256, 512 or 1024)
+         "lzma_threads" second-stage threads per CTA (512, or 1024: 256 for many windows)
   host   "slice_windows" windows per slice of the host-buffer pipelines
 
 tune_zstd() and tune_lzma2() time every candidate on a sample of the caller's
@@ -38,8 +38,8 @@ ZSTD_CANDIDATES = [
     for seg, ctas_list in ((4096, (3, 2)), (1024, (3, 2)), (8192, (3, 2)), (2048, (1,)))
     for ctas in ctas_list
 ]
-LZMA_CANDIDATES = [{"lzma_ctas": c, "lzma_threads": t} for t in (512, 256) for c in (3, 2, 1)] + [
-    {"lzma_ctas": c, "lzma_threads": 1024} for c in (2, 1)]
+# (1024 runs 256 threads where there are many windows and splits few over several CTAs, so a fixed 256 is left out)
+LZMA_CANDIDATES = [{"lzma_ctas": c, "lzma_threads": t} for t in (1024, 512) for c in (3, 2, 1)]
 SLICE_CANDIDATES = [256, 512, 1024, 2048]
 
 
