@@ -12,7 +12,7 @@
 // state machine over (pos, rep0, rep1, rep2), but its repeat offsets
 // (:259-275) decide a match only a few times per window.  So:
 // 1. Parse without repeat offsets.  Its state is the position alone.  The
-//    window is cut into 128-byte segments; every lane parses one at a time
+//    window is cut into 132-byte segments; every lane parses one at a time
 //    from the segment's start and pulls the next of its warp's when done.
 // 2. Link.  Where a segment's parse ends, it joins the list of the segment
 //    that holds that position: at once when that list has no match across it
@@ -27,10 +27,21 @@
 //    Mends lie side by side; one that starts inside an earlier one is dropped.
 //    Every literal run is then either checked or parsed exactly, so the
 //    sequences are the reference's by induction over the runs.
-// A window with many such runs (records with a fixed stride), or one that
-// overflows a list, takes the segment parse instead.
+// 5. Give up.  A window with more than kMostFixes such runs, with a mend that
+//    finds no end soon, or with no room for a list is parsed again after the
+//    CTA's other windows.  Where its matches lie close to one another (counters,
+//    sorted numbers, records with a fixed stride, pixels: the repeat offsets
+//    decide most of them), steps 1 and 2 are done with repeat offsets.  A
+//    segment's parse starts from {1,4,8} and joins a later segment's list at a
+//    match that both have with the same repeat offsets after it, nearly always
+//    its third.  Where matches are far apart (samples, floating-point numbers),
+//    or a segment does not join a list soon, the segment parse takes the window.
+//    Per 256 MiB, with the segment parse as the only way out and with both:
+//    32-bit counters 33.7 -> 5.8 ms, sorted numbers 23.6 -> 5.4, 20-byte
+//    records 11.1 -> 5.2, 8-byte records 12.2 -> 4.3, 3-byte pixels 5.8 -> 4.3,
+//    4-letter text (long continuations, step 2) 15.6 -> 3.9.
 //
-// Segment parse (zstd_seg_parse_kernel, and the lane parse's way out).  Each
+// Segment parse (zstd_seg_parse_kernel, and the lane parse's last way out).  Each
 // warp parses one segment of 2-8 KiB from a guessed state (the segment start,
 // repeat offsets {1,4,8}), then goes on past its end until one of its matches
 // equals a match of a later warp's list -- same start, length and offset, and
@@ -103,26 +114,38 @@ struct ParseScalars {
     uint32_t covered;
     uint32_t count;    // literal runs with a repeat-offset match found
     uint32_t mends;    // mends of the window
-    uint32_t bigs;     // continuations that took a long list
+    uint32_t chunks;   // chunks of continuations in use
+    uint32_t probe[2]; // matches and bytes of the window's mends
+    uint32_t again;    // 1 + the last window given up (0: none); each leads to the one before it
     uint32_t warp_sum[32];
     alignas(8) uint64_t bar;
 };
 
 // Lane parse.
-constexpr uint32_t kLSegW = 128, kLSegs = kMaxWindow / kLSegW;  // four bitmap words per segment
+// 33 words, so that the lanes of a warp start in different banks, and stay there
+// where the data has a short period (128 bytes: 32-bit counters 10.4 ms per 256
+// MiB against 5.8, 64-byte records 2.3 against 1.7, the benchmark's data alike).
+constexpr uint32_t kLSegW = 132, kLists = (kMaxWindow + kLSegW - 1) / kLSegW;
+constexpr uint32_t kLSegs = 512;                                // kLists, up to whole warps
 constexpr uint32_t kLCap = (kLSegW + 2) / 3;                    // matches that start their search in a segment
-constexpr uint32_t kLCont = 12;                                 // matches before a segment's parse joins a list ...
-constexpr uint32_t kLBig = 16, kLBigCap = 128;                  // ... and lists for the few that take more
-constexpr uint32_t kFixes = 256, kFixCap = 255;                 // mends per window, most matches per mend
+constexpr uint32_t kLCont = 12;                                 // continuation: 11 matches, then a chunk's number ...
+constexpr uint32_t kLChunks = 96, kLChunk = 32;                 // ... chunks of 31 more matches and the next one's number
+constexpr uint32_t kLMost = 255;                                // most matches before a segment's parse joins a list
+constexpr uint32_t kFixes = 256, kFixCap = 255;                 // runs recorded per window, most matches per mend
+constexpr uint32_t kMostFixes = 192;                            // most runs that are mended
+constexpr uint32_t kDense = 36;                                 // bytes per match below which a window counts as dense ...
+constexpr uint32_t kDenseCap = 48, kTryCap = 12;                // ... the most matches of a mend in one, and of one tried out
+constexpr uint32_t kMostSteps = 400;                            // most steps before a segment's parse with repeat offsets joins
 // Entries in a window's scratch: the segments' lists, then the continuations;
 // once the list of the whole parse is known it takes the lists' place, and
 // the mends that of the continuations.
-constexpr uint32_t kLContBase = kLSegs * kLCap;
-constexpr uint32_t kLBigBase = kLContBase + kLSegs * kLCont;
-constexpr uint32_t kLEntries = kLBigBase + kLBig * kLBigCap;
+constexpr uint32_t kLContBase = kLists * kLCap;
+constexpr uint32_t kLChunkBase = kLContBase + kLists * kLCont;
+constexpr uint32_t kLEntries = kLChunkBase + kLChunks * kLChunk;
 constexpr uint32_t kFixEntries = kLEntries - kLContBase;        // shared by a window's mends
 static_assert(kLContBase >= 21846, "the whole parse fits where the lists were");
-static_assert(kLCont + kLBigCap <= 255, "8-bit counts");
+static_assert(kLists <= kLSegs && kLSegs % 32 == 0, "whole warps of segments");
+static_assert(kLMost <= 255 && kFixCap <= 255, "8-bit counts");
 
 template <uint32_t kWarps>
 struct LaneSmem {
@@ -132,7 +155,6 @@ struct LaneSmem {
             uint8_t count[kLSegs];   // list entries
             uint8_t from[kLSegs];    // entry joined at, then the first entry on the chain
             uint8_t cont[kLSegs];    // continuation entries
-            uint16_t big[kLBig];     // segments whose continuation goes on in a list of kLBigCap entries
             uint32_t chain[kLSegs / 32];  // segments on the chain
         };
         struct {
@@ -466,15 +488,16 @@ __device__ __forceinline__ bool warp_step(const Win &w, const uint32_t *bm, Cand
 // ranges are read as aligned words; a byte of x ^ y is zero exactly when its
 // 0x80 flag survives ~(((d & 0x7F..) + 0x7F..) | d | 0x7F..), three flags in
 // a row mark a 3-byte match, and a multiply gathers each word's four flags.
-__device__ __forceinline__ uint32_t rep3_scan16(const Win &w, uint32_t q, uint32_t r) {
+template <uint32_t kWords>
+__device__ __forceinline__ uint32_t rep3_scan(const Win &w, uint32_t q, uint32_t r) {
     const uint32_t *wd = reinterpret_cast<const uint32_t *>(w.d - kPre);
     const uint32_t ax = q + kPre, ay = q - r + kPre;
     const uint32_t *px = wd + (ax >> 2), *py = wd + (ay >> 2);
     const uint32_t sx = (ax & 3u) * 8u, sy = (ay & 3u) * 8u;
-    uint32_t z[5];
+    uint32_t z[kWords + 1u];
     uint32_t xp = px[0], yp = py[0];
 #pragma unroll
-    for (uint32_t j = 0; j < 5; ++j) {
+    for (uint32_t j = 0; j <= kWords; ++j) {
         const uint32_t xn = px[j + 1], yn = py[j + 1];
         const uint32_t d = __funnelshift_r(xp, xn, sx) ^ __funnelshift_r(yp, yn, sy);
         z[j] = ~(((d & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | d | 0x7F7F7F7Fu);
@@ -483,7 +506,7 @@ __device__ __forceinline__ uint32_t rep3_scan16(const Win &w, uint32_t q, uint32
     }
     uint32_t m = 0;
 #pragma unroll
-    for (uint32_t j = 0; j < 4; ++j) {
+    for (uint32_t j = 0; j < kWords; ++j) {
         const uint32_t e = z[j] & __funnelshift_r(z[j], z[j + 1], 8) & __funnelshift_r(z[j], z[j + 1], 16);
         m |= ((e * 0x00204081u) >> 28) << (4u * j);
     }
@@ -989,12 +1012,14 @@ __device__ __forceinline__ uint32_t extend_lanes(const Win &w, uint32_t c, uint3
     return k;
 }
 
-// The match a parse without repeat offsets takes at its first hash-match
-// position f (lanes with act): extended, with the lazy step (:278-307).
+// The match a parse takes at its event position f (lanes with act): a hash
+// match, or with kRep one at repeat offset rep (0: hash match), extended, with
+// the lazy step (:278-307).
+template <bool kRep>
 __device__ __forceinline__ void lane_match(const Win &w, const uint32_t *bm, const uint16_t *cand, uint32_t size,
-                                           bool lazy, bool act, uint32_t f, Match &m) {
+                                           bool lazy, bool act, uint32_t f, uint32_t rep, Match &m) {
     const uint32_t fc = act ? f : 0u;
-    const uint32_t c0 = cand[fc], c1 = cand[fc + 1u];
+    const uint32_t c0 = kRep && act && rep ? fc - rep : cand[fc], c1 = cand[fc + 1u];
     // skipped when it is the same match one byte on, which is never longer (warp_step)
     const bool ltry = act && lazy && fc + 4u < size && bm_bit(bm, fc + 1u) && c1 != c0 + 1u;
     m.start = fc;
@@ -1011,7 +1036,7 @@ __device__ __forceinline__ void lane_match(const Win &w, const uint32_t *bm, con
     }
 }
 
-// List entry of a match found at hash position f: {start | (ml-3) << 16,
+// List entry of a match found at position f: {start | (ml-3) << 16,
 // offset | lazy << 16}, lazy: the match starts at f + 1.
 __device__ __forceinline__ uint2 lane_entry(const Match &m, uint32_t f) {
     return make_uint2(m.start | ((m.len - kMinMatch) << 16), m.off | ((m.start - f) << 16));
@@ -1025,8 +1050,41 @@ __device__ __forceinline__ void reps_before(const uint2 *list, uint32_t i, uint3
     c = i >= 3u ? list[i - 3u].y & 0xFFFFu : (i == 2u ? 1u : (i == 1u ? 4u : 8u));
 }
 
-// Step 1: every lane parses segments of its warp's pool without repeat offsets.
-template <uint32_t kWarps>
+// The next positions of a parse with repeat offsets r0, r1, r2, from p on (below
+// stop): ev, the position of the first event among p .. p+7 and its repeat
+// offset (0: a hash match); else a position reached, up to 64 further on.
+__device__ __forceinline__ uint32_t rep_event(const Win &w, const uint32_t *bm, uint32_t p, uint32_t stop, uint32_t r0,
+                                              uint32_t r1, uint32_t r2, uint32_t &rep, bool &ev) {
+    const uint32_t n = min(stop - p, 8u), valid = (1u << n) - 1u;
+    const uint32_t H = __funnelshift_r(bm[p >> 5], bm[(p >> 5) + 1u], p) & valid;  // (the shift counts modulo 32)
+    uint32_t hit[3];
+#pragma unroll
+    for (uint32_t k = 0; k < 3u; ++k) {
+        const uint32_t r = k == 0u ? r0 : (k == 1u ? r1 : r2);
+        const uint32_t skip = r > p ? r - p : 0u;  // positions whose source is before the window
+        hit[k] = skip < 8u ? rep3_scan<2>(w, p, r) & (valid << skip) : 0u;
+    }
+    const uint32_t any = H | ((hit[0] | hit[1] | hit[2]) & valid);
+    ev = any != 0u;
+    rep = 0;
+    if (ev) {
+        const uint32_t k = static_cast<uint32_t>(__ffs(any)) - 1u;
+        if (!((H >> k) & 1u)) rep = (hit[0] >> k) & 1u ? r0 : ((hit[1] >> k) & 1u ? r1 : r2);
+        return p + k;
+    }
+    p += n;
+    const uint32_t ro[3] = {r0, r1, r2};
+#pragma unroll 1
+    for (uint32_t i = 0; i < 4u && p + 16u <= stop && max(max(r0, r1), r2) <= p; ++i) {
+        if ((__funnelshift_r(bm[p >> 5], bm[(p >> 5) + 1u], p) & 0xFFFFu) || rep3_any16(w, p, ro, 16u)) break;
+        p += 16u;
+    }
+    return p;
+}
+
+// Step 1: every lane parses segments of its warp's pool, without repeat offsets
+// or (kRep) with them, from {1,4,8}.
+template <bool kRep, uint32_t kWarps>
 __device__ __forceinline__ void lane_parse(LaneSmem<kWarps> &N, const Win &win, const uint32_t *bm, const uint16_t *cand,
                                            uint2 *seg, uint32_t size, uint32_t nact, bool lazy) {
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5, lt = lanemask_lt();
@@ -1036,7 +1094,7 @@ __device__ __forceinline__ void lane_parse(LaneSmem<kWarps> &N, const Win &win, 
     uint32_t next = warp * pool;
     const uint32_t end = next + pool < nact ? next + pool : nact;
     bool has = false;
-    uint32_t s = 0, p = 0, n = 0;
+    uint32_t s = 0, p = 0, n = 0, r0 = 0, r1 = 0, r2 = 0;
     for (;;) {
         const uint32_t need = __ballot_sync(kFull, !has);
         if (need && next < end) {
@@ -1046,28 +1104,70 @@ __device__ __forceinline__ void lane_parse(LaneSmem<kWarps> &N, const Win &win, 
                 s = mine;
                 p = s * kLSegW;
                 n = 0;
+                if constexpr (kRep) r0 = 1u, r1 = 4u, r2 = 8u;
             }
             next += static_cast<uint32_t>(__popc(need));
         }
         if (!__any_sync(kFull, has)) break;
         const uint32_t seg_end = (s + 1u) * kLSegW;
-        const uint32_t f = has ? next_bit(bm, p, seg_end) : seg_end;
-        const bool ev = has && f < seg_end;
+        uint32_t f, rep = 0;
+        bool ev = false;
+        if constexpr (kRep) {
+            f = has ? rep_event(win, bm, p, min(seg_end, size - 3u), r0, r1, r2, rep, ev) : 0u;
+        } else {
+            f = has ? next_bit(bm, p, seg_end) : seg_end;
+            ev = has && f < seg_end;
+        }
         if (__any_sync(kFull, ev)) {
             Match m;
-            lane_match(win, bm, cand, size, lazy, ev, f, m);
+            lane_match<kRep>(win, bm, cand, size, lazy, ev, f, rep, m);
             if (ev) {
                 seg[s * kLCap + n] = lane_entry(m, f);
                 ++n;
                 p = m.start + m.len;
+                if constexpr (kRep) r2 = r1, r1 = r0, r0 = m.off;
             }
         }
-        if (has && (!ev || p >= seg_end)) {  // no match left, or the last one ends past the segment
+        if constexpr (kRep) {
+            if (has && !ev) p = f;
+            if (has && p >= min(seg_end, size - 3u)) {
+                N.count[s] = static_cast<uint8_t>(n);
+                N.link[s] = static_cast<uint16_t>(p > seg_end ? p - seg_end : 0u);
+                has = false;
+            }
+        } else if (has && (!ev || p >= seg_end)) {  // no match left, or the last one ends past the segment
             N.count[s] = static_cast<uint8_t>(n);
             N.link[s] = static_cast<uint16_t>(ev ? p - seg_end : 0u);
             has = false;
         }
     }
+}
+
+// Where a segment's continuation puts its next match.
+struct ContSlot {
+    uint32_t cur, end;  // next slot, the slot of its block's last entry (which leads to the next chunk)
+    __device__ __forceinline__ explicit ContSlot(uint32_t s) : cur(kLContBase + s * kLCont), end(cur + kLCont - 1u) {}
+    // false when there is no room for it
+    __device__ __forceinline__ bool put(ParseScalars &S, uint2 *seg, const uint2 &e) {
+        if (cur == end) {
+            const uint32_t c = atomicAdd(&S.chunks, 1u);
+            if (c >= kLChunks) return false;
+            seg[end].x = c;
+            cur = kLChunkBase + c * kLChunk;
+            end = cur + kLChunk - 1u;
+        }
+        seg[cur++] = e;
+        return true;
+    }
+};
+// Slot of match i of segment s's continuation.
+__device__ __forceinline__ uint32_t cont_slot(const uint2 *seg, uint32_t s, uint32_t i) {
+    uint32_t at = kLContBase + s * kLCont, n = kLCont - 1u;  // block and the matches it holds
+    for (; i >= n; n = kLChunk - 1u) {
+        i -= n;
+        at = kLChunkBase + seg[at + n].x * kLChunk;
+    }
+    return at + i;
 }
 
 // Step 2, first half: where each segment's parse joins a later segment's list.
@@ -1079,7 +1179,8 @@ __device__ __forceinline__ void lane_link(LaneSmem<kWarps> &N, ParseScalars &S, 
 #pragma unroll 1
     for (uint32_t s = tid; s < kLSegs; s += 32u * kWarps) {
         uint32_t E = (s + 1u) * kLSegW + (s < nact ? N.link[s] : 0u);  // position the parse has reached
-        uint32_t t = kNoWarp, j = 0, cn = 0, big = 0;
+        uint32_t t = kNoWarp, j = 0, cn = 0;
+        ContSlot slot(s);
         bool run = s < nact;
         for (;;) {
             if (run && E >= lim_pos) run = false;  // the parse is over: no link
@@ -1103,22 +1204,87 @@ __device__ __forceinline__ void lane_link(LaneSmem<kWarps> &N, ParseScalars &S, 
             const bool ev = run && f < lim_pos;
             if (run && !ev) run = false;
             Match m;
-            lane_match(win, bm, cand, size, lazy, ev, f, m);
-            if (ev && cn == kLCont) {  // goes on in a long list
-                big = atomicAdd(&S.bigs, 1u);
-                if (big < kLBig) N.big[big] = static_cast<uint16_t>(s);
-            }
-            if (ev && (cn == kLCont + kLBigCap || (cn >= kLCont && big >= kLBig))) {
-                atomicOr(&S.flags, 4u);
-                run = false;
-            } else if (ev) {
-                seg[cn < kLCont ? kLContBase + s * kLCont + cn : kLBigBase + big * kLBigCap + (cn - kLCont)] =
-                    lane_entry(m, f);
-                ++cn;
-                E = m.start + m.len;
+            lane_match<false>(win, bm, cand, size, lazy, ev, f, 0u, m);
+            if (ev) {
+                if (cn == kLMost || !slot.put(S, seg, lane_entry(m, f))) {
+                    atomicOr(&S.flags, 4u);
+                    run = false;
+                } else {
+                    ++cn;
+                    E = m.start + m.len;
+                }
             }
         }
         N.link[s] = static_cast<uint16_t>(t);
+        N.from[s] = static_cast<uint8_t>(j);
+        N.cont[s] = static_cast<uint8_t>(cn);
+        if (s >= nact) N.count[s] = 0;
+    }
+}
+
+// The same with repeat offsets: a segment's parse joins a later segment's list
+// at a match that both have, with the same repeat offsets after it.
+template <uint32_t kWarps>
+__device__ __forceinline__ void lane_link_reps(LaneSmem<kWarps> &N, ParseScalars &S, const Win &win, const uint32_t *bm,
+                                               const uint16_t *cand, uint2 *seg, uint32_t size, uint32_t nact,
+                                               uint32_t lim_pos, bool lazy) {
+#pragma unroll 1
+    for (uint32_t s = threadIdx.x; s < kLSegs; s += 32u * kWarps) {
+        bool run = s < nact;
+        uint32_t p = (s + 1u) * kLSegW, r0 = 0, r1 = 0, r2 = 0;
+        if (run) {
+            p += N.link[s];
+            reps_before(seg + s * kLCap, N.count[s], r0, r1, r2);
+        }
+        uint32_t link = kNoWarp, t = kNoWarp, j = 0, cn = 0, steps = 0, rep = 0, f = 0;
+        bool ev = false;
+        ContSlot slot(s);
+        for (;;) {
+            // (the parse is over, or some segment has found no place to join)
+            if (p >= lim_pos || (*const_cast<volatile uint32_t *>(&S.flags) & 4u)) run = false;
+            const uint32_t runs = __ballot_sync(kFull, run);
+            if (!runs) break;
+            if (run && !ev) {
+                f = rep_event(win, bm, p, lim_pos, r0, r1, r2, rep, ev);
+                if (!ev) p = f;
+                if (++steps > kMostSteps) atomicOr(&S.flags, 4u);
+            }
+            ev = ev && run;
+            // (a match takes several times as long as a step)
+            if (2u * __popc(__ballot_sync(kFull, ev)) < __popc(runs)) continue;
+            Match m;
+            lane_match<true>(win, bm, cand, size, lazy, ev, f, rep, m);
+            if (ev) {
+                ev = false;
+                const uint2 e = lane_entry(m, f);
+                if (f / kLSegW != t) {
+                    t = f / kLSegW;
+                    j = 0;
+                }
+                const uint2 *tl = seg + t * kLCap;
+                const uint32_t tc = N.count[t];
+                while (j < tc && (tl[j].x & 0xFFFFu) < m.start) ++j;
+                if (j < tc && tl[j].x == e.x && (tl[j].y & 0xFFFFu) == m.off) {
+                    uint32_t a, b, c;
+                    reps_before(tl, j, a, b, c);
+                    if (a == r0 && b == r1) {
+                        link = t;
+                        run = false;
+                    }
+                }
+                if (run) {
+                    if (cn == kLMost || !slot.put(S, seg, e)) {
+                        atomicOr(&S.flags, 4u);
+                        run = false;
+                    } else {
+                        ++cn;
+                        p = m.start + m.len;
+                        r2 = r1, r1 = r0, r0 = m.off;
+                    }
+                }
+            }
+        }
+        N.link[s] = static_cast<uint16_t>(link);
         N.from[s] = static_cast<uint8_t>(j);
         N.cont[s] = static_cast<uint8_t>(cn);
         if (s >= nact) N.count[s] = 0;
@@ -1173,6 +1339,38 @@ __device__ __forceinline__ uint32_t lane_chain(LaneSmem<kWarps> &N, ParseScalars
     return total;
 }
 
+// The chain's entries (the first `total`) in order into the output slots, then
+// from there to the front of the scratch, over the lists.
+template <bool kRef, uint32_t kWarps>
+__device__ __forceinline__ void lane_gather(const Zstd2Args &a, const LaneSmem<kWarps> &N, uint2 *seg, uint32_t wi,
+                                            uint32_t total) {
+    const uint32_t tid = threadIdx.x;
+    constexpr uint32_t kThreads = 32u * kWarps;
+    uint2 *pk = kRef ? nullptr : a.packed + static_cast<uint64_t>(wi) * a.max_seqs;
+    uint32_t *rk = kRef ? a.ref_seqs + static_cast<uint64_t>(wi) * a.max_seqs * 3u : nullptr;
+    for (uint32_t s = tid >> 2; s < kLSegs; s += kThreads / 4u) {
+        if (!((N.chain[s >> 5] >> (s & 31u)) & 1u)) continue;
+        const uint32_t from = N.from[s], ns = N.count[s], nc = N.cont[s];
+        for (uint32_t i = from + (tid & 3u); i < ns + nc; i += 4u) {
+            const uint32_t o = N.link[s] + (i - from);
+            if (o >= total) break;
+            const uint2 e = seg[i < ns ? s * kLCap + i : cont_slot(seg, s, i - ns)];
+            if constexpr (kRef) {
+                rk[3u * o] = e.x;
+                rk[3u * o + 1u] = e.y;
+            } else {
+                pk[o] = e;
+            }
+        }
+    }
+    __syncthreads();
+    for (uint32_t i = tid; i < total; i += kThreads) {
+        if constexpr (kRef) seg[i] = make_uint2(rk[3u * i], rk[3u * i + 1u]);
+        else seg[i] = pk[i];
+    }
+    __syncthreads();
+}
+
 // Step 3: runs of literals in which a repeat offset matches on 3 bytes
 // (zstd_compress.cu:259-275), into N.fix.run (unsorted, repeats possible);
 // S.count counts them.  Run i lies before entry i of the list, the last one
@@ -1207,6 +1405,7 @@ __device__ __forceinline__ void lane_check(LaneSmem<kWarps> &N, ParseScalars &S,
         }
         const uint32_t T = __shfl_sync(kFull, x, 31), before = x - nt;
         const uint32_t span = lo | (hi << 16), r12 = r1 | (r2 << 16);  // hi <= 65533
+        bool found = false;
         for (uint32_t b = warp % team * 32u; b < T; b += team * 32u) {
             const uint32_t t = b + lane;
             uint32_t o = 0;  // the run of task t: the first lane whose inclusive count is above t
@@ -1230,7 +1429,7 @@ __device__ __forceinline__ void lane_check(LaneSmem<kWarps> &N, ParseScalars &S,
                     for (uint32_t v = 0; v < 3u; ++v) {
                         const uint32_t r = v == 0u ? ro[0] : (v == 1u ? ro[1] : ro[2]);
                         const uint32_t skip = r > q0 ? r - q0 : 0u;
-                        if (skip < 16u) any |= rep3_scan16(win, q0, r) & (0xFFFFu << skip);
+                        if (skip < 16u) any |= rep3_scan<4>(win, q0, r) & (0xFFFFu << skip);
                     }
                     hit = (any & upto) != 0u;
                 }
@@ -1238,6 +1437,7 @@ __device__ __forceinline__ void lane_check(LaneSmem<kWarps> &N, ParseScalars &S,
             if (__any_sync(kFull, hit)) {
                 const uint32_t po = __shfl_up_sync(kFull, o, 1);
                 const bool ph = __shfl_up_sync(kFull, hit ? 1u : 0u, 1) != 0u;
+                found = true;
                 if (hit && !(lane > 0u && ph && po == o)) {
                     const uint32_t at = atomicAdd(&S.count, 1u);
                     if (at < kFixes) {
@@ -1247,6 +1447,8 @@ __device__ __forceinline__ void lane_check(LaneSmem<kWarps> &N, ParseScalars &S,
                 }
             }
         }
+        // too many to mend
+        if (found && __any_sync(kFull, *const_cast<volatile uint32_t *>(&S.count) > kMostFixes)) return;
     }
 }
 
@@ -1323,6 +1525,7 @@ __device__ __noinline__ void mend_run(LaneSmem<kWarps> &N, ParseScalars &S, Win 
     while (st.p + 3u < size) {
         const uint32_t *ahead = bm + (st.p >> 5);
         if ((ahead[1] | ahead[2] | ahead[3]) == 0u) st.p = skip_literals(win, bm, lim_pos, st);
+        if (__any_sync(kFull, *const_cast<volatile uint32_t *>(&S.flags) & 4u)) break;  // another one gave up
         Match m;
         if (!warp_step(win, bm, cb, size, lazy, st, m)) continue;
         for (;;) {  // first entry with start >= m.start
@@ -1342,7 +1545,7 @@ __device__ __noinline__ void mend_run(LaneSmem<kWarps> &N, ParseScalars &S, Win 
                 break;
             }
         }
-        if (n == cap) {
+        if (n == cap || (n == kDenseCap && m.start - N.fix.pos[r] < kDenseCap * kDense)) {
             if (lane == 0) atomicOr(&S.flags, 4u);
             break;
         }
@@ -1352,6 +1555,8 @@ __device__ __noinline__ void mend_run(LaneSmem<kWarps> &N, ParseScalars &S, Win 
     if (lane == 0) {
         N.fix.meet[r] = static_cast<uint16_t>(meet);
         N.fix.len[r] = static_cast<uint8_t>(n);
+        atomicAdd(&S.probe[0], n);
+        atomicAdd(&S.probe[1], st.p - N.fix.pos[r]);
     }
 }
 
@@ -1360,6 +1565,45 @@ __device__ __noinline__ void parse_segments_out(Zstd2Args a, SegSmem<kWarps> &G,
                                                 const uint32_t *bm, const uint16_t *cand, uint2 *seg, uint32_t wi,
                                                 uint32_t size, bool lazy) {
     parse_segments<kRef, kMaxWindow / kWarps>(a, G, S, win, bm, cand, seg, wi, size, lazy);
+}
+
+// Steps 1 and 2 with repeat offsets, and the output (whole CTA, S.flags clear):
+// a segment's parse starts from {1,4,8} and has the state of the parse before
+// it after a few matches.  False, with S.flags clear, where a segment does not
+// join a list soon.
+template <bool kRef, uint32_t kWarps>
+__device__ __noinline__ bool parse_lanes_reps(Zstd2Args a, LaneSmem<kWarps> &N, ParseScalars &S, Win win,
+                                              const uint32_t *bm, const uint16_t *cand, uint2 *seg, uint32_t wi,
+                                              uint32_t size, bool lazy) {
+    const uint32_t tid = threadIdx.x;
+    const uint32_t lim_pos = size - 3u, nact = (lim_pos + kLSegW - 1u) / kLSegW;  // (a match was found: size > 3)
+    lane_parse<true>(N, win, bm, cand, seg, size, nact, lazy);
+    __syncthreads();
+    lane_link_reps(N, S, win, bm, cand, seg, size, nact, lim_pos, lazy);
+    __syncthreads();
+    if (S.flags & 4u) {
+        __syncthreads();
+        if (tid == 0) S.flags = 0;
+        __syncthreads();
+        return false;
+    }
+    uint32_t total = lane_chain(N, S, true);
+    __syncthreads();
+    if (total > a.max_seqs) total = a.max_seqs;
+    lane_gather<kRef>(a, N, seg, wi, total);
+    uint32_t cov = 0;
+    for (uint32_t x = tid; x < total; x += 32u * kWarps) {
+        const uint2 e = seg[x];
+        cov += (e.x >> 16) + kMinMatch;
+        write_seq<kRef>(a, wi, x, (e.x & 0xFFFFu) - (x ? entry_end(seg[x - 1u]) : 0u), e.x >> 16, e.y & 0xFFFFu);
+    }
+    if (kRef && cov) atomicAdd(&S.covered, cov);
+    if (tid == 0) a.seq_counts[wi] = total;
+    if (a.lit_counts) {
+        __syncthreads();
+        if (tid == 0) a.lit_counts[wi] = size - S.covered;
+    }
+    return true;
 }
 
 // kCtas: CTAs of an SM.
@@ -1375,6 +1619,7 @@ __global__ void __launch_bounds__(32 * kWarps, kCtas) zstd_lane_parse_kernel(Zst
     if (tid == 0) {
         mbar_init(&S.bar, 1);
         fence_mbar_init();
+        S.again = 0;
     }
     for (uint32_t i = tid; i < kPre / 4; i += kThreads) reinterpret_cast<uint32_t *>(M.data)[i] = 0u;
     const Win win{M.data + kPre};
@@ -1390,7 +1635,8 @@ __global__ void __launch_bounds__(32 * kWarps, kCtas) zstd_lane_parse_kernel(Zst
             S.flags = 0;
             S.covered = 0;
             S.count = 0;
-            S.bigs = 0;
+            S.chunks = 0;
+            S.probe[0] = S.probe[1] = 0;
         }
         __syncthreads();
         if (warp == 0) {
@@ -1404,7 +1650,7 @@ __global__ void __launch_bounds__(32 * kWarps, kCtas) zstd_lane_parse_kernel(Zst
 
         const uint32_t lim_pos = size > 3u ? size - 3u : 0u;  // positions q < lim_pos can start a match
         const uint32_t nact = (lim_pos + kLSegW - 1u) / kLSegW;
-        lane_parse(N, win, M.bm, cand, seg, size, nact, lazy);
+        lane_parse<false>(N, win, M.bm, cand, seg, size, nact, lazy);
         __syncthreads();
         lane_link(N, S, win, M.bm, cand, seg, size, nact, lim_pos, lazy);
         __syncthreads();
@@ -1412,53 +1658,31 @@ __global__ void __launch_bounds__(32 * kWarps, kCtas) zstd_lane_parse_kernel(Zst
         __syncthreads();
         const bool capped = total > a.max_seqs;
         if (capped) total = a.max_seqs;
-        // The chain's entries in order into the output slots, then from there
-        // to the front of the scratch, over the lists.
-        uint2 *pk = kRef ? nullptr : a.packed + static_cast<uint64_t>(wi) * a.max_seqs;
-        uint32_t *rk = kRef ? a.ref_seqs + static_cast<uint64_t>(wi) * a.max_seqs * 3u : nullptr;
-        for (uint32_t s = tid >> 2; s < kLSegs; s += kThreads / 4u) {
-            if (!((N.chain[s >> 5] >> (s & 31u)) & 1u)) continue;
-            const uint32_t from = N.from[s], ns = N.count[s], nc = N.cont[s];
-            uint32_t big = 0;
-            if (nc > kLCont)
-                while (N.big[big] != s) ++big;  // a segment with more than kLCont entries has a long list
-            for (uint32_t i = from + (tid & 3u); i < ns + nc; i += 4u) {
-                const uint32_t o = N.link[s] + (i - from);
-                if (o >= total) break;
-                const uint2 e = seg[i < ns            ? s * kLCap + i
-                                    : i < ns + kLCont ? kLContBase + s * kLCont + (i - ns)
-                                                      : kLBigBase + big * kLBigCap + (i - ns - kLCont)];
-                if constexpr (kRef) {
-                    rk[3u * o] = e.x;
-                    rk[3u * o + 1u] = e.y;
-                } else {
-                    pk[o] = e;
-                }
-            }
-        }
-        __syncthreads();
-        for (uint32_t i = tid; i < total; i += kThreads) {
-            if constexpr (kRef) seg[i] = make_uint2(rk[3u * i], rk[3u * i + 1u]);
-            else seg[i] = pk[i];
-        }
-        __syncthreads();
+        lane_gather<kRef>(a, N, seg, wi, total);
         lane_check(N, S, win, seg, total, capped ? 0u : lim_pos);
         __syncthreads();
         uint32_t nfix = S.count, fcap = 0;
         if (nfix > 0u) {
-            if (capped || nfix > kFixes) {  // (uniform over the CTA)
-                if (tid == 0) S.flags = 4u;
-            } else {
+            const bool many = capped || nfix > kMostFixes;  // (uniform over the CTA)
+            // Too many: a few are tried out, unless the entries tell that the window is dense.
+            uint32_t n = capped || (total && entry_end(seg[total - 1u]) < total * kDense) ? 0u : kWarps;
+            fcap = kTryCap;
+            if (!many) {
                 if (warp == 0) {
                     nfix = sort_runs(N, nfix);
                     if (lane == 0) S.mends = nfix;
                 }
                 __syncthreads();
                 nfix = S.mends;
+                n = nfix;
                 fcap = kFixEntries / nfix < kFixCap ? kFixEntries / nfix : kFixCap;
-                for (uint32_t r = warp; r < nfix; r += kWarps)
-                    mend_run(N, S, win, M.bm, cand, seg, size, lazy, total, r, fcap);
-                __syncthreads();
+            }
+            for (uint32_t r = warp; r < n; r += kWarps)
+                mend_run(N, S, win, M.bm, cand, seg, size, lazy, total, r, fcap);
+            __syncthreads();
+            if (many) {
+                if (tid == 0) S.flags |= 4u;
+            } else {
                 if (tid == 0) {  // drop the mends that start inside an earlier one
                     uint32_t kept = 0;
                     int32_t shift = 0;
@@ -1481,10 +1705,13 @@ __global__ void __launch_bounds__(32 * kWarps, kCtas) zstd_lane_parse_kernel(Zst
             nfix = S.mends;
         }
         if (S.flags & 4u) {
-            __syncthreads();
-            if (tid == 0) S.flags = 0u;
-            __syncthreads();
-            parse_segments_out<kRef, kWarps>(a, N.seg, S, win, M.bm, cand, seg, wi, size, lazy);
+            if (tid == 0) {  // parsed again at the end
+                const bool dense = S.probe[1] < S.probe[0] * kDense ||
+                                   (total && entry_end(seg[total - 1u]) < total * kDense);
+                seg[a.seg_stride - 1u] = make_uint2(S.again, dense ? 1u : 0u);
+                S.again = wi + 1u;
+                a.seq_counts[wi] = 0u;
+            }
             continue;
         }
         const uint32_t out_n = nfix ? S.total : total;
@@ -1531,6 +1758,36 @@ __global__ void __launch_bounds__(32 * kWarps, kCtas) zstd_lane_parse_kernel(Zst
             if (tid == 0) a.lit_counts[wi] = size - S.covered;
         }
     }
+    // The windows given up, here and not above: a call in that loop costs every
+    // window registers (256 MiB of the benchmark's data 1.36 ms against 1.31).
+    __syncthreads();
+    for (uint32_t w = S.again; w;) {
+        const uint32_t wi = w - 1u;
+        uint64_t start;
+        uint32_t size;
+        window_of(a, wi, start, size);
+        const uint16_t *cand = a.cand + start;
+        uint2 *seg = a.seg + static_cast<uint64_t>(wi) * a.seg_stride;
+        const uint2 l = seg[a.seg_stride - 1u];
+        __syncthreads();
+        if (tid == 0) {
+            S.flags = 0;
+            S.covered = 0;
+            S.chunks = 0;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            if (!stage_window(M.data + kPre, a.src + start, size, &S.bar, parity, a.status) && lane == 0)
+                S.flags = 2u;
+        }
+        __syncthreads();
+        if (S.flags & 2u) return;
+        verify_window<kWarps>(win, M.bm, cand, size);
+        __syncthreads();
+        if (l.y == 0u || !parse_lanes_reps<kRef, kWarps>(a, N, S, win, M.bm, cand, seg, wi, size, lazy))
+            parse_segments_out<kRef, kWarps>(a, N.seg, S, win, M.bm, cand, seg, wi, size, lazy);
+        w = l.x;
+    }
 }
 
 }  // namespace
@@ -1540,7 +1797,7 @@ __global__ void __launch_bounds__(32 * kWarps, kCtas) zstd_lane_parse_kernel(Zst
 template <uint32_t SegW>
 constexpr uint32_t seg_entries() { return SegCfg<SegW>::kSegs * SegCfg<SegW>::kLaneCap; }
 constexpr uint32_t kSegStride = []() constexpr {
-    uint32_t m = kLEntries;
+    uint32_t m = kLEntries + 1;  // (the last one leads from a window given up to the one before it)
     if (seg_entries<2048>() > m) m = seg_entries<2048>();
     if (seg_entries<4096>() > m) m = seg_entries<4096>();
     if (seg_entries<8192>() > m) m = seg_entries<8192>();
