@@ -643,11 +643,21 @@ int zstd_host_direct(gcz_ctx *c, const uint8_t *src, size_t n, uint32_t search_d
     uint32_t *h_status = reinterpret_cast<uint32_t *>(h);
     uint64_t *h_off = reinterpret_cast<uint64_t *>(h + 16);
     uint8_t *h_rec = h + off_bytes;
-    GCZ_CUDA(c, cudaMemcpyAsync(sl.in.p, src, n, cudaMemcpyHostToDevice, sl.st));
-    if ((r = zstd_device_core(c, sl.sc, static_cast<const uint8_t *>(sl.in.p), n, search_depth, h_rec, cap, h_off,
-                              sl.st, nullptr, 0, rec_bytes == 8, h_status)) != GCZ_OK)
+    auto run = [&]() -> int {
+        GCZ_CUDA(c, cudaMemcpyAsync(sl.in.p, src, n, cudaMemcpyHostToDevice, sl.st));
+        const int r = zstd_device_core(c, sl.sc, static_cast<const uint8_t *>(sl.in.p), n, search_depth, h_rec, cap,
+                                       h_off, sl.st, nullptr, 0, rec_bytes == 8, h_status);
+        if (r != GCZ_OK) return r;
+        GCZ_CUDA(c, cudaStreamSynchronize(sl.st));
+        return GCZ_OK;
+    };
+    if ((r = run()) != GCZ_OK) {  // the copy and some kernels may be queued: src is the caller's again on return
+        std::string why;
+        why.swap(c->err);
+        drain_slots(c);
+        c->err.swap(why);
         return r;
-    GCZ_CUDA(c, cudaStreamSynchronize(sl.st));
+    }
     if (*h_status) {
         GCZ_CUDA(c, cudaMemsetAsync(c->d_status, 0, 4, sl.st));
         GCZ_CUDA(c, cudaStreamSynchronize(sl.st));

@@ -1,0 +1,60 @@
+"""Host code of the library against a fake CUDA runtime (no GPU): whichever CUDA
+call fails, a call returns with no copy of the caller's buffers still pending."""
+import ctypes
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "gpu-compressor_b200", "csrc")
+FAKE = os.path.join(ROOT, "tests", "fake_cuda", "fake_cuda.cpp")
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    d = tmp_path_factory.mktemp("fake_cuda")
+    nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+    out = str(d / "libgcz_host.so")
+    subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=compute_100a", "-O1", "-std=c++17", "-cudart", "none",
+                    "-shared", "-Xlinker", "-Bsymbolic", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr", "-I", os.path.join(ROOT, "include"),
+                    "-I", CSRC, os.path.join(CSRC, "gcz_api.cu"), FAKE, "-o", out, "-lpthread"], check=True)
+    L = ctypes.CDLL(out)
+    vp, sz = ctypes.c_void_p, ctypes.c_size_t
+    L.gcz_create.argtypes = [ctypes.c_int, ctypes.POINTER(vp)]
+    L.gcz_destroy.argtypes = [vp]
+    for f in (L.gcz_zstd_match_find, L.gcz_zstd_match_find_packed):
+        f.argtypes = [vp, vp, sz, ctypes.c_uint32, vp, sz, vp]
+    L.fake_fail_at.argtypes = [ctypes.c_long]
+    L.fake_calls.restype = ctypes.c_long
+    L.fake_pending.argtypes, L.fake_pending.restype = [vp, sz], ctypes.c_long
+    return L
+
+
+@pytest.mark.parametrize("packed", [False, True])
+@pytest.mark.parametrize("n", [1, 4096, 200_003, 262_144])
+def test_small_call_leaves_nothing_pending(lib, n, packed):
+    src = np.zeros(n, np.uint8)
+    seqs = np.zeros(n * 4 + 16, np.uint32)
+    offsets = np.zeros(8, np.uint64)
+    call = lib.gcz_zstd_match_find_packed if packed else lib.gcz_zstd_match_find
+
+    def run(fail_at):
+        h = ctypes.c_void_p()
+        lib.fake_fail_at(0)
+        assert lib.gcz_create(0, ctypes.byref(h)) == 0
+        lib.fake_fail_at(fail_at)
+        rc = call(h, src.ctypes.data, n, 16, seqs.ctypes.data, n, offsets.ctypes.data)
+        calls = lib.fake_calls()
+        lib.fake_fail_at(0)
+        left = [lib.fake_pending(a.ctypes.data, a.nbytes) for a in (src, seqs, offsets)]
+        lib.gcz_destroy(h)
+        return rc, calls, left
+
+    rc, calls, left = run(0)
+    assert rc == 0 and left == [0, 0, 0] and calls > 5
+    for k in range(1, calls + 1):
+        rc, _, left = run(k)
+        assert rc != 0, k
+        assert left == [0, 0, 0], k
