@@ -116,3 +116,36 @@ def test_not_slower_than_segment_parse(ctx, kind, windows):
         assert best() <= 1.25 * min(segments)
     finally:
         ctx.set_option("parse_seg", was)
+
+
+def test_sequence_section_of_two_distances(ctx):
+    """Encoding a window whose sequences use two distances throughout (the third
+    of the repeat history stays from its start) is no slower than one with
+    three (same lengths, on the same GPU)."""
+    import torch as t
+
+    ns, n = 16000, 65536
+    rng = np.random.default_rng(1)
+    src = t.from_numpy(rng.integers(0, 256, n, dtype=np.uint8)).cuda()
+    offs = t.tensor([0, ns], dtype=t.int64, device="cuda")
+    out = t.zeros(2 * n, dtype=t.uint8, device="cuda")
+    fo = t.zeros(2, dtype=t.int64, device="cuda")
+    st = t.cuda.current_stream().cuda_stream
+
+    def best(off):
+        s = np.zeros((ns, 4), np.uint32)  # offset, literals, match length
+        s[:, 0], s[:, 1], s[:, 2] = np.minimum(off, 1 + 4 * np.arange(ns)), 1, 3
+        d = t.from_numpy(s.view(np.int32)).cuda()
+        ms = []
+        for _ in range(8):
+            a, b = (t.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            ctx.zstd_encode_frames_device(src.data_ptr(), n, d.data_ptr(), offs.data_ptr(), out.data_ptr(), 2 * n,
+                                          fo.data_ptr(), st)
+            b.record()
+            b.synchronize()
+            ms.append(a.elapsed_time(b))
+        ctx.sync(st)
+        return min(ms[1:])
+
+    assert best(rng.choice([4, 12], ns)) <= 1.25 * best(rng.choice([4, 12, 20], ns))
