@@ -74,7 +74,8 @@ struct gcz_ctx {
     int parse_ctas = 3;    // second-stage CTAs per SM
     int seg_width = 1024;  // Zstd parse: 512 or 1024 lane parse, 2048/4096/8192 one warp per segment of that many bytes
     int sweep_warps = 7;   // warps that take turns on a window in the candidate sweep (4-7)
-    int sweep_groups = 0;  // odd: the sweep groups the lanes of every step by hash first
+    int sweep_groups = 0;    // accepted, without effect
+    bool sweep_descending = false;  // set for the length of a selftest
     int sweep_prefetch = 4;  // accepted, without effect
     int lzma_ctas = 3;     // LZMA2 second-stage CTAs per SM
     int lzma_threads = 1024;  // LZMA2 second-stage threads per CTA (256, 512 or 1024)
@@ -228,7 +229,7 @@ int zstd_device_core(gcz_ctx *c, Scratch &sc, const uint8_t *d_src, size_t n, ui
     if (split) {
         uint16_t *cand = static_cast<uint16_t *>(sc.cand.p);
         GCZ_CUDA(c, gcz::launch_cand_sweep(d_src, n, kW, (uint32_t)nb, cand, (uint32_t)nb, c->num_sms, st, wins,
-                                           c->sweep_warps, c->sweep_groups));
+                                           c->sweep_warps, c->sweep_descending));
         gcz::Zstd2Launch l{};
         l.src = d_src;
         l.cand = cand;
@@ -277,7 +278,7 @@ int lzma_run(gcz_ctx *c, Scratch &sc, const gcz::LzmaLaunch &l, cudaStream_t st)
     if (split) {
         uint16_t *cand = static_cast<uint16_t *>(sc.cand.p);
         GCZ_CUDA(c, gcz::launch_cand_sweep(l.src, l.n, l.window, l.num_windows, cand, 0u, c->num_sms, st, l.wins,
-                                           c->sweep_warps, c->sweep_groups));
+                                           c->sweep_warps, c->sweep_descending));
         gcz::LzmaLaunch lv = l;
         lv.ctas_per_sm = c->lzma_ctas;
         lv.threads = c->lzma_threads;
@@ -859,7 +860,7 @@ extern "C" int gcz_zstd_match_find_ref_layout_device(gcz_ctx *c, const uint8_t *
         ProfScope ps(c, st);
         uint16_t *cand = static_cast<uint16_t *>(c->sc.cand.p);
         GCZ_CUDA(c, gcz::launch_cand_sweep(d_input, n_eff, chunk_size, (uint32_t)nb, cand, (uint32_t)nb, c->num_sms, st, nullptr,
-                                           c->sweep_warps, c->sweep_groups));
+                                           c->sweep_warps, c->sweep_descending));
         gcz::Zstd2Launch l{};
         l.src = d_input;
         l.cand = cand;
@@ -916,6 +917,21 @@ extern "C" int gcz_lzma2_match_find_device(gcz_ctx *c, const uint8_t *d_src, siz
     DeviceGuard g(c->device);
     if (n == 0) return GCZ_OK;
     return lzma_device_core(c, c->sc, d_src, n, search_depth, d_packed, d_has_matches, pick_stream(c, stream));
+}
+
+extern "C" int gcz_selftest_sweep_redo(gcz_ctx *c, const uint8_t *d_src, size_t n, uint32_t search_depth,
+                                       uint32_t *d_packed, uint8_t *d_has_matches, void *stream) {
+    if (!c) return GCZ_EINVAL;
+    std::lock_guard<std::mutex> lk(c->mu);
+    if (n && !d_src) return fail(c, GCZ_EINVAL, "null pointer");
+    if (!aligned16(d_src)) return fail(c, GCZ_EINVAL, "d_src must be 16-byte aligned");
+    if (c->algo != 2) return fail(c, GCZ_EINVAL, "algo 1 has no sweep");
+    DeviceGuard g(c->device);
+    if (n == 0) return GCZ_OK;
+    c->sweep_descending = true;
+    const int r = lzma_device_core(c, c->sc, d_src, n, search_depth, d_packed, d_has_matches, pick_stream(c, stream));
+    c->sweep_descending = false;
+    return r;
 }
 
 namespace {
@@ -1448,7 +1464,7 @@ int server_launch(gcz_server *sv, ServerSlot &s) {
     if (nb) {
         GCZ_CUDA(c, cudaMemcpyAsync(s.wins.p, s.hwins.data(), nb * sizeof(gcz_window), cudaMemcpyHostToDevice, s.st));
         GCZ_CUDA(c, gcz::launch_cand_sweep(slab_p, slab, kW, (uint32_t)nb, cand, s.wb[kGrpLzma], c->num_sms, s.st, dw,
-                                           c->sweep_warps, c->sweep_groups));
+                                           c->sweep_warps, c->sweep_descending));
     }
     const uint32_t nz = s.wb[kGrpLzma];  // Zstd windows: sequences and frames groups
     uint64_t *d_off = static_cast<uint64_t *>(s.offsets.p);

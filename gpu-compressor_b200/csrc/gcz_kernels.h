@@ -72,14 +72,14 @@ struct Zstd2Launch {
 };
 
 cudaError_t launch_zstd_match(const ZstdLaunch &l, cudaStream_t st);
-// sweep_warps: warps that take turns on a window (4-7).  sweep_groups: odd
-// values group the lanes of a step by hash first (several times slower; the
-// path an unexpected order of colliding lanes would take).  Schedule only.
+// sweep_warps: warps that take turns on a window (4-7; schedule only).
+// descending (selftest): the steps of a turn last to first, which sends the
+// CTAs that meet equal hashes in a turn through the grouped sweep.
 // zero_windows: positions without a candidate get 0 (what the Zstd kernels
 // read) in the first zero_windows windows, 0xFFFF (LZMA2) in the others.
 cudaError_t launch_cand_sweep(const uint8_t *src, uint64_t n, uint32_t window, uint32_t num_windows, uint16_t *cand,
                               uint32_t zero_windows, int num_sms, cudaStream_t st, const WinDesc *wins = nullptr,
-                              int sweep_warps = 7, int sweep_groups = 0);
+                              int sweep_warps = 7, bool descending = false);
 size_t zstd2_seg_scratch_entries(uint32_t num_windows);
 cudaError_t launch_zstd_parse(const Zstd2Launch &l, cudaStream_t st);
 cudaError_t launch_scan_counts(const uint32_t *counts, uint32_t num, uint64_t *offsets, cudaStream_t st);

@@ -127,9 +127,10 @@ __device__ void sweep_window_grouped(uint32_t *T, uint16_t *out, const uint32_t 
     }
 }
 
-// kWarps warps take turns on a window (a schedule knob, 4-7).  kGrouped: every
-// window takes the grouped sweep (what an unexpected lane order would lead to).
-template <int kWarps, bool kGrouped>
+// kWarps warps take turns on a window (a schedule knob, 4-7).  kDescending: the
+// steps of a turn are exchanged last to first, an order that the check finds
+// wherever two of a turn's positions share a bucket (selftest).
+template <int kWarps, bool kDescending>
 __global__ void __launch_bounds__(32 * kWarps, kSweepCtas) cand_sweep_kernel(SweepArgs a) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     SweepSmem<kWarps> &S = *reinterpret_cast<SweepSmem<kWarps> *>(smem_raw);
@@ -139,76 +140,77 @@ __global__ void __launch_bounds__(32 * kWarps, kSweepCtas) cand_sweep_kernel(Swe
         uint4 *T4 = reinterpret_cast<uint4 *>(S.T);
         for (uint32_t i = tid; i < kHashSize / 4; i += kThreads) T4[i] = make_uint4(0u, 0u, 0u, 0u);
     };
-    if (tid == 0) S.redo = kGrouped ? 1u : 0u;
+    if (tid == 0) S.redo = 0u;
     clear();
     __syncthreads();
     bool bad = false;
-    if constexpr (!kGrouped) {
-        uint32_t first = 0;  // warp whose turn the window's first chunk is
-        uint32_t epoch = 0;
-        bool begun = false;  // some chunk of this CTA has been handed out
-        for (uint32_t w = blockIdx.x; w < a.num_windows; w += gridDim.x) {
-            if (++epoch == 0x10000u) {
-                __syncthreads();
-                clear();
-                __syncthreads();
-                epoch = 1u;
-            }
-            uint64_t start;
-            uint32_t size;
-            window_of(a, w, start, size);
-            const uint32_t *src32 = reinterpret_cast<const uint32_t *>(a.src + start);
-            uint16_t *out = a.cand + start;
-            const uint32_t nwords = (size + 3u) >> 2;
-            const uint32_t nch = (size + kChunkPos - 1u) / kChunkPos;
-            const bool last_window = a.num_windows - w <= gridDim.x;
-            const uint32_t none = w < a.zero_windows ? 0u : 0xFFFFu;
-            uint32_t ch = warp >= first ? warp - first : warp + kWarps - first;  // this warp's first chunk
-            ChunkWords cw = load_chunk(src32, nwords, ch);
-            for (; ch < nch; ch += kWarps) {
-                uint32_t nx = __shfl_down_sync(kFull, cw.a.x, 1);
-                const uint32_t b0 = __shfl_sync(kFull, cw.b.x, 0);
-                if (lane == 31u) nx = b0;
-                uint32_t ny = __shfl_down_sync(kFull, cw.b.x, 1);
-                if (lane == 31u) ny = cw.next;
-                uint4 *hb = reinterpret_cast<uint4 *>(S.h[warp]);
-                hb[lane] = bucket_offsets(cw.a, nx);
-                hb[32u + lane] = bucket_offsets(cw.b, ny);
-                __syncwarp();
-                cw = load_chunk(src32, nwords, ch + kWarps);  // the next chunk's words arrive while others take turns
-                uint32_t h[kChunkSteps], old[kChunkSteps];
-#pragma unroll
-                for (uint32_t j = 0; j < kChunkSteps; ++j) h[j] = S.h[warp][32u * j + lane];
-                const uint32_t q0 = ch * kChunkPos + lane, e0 = epoch << 16;
-                uint8_t *T = reinterpret_cast<uint8_t *>(S.T);
-                if (begun || ch > 0u) turn_wait(1u + warp);
-                const bool full = (ch + 1u) * kChunkPos + 3u <= size;  // every position has its four bytes
-                if (full) {
-#pragma unroll
-                    for (uint32_t j = 0; j < kChunkSteps; ++j)
-                        old[j] = atomicExch(reinterpret_cast<uint32_t *>(T + h[j]), e0 + q0 + 32u * j);
-                } else {
-#pragma unroll
-                    for (uint32_t j = 0; j < kChunkSteps; ++j) {
-                        old[j] = 0u;
-                        if (q0 + 32u * j + 3u < size)
-                            old[j] = atomicExch(reinterpret_cast<uint32_t *>(T + h[j]), e0 + q0 + 32u * j);
-                    }
-                }
-                if (!(last_window && ch + 1u == nch)) turn_pass(1u + (warp + 1u == kWarps ? 0u : warp + 1u));
-#pragma unroll
-                for (uint32_t j = 0; j < kChunkSteps; ++j) {
-                    const uint32_t q = q0 + 32u * j;
-                    bad = bad || old[j] >= e0 + q;
-                    const uint32_t c = old[j] - e0;  // an earlier epoch's entry is below e0: none
-                    if (full || q < size) out[q] = static_cast<uint16_t>(c < 0x10000u ? c : none);
-                }
-            }
-            if (nch) begun = true;
-            first = (first + nch) % kWarps;
+    uint32_t first = 0;  // warp whose turn the window's first chunk is
+    uint32_t epoch = 0;
+    bool begun = false;  // some chunk of this CTA has been handed out
+    for (uint32_t w = blockIdx.x; w < a.num_windows; w += gridDim.x) {
+        if (++epoch == 0x10000u) {
+            __syncthreads();
+            clear();
+            __syncthreads();
+            epoch = 1u;
         }
-        if (bad) S.redo = 1u;
+        uint64_t start;
+        uint32_t size;
+        window_of(a, w, start, size);
+        const uint32_t *src32 = reinterpret_cast<const uint32_t *>(a.src + start);
+        uint16_t *out = a.cand + start;
+        const uint32_t nwords = (size + 3u) >> 2;
+        const uint32_t nch = (size + kChunkPos - 1u) / kChunkPos;
+        const bool last_window = a.num_windows - w <= gridDim.x;
+        const uint32_t none = w < a.zero_windows ? 0u : 0xFFFFu;
+        uint32_t ch = warp >= first ? warp - first : warp + kWarps - first;  // this warp's first chunk
+        ChunkWords cw = load_chunk(src32, nwords, ch);
+        for (; ch < nch; ch += kWarps) {
+            uint32_t nx = __shfl_down_sync(kFull, cw.a.x, 1);
+            const uint32_t b0 = __shfl_sync(kFull, cw.b.x, 0);
+            if (lane == 31u) nx = b0;
+            uint32_t ny = __shfl_down_sync(kFull, cw.b.x, 1);
+            if (lane == 31u) ny = cw.next;
+            uint4 *hb = reinterpret_cast<uint4 *>(S.h[warp]);
+            hb[lane] = bucket_offsets(cw.a, nx);
+            hb[32u + lane] = bucket_offsets(cw.b, ny);
+            __syncwarp();
+            cw = load_chunk(src32, nwords, ch + kWarps);  // the next chunk's words arrive while others take turns
+            uint32_t h[kChunkSteps], old[kChunkSteps];
+#pragma unroll
+            for (uint32_t j = 0; j < kChunkSteps; ++j) h[j] = S.h[warp][32u * j + lane];
+            const uint32_t q0 = ch * kChunkPos + lane, e0 = epoch << 16;
+            uint8_t *T = reinterpret_cast<uint8_t *>(S.T);
+            if (begun || ch > 0u) turn_wait(1u + warp);
+            const bool full = (ch + 1u) * kChunkPos + 3u <= size;  // every position has its four bytes
+            if (full) {
+#pragma unroll
+                for (uint32_t i = 0; i < kChunkSteps; ++i) {
+                    const uint32_t j = kDescending ? kChunkSteps - 1u - i : i;
+                    old[j] = atomicExch(reinterpret_cast<uint32_t *>(T + h[j]), e0 + q0 + 32u * j);
+                }
+            } else {
+#pragma unroll
+                for (uint32_t i = 0; i < kChunkSteps; ++i) {
+                    const uint32_t j = kDescending ? kChunkSteps - 1u - i : i;
+                    old[j] = 0u;
+                    if (q0 + 32u * j + 3u < size)
+                        old[j] = atomicExch(reinterpret_cast<uint32_t *>(T + h[j]), e0 + q0 + 32u * j);
+                }
+            }
+            if (!(last_window && ch + 1u == nch)) turn_pass(1u + (warp + 1u == kWarps ? 0u : warp + 1u));
+#pragma unroll
+            for (uint32_t j = 0; j < kChunkSteps; ++j) {
+                const uint32_t q = q0 + 32u * j;
+                bad = bad || old[j] >= e0 + q;
+                const uint32_t c = old[j] - e0;  // an earlier epoch's entry is below e0: none
+                if (full || q < size) out[q] = static_cast<uint16_t>(c < 0x10000u ? c : none);
+            }
+        }
+        if (nch) begun = true;
+        first = (first + nch) % kWarps;
     }
+    if (bad) S.redo = 1u;
     __syncthreads();
     if (S.redo && warp == 0) {
         for (uint32_t w = blockIdx.x; w < a.num_windows; w += gridDim.x) {
@@ -222,16 +224,16 @@ __global__ void __launch_bounds__(32 * kWarps, kSweepCtas) cand_sweep_kernel(Swe
     }
 }
 
-template <int kWarps, bool kGrouped>
+template <int kWarps, bool kDescending>
 cudaError_t launch_sweep_variant(const SweepArgs &a, int num_sms, cudaStream_t st) {
     const uint32_t smem = sizeof(SweepSmem<kWarps>);
     static_assert((sizeof(SweepSmem<kWarps>) + 1024) * kSweepCtas <= 233472, "three CTAs per SM must fit");
     static SmemOnce smem_set{0};
-    cudaError_t e = set_smem_once(cand_sweep_kernel<kWarps, kGrouped>, smem, smem_set);
+    cudaError_t e = set_smem_once(cand_sweep_kernel<kWarps, kDescending>, smem, smem_set);
     if (e != cudaSuccess) return e;
     uint32_t ctas = static_cast<uint32_t>(num_sms) * kSweepCtas;
     if (ctas > a.num_windows) ctas = a.num_windows;
-    cand_sweep_kernel<kWarps, kGrouped><<<ctas, 32 * kWarps, smem, st>>>(a);
+    cand_sweep_kernel<kWarps, kDescending><<<ctas, 32 * kWarps, smem, st>>>(a);
     return cudaGetLastError();
 }
 
@@ -239,15 +241,15 @@ cudaError_t launch_sweep_variant(const SweepArgs &a, int num_sms, cudaStream_t s
 
 cudaError_t launch_cand_sweep(const uint8_t *src, uint64_t n, uint32_t window, uint32_t num_windows, uint16_t *cand,
                               uint32_t zero_windows, int num_sms, cudaStream_t st, const WinDesc *wins,
-                              int sweep_warps, int sweep_groups) {
+                              int sweep_warps, bool descending) {
     if (num_windows == 0) return cudaSuccess;
     SweepArgs a{src, n, window, num_windows, cand, wins, zero_windows};
-    const bool grouped = (sweep_groups & 1) != 0;
+    if (descending) return launch_sweep_variant<7, true>(a, num_sms, st);
     switch (sweep_warps) {
-    case 4: return grouped ? launch_sweep_variant<4, true>(a, num_sms, st) : launch_sweep_variant<4, false>(a, num_sms, st);
-    case 5: return grouped ? launch_sweep_variant<5, true>(a, num_sms, st) : launch_sweep_variant<5, false>(a, num_sms, st);
-    case 6: return grouped ? launch_sweep_variant<6, true>(a, num_sms, st) : launch_sweep_variant<6, false>(a, num_sms, st);
-    default: return grouped ? launch_sweep_variant<7, true>(a, num_sms, st) : launch_sweep_variant<7, false>(a, num_sms, st);
+    case 4: return launch_sweep_variant<4, false>(a, num_sms, st);
+    case 5: return launch_sweep_variant<5, false>(a, num_sms, st);
+    case 6: return launch_sweep_variant<6, false>(a, num_sms, st);
+    default: return launch_sweep_variant<7, false>(a, num_sms, st);
     }
 }
 

@@ -69,6 +69,7 @@ SIGNATURES = {
     "gcz_zstd_compress_frames_gpu": (_i, [_vp, _vp, _sz, _u32, _vp, _sz, _vp, ctypes.POINTER(_sz)]),
     "gcz_zstd_encode_frames_device": (_i, [_vp, _vp, _sz, _vp, _vp, _vp, _sz, _vp, _vp]),
     "gcz_selftest_wait_timeout": (_i, [_vp, _u32]),
+    "gcz_selftest_sweep_redo": (_i, [_vp, _vp, _sz, _u32, _vp, _vp, _vp]),
     "gcz_zstd_encode_frames_batch_device": (_i, [_vp, _vp, _u64, _vp, _u32, _vp, _vp, _vp, _sz, _vp, _vp]),
     "gcz_zstd_compress_files_gpu": (_i, [_vp, _vp, _vp, _sz, _u32, _vp, _sz, _vp, ctypes.POINTER(_sz)]),
     "gcz_profile_start": (_i, [_vp]),

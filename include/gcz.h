@@ -79,11 +79,8 @@ const char *gcz_version(void);
  * parse: 1024 (default) or 512, one lane per 128-byte segment without repeat
  * offsets, which are checked and mended afterwards; 2048, 4096 or 8192, one
  * warp per segment of that many bytes with them; "sweep_warps" = warps that take turns on
- * a window in the candidate sweep (4-7, default 7); "sweep_groups" = 0 (default)
- * or 2: the sweep exchanges positions through its table and checks the order of
- * colliding lanes, 1 or 3: it groups the lanes of every step by hash first
- * (several times slower; the path an unexpected order leads to);
- * "sweep_prefetch" = accepted (0 to 64) and without effect;
+ * a window in the candidate sweep (4-7, default 7); "sweep_groups" (0 to 3) and
+ * "sweep_prefetch" (0 to 64) = accepted and without effect;
  * "lzma_ctas" = LZMA2 second-stage CTAs per SM (1-8, default 3; values above
  * what fits on an SM -- 3, or 2 with 1024 threads -- run as that many);
  * "lzma_threads" = LZMA2 second-stage threads per CTA (256, 512 or 1024,
@@ -377,6 +374,11 @@ int gcz_zstd_compress_files_gpu(gcz_ctx *ctx, const uint8_t *const *srcs, const 
  * max_iterations tries and the kernel records it, so this returns GCZ_EDEVICE
  * and the context stays usable.  No fault, trap or hang is involved. */
 int gcz_selftest_wait_timeout(gcz_ctx *ctx, uint32_t max_iterations);
+/* gcz_lzma2_match_find_device with a candidate sweep that takes its steps in an
+ * order its own check finds wrong, so that it sweeps again the exact way: the
+ * results have to be the same. */
+int gcz_selftest_sweep_redo(gcz_ctx *ctx, const uint8_t *d_src, size_t n, uint32_t search_depth, uint32_t *d_packed,
+                            uint8_t *d_has_matches, void *stream);
 
 /* Between gcz_profile_start and gcz_profile_stop every match-find step this
  * context launches is bracketed by CUDA events on its own launch stream.

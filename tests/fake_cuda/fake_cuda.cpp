@@ -93,7 +93,7 @@ namespace gcz {
 cudaError_t launch_zstd_match(const ZstdLaunch &, cudaStream_t) { return done(); }
 cudaError_t launch_lzma_match(const LzmaLaunch &, cudaStream_t) { return done(); }
 cudaError_t launch_cand_sweep(const uint8_t *, uint64_t, uint32_t, uint32_t, uint16_t *, uint32_t, int, cudaStream_t,
-                              const WinDesc *, int, int) {
+                              const WinDesc *, int, bool) {
     return done();
 }
 size_t zstd2_seg_scratch_entries(uint32_t n) { return n * 1024ull; }
