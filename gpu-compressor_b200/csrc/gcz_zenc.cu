@@ -1485,18 +1485,31 @@ __device__ uint32_t encode_sequences(const ZencArgs &a, SeqSmem &G, uint32_t b, 
     __syncthreads();
     // ---- R: Offset_Values and code counts
     // The guessed history: the three different offsets used last before the run,
-    // each thread's own first (0: none), then those of the threads before it.
+    // by a scan of each thread's own (0: none).
     uint32_t l1 = 0, l2 = 0, l3 = 0;
     for (uint32_t i = i1; i > i0 && l3 == 0u; --i) recent(l1, l2, l3, sq[i - 1u].x);
-    G.out_state[0][tid] = l1;
-    G.out_state[1][tid] = l2;
-    G.out_state[2][tid] = l3;
+#pragma unroll
+    for (uint32_t d = 1; d < 32u; d <<= 1) {  // with those of the lanes before it
+        const uint32_t a1 = __shfl_up_sync(kFull, l1, d), a2 = __shfl_up_sync(kFull, l2, d),
+                       a3 = __shfl_up_sync(kFull, l3, d);
+        if (lane >= d) {
+            recent(l1, l2, l3, a1);
+            recent(l1, l2, l3, a2);
+            recent(l1, l2, l3, a3);
+        }
+    }
+    if (lane == 31u) {
+        G.out_state[0][warp] = l1;
+        G.out_state[1][warp] = l2;
+        G.out_state[2][warp] = l3;
+    }
+    uint32_t in1 = __shfl_up_sync(kFull, l1, 1), in2 = __shfl_up_sync(kFull, l2, 1), in3 = __shfl_up_sync(kFull, l3, 1);
+    if (lane == 0u) in1 = in2 = in3 = 0u;
     __syncthreads();
-    uint32_t in1 = 0, in2 = 0, in3 = 0;
-    for (uint32_t t = tid; t > 0u && in3 == 0u; --t) {
-        recent(in1, in2, in3, G.out_state[0][t - 1u]);
-        recent(in1, in2, in3, G.out_state[1][t - 1u]);
-        recent(in1, in2, in3, G.out_state[2][t - 1u]);
+    for (uint32_t v = warp; v > 0u; --v) {  // and of the warps before it
+        recent(in1, in2, in3, G.out_state[0][v - 1u]);
+        recent(in1, in2, in3, G.out_state[1][v - 1u]);
+        recent(in1, in2, in3, G.out_state[2][v - 1u]);
     }
     recent(in1, in2, in3, 1u);
     recent(in1, in2, in3, 4u);
