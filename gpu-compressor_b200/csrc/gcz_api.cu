@@ -1277,7 +1277,7 @@ double now_ms() {
 
 // Device bytes per input byte of one slot, pre-sized at creation for a batch of
 // max_batch_bytes of any mix of kinds: slab 1, candidates 2, Zstd speculative
-// lists 3.9 (sized for the widest segment layout), packed sequences 2.67, ZSTD_Sequence output 5.33, LZMA2 packed
+// lists 4 (sized for the widest segment layout), packed sequences 2.67, ZSTD_Sequence output 5.33, LZMA2 packed
 // matches 4, and for frames the frames 1.02, frame slots 1.02, offset codes
 // 1.33 and plans 0.03.
 constexpr double kDeviceBytesPerInputByte = 23.0;

@@ -27,23 +27,27 @@
 //    Mends lie side by side; one that starts inside an earlier one is dropped.
 //    Every literal run is then either checked or parsed exactly, so the
 //    sequences are the reference's by induction over the runs.
-// 5. Give up.  A window with more than kMostFixes such runs, with a mend that
-//    finds no end soon, or with no room for a list is parsed again after the
-//    CTA's other windows.  Where its matches lie close to one another (counters,
-//    sorted numbers, records with a fixed stride, pixels: the repeat offsets
-//    decide most of them), steps 1 and 2 are done with repeat offsets.  A
-//    segment's parse starts from {1,4,8} and joins a later segment's list at a
-//    match that both have with the same repeat offsets after it, nearly always
-//    its third.  Where matches are far apart (samples, floating-point numbers),
-//    or a segment does not join a list soon, the segment parse takes the window.
-//    Per 256 MiB, with the segment parse as the only way out and with both:
-//    32-bit counters 33.7 -> 5.8 ms, sorted numbers 23.6 -> 5.4, 20-byte
-//    records 11.1 -> 5.2, 8-byte records 12.2 -> 4.3, 3-byte pixels 5.8 -> 4.3,
-//    4-letter text (long continuations, step 2) 15.6 -> 3.9.
+// 5. Give up.  A window with more than kMostFixes such runs, with runs that
+//    have such matches all over them, with a mend that finds no end soon, or
+//    with no room for a list is parsed again after the CTA's other windows, and
+//    some windows after it are given up at once.  How depends on how close to
+//    one another the matches lie, by the entries or by a few mends tried out:
+//    - close (counters, records with a fixed stride, 4-letter text): steps 1 and
+//      2 with repeat offsets.  A segment's parse starts from {1,4,8} and joins a
+//      later segment's list at a match that both have with the same repeat
+//      offsets after it, nearly always its third;
+//    - far apart (samples, floating-point numbers): the segment parse by warps;
+//    - else (pixels, sorted numbers), and where a segment does not join a list
+//      soon: the segment parse by 8-lane groups.
+//    Per 256 MiB, with the segment parse by warps as the only way out and now:
+//    32-bit counters 33.7 -> 4.3 ms, sorted numbers 23.5 -> 3.5, 20-byte records
+//    11.1 -> 3.6, 8-byte records 12.2 -> 3.5, 3-byte pixels 5.8 -> 2.9, 4-letter
+//    text (long continuations, step 2) 15.6 -> 3.9.
 //
-// Segment parse (zstd_seg_parse_kernel, and the lane parse's last way out).  Each
-// warp parses one segment of 2-8 KiB from a guessed state (the segment start,
-// repeat offsets {1,4,8}), then goes on past its end until one of its matches
+// Segment parse (zstd_seg_parse_kernel, and ways out of the lane parse).  Each
+// warp parses one segment of 2-8 KiB, or each 8-lane group one of 1 KiB, from a
+// guessed state (the segment start, repeat offsets {1,4,8}), then goes on past
+// its end until one of its matches
 // equals a match of a later warp's list -- same start, length and offset, and
 // the same repeat offsets afterwards.  A chain walk from warp 0 picks the
 // lists; every list on the chain is exact by induction.  A warp step takes the
@@ -72,18 +76,21 @@ namespace {
 constexpr uint32_t kMinMatch = 3;                 // MIN_MATCH_LEN, zstd_compress.cu:28
 
 // Segment parse: segment width (a schedule knob: 2, 4 or 8 KiB, one warp each;
-// it never changes the sequences).
-template <uint32_t SegW>
+// it never changes the sequences), or 1 KiB, one 8-lane group each.
+template <uint32_t SegW, uint32_t GL = 32>
 struct SegCfg {
     static constexpr uint32_t kSegW = SegW;
     static constexpr uint32_t kSegs = kMaxWindow / SegW;
-    static constexpr uint32_t kThreads = kSegs * 32;
+    static constexpr uint32_t kThreads = kSegs * GL;
     // A segment's own parse ends with a step that starts before seg_end and
-    // looks at most 128 positions ahead, the lazy step one more; matches do
-    // not overlap and are >= 3 bytes, so a list holds at most
-    // (SegW + 128) / 3 + 1 entries; lists are written in 32-entry blocks.
-    static constexpr uint32_t kSpecCap = ((SegW + 128) / 3 + 1 + 31) / 32 * 32;
-    static constexpr uint32_t kContCap = 256;  // continuation matches before giving up (three meet nearly always)
+    // looks at most kLook positions ahead (a warp's wide scan 128, a group's
+    // scan 32), the lazy step one more; matches do not overlap and are >= 3
+    // bytes, so a list holds at most (SegW + kLook) / 3 + 1 entries; lists are
+    // written in 32-entry blocks.
+    static constexpr uint32_t kLook = GL == 32 ? 128 : 32;
+    static constexpr uint32_t kSpecCap = ((SegW + kLook) / 3 + 1 + 31) / 32 * 32;
+    // continuation matches before giving up (three meet nearly always)
+    static constexpr uint32_t kContCap = GL == 32 ? 256 : 128;
     static constexpr uint32_t kLaneCap = kSpecCap + kContCap;
     static constexpr uint32_t kMinBlocks = kThreads >= 1024 ? 1 : 3;
 };
@@ -109,7 +116,7 @@ struct SegSmem {
 };
 
 struct ParseScalars {
-    uint32_t flags;    // 1: the segment parse gives up, 2: staging failed, 4: the lane parse gives up
+    uint32_t flags;    // 1: the segment parse gives up, 2: staging failed, 4: the lane parse gives up, 16: at once
     uint32_t total;
     uint32_t covered;
     uint32_t count;    // literal runs with a repeat-offset match found
@@ -117,6 +124,8 @@ struct ParseScalars {
     uint32_t chunks;   // chunks of continuations in use
     uint32_t probe[2]; // matches and bytes of the window's mends
     uint32_t again;    // 1 + the last window given up (0: none); each leads to the one before it
+    uint32_t how;      // how to parse the windows given up: 1 lanes, 0 groups, 2 warps
+    uint32_t skip, streak;  // windows to give up at once; of the last time
     uint32_t warp_sum[32];
     alignas(8) uint64_t bar;
 };
@@ -129,13 +138,17 @@ constexpr uint32_t kLSegW = 132, kLists = (kMaxWindow + kLSegW - 1) / kLSegW;
 constexpr uint32_t kLSegs = 512;                                // kLists, up to whole warps
 constexpr uint32_t kLCap = (kLSegW + 2) / 3;                    // matches that start their search in a segment
 constexpr uint32_t kLCont = 12;                                 // continuation: 11 matches, then a chunk's number ...
-constexpr uint32_t kLChunks = 96, kLChunk = 32;                 // ... chunks of 31 more matches and the next one's number
+constexpr uint32_t kLChunks = 224, kLChunk = 16;                // ... chunks of 15 more matches and the next one's number
 constexpr uint32_t kLMost = 255;                                // most matches before a segment's parse joins a list
 constexpr uint32_t kFixes = 256, kFixCap = 255;                 // runs recorded per window, most matches per mend
 constexpr uint32_t kMostFixes = 192;                            // most runs that are mended
-constexpr uint32_t kDense = 36;                                 // bytes per match below which a window counts as dense ...
-constexpr uint32_t kDenseCap = 48, kTryCap = 12;                // ... the most matches of a mend in one, and of one tried out
-constexpr uint32_t kMostSteps = 400;                            // most steps before a segment's parse with repeat offsets joins
+// Bytes per match of a window given up: lanes below kDense (kTryDense by the
+// few matches tried out), warps from kSparse on, groups between.  64 MiB of 16-bit
+// samples: with a match every 31 bytes 1.8 ms with lanes tried first, 1.04 by
+// groups, 1.30 by warps; every 47 bytes 2.7 by groups, 1.2 by warps.
+constexpr uint32_t kDense = 16, kTryDense = 12, kSparse = 44;
+constexpr uint32_t kDenseCap = 48, kTryCap = 4;                 // most matches of a dense mend, and of one only tried out
+constexpr uint32_t kMostSteps = 128;                            // most steps before a parse with repeat offsets joins a list
 // Entries in a window's scratch: the segments' lists, then the continuations;
 // once the list of the whole parse is known it takes the lists' place, and
 // the mends that of the continuations.
@@ -145,7 +158,7 @@ constexpr uint32_t kLEntries = kLChunkBase + kLChunks * kLChunk;
 constexpr uint32_t kFixEntries = kLEntries - kLContBase;        // shared by a window's mends
 static_assert(kLContBase >= 21846, "the whole parse fits where the lists were");
 static_assert(kLists <= kLSegs && kLSegs % 32 == 0, "whole warps of segments");
-static_assert(kLMost <= 255 && kFixCap <= 255, "8-bit counts");
+static_assert(kLMost <= 255, "8-bit counts");
 
 template <uint32_t kWarps>
 struct LaneSmem {
@@ -165,7 +178,8 @@ struct LaneSmem {
             uint8_t len[kFixes];     // entries of the mend
             uint8_t list[kFixes];    // the mend's list in the scratch
         } fix;
-        SegSmem<kWarps> seg;
+        SegSmem<64> seg;
+        SegSmem<kWarps> segw;
     };
 };
 
@@ -554,6 +568,132 @@ __device__ __forceinline__ bool rep3_any16(const Win &w, uint32_t q, const uint3
     return ((a[0] | a[1] | a[2] | a[3]) & 0x80808080u) != 0u;
 }
 
+// Group-wide extension: the lanes of each GL-lane group compare 4 bytes each
+// (4 * GL per iteration) of their group's own (c, q, lim) and get the first
+// index in [0, lim) where bytes c+i and q+i differ, else lim; groups with
+// act == false get 0.  All 32 lanes call it (the loop runs while any group
+// is still extending).
+template <uint32_t GL>
+__device__ __forceinline__ uint32_t extend_group(const Win &w, uint32_t c, uint32_t q, uint32_t lim, bool act) {
+    const uint32_t lane = lane_id(), gl = lane & (GL - 1u), gb = lane & ~(GL - 1u);
+    uint32_t len = 0, out = 0;
+    bool done = !act;
+    while (__any_sync(kFull, !done)) {
+        const uint32_t k = len + 8u * gl;  // 8 bytes per lane
+        uint32_t res = k;
+        if (!done && k < lim) {
+            uint32_t ql, qh, cl, ch;
+            w.u64(static_cast<int>(q + k), ql, qh);
+            w.u64(static_cast<int>(c + k), cl, ch);
+            const uint32_t dl = ql ^ cl, dh = qh ^ ch;
+            const uint32_t fb = dl ? (static_cast<uint32_t>(__ffs(dl)) - 1u) >> 3
+                                   : (dh ? 4u + ((static_cast<uint32_t>(__ffs(dh)) - 1u) >> 3) : 8u);
+            const uint32_t rem = lim - k;
+            res = k + (fb < rem ? fb : rem);
+        }
+        const uint32_t sb = (__ballot_sync(kFull, !done && res < k + 8u) >> gb) & ((1u << GL) - 1u);
+        const uint32_t v = __shfl_sync(kFull, res, gb + (sb ? static_cast<uint32_t>(__ffs(sb)) - 1u : 0u));
+        if (!done && sb) {
+            out = v;
+            done = true;
+        }
+        len += 8u * GL;
+    }
+    return out;
+}
+
+// One step of the exact parse for every 8-lane group of the warp at once, each
+// from its own state s (group-uniform); groups with run == false keep theirs.
+// A group looks at the 32 positions from s.p: the hash-match bits come from the
+// bitmap, and six lanes test the three repeat offsets among the positions
+// before the first hash match (zstd_compress.cu:259-275), 16 positions each.
+// The first event is the match, extended 64 bytes per group iteration, with the
+// lazy step (:278-307) at f+1; with no event the group moves over the 32
+// positions.  Returns whether the group found a match (m set, s advanced past
+// it, repeat offsets updated).
+template <uint32_t GL>
+__device__ __forceinline__ bool group_step(const Win &w, const uint32_t *bm, const uint16_t *cand, uint32_t size,
+                                           bool lazy, bool run, PState &s, Match &m) {
+    static_assert(GL == 8, "8-lane groups");
+    const uint32_t lane = lane_id(), gl = lane & (GL - 1u), gb = lane & ~(GL - 1u);
+    const uint32_t p = run ? s.p : 0u;
+    const uint32_t lim = run ? size - 3u - p : 0u;
+    const uint32_t n32 = lim < 32u ? lim : 32u;
+    uint32_t H = __funnelshift_r(bm[p >> 5], bm[(p >> 5) + 1], p & 31u);
+    if (n32 < 32u) H &= (1u << n32) - 1u;
+    const uint32_t nh = H ? static_cast<uint32_t>(__ffs(H)) - 1u : n32;  // positions without a hash match
+    // The candidates at the first hash match and the position after it are
+    // loaded before the repeat-offset test, so that their latency overlaps
+    // it: the event is that hash match unless a repeat offset hits earlier
+    // (a few times per window), and only then is cand(f+1) loaded again.
+    const uint32_t fh = nh < n32 ? p + nh : 0u;
+    const uint32_t ch0 = cand[fh], ch1 = cand[fh + 1u];
+    uint32_t m0, m1, m2;  // per repeat offset: hits among the 32 positions
+    {
+        // Lane 2k+h (k < 3) tests repeat offset k on the 16 positions from
+        // p + 16h that come before the first hash match and whose source lies
+        // in the window; lanes 6 and 7 test nothing.
+        const uint32_t rk = gl >> 1, hh = gl & 1u;
+        const uint32_t q0 = p + 16u * hh;
+        const uint32_t rv = rk == 0u ? s.r0 : (rk == 1u ? s.r1 : s.r2);
+        const uint32_t lo = rv > q0 ? (rv - q0 < 16u ? rv - q0 : 16u) : 0u;
+        const uint32_t hi = (rk < 3u && nh > 16u * hh) ? (nh - 16u * hh < 16u ? nh - 16u * hh : 16u) : 0u;
+        const uint32_t vm = ((1u << hi) - 1u) & ~((1u << lo) - 1u);
+        const uint32_t mk = rep3_scan<4>(w, q0, rv <= q0 + 16u ? rv : 0u) & vm;
+        const uint32_t mo = __shfl_xor_sync(kFull, mk, 1);
+        const uint32_t mf = hh ? (mo | (mk << 16)) : (mk | (mo << 16));  // offset rk over all 32 positions
+        m0 = __shfl_sync(kFull, mf, gb);
+        m1 = __shfl_sync(kFull, mf, gb + 2u);
+        m2 = __shfl_sync(kFull, mf, gb + 4u);
+    }
+    const uint32_t al = m0 | m1 | m2;
+    const bool rep = al != 0u;
+    const bool ev = run && (rep || nh < n32);
+    uint32_t f = p + nh, r = 0;
+    if (rep) {
+        const uint32_t t = static_cast<uint32_t>(__ffs(al)) - 1u;
+        f = p + t;
+        r = (m0 >> t) & 1u ? 0u : ((m1 >> t) & 1u ? 1u : 2u);
+    }
+    const uint32_t fc = ev ? f : 0u;
+    const uint32_t cf = ch0;
+    uint32_t cf1 = ch1;
+    if (rep) cf1 = cand[fc + 1u];
+    uint32_t off, c0;
+    if (!rep) {
+        off = fc - cf;
+        c0 = cf;
+    } else {  // first repeat offset with 3 equal bytes wins
+        off = r == 0u ? s.r0 : (r == 1u ? s.r1 : s.r2);
+        c0 = fc - off;
+    }
+    // The lazy candidate at f+1 is skipped when it is the same match one byte on
+    // (cand(f+1) == c0 + 1): it is exactly one byte shorter, never taken.
+    const bool ltry = ev && lazy && fc + 4u < size && bm_bit(bm, fc + 1u) && cf1 != c0 + 1u;
+    const uint32_t e1 = extend_group<GL>(w, c0 + kMinMatch, fc + kMinMatch, ev ? size - fc - kMinMatch : 0u, ev);
+    const uint32_t e2 =
+        extend_group<GL>(w, cf1 + kMinMatch, fc + 1u + kMinMatch, ltry ? size - fc - 1u - kMinMatch : 0u, ltry);
+    uint32_t len = e1 + kMinMatch;
+    f = fc;
+    if (ltry && e2 + kMinMatch > len + 1u) {
+        f = fc + 1u;
+        len = e2 + kMinMatch;
+        off = f - cf1;
+    }
+    if (ev) {
+        m.start = f;
+        m.len = len;
+        m.off = off;
+        s.r2 = s.r1;
+        s.r1 = s.r0;
+        s.r0 = off;
+        s.p = f + len;
+    } else if (run) {
+        s.p = p + n32;
+    }
+    return ev;
+}
+
 __device__ __forceinline__ uint2 pack_entry(const Match &m) {
     return make_uint2(m.start | ((m.len - kMinMatch) << 16), m.off);
 }
@@ -661,63 +801,221 @@ __device__ __forceinline__ void write_seq(const Zstd2Args &a, uint32_t wi, uint3
 // ---------------------------------------------------------------- segment parse
 // All threads of the CTA (SegCfg<SegW>::kThreads) call it with the window
 // staged and verified, S.flags & 1 clear and S.covered zero.
-template <bool kRef, uint32_t SegW>
-__device__ __forceinline__ void parse_segments(const Zstd2Args &a, SegSmem<SegCfg<SegW>::kSegs> &G, ParseScalars &S,
+template <bool kRef, uint32_t SegW, uint32_t GL = 32>
+__device__ __forceinline__ void parse_segments(const Zstd2Args &a, SegSmem<SegCfg<SegW, GL>::kSegs> &G, ParseScalars &S,
                                                const Win &win, const uint32_t *bm, const uint16_t *cand, uint2 *seg,
                                                uint32_t wi, uint32_t size, bool lazy) {
-    using C = SegCfg<SegW>;
+    using C = SegCfg<SegW, GL>;
     constexpr uint32_t kSegW = C::kSegW, kSegs = C::kSegs;
     constexpr uint32_t kSpecCap = C::kSpecCap, kLaneCap = C::kLaneCap, kContCap = C::kContCap;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t lim_pos = size > 3u ? size - 3u : 0u;  // positions q < lim_pos can start a match
-    // ---- 2a. speculative parse of each segment (one warp each)
-    const uint32_t seg_start = warp * kSegW, seg_end = seg_start + kSegW;
-    const bool active = seg_start < lim_pos;
-    const bool last_active = !(seg_end < lim_pos);
-    ListWriter lw(seg + warp * kLaneCap);
-    PState s{seg_start, 1u, 4u, 8u};
-    CandBuf cb{cand, size, 0u, 0u, 0u, 0u};
-    if (active) cb.init(seg_start);
-    if (active) {
-        const uint32_t stop = last_active ? size : seg_end;
-        Match m;
-        while (s.p < stop && s.p + 3u < size) {
-            if (warp_step(win, bm, cb, size, lazy, s, m)) lw.put(pack_entry(m));
-        }
-        lw.flush();
-    }
-    if (lane == 0) {
-        G.spec_count[warp] = lw.n;
-        G.cont_count[warp] = 0;
-        G.sync_warp[warp] = kNoWarp;
-        G.sync_idx[warp] = 0;
-    }
-    __syncthreads();
-
-    // ---- 2b. continue each warp's parse until it meets a later warp's list
-    if (active && !last_active) {
-        ListWriter cw(seg + warp * kLaneCap + kSpecCap);
-        uint32_t t = kNoWarp, j = 0;
-        Match m;
-        while (s.p + 3u < size) {
-            if (!warp_step(win, bm, cb, size, lazy, s, m)) continue;
-            const uint32_t tw = m.start / kSegW;  // warp whose segment holds this match start
-            if (tw != t) {
-                t = tw;
-                j = 0;
+    if constexpr (GL == 32) {
+        // ---- 2a. speculative parse of each segment (one warp each)
+        const uint32_t seg_start = warp * kSegW, seg_end = seg_start + kSegW;
+        const bool active = seg_start < lim_pos;
+        const bool last_active = !(seg_end < lim_pos);
+        ListWriter lw(seg + warp * kLaneCap);
+        PState s{seg_start, 1u, 4u, 8u};
+        CandBuf cb{cand, size, 0u, 0u, 0u, 0u};
+        if (active) cb.init(seg_start);
+        if (active) {
+            const uint32_t stop = last_active ? size : seg_end;
+            Match m;
+            while (s.p < stop && s.p + 3u < size) {
+                if (warp_step(win, bm, cb, size, lazy, s, m)) lw.put(pack_entry(m));
             }
-            const uint32_t tcount = G.spec_count[t];
-            const uint2 *tl = seg + t * kLaneCap;
-            // first entry of t's list with start >= m.start (lists are sorted by start)
-            for (;;) {
-                const uint32_t idx = j + lane;
-                const bool ge = idx >= tcount || (tl[idx].x & 0xFFFFu) >= m.start;
-                const uint32_t b = __ballot_sync(kFull, ge);
-                if (b) {
-                    j += static_cast<uint32_t>(__ffs(b)) - 1u;
+            lw.flush();
+        }
+        if (lane == 0) {
+            G.spec_count[warp] = lw.n;
+            G.cont_count[warp] = 0;
+            G.sync_warp[warp] = kNoWarp;
+            G.sync_idx[warp] = 0;
+        }
+        __syncthreads();
+
+        // ---- 2b. continue each warp's parse until it meets a later warp's list
+        if (active && !last_active) {
+            ListWriter cw(seg + warp * kLaneCap + kSpecCap);
+            uint32_t t = kNoWarp, j = 0;
+            Match m;
+            while (s.p + 3u < size) {
+                if (!warp_step(win, bm, cb, size, lazy, s, m)) continue;
+                const uint32_t tw = m.start / kSegW;  // warp whose segment holds this match start
+                if (tw != t) {
+                    t = tw;
+                    j = 0;
+                }
+                const uint32_t tcount = G.spec_count[t];
+                const uint2 *tl = seg + t * kLaneCap;
+                // first entry of t's list with start >= m.start (lists are sorted by start)
+                for (;;) {
+                    const uint32_t idx = j + lane;
+                    const bool ge = idx >= tcount || (tl[idx].x & 0xFFFFu) >= m.start;
+                    const uint32_t b = __ballot_sync(kFull, ge);
+                    if (b) {
+                        j += static_cast<uint32_t>(__ffs(b)) - 1u;
+                        break;
+                    }
+                    j += 32u;
+                }
+                bool met = false;
+                if (j < tcount) {
+                    const uint2 e = tl[j];
+                    if (e.x == pack_entry(m).x && e.y == m.off) {
+                        uint32_t e0, e1, e2;
+                        reps_after(tl, j, e0, e1, e2);
+                        met = e0 == s.r0 && e1 == s.r1 && e2 == s.r2;
+                    }
+                }
+                if (met) {
+                    if (lane == 0) {
+                        G.sync_warp[warp] = t;
+                        G.sync_idx[warp] = j;
+                    }
                     break;
                 }
-                j += 32u;
+                if (cw.n == kContCap) {
+                    if (lane == 0) atomicOr(&S.flags, 1u);  // give up: exact fallback below
+                    break;
+                }
+                cw.put(pack_entry(m));
+            }
+            cw.flush();
+            if (lane == 0) G.cont_count[warp] = cw.n;
+        }
+        __syncthreads();
+    } else {
+        // ---- 2a. speculative parse of each segment (one 8-lane group each)
+        const uint32_t sg = tid / GL, gl = lane & (GL - 1u), gb = lane & ~(GL - 1u);
+        const uint32_t seg_start = sg * kSegW, seg_end = seg_start + kSegW;
+        const bool active = sg < kSegs && seg_start < lim_pos;
+        const bool last_active = !(seg_end < lim_pos);
+        const uint32_t stop = last_active ? size : seg_end;
+        uint2 *lst = seg + sg * kLaneCap;
+        PState s{seg_start, 1u, 4u, 8u};
+        uint32_t n = 0;
+        for (;;) {
+            const bool run = active && s.p < stop && s.p + 3u < size;
+            if (!__any_sync(kFull, run)) break;
+            Match m;
+            if (group_step<GL>(win, bm, cand, size, lazy, run, s, m)) {
+                if (gl == 0) lst[n] = pack_entry(m);
+                ++n;
+            }
+        }
+        if (gl == 0 && sg < kSegs) {
+            G.spec_count[sg] = n;
+            G.cont_count[sg] = 0;
+            G.sync_warp[sg] = kNoWarp;
+            G.sync_idx[sg] = 0;
+        }
+        __syncthreads();
+
+        // ---- 2b. continue each group's parse until it meets a later segment's list
+        bool crun = active && !last_active;
+        uint32_t t = kNoWarp, j = 0, cn = 0;
+        uint2 *cl = lst + kSpecCap;
+        for (;;) {
+            const bool run = crun && s.p + 3u < size;
+            const uint32_t runners = __ballot_sync(kFull, run && gl == 0u);
+            if (!runners) break;
+            if ((runners & (runners - 1u)) == 0u) {
+                // Only one group of the warp still runs (the slow tail of the
+                // phase): the whole warp takes over its parse with warp-wide
+                // steps (up to 128 positions scanned, 128 bytes extended per
+                // iteration), same meeting test, then the loop ends.
+                const uint32_t L = static_cast<uint32_t>(__ffs(runners)) - 1u;
+                PState ws{__shfl_sync(kFull, s.p, L), __shfl_sync(kFull, s.r0, L), __shfl_sync(kFull, s.r1, L),
+                          __shfl_sync(kFull, s.r2, L)};
+                const uint32_t wsg = __shfl_sync(kFull, sg, L);
+                uint32_t wt = __shfl_sync(kFull, t, L), wj = __shfl_sync(kFull, j, L),
+                         wcn = __shfl_sync(kFull, cn, L);
+                uint2 *wcl = seg + wsg * kLaneCap + kSpecCap;
+                CandBuf wcb{cand, size, 0u, 0u, 0u, 0u};
+                wcb.init(ws.p);
+                while (ws.p + 3u < size) {
+                    Match m;
+                    if (!warp_step(win, bm, wcb, size, lazy, ws, m)) continue;
+                    const uint32_t tw = m.start / kSegW;  // segment that holds this match start
+                    if (tw != wt) {
+                        wt = tw;
+                        wj = 0;
+                    }
+                    const uint32_t tcount = G.spec_count[wt];
+                    const uint2 *tl = seg + wt * kLaneCap;
+                    // first entry of wt's list with start >= m.start, 32 per step
+                    for (;;) {
+                        const uint32_t idx = wj + lane;
+                        const bool ge = idx >= tcount || (tl[idx].x & 0xFFFFu) >= m.start;
+                        const uint32_t b = __ballot_sync(kFull, ge);
+                        if (b) {
+                            wj += static_cast<uint32_t>(__ffs(b)) - 1u;
+                            break;
+                        }
+                        wj += 32u;
+                    }
+                    bool met = false;
+                    if (wj < tcount) {
+                        const uint2 e = tl[wj];
+                        if (e.x == pack_entry(m).x && e.y == m.off) {
+                            uint32_t e0, e1, e2;
+                            reps_after(tl, wj, e0, e1, e2);
+                            met = e0 == ws.r0 && e1 == ws.r1 && e2 == ws.r2;
+                        }
+                    }
+                    if (met) {
+                        if (lane == 0) {
+                            G.sync_warp[wsg] = wt;
+                            G.sync_idx[wsg] = wj;
+                        }
+                        break;
+                    }
+                    if (wcn == kContCap) {
+                        if (lane == 0) atomicOr(&S.flags, 1u);  // give up: exact fallback below
+                        break;
+                    }
+                    if (lane == 0) wcl[wcn] = pack_entry(m);
+                    ++wcn;
+                }
+                if (lane >= L && lane < L + GL) {
+                    cn = wcn;
+                    crun = false;
+                }
+                break;
+            }
+            Match m;
+            const bool ev = group_step<GL>(win, bm, cand, size, lazy, run, s, m);
+            uint32_t tcount = 0;
+            const uint2 *tl = seg;
+            if (ev) {
+                const uint32_t tw = m.start / kSegW;  // segment that holds this match start
+                if (tw != t) {
+                    t = tw;
+                    j = 0;
+                }
+                tcount = G.spec_count[t];
+                tl = seg + t * kLaneCap;
+            }
+            // first entry of t's list with start >= m.start (lists are sorted by start), 8 per step
+            bool found = !ev;
+            while (__any_sync(kFull, !found)) {
+                const uint32_t idx = j + gl;
+                const bool ge = !found && (idx >= tcount || (tl[idx].x & 0xFFFFu) >= m.start);
+                const uint32_t b = (__ballot_sync(kFull, ge) >> gb) & ((1u << GL) - 1u);
+                if (!found) {
+                    if (b) {
+                        j += static_cast<uint32_t>(__ffs(b)) - 1u;
+                        found = true;
+                    } else {
+                        j += GL;
+                    }
+                }
+            }
+            if (!ev) {
+                if (!run) crun = false;
+                continue;
             }
             bool met = false;
             if (j < tcount) {
@@ -729,22 +1027,22 @@ __device__ __forceinline__ void parse_segments(const Zstd2Args &a, SegSmem<SegCf
                 }
             }
             if (met) {
-                if (lane == 0) {
-                    G.sync_warp[warp] = t;
-                    G.sync_idx[warp] = j;
+                if (gl == 0) {
+                    G.sync_warp[sg] = t;
+                    G.sync_idx[sg] = j;
                 }
-                break;
+                crun = false;
+            } else if (cn == kContCap) {
+                if (gl == 0) atomicOr(&S.flags, 1u);  // give up: exact fallback below
+                crun = false;
+            } else {
+                if (gl == 0) cl[cn] = pack_entry(m);
+                ++cn;
             }
-            if (cw.n == kContCap) {
-                if (lane == 0) atomicOr(&S.flags, 1u);  // give up: exact fallback below
-                break;
-            }
-            cw.put(pack_entry(m));
         }
-        cw.flush();
-        if (lane == 0) G.cont_count[warp] = cw.n;
+        if (gl == 0 && sg < kSegs) G.cont_count[sg] = cn;
+        __syncthreads();
     }
-    __syncthreads();
 
     if (!(S.flags & 1u)) {
         // ---- 3. chain walk, then copy in chain order.  Nearly always every
@@ -844,13 +1142,13 @@ __device__ __forceinline__ void parse_segments(const Zstd2Args &a, SegSmem<SegCf
         // its start minus the end of the entry before it -- the previous
         // entry of the same list, or for a segment's first copied entry the
         // last entry contributed before it, which the chain walk located.
-        const uint32_t csg = tid / 32u, csl = tid % 32u;  // segment whose list this thread copies
-        if (G.on_chain[csg]) {
+        const uint32_t csg = tid / GL, csl = tid % GL;  // segment whose list this thread copies
+        if (csg < kSegs && G.on_chain[csg]) {
             const uint32_t from = G.chain_from[csg], ns = G.spec_count[csg], nc = G.cont_count[csg];
             const uint32_t base = G.out_off[csg];
             const uint2 *mine = seg + csg * kLaneCap;
             uint32_t cov = 0;
-            for (uint32_t i = from + csl; i < ns + nc; i += 32u) {
+            for (uint32_t i = from + csl; i < ns + nc; i += GL) {
                 const uint32_t o = base + (i - from);
                 if (o >= keep) break;
                 const uint2 e = mine[i < ns ? i : kSpecCap + (i - ns)];
@@ -1567,6 +1865,15 @@ __device__ __noinline__ void parse_segments_out(Zstd2Args a, SegSmem<kWarps> &G,
     parse_segments<kRef, kMaxWindow / kWarps>(a, G, S, win, bm, cand, seg, wi, size, lazy);
 }
 
+// The segment parse by 8-lane groups, 64 of them whatever the CTA's warps.
+template <bool kRef>
+__device__ __noinline__ void parse_groups_out(Zstd2Args a, SegSmem<64> &G, ParseScalars &S, Win win, const uint32_t *bm,
+                                              const uint16_t *cand, uint2 *seg, uint32_t wi, uint32_t size, bool lazy) {
+    using C = SegCfg<1024, 8>;
+    static_assert(C::kThreads == 512 && C::kMinBlocks == 3, "what the smallest form of the lane parse has");
+    parse_segments<kRef, 1024, 8>(a, G, S, win, bm, cand, seg, wi, size, lazy);
+}
+
 // Steps 1 and 2 with repeat offsets, and the output (whole CTA, S.flags clear):
 // a segment's parse starts from {1,4,8} and has the state of the parse before
 // it after a few matches.  False, with S.flags clear, where a segment does not
@@ -1576,7 +1883,7 @@ __device__ __noinline__ bool parse_lanes_reps(Zstd2Args a, LaneSmem<kWarps> &N, 
                                               const uint32_t *bm, const uint16_t *cand, uint2 *seg, uint32_t wi,
                                               uint32_t size, bool lazy) {
     const uint32_t tid = threadIdx.x;
-    const uint32_t lim_pos = size - 3u, nact = (lim_pos + kLSegW - 1u) / kLSegW;  // (a match was found: size > 3)
+    const uint32_t lim_pos = size - 3u, nact = (lim_pos + kLSegW - 1u) / kLSegW;  // (no window of up to 3 bytes is given up)
     lane_parse<true>(N, win, bm, cand, seg, size, nact, lazy);
     __syncthreads();
     lane_link_reps(N, S, win, bm, cand, seg, size, nact, lim_pos, lazy);
@@ -1606,6 +1913,13 @@ __device__ __noinline__ bool parse_lanes_reps(Zstd2Args a, LaneSmem<kWarps> &N, 
     return true;
 }
 
+// Window wi to be parsed again in the way S.how (one thread).
+__device__ __forceinline__ void give_up(const Zstd2Args &a, ParseScalars &S, uint32_t wi) {
+    a.seg[static_cast<uint64_t>(wi + 1u) * a.seg_stride - 1u] = make_uint2(S.again, S.how);
+    S.again = wi + 1u;
+    a.seq_counts[wi] = 0u;
+}
+
 // kCtas: CTAs of an SM.
 template <bool kRef, uint32_t kWarps, int kCtas>
 __global__ void __launch_bounds__(32 * kWarps, kCtas) zstd_lane_parse_kernel(Zstd2Args a) {
@@ -1619,7 +1933,7 @@ __global__ void __launch_bounds__(32 * kWarps, kCtas) zstd_lane_parse_kernel(Zst
     if (tid == 0) {
         mbar_init(&S.bar, 1);
         fence_mbar_init();
-        S.again = 0;
+        S.again = S.skip = S.streak = 0;
     }
     for (uint32_t i = tid; i < kPre / 4; i += kThreads) reinterpret_cast<uint32_t *>(M.data)[i] = 0u;
     const Win win{M.data + kPre};
@@ -1637,8 +1951,14 @@ __global__ void __launch_bounds__(32 * kWarps, kCtas) zstd_lane_parse_kernel(Zst
             S.count = 0;
             S.chunks = 0;
             S.probe[0] = S.probe[1] = 0;
+            if (S.skip && size > 3u) {
+                --S.skip;
+                S.flags = 16u;
+                give_up(a, S, wi);
+            }
         }
         __syncthreads();
+        if (S.flags & 16u) continue;
         if (warp == 0) {
             if (!stage_window(M.data + kPre, a.src + start, size, &S.bar, parity, a.status) && lane == 0)
                 S.flags = 2u;
@@ -1663,19 +1983,23 @@ __global__ void __launch_bounds__(32 * kWarps, kCtas) zstd_lane_parse_kernel(Zst
         __syncthreads();
         uint32_t nfix = S.count, fcap = 0;
         if (nfix > 0u) {
-            const bool many = capped || nfix > kMostFixes;  // (uniform over the CTA)
-            // Too many: a few are tried out, unless the entries tell that the window is dense.
-            uint32_t n = capped || (total && entry_end(seg[total - 1u]) < total * kDense) ? 0u : kWarps;
-            fcap = kTryCap;
+            bool many = capped || nfix > kMostFixes;  // (uniform over the CTA)
+            uint32_t n = kWarps;
             if (!many) {
+                const uint32_t found = nfix;
                 if (warp == 0) {
                     nfix = sort_runs(N, nfix);
                     if (lane == 0) S.mends = nfix;
                 }
                 __syncthreads();
                 nfix = S.mends;
-                n = nfix;
-                fcap = kFixEntries / nfix < kFixCap ? kFixEntries / nfix : kFixCap;
+                many = found * 512u >= size && found >= 8u * nfix;  // few runs with matches all over them
+                if (!many || nfix < n) n = nfix;
+            }
+            fcap = kFixEntries / nfix < kFixCap ? kFixEntries / nfix : kFixCap;
+            if (many) {  // a few are tried out, unless the entries tell how dense the window is
+                fcap = kTryCap;
+                if (capped || (total && entry_end(seg[total - 1u]) < total * kDense)) n = 0;
             }
             for (uint32_t r = warp; r < n; r += kWarps)
                 mend_run(N, S, win, M.bm, cand, seg, size, lazy, total, r, fcap);
@@ -1705,12 +2029,14 @@ __global__ void __launch_bounds__(32 * kWarps, kCtas) zstd_lane_parse_kernel(Zst
             nfix = S.mends;
         }
         if (S.flags & 4u) {
-            if (tid == 0) {  // parsed again at the end
-                const bool dense = S.probe[1] < S.probe[0] * kDense ||
-                                   (total && entry_end(seg[total - 1u]) < total * kDense);
-                seg[a.seg_stride - 1u] = make_uint2(S.again, dense ? 1u : 0u);
-                S.again = wi + 1u;
-                a.seq_counts[wi] = 0u;
+            if (tid == 0) {  // parsed again at the end, as are 3 windows after it at once, later 7
+                const uint32_t end = total ? entry_end(seg[total - 1u]) : 0u;
+                const bool dense = S.probe[1] < S.probe[0] * kTryDense || end < total * kDense;
+                const bool sparse = S.probe[1] >= S.probe[0] * kSparse && end >= total * kSparse;
+                S.how = dense ? 1u : (sparse ? 2u : 0u);
+                S.streak = S.streak ? 7u : 3u;
+                S.skip = S.streak;
+                give_up(a, S, wi);
             }
             continue;
         }
@@ -1752,7 +2078,10 @@ __global__ void __launch_bounds__(32 * kWarps, kCtas) zstd_lane_parse_kernel(Zst
             }
         }
         if (kRef && cov) atomicAdd(&S.covered, cov);
-        if (tid == 0) a.seq_counts[wi] = keep;
+        if (tid == 0) {
+            a.seq_counts[wi] = keep;
+            S.streak = 0;
+        }
         if (a.lit_counts) {
             __syncthreads();
             if (tid == 0) a.lit_counts[wi] = size - S.covered;
@@ -1784,8 +2113,10 @@ __global__ void __launch_bounds__(32 * kWarps, kCtas) zstd_lane_parse_kernel(Zst
         if (S.flags & 2u) return;
         verify_window<kWarps>(win, M.bm, cand, size);
         __syncthreads();
-        if (l.y == 0u || !parse_lanes_reps<kRef, kWarps>(a, N, S, win, M.bm, cand, seg, wi, size, lazy))
-            parse_segments_out<kRef, kWarps>(a, N.seg, S, win, M.bm, cand, seg, wi, size, lazy);
+        if (l.y == 2u)
+            parse_segments_out<kRef, kWarps>(a, N.segw, S, win, M.bm, cand, seg, wi, size, lazy);
+        else if (l.y == 0u || !parse_lanes_reps<kRef, kWarps>(a, N, S, win, M.bm, cand, seg, wi, size, lazy))
+            parse_groups_out<kRef>(a, N.seg, S, win, M.bm, cand, seg, wi, size, lazy);
         w = l.x;
     }
 }
@@ -1794,10 +2125,11 @@ __global__ void __launch_bounds__(32 * kWarps, kCtas) zstd_lane_parse_kernel(Zst
 
 // Scratch entries per window: the largest of the layouts, so that a buffer
 // sized once serves every segment width.
-template <uint32_t SegW>
-constexpr uint32_t seg_entries() { return SegCfg<SegW>::kSegs * SegCfg<SegW>::kLaneCap; }
+template <uint32_t SegW, uint32_t GL = 32>
+constexpr uint32_t seg_entries() { return SegCfg<SegW, GL>::kSegs * SegCfg<SegW, GL>::kLaneCap; }
 constexpr uint32_t kSegStride = []() constexpr {
     uint32_t m = kLEntries + 1;  // (the last one leads from a window given up to the one before it)
+    if (seg_entries<1024, 8>() > m) m = seg_entries<1024, 8>();
     if (seg_entries<2048>() > m) m = seg_entries<2048>();
     if (seg_entries<4096>() > m) m = seg_entries<4096>();
     if (seg_entries<8192>() > m) m = seg_entries<8192>();

@@ -80,6 +80,31 @@ def test_among_other_windows(ctx):
     np.testing.assert_array_equal(seqs, o_seqs)
 
 
+@pytest.mark.parametrize("kind", ["counters", "pixels", "wave"])
+def test_small_windows_after_given_up_ones(ctx, kind):
+    """A CTA that has given up a window gives up the next ones at once: windows of
+    a few bytes, of ordinary data and of other kinds among them."""
+    import torch as t
+
+    ctas = 3 * t.cuda.get_device_properties(0).multi_processor_count
+    rng = np.random.default_rng(9)
+    rows = [[_make(kind, 65536 if i % 5 else 4096, i) for i in range(ctas)],
+            [rng.integers(0, 3, i % 7, dtype=np.uint8) for i in range(ctas)],
+            [orc.gen_synthetic(i, 3000 + i) for i in range(ctas)],
+            [_make("bases", 300 + 7 * i, i) for i in range(ctas)],
+            [np.zeros(i % 40 + 1, np.uint8) for i in range(ctas)]]
+    files = [f for row in rows for f in row]
+    seqs, offsets = ctx.zstd_match_find_files(files, 16)
+    w = 0
+    for f in files:
+        if f.size == 0:
+            continue
+        want = orc.zstd_sequences(f, 16, threads=1)[0]
+        np.testing.assert_array_equal(seqs[int(offsets[w]):int(offsets[w + 1])], want)
+        w += 1
+    assert w + 1 == offsets.size
+
+
 @pytest.mark.parametrize("kind,windows", [("counters", 16), ("sorted_ids", 16), ("bases", 16), ("fields64", 256),
                                           ("counters", 2048), ("fields8", 2048)])
 def test_not_slower_than_segment_parse(ctx, kind, windows):
