@@ -968,6 +968,13 @@ int lzma_host_slices(gcz_ctx *c, const uint8_t *src, size_t n, uint32_t depth, u
                                   static_cast<uint32_t *>(sl.lz_packed.p), static_cast<uint8_t *>(sl.lz_has.p),
                                   sl.st)) != GCZ_OK)
             break;
+        // The has bytes go through pinned memory: a copy to pageable memory would hold up the host until the slice is
+        // done.  The packed copy may be such a one, so they go first (1000 bytes: 64.9 -> 60.0 us a call, 64 KiB
+        // 112 -> 107).
+        if (has_out) {
+            if ((r = ensure_host(c, sl.h_has, sb)) != GCZ_OK) break;
+            GCZ_CUDA(c, cudaMemcpyAsync(sl.h_has.p, sl.lz_has.p, sb, cudaMemcpyDeviceToHost, sl.st));
+        }
         if (copy_packed) {  // a has-only call (packed == NULL) copies back one byte per window
             uint32_t *dst = packed_out ? packed_out + sl.off : nullptr;
             if (!dst) {
@@ -975,10 +982,6 @@ int lzma_host_slices(gcz_ctx *c, const uint8_t *src, size_t n, uint32_t depth, u
                 dst = static_cast<uint32_t *>(sl.h_packed.p);
             }
             GCZ_CUDA(c, cudaMemcpyAsync(dst, sl.lz_packed.p, sl.len * 4, cudaMemcpyDeviceToHost, sl.st));
-        }
-        if (has_out) {  // through pinned memory: a copy to pageable memory would hold up the host until the slice is done
-            if ((r = ensure_host(c, sl.h_has, sb)) != GCZ_OK) break;
-            GCZ_CUDA(c, cudaMemcpyAsync(sl.h_has.p, sl.lz_has.p, sb, cudaMemcpyDeviceToHost, sl.st));
         }
         GCZ_CUDA(c, cudaEventRecord(sl.ev, sl.st));
         sl.busy = true;

@@ -19,14 +19,21 @@ struct Copy {
 std::map<cudaStream_t, std::vector<Copy>> g_pending;
 long g_calls = 0, g_fail_at = 0;
 size_t g_handles = 0;
+std::map<cudaStream_t, void *> g_last_to;
 
 bool fails() { return ++g_calls == g_fail_at; }
 cudaError_t done(cudaError_t e = cudaErrorUnknown) { return fails() ? e : cudaSuccess; }
 }  // namespace
 
 extern "C" {
-void fake_fail_at(long call) { g_calls = 0, g_fail_at = call; }
+void fake_fail_at(long call) { g_calls = 0, g_fail_at = call, g_last_to.clear(); }
 long fake_calls() { return g_calls; }
+// Whether the last copy of a stream went to p.
+int fake_last_to(void *p) {
+    for (auto &s : g_last_to)
+        if (s.second == p) return 1;
+    return 0;
+}
 // Copies not waited for that read or write [p, p + n).
 long fake_pending(const char *p, size_t n) {
     long k = 0;
@@ -57,7 +64,7 @@ cudaError_t cudaMemsetAsync(void *p, int v, size_t n, cudaStream_t) { return cud
 cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) { return memcpy(d, s, n), done(); }
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t st) {
     if (fails()) return cudaErrorUnknown;
-    memcpy(d, s, n);
+    memcpy(g_last_to[st] = d, s, n);
     g_pending[st].push_back({static_cast<const char *>(s), n});
     g_pending[st].push_back({static_cast<const char *>(d), n});
     return cudaSuccess;

@@ -1,5 +1,6 @@
 """Host code of the library against a fake CUDA runtime (no GPU): whichever CUDA
-call fails, a call returns with no copy of the caller's buffers still pending."""
+call fails, a call returns with no copy of the caller's buffers still pending.
+And the order of the copies that a small call waits for."""
 import ctypes
 import os
 import subprocess
@@ -26,6 +27,8 @@ def lib(tmp_path_factory):
     L.gcz_destroy.argtypes = [vp]
     for f in (L.gcz_zstd_match_find, L.gcz_zstd_match_find_packed):
         f.argtypes = [vp, vp, sz, ctypes.c_uint32, vp, sz, vp]
+    L.gcz_lzma2_match_find.argtypes = [vp, vp, sz, ctypes.c_uint32, vp, vp]
+    L.fake_last_to.argtypes = [vp]
     L.fake_fail_at.argtypes = [ctypes.c_long]
     L.fake_calls.restype = ctypes.c_long
     L.fake_pending.argtypes, L.fake_pending.restype = [vp, sz], ctypes.c_long
@@ -58,3 +61,16 @@ def test_small_call_leaves_nothing_pending(lib, n, packed):
         rc, _, left = run(k)
         assert rc != 0, k
         assert left == [0, 0, 0], k
+
+
+@pytest.mark.parametrize("n", [1, 4096, 200_003])
+def test_lzma_results_leave_last(lib, n):
+    """A copy to pageable memory holds the host up: nothing may be queued behind it."""
+    src, packed, has = np.zeros(n, np.uint8), np.zeros(n, np.uint32), np.zeros(4, np.uint8)
+    h = ctypes.c_void_p()
+    lib.fake_fail_at(0)
+    assert lib.gcz_create(0, ctypes.byref(h)) == 0
+    assert lib.gcz_lzma2_match_find(h, src.ctypes.data, n, 32, packed.ctypes.data, has.ctypes.data) == 0
+    last = lib.fake_last_to(packed.ctypes.data)
+    lib.gcz_destroy(h)
+    assert last
