@@ -2178,7 +2178,7 @@ cudaError_t launch_parse_ref(const Zstd2Args &a, uint32_t seg_width, int num_sms
     // the SM's registers.  Sweep to records, 1 window 100.3 -> 89.3 us, 148
     // windows 109.6 -> 96.6; a 4 KiB window takes the same 26.7.  At most two:
     // 16 warps each, 64 registers instead of 40 and no spills, 256 windows
-    // 127.7 -> 121.4.  More: three CTAs per SM (4096 windows 1.31 ms, two 1.72).
+    // 127.7 -> 120.4.  More: three CTAs per SM (4096 windows 1.31 ms, two 1.72).
     const uint32_t sms = static_cast<uint32_t>(num_sms);
     if (a.num_windows <= sms) return launch_lane_parse<kRef, 32, 1>(a, num_sms, ctas_per_sm, st);
     if (a.num_windows <= 2u * sms) return launch_lane_parse<kRef, 16, 2>(a, num_sms, ctas_per_sm, st);

@@ -75,14 +75,17 @@ const char *gcz_version(void);
  * the candidate sweep then the per-window second stage, 1 the fused
  * single-warp kernels; "staged" (algo 1) = 1 stages each window into shared
  * memory with bulk copies, 0 reads it through L1; "parse_ctas" = Zstd
- * second-stage CTAs per SM (1-8); "parse_seg" = the Zstd second stage's
- * parse: 1024 (default) or 512, one lane per 128-byte segment without repeat
- * offsets, which are checked and mended afterwards; 2048, 4096 or 8192, one
+ * second-stage CTAs per SM (1-8; the lane parse runs at most 3, 2 where there
+ * are up to two windows per SM, 1 up to one); "parse_seg" = the Zstd second
+ * stage's parse: 1024 (default) or 512, one lane per 132-byte segment without
+ * repeat offsets, which are checked and mended afterwards, windows that are
+ * full of them parsed with them; 2048, 4096 or 8192, one
  * warp per segment of that many bytes with them; "sweep_warps" = warps that take turns on
  * a window in the candidate sweep (4-7, default 7); "sweep_groups" (0 to 3) and
  * "sweep_prefetch" (0 to 64) = accepted and without effect;
  * "lzma_ctas" = LZMA2 second-stage CTAs per SM (1-8, default 3; values above
- * what fits on an SM -- 3, or 2 with 1024 threads -- run as that many);
+ * what fits on an SM -- 3, or 2 with 1024 threads -- run as that many; without effect
+ * where 2, 4 or 8 CTAs share each of a few windows);
  * "lzma_threads" = LZMA2 second-stage threads per CTA (256, 512 or 1024,
  * default 1024, which takes 256 where there are several windows per CTA);
  * "slice_windows" = windows per slice of the host-buffer
