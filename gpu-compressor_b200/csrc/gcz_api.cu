@@ -611,10 +611,35 @@ size_t next_slice(size_t b0, size_t nb, size_t maxw) {
 }
 
 int drain_slots(gcz_ctx *c) {
-    for (Slot &sl : c->slots) GCZ_CUDA(c, cudaStreamSynchronize(sl.st));
-    GCZ_CUDA(c, cudaStreamSynchronize(c->out_stream));
+    cudaError_t first = cudaStreamSynchronize(c->out_stream);
+    for (Slot &sl : c->slots) {  // all of them, whatever one returns
+        const cudaError_t e = cudaStreamSynchronize(sl.st);
+        if (first == cudaSuccess) first = e;
+    }
+    GCZ_CUDA(c, first);
     return read_status(c, c->stream);
 }
+
+// Waits for the slots' streams where a host-buffer call is left by an error:
+// the buffers are the caller's again when it returns.
+struct DrainOnError {
+    gcz_ctx *c;
+    bool armed = true;
+    ~DrainOnError() {
+        if (!armed) return;
+        std::string why;
+        why.swap(c->err);
+        for (Slot &sl : c->slots) sl.busy = false;
+        drain_slots(c);
+        c->err.swap(why);
+    }
+    int finish(int r) {  // the regular end: the first error counts
+        armed = r != GCZ_OK;
+        if (armed) return r;
+        for (Slot &sl : c->slots) sl.busy = false;
+        return drain_slots(c);
+    }
+};
 }  // namespace
 
 // Slices of slice_windows windows rotate over the S = 4 slots (streams): the
@@ -644,21 +669,13 @@ int zstd_host_direct(gcz_ctx *c, const uint8_t *src, size_t n, uint32_t search_d
     uint32_t *h_status = reinterpret_cast<uint32_t *>(h);
     uint64_t *h_off = reinterpret_cast<uint64_t *>(h + 16);
     uint8_t *h_rec = h + off_bytes;
-    auto run = [&]() -> int {
-        GCZ_CUDA(c, cudaMemcpyAsync(sl.in.p, src, n, cudaMemcpyHostToDevice, sl.st));
-        const int r = zstd_device_core(c, sl.sc, static_cast<const uint8_t *>(sl.in.p), n, search_depth, h_rec, cap,
-                                       h_off, sl.st, nullptr, 0, rec_bytes == 8, h_status);
-        if (r != GCZ_OK) return r;
-        GCZ_CUDA(c, cudaStreamSynchronize(sl.st));
-        return GCZ_OK;
-    };
-    if ((r = run()) != GCZ_OK) {  // the copy and some kernels may be queued: src is the caller's again on return
-        std::string why;
-        why.swap(c->err);
-        drain_slots(c);
-        c->err.swap(why);
+    DrainOnError drain{c};
+    GCZ_CUDA(c, cudaMemcpyAsync(sl.in.p, src, n, cudaMemcpyHostToDevice, sl.st));
+    if ((r = zstd_device_core(c, sl.sc, static_cast<const uint8_t *>(sl.in.p), n, search_depth, h_rec, cap, h_off,
+                              sl.st, nullptr, 0, rec_bytes == 8, h_status)) != GCZ_OK)
         return r;
-    }
+    GCZ_CUDA(c, cudaStreamSynchronize(sl.st));
+    drain.armed = false;
     if (*h_status) {
         GCZ_CUDA(c, cudaMemsetAsync(c->d_status, 0, 4, sl.st));
         GCZ_CUDA(c, cudaStreamSynchronize(sl.st));
@@ -685,6 +702,7 @@ int zstd_host_pipeline(gcz_ctx *c, const uint8_t *src, size_t n, uint32_t search
     if (n <= kDirectBytes && nb <= c->slice_windows)
         return zstd_host_direct(c, src, n, search_depth, seqs, seq_capacity, offsets, rec_bytes);
     int r = GCZ_OK;
+    DrainOnError drain{c};
     uint64_t done = 0;  // sequences copied so far
     constexpr size_t kS = sizeof(c->slots) / sizeof(c->slots[0]);
     size_t k = 0;
@@ -718,9 +736,7 @@ int zstd_host_pipeline(gcz_ctx *c, const uint8_t *src, size_t n, uint32_t search
         Slot &rest = c->slots[j % kS];
         if (rest.busy) r = zstd_finish_slot(c, rest, seqs, seq_capacity, offsets, done, rec_bytes);
     }
-    for (Slot &sl : c->slots) sl.busy = false;
-    const int r2 = drain_slots(c);
-    return r != GCZ_OK ? r : r2;
+    return drain.finish(r);
 }
 }  // namespace
 
@@ -778,6 +794,7 @@ extern "C" int gcz_zstd_compress_frames_gpu(gcz_ctx *c, const uint8_t *src, size
     const size_t nb = nwin(n);
     size_t written = 0;
     int r = GCZ_OK;
+    DrainOnError drain{c};
     auto finish = [&](Slot &sl) -> int {
         GCZ_CUDA(c, cudaEventSynchronize(sl.ev));
         sl.busy = false;
@@ -830,10 +847,8 @@ extern "C" int gcz_zstd_compress_frames_gpu(gcz_ctx *c, const uint8_t *src, size
         Slot &rest = c->slots[j % kFrameSlots];
         if (rest.busy) r = finish(rest);
     }
-    for (Slot &sl : c->slots) sl.busy = false;
-    const int r2 = drain_slots(c);
-    if (r == GCZ_OK && r2 == GCZ_OK) *out_size = written;
-    return r != GCZ_OK ? r : r2;
+    if ((r = drain.finish(r)) == GCZ_OK) *out_size = written;
+    return r;
 }
 
 extern "C" int gcz_zstd_match_find_ref_layout_device(gcz_ctx *c, const uint8_t *d_input, uint32_t *d_sequences,
@@ -944,6 +959,7 @@ int lzma_host_slices(gcz_ctx *c, const uint8_t *src, size_t n, uint32_t depth, u
                      uint8_t *has_out, bool copy_packed, Consume consume) {
     const size_t nb = nwin(n);
     int r = GCZ_OK;
+    DrainOnError drain{c};
     auto finish = [&](Slot &sl) -> int {
         GCZ_CUDA(c, cudaEventSynchronize(sl.ev));
         sl.busy = false;
@@ -994,9 +1010,7 @@ int lzma_host_slices(gcz_ctx *c, const uint8_t *src, size_t n, uint32_t depth, u
         Slot &rest = c->slots[j % kS];
         if (rest.busy) r = finish(rest);
     }
-    for (Slot &sl : c->slots) sl.busy = false;
-    const int r2 = drain_slots(c);
-    return r != GCZ_OK ? r : r2;
+    return drain.finish(r);
 }
 }  // namespace
 

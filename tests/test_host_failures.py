@@ -28,6 +28,9 @@ def lib(tmp_path_factory):
     for f in (L.gcz_zstd_match_find, L.gcz_zstd_match_find_packed):
         f.argtypes = [vp, vp, sz, ctypes.c_uint32, vp, sz, vp]
     L.gcz_lzma2_match_find.argtypes = [vp, vp, sz, ctypes.c_uint32, vp, vp]
+    L.gcz_zstd_compress_frames_gpu.argtypes = [vp, vp, sz, ctypes.c_uint32, vp, sz, vp, vp]
+    L.gcz_set_option.argtypes = [vp, ctypes.c_char_p, ctypes.c_long]
+    L.gcz_last_error.argtypes, L.gcz_last_error.restype = [vp], ctypes.c_char_p
     L.fake_last_to.argtypes = [vp]
     L.fake_fail_at.argtypes = [ctypes.c_long]
     L.fake_calls.restype = ctypes.c_long
@@ -74,3 +77,41 @@ def test_lzma_results_leave_last(lib, n):
     last = lib.fake_last_to(packed.ctypes.data)
     lib.gcz_destroy(h)
     assert last
+
+
+@pytest.mark.parametrize("kind", ["sequences", "packed", "lzma", "triage", "frames"])
+@pytest.mark.parametrize("n", [65536, 9 * 65536 + 1])
+def test_sliced_call_leaves_nothing_pending(lib, n, kind):
+    nb = (n + 65535) // 65536
+    src, out = np.zeros(n, np.uint8), np.zeros(n * 4 + 1024 * nb, np.uint32)
+    small, size = np.zeros(nb + 1, np.uint64), np.zeros(1, np.uint64)
+    s, o, m = src.ctypes.data, out.ctypes.data, small.ctypes.data
+    call = {
+        "sequences": lambda h: lib.gcz_zstd_match_find(h, s, n, 16, o, n, m),
+        "packed": lambda h: lib.gcz_zstd_match_find_packed(h, s, n, 16, o, n, m),
+        "lzma": lambda h: lib.gcz_lzma2_match_find(h, s, n, 32, o, m),
+        "triage": lambda h: lib.gcz_lzma2_match_find(h, s, n, 32, None, m),
+        "frames": lambda h: lib.gcz_zstd_compress_frames_gpu(h, s, n, 1, o, out.nbytes, m, size.ctypes.data),
+    }[kind]
+
+    def run(fail_at):
+        h = ctypes.c_void_p()
+        lib.fake_fail_at(0)
+        assert lib.gcz_create(0, ctypes.byref(h)) == 0
+        for key in (b"slice_windows", b"frames_slice_windows"):
+            assert lib.gcz_set_option(h, key, 2) == 0
+        lib.fake_fail_at(fail_at)
+        rc = call(h)
+        calls = lib.fake_calls()
+        lib.fake_fail_at(0)
+        left = [lib.fake_pending(a.ctypes.data, a.nbytes) for a in (src, out, small)]
+        why = lib.gcz_last_error(h)
+        lib.gcz_destroy(h)
+        return rc, calls, left, why
+
+    rc, calls, left, _ = run(0)
+    assert rc == 0 and left == [0, 0, 0] and calls > 5
+    for k in range(1, calls + 1):
+        rc, _, left, why = run(k)
+        assert rc != 0 and why, k
+        assert left == [0, 0, 0], k
